@@ -58,9 +58,8 @@ size_t control_bytes(uint32_t n) {
 // pass's open-node buffers, the control block and the look-back words.
 size_t arena_bytes(uint32_t cap) {
     const size_t groups = emit_groups(cap);
-    return 4 * align_up((size_t)cap * 4) + align_up((size_t)cap * 12) + align_up((size_t)cap * 32) + align_up((size_t)cap) +
-           align_up(groups * kOpenCap * sizeof(OpenItem)) + align_up(groups * sizeof(uint32_t)) +
-           align_up(sizeof(uint32_t)) + control_bytes(cap);
+    return 3 * align_up((size_t)cap * 4) + align_up((size_t)cap * 12) +
+           align_up(groups * kOpenCap * sizeof(OpenItem)) + align_up(2 * groups * sizeof(uint32_t)) + control_bytes(cap);
 }
 
 struct GraphKey {
@@ -113,9 +112,7 @@ struct lvbh_ctx {
     uint32_t *keys_a = nullptr;  // unsorted Morton keys (input of the first sort pass)
     float *cen = nullptr;        // triangle centroids, x / y / z arrays of `cap` floats
     OpenItem *items = nullptr;
-    uint32_t *counts = nullptr, *arrive = nullptr, *epoch = nullptr;
-    float4 *pend = nullptr;
-    uint8_t *pend_d = nullptr;
+    uint32_t *counts = nullptr;  // open items and a straddling-pass counter per tree block
     Control *ctl = nullptr;
     uint32_t *lookback = nullptr;  // the sort's tile and chunk histograms
     // staging for host input
@@ -225,7 +222,7 @@ size_t batch_bytes(uint32_t segs, uint32_t tiles, uint32_t blocks) {
     const size_t lb = (size_t)kSortPasses * tiles * kDigits * 4;
     return rows + align_up(tiles * 4ull) + 2 * align_up(blocks * 4ull) + align_up(ord + hist + lb) +
            align_up((size_t)segs * 6 * 4) + align_up((size_t)blocks * kOpenCap * sizeof(OpenItem)) +
-           align_up(blocks * 4ull);
+           align_up(2 * blocks * 4ull);
 }
 
 // Batch scratch for up to `segs` segments, `tiles` sort tiles and `blocks` tree blocks.
@@ -262,7 +259,7 @@ int ensure_batch(lvbh_ctx *ctx, uint32_t segs, uint32_t tiles, uint32_t blocks) 
     c += zero;
     ctx->b_bounds = reinterpret_cast<float *>(c); c += bnd;
     ctx->b_items = reinterpret_cast<OpenItem *>(c); c += align_up((size_t)blocks * kOpenCap * sizeof(OpenItem));
-    ctx->b_counts = reinterpret_cast<uint32_t *>(c);  // open items per tree block
+    ctx->b_counts = reinterpret_cast<uint32_t *>(c);  // as counts
     char *hc = static_cast<char *>(h);
     ctx->b_host = h;
     ctx->bh_rows = reinterpret_cast<SegRow *>(hc); hc += rows;
@@ -288,19 +285,12 @@ int ensure_arena(lvbh_ctx *ctx, uint32_t n) {
     const size_t groups = emit_groups(cap);
     ctx->keys_b = reinterpret_cast<uint32_t *>(c); c += kb;
     ctx->vals_b = reinterpret_cast<uint32_t *>(c); c += kb;
-    ctx->arrive = reinterpret_cast<uint32_t *>(c); c += kb;
     ctx->keys_a = reinterpret_cast<uint32_t *>(c); c += kb;
     ctx->cen = reinterpret_cast<float *>(c); c += align_up((size_t)cap * 12);
-    ctx->pend = reinterpret_cast<float4 *>(c); c += align_up((size_t)cap * 32);
-    ctx->pend_d = reinterpret_cast<uint8_t *>(c); c += align_up((size_t)cap);
     ctx->items = reinterpret_cast<OpenItem *>(c); c += align_up(groups * kOpenCap * sizeof(OpenItem));
-    ctx->counts = reinterpret_cast<uint32_t *>(c); c += align_up(groups * sizeof(uint32_t));  // per tree block
-    ctx->epoch = reinterpret_cast<uint32_t *>(c); c += align_up(sizeof(uint32_t));
+    ctx->counts = reinterpret_cast<uint32_t *>(c); c += align_up(2 * groups * sizeof(uint32_t));
     ctx->ctl = reinterpret_cast<Control *>(c);
     ctx->lookback = reinterpret_cast<uint32_t *>(c + align_up(sizeof(Control)));
-    // arrival words and the epoch start at zero; from then on the epoch keeps them valid
-    LVBH_CUDA(ctx, cudaMemset(ctx->arrive, 0, kb));
-    LVBH_CUDA(ctx, cudaMemset(ctx->epoch, 0, sizeof(uint32_t)));
     // the control block's test words (zero unless lvbh_test_stall_lookback set them)
     const uint32_t test_words[2] = {ctx->test_stall1, ctx->test_spin};
     LVBH_CUDA(ctx, cudaMemcpy(ctx->ctl, test_words, sizeof test_words, cudaMemcpyHostToDevice));
@@ -353,10 +343,10 @@ cudaError_t enqueue_build(lvbh_ctx *ctx, const float4 *tri, uint32_t n, const Ho
     // unsorted keys go to keys_a, so that the three passes ping-pong keys_a -> result ->
     // scratch -> result
     uint32_t *keys_a = ctx->keys_a;
-    if (mesh) launch_morton_mesh(mesh->verts, mesh->nverts, mesh->idx3, n, hb, ctx->ctl, keys_a, ctx->epoch,
+    if (mesh) launch_morton_mesh(mesh->verts, mesh->nverts, mesh->idx3, n, hb, ctx->ctl, keys_a,
                                  ctx->lookback, s);
-    else if (cen_path) launch_morton_cen(ctx->cen, ctx->cap, n, ctx->ctl, keys_a, ctx->epoch, ctx->lookback, s);
-    else if (pre != kPreKeys) launch_morton(tri, n, hb, ctx->ctl, keys_a, ctx->epoch, ctx->lookback, s);
+    else if (cen_path) launch_morton_cen(ctx->cen, ctx->cap, n, ctx->ctl, keys_a, ctx->lookback, s);
+    else if (pre != kPreKeys) launch_morton(tri, n, hb, ctx->ctl, keys_a, ctx->lookback, s);
     if (profile) cudaEventRecord(ctx->ev[3], s);
     launch_sort_pass(keys_a, nullptr, out->morton, out->leaf_index, n, 0, true, ctx->ctl, ctx->lookback, s);
     launch_sort_pass(out->morton, out->leaf_index, ctx->keys_b, ctx->vals_b, n, 1, false, ctx->ctl, ctx->lookback, s);
@@ -366,13 +356,12 @@ cudaError_t enqueue_build(lvbh_ctx *ctx, const float4 *tri, uint32_t n, const Ho
         uint32_t *sidx = static_cast<uint32_t *>(out->tris);
         launch_leaf_idx(mesh->idx3, out->leaf_index, n, sidx, s);
         launch_emit_mesh(mesh->verts, mesh->nverts, sidx, out->morton, n, static_cast<float4 *>(out->nodes),
-                         out->parents, ctx->items, ctx->counts, ctx->arrive, ctx->pend, ctx->pend_d, ctx->epoch,
-                         ctx->ctl, s, profile ? ctx->ev + 5 : nullptr);
+                         out->parents, ctx->items, ctx->counts, ctx->ctl, s, profile ? ctx->ev + 5 : nullptr);
         return cudaSuccess;
     }
     return launch_emit(tri, out->leaf_index, out->morton, n, static_cast<float4 *>(out->tris),
                        static_cast<float4 *>(out->nodes), out->parents, ctx->items, ctx->counts,
-                       ctx->arrive, ctx->pend, ctx->pend_d, ctx->epoch, ctx->ctl, s,
+                       ctx->ctl, s,
                        profile ? ctx->ev + 5 : nullptr);
 }
 
@@ -397,7 +386,7 @@ cudaError_t enqueue_batch(lvbh_ctx *ctx, const float4 *tri, const BatchPlan &bp,
     if (profile) cudaEventRecord(ctx->ev[2], s);
     uint32_t *keys_a = ctx->keys_a;
     launch_morton_batch(bp, tri, use_bounds ? ctx->b_bounds : nullptr, ctx->b_ord, ctx->b_hist,
-                        ctx->ctl, keys_a, ctx->epoch, s);
+                        ctx->ctl, keys_a, s);
     if (profile) cudaEventRecord(ctx->ev[3], s);
     // ping-pong so that the last pass lands in the result buffers
     uint32_t *kb = ctx->keys_b, *vb = ctx->vals_b, *ko = out->morton, *vo = out->leaf_index;
@@ -414,7 +403,7 @@ cudaError_t enqueue_batch(lvbh_ctx *ctx, const float4 *tri, const BatchPlan &bp,
     if (profile) cudaEventRecord(ctx->ev[4], s);
     return launch_emit_batch(bp, tri, out->leaf_index, out->morton, static_cast<float4 *>(out->tris),
                              static_cast<float4 *>(out->nodes), out->parents, ctx->b_items,
-                             ctx->b_counts, ctx->arrive, ctx->pend, ctx->pend_d, ctx->epoch, ctx->ctl, s,
+                             ctx->b_counts, ctx->ctl, s,
                              profile ? ctx->ev + 5 : nullptr);
 }
 
@@ -621,7 +610,7 @@ int upload_chunked(lvbh_ctx *ctx, const float *host, uint32_t n, const float *mo
                                        cudaMemcpyHostToDevice, ctx->copy_stream));
         LVBH_CUDA(ctx, cudaEventRecord(ctx->up_ev[1 + c], ctx->copy_stream));
         LVBH_CUDA(ctx, cudaStreamWaitEvent(s, ctx->up_ev[1 + c], 0));
-        if (hb.use) launch_morton_chunks(tri, n, hb, ctx->ctl, ctx->keys_a, ctx->epoch, ctx->lookback, u0, u1, s);
+        if (hb.use) launch_morton_chunks(tri, n, hb, ctx->ctl, ctx->keys_a, ctx->lookback, u0, u1, s);
         else launch_bounds_cen(tri, t0, t1, ctx->cen, ctx->cap, ctx->ctl, s);
     }
     *pre = hb.use ? kPreKeys : kPreCen;
@@ -874,7 +863,7 @@ int lvbh_build_batched(lvbh_ctx *ctx, const float *tri_array, const uint32_t *se
     if (int rc = ensure_batch(ctx, num_segs, (uint32_t)tiles, (uint32_t)blocks128)) return rc;
     if (seg_bounds) std::memcpy(ctx->bh_bounds, seg_bounds, num_segs * 6ull * sizeof(float));
     // segment table for tree blocks of 2^log_block leaves: first triangle, first sort tile,
-    // first tree block and first straddling-pass group (16 blocks of one segment) per segment
+    // first tree block and first straddling-pass group (blocks of one segment) per segment
     auto plan = [&](const Tunables &t) {
         uint32_t tile = 0, blk = 0, grp = 0;
         for (uint32_t i = 0; i <= num_segs; ++i) {

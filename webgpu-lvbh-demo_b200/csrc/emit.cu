@@ -32,9 +32,9 @@
 //                        arrives (the parent straddles the block boundary), leaves as an
 //                        "open item" (at most 2 x 64 per block: they hang off the two boundary
 //                        paths of a tree at most 64 deep).
-//   K3c (k_top_group)    the nodes that straddle blocks (~3 % of them), built bottom-up from
-//                        the open items: per group of blocks in shared memory, then with
-//                        arrival words in global memory (see below).
+//   K3c (k_top_group)    the nodes that straddle blocks (~3 % of them), from the open items: per
+//                        group of blocks in shared memory, each node on its own thread, then per
+//                        group of groups, up to the root (see below).
 #include <cstring>
 #include <cuda.h>  // CUtensorMap
 #include <cudaTypedefs.h>
@@ -65,7 +65,6 @@ struct TreeGeo {
     static __device__ __forceinline__ int rdl(uint32_t p) { return (int)((p >> (2 * LOG)) & 127u) - 1; }
     static __device__ __forceinline__ int rdr(uint32_t p) { return (int)(p >> (2 * LOG + 7)) - 1; }
 };
-constexpr int kTopLanes = 8;                   // K3c threads per block of K3b
 constexpr int kFreeClimb = 64;                 // K3b items left when compaction stops
 
 // Where a block of EB sorted leaves lives.  A batched build is a list of segments (meshes)
@@ -319,6 +318,7 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
         if (blk - grid >= (int)blockIdx.x) {
             const int o = S.open[buf ^ 1];
             out_counts[blk - grid] = (uint32_t)min(o, kOpenCap);
+            out_counts[nblk + blk - grid] = 0u;  // a counter of the straddling pass
             if (o > kOpenCap) atomicOr(&ctl->err, ERR_CLIMB);
         }
         S.open[buf ^ 1] = 0;
@@ -537,310 +537,379 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
     if (t == 0 && last >= 0) {
         const int o = S.open[last_buf];
         out_counts[last] = (uint32_t)min(o, kOpenCap);
+        out_counts[nblk + last] = 0u;
         if (o > kOpenCap) atomicOr(&ctl->err, ERR_CLIMB);
     }
     if (bad_perm) atomicOr(&ctl->err, ERR_CLIMB);
     if (copy_timeout) atomicOr(&ctl->err, ERR_COPY_TIMEOUT);
 }
 
-// K3c, the arrival-word climb: each thread climbs an open item through the splits above it
-// (k_top_group calls it for what leaves a group; k_emit_top, with kTopLanes threads per K3b
-// block, over the blocks' items directly).  At a split the
-// first arriving child parks its box, link and far range end in pend[] and its far end's
-// separator in pend_d[], both at its own index (r when it is a left child, l when a right child -
-// no two pending children ever share one), and exchanges the build's epoch into the split's
-// arrival word with release-acquire semantics; the second, seeing the epoch already there,
-// reads its sibling back,
-// merges, and has the parent's range, both end separators and so its Karras index without
-// touching the keys.  A completed record and its two parent links are stored after the next
-// split's exchange, so that exchange's release waits for the parked rows only.
-// Nothing waits, so the kernel cannot hang; climbs are bounded and every index is
-// range-checked.  The epoch makes the arrival words reusable without clearing: a word left by
-// an older build never equals the current epoch.
+// K3c: the nodes that straddle tree blocks, without a climb.  The open items of consecutive
+// blocks, in leaf order, partition those blocks' leaves; with the separators between and around
+// them they are a shorter instance of the same problem: the node of the separator at split s
+// covers the items between the nearest smaller separators on either side, its parent is the node
+// of the larger of those two, its index follows from its own range, and its box is the union of a
+// range of items.  So every node of such a run is found on its own thread (reduce_run).  A node
+// with no smaller separator on one side within the run extends past it; the maximal subtrees
+// below such nodes (at most 2 x 64: they hang off the run's two boundary paths) are the run's own
+// open items.
 //
-// One open item's climb through the splits above it with the arrival words, in a
-// segment of n triangles whose node, parent, arrival and pending arrays start at the pointers
-// given.  False if the climb broke off (a range inconsistent with the tree, or more levels than
-// any tree has).
-__device__ __forceinline__ bool top_climb(const OpenItem &it, int n, float4 *nodes, int32_t *parents, uint32_t *arrive,
-                                          float4 *pend, uint8_t *pend_d, uint32_t epoch) {
-    int l = it.xl, r = it.xr, ref = __float_as_int(it.lo.w);
-    float nx = it.lo.x, ny = it.lo.y, nz = it.lo.z, xx = it.hi.x, xy = it.hi.y, xz = it.hi.z;
-    int dl = it.pad0, dr = __float_as_int(it.hi.w);
-    // the record completed at the previous split, stored after the next exchange
-    bool have = false;
-    float4 w0, w1, w2, w3;
-    int wP = 0, wl = 0, wr = 0;
-    auto flush = [&]() {
-        if (!have) return;
-        float4 *rc = nodes + 4ull * wP;
-        rc[0] = w0; rc[1] = w1; rc[2] = w2; rc[3] = w3;
-        parents[wl >= 0 ? wl : n - (wl + 1)] = wP;
-        parents[wr >= 0 ? wr : n - (wr + 1)] = wP;
-        have = false;
-    };
-    bool done = false;
-    for (int level = 0; level < 160; ++level) {
-        if (l == 0 && r == n - 1) { done = true; break; }  // root complete
-        const bool is_left = dr > dl;
-        const int s = is_left ? r : l - 1;
-        if (s < 0 || s >= n - 1 || l < 0 || r >= n) break;
-        const int own = is_left ? r : l, sib = is_left ? s + 1 : s;
-        const float4 h0 = make_float4(nx, ny, nz, __int_as_float(ref));
-        const float4 h1 = make_float4(xx, xy, xz, __int_as_float(is_left ? l : r));
-        pend[2ull * own] = h0;
-        pend[2ull * own + 1] = h1;
-        pend_d[own] = (uint8_t)((is_left ? dl : dr) + 1);
-        const bool first = atom_exch_acq_rel_gpu(arrive + s, epoch) != epoch;
-        flush();
-        if (first) { done = true; break; }  // the sibling completes the parent
-        const float4 g0 = __ldcg(pend + 2ull * sib), g1 = __ldcg(pend + 2ull * sib + 1);
-        const int gd = (int)__ldcg(pend_d + sib) - 1;
-        const int sib_ref = __float_as_int(g0.w), sib_far = __float_as_int(g1.w);
-        const int L = is_left ? l : sib_far, R = is_left ? sib_far : r;
-        if (L < 0 || R >= n || L > l || R < r || sib_ref < -n || sib_ref >= n - 1) break;
-        const float4 lo0 = is_left ? h0 : g0, lo1 = is_left ? h1 : g1;
-        const float4 hi0 = is_left ? g0 : h0, hi1 = is_left ? g1 : h1;
-        nx = fminf(nx, g0.x); ny = fminf(ny, g0.y); nz = fminf(nz, g0.z);
-        xx = fmaxf(xx, g1.x); xy = fmaxf(xy, g1.y); xz = fmaxf(xz, g1.z);
-        const int ndl = is_left ? dl : gd, ndr = is_left ? gd : dr;
-        const int P = (L == 0 && R == n - 1) ? 0 : (ndr > ndl ? R : L);
-        w0 = lo0;
-        w1 = make_float4(lo1.x, lo1.y, lo1.z, __int_as_float(2));
-        w2 = hi0;
-        w3 = make_float4(hi1.x, hi1.y, hi1.z, __int_as_float(0));
-        wP = P;
-        wl = __float_as_int(lo0.w);
-        wr = __float_as_int(hi0.w);
-        have = true;
-        l = L; r = R; ref = P; dl = ndl; dr = ndr;
-    }
-    flush();
-    return done;
-}
+// One block reduces a group of kGroupBlocks tree blocks; the last of kFan neighbouring groups to
+// finish (a counter per parent, nothing waits) goes on with what those groups left as one run,
+// and so on up to the root: three levels at 2^20 triangles, four at 2^24.  Latency bounds it: a
+// level is about eight block barriers and four dependent L2 accesses, 5 to 6 us.  Before, each
+// open item climbed one level of the tree at a time, parking and merging through shared-memory
+// hashes and then arrival words in L2 (0.5 to 2.6 us a level, up to 31 levels).  The pass, climbs
+// -> runs (B200): 4,098 triangles 19 -> 6 us, 65,536 uniform 35 -> 11, 1,000,003 clustered 63 ->
+// 26, the 2 M sphere 65 -> 34, 2^24 clustered 130 -> 91, 1,024 meshes of 33 M triangles 203 ->
+// 155; the scratch of arrival words and parked children (37 B per triangle) is gone.
+//
+// Sizes: a run holds at most 256 items, one per thread: a child's open items (<= kOpenCap) always
+// fit beside what the children before it left (<= kOpenCap), so a run that would be longer is
+// reduced a few children at a time.  A tree block leaves 8.1 items on average (uniform and
+// clustered triangles), so a group of 24 blocks leaves 60 of 256 threads idle and rarely needs a
+// second turn.  24 blocks against 16 (more levels, more idle threads) at 2^24 and the batch:
+// 91 and 155 us against 109 and 173; 512 threads and 32 blocks: 117 and 231; 384 and 24: 110 and
+// 207 (fewer, longer blocks hide each other's latency less).
+constexpr int kRunCap = 256;
+constexpr int kRunWarps = kRunCap / 32;
+static_assert(kRunCap >= 2 * kOpenCap && kGroupBlocks <= 32 && kFan <= 32, "a run takes two children; one warp counts them");
 
-template <class Segs, int LANES = kTopLanes>
-__global__ void __launch_bounds__(256) k_emit_top(Segs segs, const OpenItem *__restrict__ items, int cap,
-                                                  const uint32_t *__restrict__ counts,
-                                                  float4 *nodes_all, int32_t *parents_all,
-                                                  uint32_t *arrive_all, float4 *pend_all,
-                                                  uint8_t *pend_d_all,
-                                                  const uint32_t *__restrict__ epoch_p,
-                                                  Control *ctl) {
-    const int gw = (blockIdx.x * 256 + threadIdx.x) / LANES, lane = threadIdx.x % LANES;
-    if (gw >= segs.blocks()) return;
-    if (ld_relaxed_gpu(&ctl->err) & ERR_LOOKBACK_TIMEOUT) return;  // unsorted keys: nothing to build
-    const int cnt = (int)min(counts[gw], (uint32_t)cap);
-    if (lane >= cnt) return;
-    const uint32_t epoch = *epoch_p;
-    const Span sp = segs.span(gw);
-    for (int q = lane; q < cnt; q += LANES)
-        if (!top_climb(items[segs.item_base(gw, cap) + q], sp.n, nodes_all + 4ull * sp.start,
-                       parents_all + 2ull * sp.start, arrive_all + sp.start, pend_all + 2ull * sp.start,
-                       pend_d_all + sp.start, epoch))
-            atomicOr(&ctl->err, ERR_CLIMB);
-}
-
-// K3c, first level: one block per group of Groups::kBlocks consecutive K3b blocks
-// climbs the group's open items through every split both of whose sides lie in the group, in
-// shared memory - the same park / merge handshake as K3b, splits found through a hash table,
-// each item climbing on its own thread with no barrier between levels - and writes those
-// records and parent links.  What is left (items whose next split leaves the group, children
-// parked at a split whose sibling never came; about 1 / kBlocks of the items) then climbs on in
-// the same block with the arrival words of k_emit_top (top_climb), while other groups still run
-// their shared-memory climbs: those touch only splits inside their own groups, the arrival words
-// only splits that straddle a group.  (As a kernel of its own after the group pass the global
-// climb took 80 us of the 16.7 M build's 155; in the group kernel the pass takes 151 us: the
-// chain of arrivals up to the root, not the launch, sets its length.)  A plain build's groups
-// span 4096 leaves (16 blocks of 256, or 32 of 128), a batched build's 16 blocks of its meshes.
-// A group with more than kGroupCap items climbs them all with the arrival words.
-constexpr int kGroupBlocks = 16;  // a batched build's blocks per group
-constexpr int kMaxGroupBlocks = 32;
-constexpr int kGroupCap = 256;
-constexpr int kGroupHash = 512;   // slots (power of two); distinct splits <= 2 x items
-constexpr int kGroupThreads = 128;
-
-struct GroupSmem {
-    OpenItem it[kGroupCap];
-    int out[kGroupCap];
-    int hkey[kGroupHash];
-    uint32_t hmask[kGroupHash];
-    int hidx[kGroupHash][2];
-    int bstart[kMaxGroupBlocks + 1];
-    int cnt[1];
-    int nout;
+struct RunSmem {
+    float4 lo[4][kRunCap], hi[4][kRunCap];    // boxes of 1, 4, 16 and 64 items from each item on
+    float4 clo[2][kRunCap], chi[2][kRunCap];  // left and right child of each separator's node: box, link
+    uint32_t below[64][kRunWarps];  // separators below v among 32 w .. 32 w + 31, at [v][w]
+    int xl[kRunCap + 1];            // first leaf of each item, then the end of the last one
+    int sep[kRunCap + 1];           // the separators around and between the items
+    int out[kRunCap];               // what leaves the run from item i on: -1 nothing, 0 the item,
+                                    // else the node of separator out[i]
+    uint8_t done[kRunCap];          // separators whose node lies in the run
+    int cstart[33];                 // the children's first items among those loaded together
+    int warp[kRunWarps];
+    int take, last;
 };
 
-// Where group g lies: its segment (first triangle, size), its tree blocks [blk0, blk1) as
-// global block numbers and its first leaf within the segment.  A group never crosses a segment.
+__device__ __forceinline__ void box_join(float4 &lo, float4 &hi, const float4 &l, const float4 &h) {
+    lo.x = fminf(lo.x, l.x); lo.y = fminf(lo.y, l.y); lo.z = fminf(lo.z, l.z);
+    hi.x = fmaxf(hi.x, h.x); hi.y = fmaxf(hi.y, h.y); hi.z = fmaxf(hi.z, h.z);
+}
+
+// The union of items [u, v): at most four windows of the largest length that fits (the last one
+// ends at v, overlapping the one before), their loads all in flight.
+__device__ __forceinline__ void run_box(const RunSmem &S, int u, int v, float4 &lo, float4 &hi) {
+    const int len = v - u, w = len >= 64 ? 3 : len >= 16 ? 2 : len >= 4 ? 1 : 0, step = 1 << (2 * w), z = v - step;
+    lo = S.lo[w][z];
+    hi = S.hi[w][z];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        if (u + k * step < z) box_join(lo, hi, S.lo[w][u + k * step], S.hi[w][u + k * step]);
+}
+
+// The open item of leaves [xl, xr]; dl, dr: the separators before and after it.
+__device__ __forceinline__ OpenItem open_item(float4 lo, float4 hi, int ref, int xl, int xr, int dl, int dr) {
+    OpenItem o;
+    o.lo = make_float4(lo.x, lo.y, lo.z, __int_as_float(ref));
+    o.hi = make_float4(hi.x, hi.y, hi.z, __int_as_float(dr));
+    o.xl = xl;
+    o.xr = xr;
+    o.pad0 = dl;
+    o.pad1 = 0;
+    return o;
+}
+
+// Every node of the run of M items in S (lo[0] with the links, hi[0], xl[0 .. M], sep[0 .. M]
+// set, a barrier since): records and parent links to memory; the run's own open items, in leaf
+// order, to dst (at most kOpenCap of them) or, when dst is null, back to S as the next run.
+// Returns their number (uniform).  ok: false when an index lies outside the segment (nothing is
+// written for it).
+//
+// Thread j: the node of separator j (split xl[j] - 1), which covers items a .. b - 1 between the
+// nearest smaller separators a, b on either side; it takes the node's box as the union of those
+// items and hands box and index to its parent's node (that of the larger of separators a, b).
+// Thread i also hands item i to its parent's node.
+__device__ __forceinline__ int reduce_run(RunSmem &S, int M, int n, float4 *nodes, int32_t *parents, OpenItem *dst,
+                                          bool &ok) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int mysep = t < M ? S.sep[t] : 64;
+    // which separators lie below each value, one ballot per value
+    uint32_t keep0 = 0, keep1 = 0;  // the ballots of v = lane and v = 32 + lane
+    if (32 * warp < M) {
+#pragma unroll 8
+        for (int v = 0; v < 32; ++v) {
+            const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, mysep < v), b1 = __ballot_sync(0xFFFFFFFFu, mysep < 32 + v);
+            keep0 = lane == v ? b0 : keep0;
+            keep1 = lane == v ? b1 : keep1;
+        }
+    }
+    S.below[lane][warp] = keep0;
+    S.below[32 + lane][warp] = keep1;
+    S.out[t] = -1;
+    // windows of 4, 16 and 64 items
+#pragma unroll
+    for (int w = 1; w < 4; ++w) {
+        const int len = 1 << (2 * w), part = len / 4;
+        if (M < len) break;  // uniform
+        if (t + len <= M) {
+            float4 lo = S.lo[w - 1][t], hi = S.hi[w - 1][t];
+#pragma unroll
+            for (int k = 1; k < 4; ++k) box_join(lo, hi, S.lo[w - 1][t + k * part], S.hi[w - 1][t + k * part]);
+            S.lo[w][t] = lo;
+            S.hi[w][t] = hi;
+        }
+        __syncthreads();
+    }
+    if (M < 4) __syncthreads();  // (the ballots)
+    const int j = t;
+    int na = -1, nb = 0, P = 0, np = 0, ip = 0;  // node's ends, index, its and the item's parent separator
+    float4 nlo, nhi;
+    if (j >= 1 && j < M) {
+        if (mysep < 0) ok = false;  // only a segment's ends have separator -1
+        const uint4 *row = reinterpret_cast<const uint4 *>(S.below[max(mysep, 0)]);
+        uint32_t wd[kRunWarps];
+#pragma unroll
+        for (int w = 0; w < kRunWarps; w += 4) {
+            const uint4 r = row[w / 4];
+            wd[w] = r.x; wd[w + 1] = r.y; wd[w + 2] = r.z; wd[w + 3] = r.w;
+        }
+        int a = -1, b = S.sep[M] < mysep ? M : M + 1;  // -1 and M + 1: none in the run
+#pragma unroll
+        for (int w = 0; w < kRunWarps; ++w) {  // the words below j's, the last non-zero one wins
+            const uint32_t m = w < warp ? wd[w] : w == warp ? wd[w] & lanemask_lt() : 0u;
+            if (m) a = 32 * w + 31 - __clz(m);
+        }
+#pragma unroll
+        for (int w = kRunWarps - 1; w >= 0; --w) {  // and above (bit j itself is never set)
+            const uint32_t m = w > warp ? wd[w] : w == warp ? wd[w] & ~lanemask_lt() : 0u;
+            if (m) b = 32 * w + __ffs(m) - 1;
+        }
+        const bool in = a >= 0 && b <= M;
+        S.done[j] = in;
+        if (in) {
+            na = a;
+            nb = b;
+            const int L = S.xl[a], R = S.xl[b] - 1;
+            const bool left = S.sep[b] > S.sep[a];  // the node is its parent's left child
+            const bool root = L == 0 && R == n - 1;
+            P = root ? 0 : left ? R : L;
+            np = root ? -1 : left ? b : a;
+            run_box(S, a, b, nlo, nhi);
+            nlo.w = __int_as_float(P);
+            if (np > 0 && np < M) {
+                S.clo[left ? 0 : 1][np] = nlo;
+                S.chi[left ? 0 : 1][np] = nhi;
+            }
+        }
+    }
+    if (t < M) {
+        const bool left = S.sep[t + 1] > mysep;
+        ip = left ? t + 1 : t;
+        if (ip > 0 && ip < M) {
+            S.clo[left ? 0 : 1][ip] = S.lo[0][t];
+            S.chi[left ? 0 : 1][ip] = S.hi[0][t];
+        }
+    }
+    __syncthreads();
+    // the records; and what leaves: items and nodes of the run whose parent's node does not lie in it
+    auto leaves = [&](int p) { return p == 0 || p == M || (p > 0 && !S.done[p]); };
+    if (t < M && leaves(ip)) S.out[t] = 0;
+    if (na >= 0) {
+        const float4 ll = S.clo[0][j], lh = S.chi[0][j], rl = S.clo[1][j], rh = S.chi[1][j];
+        const int lref = __float_as_int(ll.w), rref = __float_as_int(rl.w);
+        if ((uint32_t)P < (uint32_t)(n - 1) && lref >= -n && lref < n - 1 && rref >= -n && rref < n - 1) {
+            float4 *rec = nodes + 4ull * P;
+            rec[0] = ll;
+            rec[1] = make_float4(lh.x, lh.y, lh.z, __int_as_float(2));
+            rec[2] = rl;
+            rec[3] = make_float4(rh.x, rh.y, rh.z, __int_as_float(0));
+            parents[lref >= 0 ? lref : n - (lref + 1)] = P;
+            parents[rref >= 0 ? rref : n - (rref + 1)] = P;
+        } else {
+            ok = false;
+        }
+        if (leaves(np)) {
+            S.out[na] = j;
+            nhi.w = __int_as_float(nb);
+            S.lo[1][j] = nlo;  // the windows are read
+            S.hi[1][j] = nhi;
+        }
+    }
+    __syncthreads();
+    const int o = S.out[t];
+    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, o >= 0);
+    if (lane == 0) S.warp[warp] = __popc(bal);
+    float4 lo, hi;
+    int ref = 0, xl = 0, xr = 0, dl = 0, dr = 0;
+    if (o >= 0) {
+        lo = S.lo[o ? 1 : 0][o ? o : t];
+        hi = S.hi[o ? 1 : 0][o ? o : t];
+        const int b = o ? __float_as_int(hi.w) : t + 1;
+        ref = __float_as_int(lo.w);
+        xl = S.xl[t];
+        xr = S.xl[b] - 1;
+        dl = S.sep[t];
+        dr = S.sep[b];
+    }
+    const int end_xl = S.xl[M], end_sep = S.sep[M];
+    __syncthreads();
+    int at = __popc(bal & lanemask_lt()), total = 0;
+#pragma unroll
+    for (int w = 0; w < kRunWarps; ++w) {
+        const int c = S.warp[w];
+        at += w < warp ? c : 0;
+        total += c;
+    }
+    if (dst) {
+        if (o >= 0 && at < kOpenCap) dst[at] = open_item(lo, hi, ref, xl, xr, dl, dr);
+        return total;
+    }
+    if (o >= 0) {
+        lo.w = __int_as_float(ref);
+        S.lo[0][at] = lo;
+        S.hi[0][at] = hi;
+        S.xl[at] = xl;
+        S.sep[at] = dl;
+    }
+    if (t == 0) { S.xl[total] = end_xl; S.sep[total] = end_sep; }
+    __syncthreads();
+    return total;
+}
+
+// The tree blocks of one segment as the straddling pass sees them: its first triangle and size,
+// its tree blocks [blk0, blk1) as global block numbers and the group's number within it.
 struct GroupSpan {
     size_t start;
-    int n, blk0, blk1, leaf0;
+    int n, blk0, blk1, grp;
 };
 template <int LOG>
-struct OneSegGroups {  // plain build: blocks kBlocks g .. kBlocks g + kBlocks - 1 of the one segment
-    static constexpr int kBlocks = 4096 >> LOG;
-    static_assert(kBlocks <= kMaxGroupBlocks, "one warp scans a group's blocks");
+struct OneSegGroups {
+    static constexpr int kCtas = 3;  // 80 registers
     int n;
     __device__ __forceinline__ GroupSpan group(int g) const {
-        const int nblk = (n + (1 << LOG) - 1) >> LOG, b0 = g * kBlocks;
-        return GroupSpan{0, n, b0, min(nblk, b0 + kBlocks), b0 << LOG};
+        return GroupSpan{0, n, 0, (n + (1 << LOG) - 1) >> LOG, g};
     }
 };
-template <int LOG>
-struct ManySegGroups {  // batched build: a segment's blocks in groups of 16, from its first group
-    static constexpr int kBlocks = kGroupBlocks;
+struct ManySegGroups {  // groups never cross a segment; each starts at its segment's first group
+    static constexpr int kCtas = 4;  // many runs at once: 173 us at 4 against 185 at 3
     const SegRow *rows;
     const uint32_t *grp_seg;
     __device__ __forceinline__ GroupSpan group(int g) const {
         const uint32_t sg = __ldg(grp_seg + g);
         const uint32_t t0 = __ldg(&rows[sg].tri), t1 = __ldg(&rows[sg + 1].tri);
-        const int first = (int)__ldg(&rows[sg].blk), end = (int)__ldg(&rows[sg + 1].blk);
-        const int b0 = first + (g - (int)__ldg(&rows[sg].grp)) * kGroupBlocks;
-        return GroupSpan{t0, (int)(t1 - t0), b0, min(end, b0 + kGroupBlocks), (b0 - first) << LOG};
+        return GroupSpan{t0, (int)(t1 - t0), (int)__ldg(&rows[sg].blk), (int)__ldg(&rows[sg + 1].blk),
+                         g - (int)__ldg(&rows[sg].grp)};
     }
 };
 
-template <int LOG, class Groups>
-__global__ void __launch_bounds__(kGroupThreads) k_top_group(Groups groups, const OpenItem *__restrict__ items,
-                                                   const uint32_t *__restrict__ counts, float4 *nodes_all,
-                                                   int32_t *parents_all, uint32_t *arrive_all, float4 *pend_all,
-                                                   uint8_t *pend_d_all, const uint32_t *__restrict__ epoch_p,
-                                                   Control *ctl) {
-    constexpr int EB = 1 << LOG, GB = Groups::kBlocks;
+// counts: per tree block its open items, then (n_counts words on) the counters of the units that
+// start there, cleared by the tree pass.  A unit's open items are in its first block's slots.
+template <class Groups>
+__global__ void __launch_bounds__(kRunCap, Groups::kCtas) k_top_group(Groups groups, OpenItem *items, uint32_t *counts,
+                                                           uint32_t n_counts, float4 *nodes_all, int32_t *parents_all,
+                                                           Control *ctl) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    GroupSmem &S = *reinterpret_cast<GroupSmem *>(smem_raw);
+    RunSmem &S = *reinterpret_cast<RunSmem *>(smem_raw);
     const int t = threadIdx.x;
-    const int g = blockIdx.x;
     chain_wait();
     if (ld_relaxed_gpu(&ctl->err) & ERR_LOOKBACK_TIMEOUT) return;  // unsorted keys: nothing to build
-    const GroupSpan gs = groups.group(g);
-    const int n = gs.n, blk0 = gs.blk0, blk1 = gs.blk1;
-    const int lo_leaf = gs.leaf0, hi_leaf = min(n, gs.leaf0 + (blk1 - blk0) * EB);
+    const GroupSpan gs = groups.group(blockIdx.x);
+    const int n = gs.n, nblk = gs.blk1 - gs.blk0;
+    if (nblk < 2) return;  // one tree block: its root is complete
     float4 *nodes = nodes_all + 4ull * gs.start;
     int32_t *parents = parents_all + 2ull * gs.start;
-    uint32_t *arrive = arrive_all + gs.start;
-    float4 *pend = pend_all + 2ull * gs.start;
-    uint8_t *pend_d = pend_d_all + gs.start;
-    const uint32_t epoch = *epoch_p;
-    if (t < 32) {  // the blocks' item counts and their exclusive prefix (one warp)
-        const int c = (t < GB && blk0 + t < blk1) ? (int)min(counts[blk0 + t], (uint32_t)kOpenCap) : 0;
-        int incl = c;
+    bool ok = true;
+    // level 1: unit = group, children = tree blocks; each later level kFan times as wide
+    int unit = gs.grp;
+    long long stride = 1;  // tree blocks per child
+    for (int level = 1, fan = kGroupBlocks;; ++level, stride *= fan, fan = kFan, unit /= fan) {
+        const int first = (int)(unit * stride * fan);  // the unit's first block within the segment
+        const int nchild = (int)min((long long)fan, (nblk - first + stride - 1) / stride);
+        const size_t blk0 = (size_t)gs.blk0 + first;
+        if (level > 1) {
+            // the last child to come goes on with all of them; a single child is the unit
+            if (nchild > 1) {
+                __syncthreads();  // this block's items and count are written
+                if (t == 0) {
+                    uint32_t *tally = counts + n_counts + blk0 + (level - 1);
+                    S.last = atom_add_acq_rel_gpu(tally, 1u) == (uint32_t)(nchild - 1);
+                }
+                __syncthreads();
+                if (!S.last) break;
+            }
+        }
+        if (nchild > 1 || level == 1) {
+            // the children's items, as many children at a time as fit beside what is left of those
+            // before; a run of what came so far is reduced in between
+            int M = 0, c = 0;
+            while (c < nchild) {
+                if (t < 32) {
+                    const bool child = c + t < nchild;  // at most 32
+                    int incl = child ? (int)min(__ldcg(counts + blk0 + (c + t) * stride), (uint32_t)kOpenCap) : 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (t >= o) incl += y;
-        }
-        if (t < GB) S.bstart[t] = incl - c;
-        if (t == 31) {
-            S.bstart[GB] = incl;  // lanes from GB on count zero
-            S.cnt[0] = min(incl, kGroupCap);
-            S.nout = 0;
-        }
-    }
-    for (int h = t; h < kGroupHash; h += kGroupThreads) {
-        S.hkey[h] = -1;
-        S.hmask[h] = 0u;
-    }
-    __syncthreads();
-    const int total = S.bstart[GB];  // blocks past blk1 count zero
-    if (total > kGroupCap) {
-        // more items than shared memory holds: every item climbs with the arrival words
-        for (int b = blk0; b < blk1; ++b) {
-            const int c = S.bstart[b - blk0 + 1] - S.bstart[b - blk0];
-            for (int k = t; k < c; k += kGroupThreads)
-                if (!top_climb(items[(size_t)b * kOpenCap + k], n, nodes, parents, arrive, pend, pend_d, epoch))
-                    atomicOr(&ctl->err, ERR_CLIMB);
-        }
-        return;
-    }
-    // The group's items into shared memory: item `at` of the group is item at - bstart[b] of
-    // block blk0 + b.  Each thread holds at most two, and issues both loads before storing
-    // either (a loop over the blocks waited for one load per block in turn).
-    static_assert(kGroupCap <= 2 * kGroupThreads, "at most two items per thread");
-    auto src = [&](int at) -> const OpenItem & {
-        int b = 0;
-        while (S.bstart[b + 1] <= at) ++b;  // bstart[GB] = total > at: ends at a non-empty block
-        return items[(size_t)(blk0 + b) * kOpenCap + (at - S.bstart[b])];
-    };
-    {
-        const int a0 = t, a1 = t + kGroupThreads;
-        OpenItem i0, i1;
-        if (a0 < total) i0 = src(a0);
-        if (a1 < total) i1 = src(a1);
-        if (a0 < total) S.it[a0] = i0;
-        if (a1 < total) S.it[a1] = i1;
-    }
-    auto push_out = [&](int i) {
-        const int at = atomicAdd(&S.nout, 1);
-        S.out[at] = i;  // at most one entry per item: < kGroupCap
-    };
-    __syncthreads();
-    // Every item climbs on its own thread, with no barrier between levels: S.it[i] holds item
-    // i's current node; at a split the first child parks (its row and index published by the
-    // release of the arrival mask), the second merges both and climbs on with the parent.
-    const int count = S.cnt[0];
-    for (int i = t; i < count; i += kGroupThreads) {
-        OpenItem it = S.it[i];
-        for (int step = 0; step < 4 * EB; ++step) {
-            const int l = it.xl, r = it.xr, dl = it.pad0, dr = __float_as_int(it.hi.w);
-            const bool is_left = dr > dl;
-            const int s = is_left ? r : l - 1;
-            if (s < lo_leaf || s + 1 >= hi_leaf || s < 0 || s >= n - 1) {
-                push_out(i);
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                        if (t >= o) incl += y;
+                    }
+                    S.cstart[t + 1] = incl;
+                    if (t == 0) S.cstart[0] = 0;
+                    const uint32_t fits = __ballot_sync(0xFFFFFFFFu, child && M + incl <= kRunCap);
+                    if (t == 0) S.take = max(1, __popc(fits));
+                }
+                __syncthreads();
+                const int take = S.take, add = min(S.cstart[take], kRunCap - M);
+                // item t of them: child b's (a tree block's items are unordered: their place is their
+                // rank by first leaf)
+                OpenItem it;
+                int at = t, b0 = 0, b1 = 0;
+                if (t < add) {
+                    int b = 0;  // the last child that starts at or before t
+#pragma unroll
+                    for (int h = 16; h > 0; h >>= 1) b += b + h < take && S.cstart[b + h] <= t ? h : 0;
+                    b0 = S.cstart[b];
+                    b1 = min(S.cstart[b + 1], add);
+                    const OpenItem *src = items + (blk0 + (c + b) * stride) * kOpenCap + (t - b0);
+                    it.lo = __ldcg(&src->lo);
+                    it.hi = __ldcg(&src->hi);
+                    const int4 x = __ldcg(reinterpret_cast<const int4 *>(&src->xl));
+                    it.xl = x.x;
+                    it.xr = x.y;
+                    it.pad0 = x.z;
+                    S.out[t] = x.x;
+                    // every first leaf inside the segment: what is derived from it then is too
+                    if (x.x < 0 || x.y < x.x || x.y >= n || x.z < -1 || x.z > 63) ok = false;
+                }
+                if (level == 1) {  // uniform
+                    __syncthreads();
+                    if (t < add) {
+                        at = b0;
+#pragma unroll 4
+                        for (int k = b0; k < b1; ++k) at += S.out[k] < it.xl;
+                    }
+                }
+                if (t < add) {
+                    const int x = M + at;
+                    S.lo[0][x] = it.lo;
+                    S.hi[0][x] = it.hi;
+                    S.xl[x] = it.xl;
+                    S.sep[x] = it.pad0;
+                    if (at == add - 1) {  // the run's end
+                        S.xl[x + 1] = it.xr + 1;
+                        S.sep[x + 1] = __float_as_int(it.hi.w);
+                    }
+                }
+                M += add;
+                c += take;
+                if (__syncthreads_or(!ok)) { M = 0; ok = false; break; }  // inconsistent items: build nothing from them
+                if (M > 0) M = reduce_run(S, M, n, nodes, parents, c < nchild ? nullptr : items + blk0 * kOpenCap, ok);
+                if (M > kOpenCap) { ok = false; M = kOpenCap; }
+            }
+            if (t == 0) counts[blk0] = (uint32_t)M;
+            if (first == 0 && stride * fan >= nblk) {  // the whole segment: nothing may be left
+                if (M != 0) ok = false;
                 break;
             }
-            uint32_t h = ((uint32_t)s * 2654435761u) & (kGroupHash - 1);
-            for (int probe = 0; probe < kGroupHash; ++probe) {
-                const int prev = atomicCAS(&S.hkey[h], -1, s);
-                if (prev == -1 || prev == s) break;
-                h = (h + 1) & (kGroupHash - 1);
-            }
-            const int side = is_left ? 0 : 1;
-            S.hidx[h][side] = i;
-            if (atom_or_acq_rel_cta(&S.hmask[h], 1u << side) == 0u) break;  // first parks
-            const int j = S.hidx[h][side ^ 1];
-            const OpenItem sb = S.it[j];
-            const int L = is_left ? l : sb.xl, R = is_left ? sb.xr : r;
-            const int ndl = is_left ? dl : sb.pad0, ndr = is_left ? __float_as_int(sb.hi.w) : dr;
-            const bool root = L == 0 && R == n - 1;
-            const int P = root ? 0 : (ndr > ndl ? R : L);
-            const OpenItem &lc = is_left ? it : sb;
-            const OpenItem &rc = is_left ? sb : it;
-            float4 *rec = nodes + 4ull * P;
-            rec[0] = lc.lo;
-            rec[1] = make_float4(lc.hi.x, lc.hi.y, lc.hi.z, __int_as_float(2));
-            rec[2] = rc.lo;
-            rec[3] = make_float4(rc.hi.x, rc.hi.y, rc.hi.z, __int_as_float(0));
-            const int lref = __float_as_int(lc.lo.w), rref = __float_as_int(rc.lo.w);
-            parents[lref >= 0 ? lref : n - (lref + 1)] = P;
-            parents[rref >= 0 ? rref : n - (rref + 1)] = P;
-            if (root) break;
-            OpenItem pa;
-            pa.lo = make_float4(fminf(it.lo.x, sb.lo.x), fminf(it.lo.y, sb.lo.y), fminf(it.lo.z, sb.lo.z),
-                                __int_as_float(P));
-            pa.hi = make_float4(fmaxf(it.hi.x, sb.hi.x), fmaxf(it.hi.y, sb.hi.y), fmaxf(it.hi.z, sb.hi.z),
-                                __int_as_float(ndr));
-            pa.xl = L;
-            pa.xr = R;
-            pa.pad0 = ndl;
-            pa.pad1 = 0;
-            S.it[i] = pa;
-            it = pa;
         }
     }
-    __syncthreads();
-    // a child parked at a split whose sibling never came: its parent leaves the group
-    for (int h = t; h < kGroupHash; h += kGroupThreads) {
-        const uint32_t mk = S.hmask[h];
-        if (mk == 1u || mk == 2u) push_out(S.hidx[h][mk == 1u ? 0 : 1]);
-    }
-    __syncthreads();
-    // what leaves the group climbs on at once with the arrival words, beside the other groups'
-    // shared-memory climbs (those touch only splits inside their groups)
-    const int nout = S.nout;
-    for (int k = t; k < nout; k += kGroupThreads)
-        if (!top_climb(S.it[S.out[k]], n, nodes, parents, arrive, pend, pend_d, epoch)) atomicOr(&ctl->err, ERR_CLIMB);
+    if (!ok) atomicOr(&ctl->err, ERR_CLIMB);
 }
 
 // the layout plus the slack that puts it on a 128-byte boundary
@@ -873,11 +942,9 @@ cudaError_t soup_tensor_map(CUtensorMap *m, const float4 *tri, uint32_t rows) {
 
 template <int LOG, class Segs, class Leaves>
 void launch_emit_impl(Segs segs, int groups, Leaves lv, const CUtensorMap &soup_map, const uint32_t *keys,
-                      float4 *nodes, int32_t *parents,
-                      OpenItem *items, uint32_t *counts, uint32_t *arrive, float4 *pend,
-                      uint8_t *pend_d, const uint32_t *epoch, Control *ctl, bool top,
-                      cudaStream_t s, cudaEvent_t *ev, int ctas_per_sm,
-                      const uint32_t *grp_seg = nullptr, int ngroups = 0) {
+                      float4 *nodes, int32_t *parents, OpenItem *items, uint32_t *counts, Control *ctl,
+                      cudaStream_t s, cudaEvent_t *ev, int ctas_per_sm, const uint32_t *grp_seg = nullptr,
+                      int ngroups = 0) {
     if (ev) cudaEventRecord(ev[0], s);  // the leaf gather runs inside the tree pass
     const int per_sm = ctas_per_sm > 0 && ctas_per_sm < TreeGeo<LOG>::kCtasPerSm ? ctas_per_sm
                                                                                 : TreeGeo<LOG>::kCtasPerSm;
@@ -888,23 +955,14 @@ void launch_emit_impl(Segs segs, int groups, Leaves lv, const CUtensorMap &soup_
     launch_chained(chain, k_tree_climb<LOG, Segs, Leaves>, grid, TreeGeo<LOG>::EB, leaves_smem_bytes<LOG, Segs, Leaves>(), s,
                    segs, keys, lv, nodes, parents, items, counts, ctl, soup_map);
     if (ev) cudaEventRecord(ev[1], s);
-    if (top) {
-        if constexpr (std::is_same<Segs, OneSeg<LOG>>::value) {
-            constexpr int GB = OneSegGroups<LOG>::kBlocks;
-            const int ngroups = (groups + GB - 1) / GB;
-            launch_chained(chain, k_top_group<LOG, OneSegGroups<LOG>>, ngroups, kGroupThreads, sizeof(GroupSmem), s,
-                           OneSegGroups<LOG>{segs.n}, items, counts, nodes, parents, arrive, pend, pend_d, epoch, ctl);
-        } else if (grp_seg) {
-            // batched: the same over groups of 16 blocks that never cross a mesh
-            const ManySegGroups<LOG> gr{segs.rows, grp_seg};
-            if (ngroups > 0)
-                launch_chained(chain, k_top_group<LOG, ManySegGroups<LOG>>, ngroups, kGroupThreads, sizeof(GroupSmem), s, gr,
-                               items, counts, nodes, parents, arrive, pend, pend_d, epoch, ctl);
-        } else {
-            k_emit_top<<<(groups * kTopLanes + 255) / 256, 256, 0, s>>>(segs, items, kOpenCap, counts, nodes,
-                                                                         parents, arrive, pend, pend_d,
-                                                                         epoch, ctl);
-        }
+    if constexpr (std::is_same<Segs, OneSeg<LOG>>::value) {
+        if (groups > 1)
+            launch_chained(chain, k_top_group<OneSegGroups<LOG>>, straddle_groups((uint32_t)groups), kRunCap,
+                           sizeof(RunSmem), s, OneSegGroups<LOG>{segs.n}, items, counts, (uint32_t)groups, nodes,
+                           parents, ctl);
+    } else if (ngroups > 0) {
+        launch_chained(chain, k_top_group<ManySegGroups>, ngroups, kRunCap, sizeof(RunSmem), s,
+                       ManySegGroups{segs.rows, grp_seg}, items, counts, (uint32_t)groups, nodes, parents, ctl);
     }
     if (ev) cudaEventRecord(ev[2], s);
 }
@@ -929,49 +987,41 @@ cudaError_t emit_init() {
     if (e == cudaSuccess)
         e = prefer_shared(k_tree_climb<L, OneSeg<L>, MeshLeaves>, leaves_smem_bytes<L, OneSeg<L>, MeshLeaves>());
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_top_group<kLogEmitBlock, OneSegGroups<kLogEmitBlock>>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmem));
+        e = cudaFuncSetAttribute(k_top_group<OneSegGroups<L>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(RunSmem));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_top_group<8, ManySegGroups<8>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(GroupSmem));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_top_group<7, ManySegGroups<7>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(GroupSmem));
+        e = cudaFuncSetAttribute(k_top_group<ManySegGroups>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(RunSmem));
     return e;
 }
 
 cudaError_t launch_emit(const float4 *tri, const uint32_t *perm, const uint32_t *keys, uint32_t n,
                         float4 *otri, float4 *nodes, int32_t *parents, OpenItem *items,
-                        uint32_t *counts, uint32_t *arrive, float4 *pend, uint8_t *pend_d,
-                        const uint32_t *epoch, Control *ctl, cudaStream_t s, cudaEvent_t *ev) {
+                        uint32_t *counts, Control *ctl, cudaStream_t s, cudaEvent_t *ev) {
     if (n == 0) return cudaSuccess;
     CUtensorMap map;
     const cudaError_t e = soup_tensor_map(&map, tri, n);
     if (e != cudaSuccess) return e;
     const int groups = (int)emit_groups(n, kLogEmitBlock);
     launch_emit_impl<kLogEmitBlock>(OneSeg<kLogEmitBlock>{(int)n}, groups, SoupLeaves{tri, perm, otri}, map, keys,
-                                    nodes, parents, items, counts, arrive, pend, pend_d, epoch,
-                                    ctl, groups > 1, s, ev, 0);
+                                    nodes, parents, items, counts, ctl, s, ev, 0);
     return cudaSuccess;
 }
 
 void launch_emit_mesh(const float4 *verts, uint32_t num_verts, const uint32_t *sidx, const uint32_t *keys,
                       uint32_t n, float4 *nodes, int32_t *parents, OpenItem *items, uint32_t *counts,
-                      uint32_t *arrive, float4 *pend, uint8_t *pend_d, const uint32_t *epoch, Control *ctl,
-                      cudaStream_t s, cudaEvent_t *ev) {
+                      Control *ctl, cudaStream_t s, cudaEvent_t *ev) {
     if (n == 0) return;
     const int groups = (int)emit_groups(n, kLogEmitBlock);
     CUtensorMap unused;  // mesh leaves come by cp.async
     std::memset(&unused, 0, sizeof unused);
     launch_emit_impl<kLogEmitBlock>(OneSeg<kLogEmitBlock>{(int)n}, groups, MeshLeaves{verts, sidx, num_verts},
-                                    unused, keys, nodes, parents, items, counts, arrive, pend, pend_d, epoch, ctl,
-                                    groups > 1, s, ev, 0);
+                                    unused, keys, nodes, parents, items, counts, ctl, s, ev, 0);
 }
 
 cudaError_t launch_emit_batch(const BatchPlan &bp, const float4 *tri, const uint32_t *perm,
                               const uint32_t *keys, float4 *otri, float4 *nodes, int32_t *parents,
-                              OpenItem *items, uint32_t *counts, uint32_t *arrive, float4 *pend,
-                              uint8_t *pend_d, const uint32_t *epoch, Control *ctl, cudaStream_t s,
+                              OpenItem *items, uint32_t *counts, Control *ctl, cudaStream_t s,
                               cudaEvent_t *ev) {
     if (bp.blocks == 0) return cudaSuccess;
     CUtensorMap map;
@@ -979,12 +1029,12 @@ cudaError_t launch_emit_batch(const BatchPlan &bp, const float4 *tri, const uint
     if (e != cudaSuccess) return e;
     if (bp.log_block == 7)
         launch_emit_impl<7>(ManySegs<7>{bp.rows, bp.blk_seg, (int)bp.blocks}, (int)bp.blocks,
-                            SoupLeaves{tri, perm, otri}, map, keys, nodes, parents, items, counts, arrive, pend,
-                            pend_d, epoch, ctl, true, s, ev, bp.tree_ctas_per_sm, bp.grp_seg, (int)bp.groups);
+                            SoupLeaves{tri, perm, otri}, map, keys, nodes, parents, items, counts, ctl, s, ev,
+                            bp.tree_ctas_per_sm, bp.grp_seg, (int)bp.groups);
     else
         launch_emit_impl<8>(ManySegs<8>{bp.rows, bp.blk_seg, (int)bp.blocks}, (int)bp.blocks,
-                            SoupLeaves{tri, perm, otri}, map, keys, nodes, parents, items, counts, arrive, pend,
-                            pend_d, epoch, ctl, true, s, ev, bp.tree_ctas_per_sm, bp.grp_seg, (int)bp.groups);
+                            SoupLeaves{tri, perm, otri}, map, keys, nodes, parents, items, counts, ctl, s, ev,
+                            bp.tree_ctas_per_sm, bp.grp_seg, (int)bp.groups);
     return cudaSuccess;
 }
 

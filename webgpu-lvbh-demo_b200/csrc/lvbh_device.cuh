@@ -74,11 +74,6 @@ __device__ __forceinline__ bool finite3(float4 v) {
     return isfinite(v.x) && isfinite(v.y) && isfinite(v.z);
 }
 
-// Acquire-release fences: order this thread's earlier memory operations before its later
-// ones for the given scope (the park / merge handshakes need no sequential consistency).
-__device__ __forceinline__ void fence_acq_rel_cta() { asm volatile("fence.acq_rel.cta;" ::: "memory"); }
-__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-
 // Programmatic dependent launch.  A kernel launched by launch_chained starts launching once
 // every block of the kernel before it on the stream has exited, before that kernel's
 // completion is flushed; chain_wait blocks until the kernel before has completed and its
@@ -99,11 +94,11 @@ __device__ __forceinline__ uint32_t atom_or_acq_rel_cta(uint32_t *p, uint32_t v)
     return old;
 }
 
-// Global-memory atomic exchange with acquire-release semantics at GPU scope (the park / merge
-// handshake across CTAs, as atom_or_acq_rel_cta is within one).
-__device__ __forceinline__ uint32_t atom_exch_acq_rel_gpu(uint32_t *p, uint32_t v) {
+// Global-memory atomic add with acquire-release semantics at GPU scope: after a block barrier it
+// publishes the whole block's writes to a thread that later reads a value at least as new.
+__device__ __forceinline__ uint32_t atom_add_acq_rel_gpu(uint32_t *p, uint32_t v) {
     uint32_t old;
-    asm volatile("atom.acq_rel.gpu.global.exch.b32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
     return old;
 }
 

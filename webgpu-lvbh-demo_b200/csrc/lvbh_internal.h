@@ -154,20 +154,20 @@ size_t ctx_device_bytes(const lvbh_ctx *ctx);
 void launch_bounds(const float4 *tri, uint32_t n, Control *ctl, cudaStream_t s);
 // K1b: triangle box centroid -> Morton key (input order), the first sort pass's tile
 // histograms, chunk sums (sort_scratch) and global digit counts (ctl->hist_part, zero before); flags
-// non-finite vertices in ctl->err and advances the build epoch *epoch used by K3c.
+// non-finite vertices in ctl->err.
 void launch_morton(const float4 *tri, uint32_t n, HostBounds hb, Control *ctl,
-                   uint32_t *keys_out, uint32_t *epoch, uint32_t *sort_scratch, cudaStream_t s);
+                   uint32_t *keys_out, uint32_t *sort_scratch, cudaStream_t s);
 // K1b over the sort-tile chunks [c0, c1) only (chunk = sort_chunk_tiles(n) tiles): the keys of
 // a soup uploaded chunk by chunk, each part launched once its triangles have landed.
 void launch_morton_chunks(const float4 *tri, uint32_t n, HostBounds hb, Control *ctl, uint32_t *keys,
-                          uint32_t *epoch, uint32_t *sort_scratch, uint32_t c0, uint32_t c1, cudaStream_t s);
+                          uint32_t *sort_scratch, uint32_t c0, uint32_t c1, cudaStream_t s);
 // K1a + K1b split for a soup whose box is reduced on the device: K1a over triangles [t0, t1)
 // also stores each triangle's centroid (cen[t], cen[stride + t], cen[2 stride + t]); K1b then
 // quantises the centroids (12 bytes per triangle instead of the 48-byte soup).
 void launch_bounds_cen(const float4 *tri, uint32_t t0, uint32_t t1, float *cen, uint32_t cen_stride,
                        Control *ctl, cudaStream_t s);
 void launch_morton_cen(const float *cen, uint32_t cen_stride, uint32_t n, Control *ctl, uint32_t *keys,
-                       uint32_t *epoch, uint32_t *sort_scratch, cudaStream_t s);
+                       uint32_t *sort_scratch, cudaStream_t s);
 cudaError_t morton_init();  // once per device, before the first launch
 // K2: one reduce-then-scan pass over 10-bit digit `pass` (0..2) of 30-bit keys.  counted: the
 // tile histograms, chunk sums and global digit counts (ctl->hist_part) of this pass are there
@@ -186,18 +186,17 @@ void launch_onesweep32(const uint32_t *keys_in, const uint32_t *vals_in, uint32_
 cudaError_t sort_init();  // once per device, before the first launch
 // K3: leaf gather + rearrange + in-block radix tree and refit (K3b), straddling nodes (K3c)
 // -> BVH nodes, parent links, sorted triangles.  Scratch: items (emit_groups(n) * kOpenCap)
-// and counts (emit_groups(n)), arrive (n words, zero or older epochs), pend (2n float4),
-// pend_d (n bytes); *epoch is this build's epoch (advanced by K1b).
+// and counts (2 emit_groups(n): a tree block's open items and a counter of the straddling pass).
 size_t emit_groups(uint32_t n, int log_eb = kLogEmitBlock);
 // Groups of the straddling pass's first level over `blocks` tree blocks of one segment.
-inline uint32_t straddle_groups(uint32_t blocks) { return (blocks + 15u) / 16u; }
+constexpr int kGroupBlocks = 24, kFan = 16;  // tree blocks per group; groups per later unit
+inline uint32_t straddle_groups(uint32_t blocks) { return (blocks + kGroupBlocks - 1u) / kGroupBlocks; }
 cudaError_t emit_init();  // once per device, before the first launch
 // ev (may be nullptr): three events, recorded before K3b, after K3b and after K3c.  An error:
 // the soup's tensor map (K3b's gather) could not be made; nothing was launched.
 cudaError_t launch_emit(const float4 *tri, const uint32_t *perm, const uint32_t *keys, uint32_t n,
                         float4 *otri, float4 *nodes, int32_t *parents, OpenItem *items,
-                        uint32_t *counts, uint32_t *arrive, float4 *pend, uint8_t *pend_d,
-                        const uint32_t *epoch, Control *ctl, cudaStream_t s, cudaEvent_t *ev);
+                        uint32_t *counts, Control *ctl, cudaStream_t s, cudaEvent_t *ev);
 // Batched forms of K1a, K1b, K2 and K3 over the segments of `bp`.  seg_ord holds 6 ordered
 // bound words per segment (zeroed before K1a; min at 0-2 as ~ord_lo, max at 3-5 as ord_lo),
 // seg_hist 4 x 256 digit counts per segment (zeroed before K1b); host_bounds, when not null,
@@ -210,17 +209,16 @@ void launch_bounds_batch(const BatchPlan &bp, const float4 *tri, const float *ho
 // seg_hist: kHistWords per segment, pass-major (bp.digit_bits wide digits).
 void launch_morton_batch(const BatchPlan &bp, const float4 *tri, const float *host_bounds,
                          const uint32_t *seg_ord, uint32_t *seg_hist, Control *ctl,
-                         uint32_t *keys_out, uint32_t *epoch, cudaStream_t s);
+                         uint32_t *keys_out, cudaStream_t s);
 void launch_onesweep_batch(const BatchPlan &bp, const uint32_t *keys_in, const uint32_t *vals_in,
                            uint32_t *keys_out, uint32_t *vals_out, int pass,
                            const uint32_t *seg_hist, Control *ctl, uint32_t *lookback,
                            cudaStream_t s);
-// items / counts: bp.blocks * kOpenCap / bp.blocks entries (open items per tree block).
+// items / counts: bp.blocks * kOpenCap / 2 bp.blocks entries.
 // Errors as launch_emit.
 cudaError_t launch_emit_batch(const BatchPlan &bp, const float4 *tri, const uint32_t *perm,
                               const uint32_t *keys, float4 *otri, float4 *nodes, int32_t *parents,
-                              OpenItem *items, uint32_t *counts, uint32_t *arrive, float4 *pend,
-                              uint8_t *pend_d, const uint32_t *epoch, Control *ctl, cudaStream_t s,
+                              OpenItem *items, uint32_t *counts, Control *ctl, cudaStream_t s,
                               cudaEvent_t *ev);
 // Indexed mesh -> 48-byte soup (pad 0).  An index >= num_verts sets ERR_BAD_INDEX in
 // *err and gathers zeros instead of reading out of bounds.
@@ -237,12 +235,11 @@ void launch_trace(const float4 *nodes, const float4 *tris, uint32_t n, const flo
 void launch_bounds_mesh(const float4 *verts, uint32_t nverts, const uint32_t *idx3, uint32_t n, Control *ctl,
                         cudaStream_t s);
 void launch_morton_mesh(const float4 *verts, uint32_t nverts, const uint32_t *idx3, uint32_t n, HostBounds hb,
-                        Control *ctl, uint32_t *keys, uint32_t *epoch, uint32_t *sort_scratch, cudaStream_t s);
+                        Control *ctl, uint32_t *keys, uint32_t *sort_scratch, cudaStream_t s);
 void launch_leaf_idx(const uint32_t *idx3, const uint32_t *perm, uint32_t n, uint32_t *sidx, cudaStream_t s);
 void launch_emit_mesh(const float4 *verts, uint32_t num_verts, const uint32_t *sidx, const uint32_t *keys,
                       uint32_t n, float4 *nodes, int32_t *parents, OpenItem *items, uint32_t *counts,
-                      uint32_t *arrive, float4 *pend, uint8_t *pend_d, const uint32_t *epoch, Control *ctl,
-                      cudaStream_t s, cudaEvent_t *ev);
+                      Control *ctl, cudaStream_t s, cudaEvent_t *ev);
 // K5 over the indexed leaf format: leaf i's vertices are verts[sidx[3i..3i+2]].
 void launch_trace_mesh(const float4 *nodes, const float4 *verts, uint32_t num_verts, const uint32_t *sidx, uint32_t n,
                        const float4 *rays, uint32_t num_rays, int32_t *hit_prim, float *hit_t,

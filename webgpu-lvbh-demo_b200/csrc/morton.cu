@@ -151,7 +151,7 @@ template <int SRC, int THREADS = kThreads>
 __global__ void __launch_bounds__(THREADS) k_morton(const float4 *__restrict__ tri, uint32_t n,
                                                      HostBounds hb, Control *__restrict__ ctl,
                                                      uint32_t *__restrict__ keys,
-                                                     uint32_t *__restrict__ epoch, uint32_t chunk_tiles,
+                                                     uint32_t chunk_tiles,
                                                      uint32_t *__restrict__ tile_hist,
                                                      uint32_t *__restrict__ chunk_sum,
                                                      const uint32_t *__restrict__ idx3, uint32_t nverts,
@@ -162,10 +162,6 @@ __global__ void __launch_bounds__(THREADS) k_morton(const float4 *__restrict__ t
     constexpr int WARPS = THREADS / 32;
     __shared__ float4 stage[MESH ? 1 : WARPS][96];
     __shared__ uint32_t th[kDigits];
-    if (chunk == 0 && threadIdx.x == 0) {  // new arrival epoch for K3c; 0 is never used
-        const uint32_t e = *epoch + 1u;
-        *epoch = e == 0u ? 1u : e;
-    }
 
     float umin[3], umax[3];
     if (hb.use) {
@@ -291,8 +287,7 @@ struct CenSmem {
 };
 __global__ void __launch_bounds__(kCenThreads) k_morton_cen(const float *__restrict__ cen, uint32_t cen_stride,
                                                             uint32_t n, Control *__restrict__ ctl,
-                                                            uint32_t *__restrict__ keys, uint32_t *__restrict__ epoch,
-                                                            uint32_t chunk_tiles, uint32_t *__restrict__ tile_hist,
+                                                            uint32_t *__restrict__ keys, uint32_t chunk_tiles, uint32_t *__restrict__ tile_hist,
                                                             uint32_t *__restrict__ chunk_sum) {
     constexpr int WARPS = kCenThreads / 32, P = kDigits / kCenThreads, R = kSortTile / 32 / WARPS;
     static_assert(R * WARPS * 32 == kSortTile && P * kCenThreads == kDigits, "whole rows and digits");
@@ -301,10 +296,6 @@ __global__ void __launch_bounds__(kCenThreads) k_morton_cen(const float *__restr
     __shared__ uint32_t th[2][kDigits];  // a tile's counts, alternating with the buffers
     const uint32_t chunk = blockIdx.x;
     chain_wait();
-    if (chunk == 0 && threadIdx.x == 0) {  // new arrival epoch for K3c; 0 is never used
-        const uint32_t e = *epoch + 1u;
-        *epoch = e == 0u ? 1u : e;
-    }
     float umin[3], umax[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -471,16 +462,11 @@ __global__ void __launch_bounds__(kThreads) k_morton_batch(const float4 *__restr
                                                            const uint32_t *__restrict__ seg_ord,
                                                            uint32_t *__restrict__ seg_hist,
                                                            Control *__restrict__ ctl,
-                                                           uint32_t *__restrict__ keys,
-                                                           uint32_t *__restrict__ epoch) {
+                                                           uint32_t *__restrict__ keys) {
     constexpr int D = 1 << BITS, NP = BITS == kDigitBits ? kSortPasses : kSortPasses32;
     static_assert(NP * D <= kHistWords, "per-segment counts");
     __shared__ float4 stage[kWarps][96];
     __shared__ uint32_t hist[NP][D];
-    if (blockIdx.x == 0 && threadIdx.x == 0) {  // new arrival epoch for K3c; 0 is never used
-        const uint32_t e = *epoch + 1u;
-        *epoch = e == 0u ? 1u : e;
-    }
     for (int i = threadIdx.x; i < NP * D; i += kThreads) (&hist[0][0])[i] = 0;
     const uint32_t tile = blockIdx.x, sg = __ldg(tile_seg + tile);
     const uint32_t t0 = __ldg(&rows[sg].tri), t1 = __ldg(&rows[sg + 1].tri);
@@ -596,15 +582,15 @@ void launch_bounds(const float4 *tri, uint32_t n, Control *ctl, cudaStream_t s) 
 }
 
 void launch_morton(const float4 *tri, uint32_t n, HostBounds hb, Control *ctl, uint32_t *keys,
-                   uint32_t *epoch, uint32_t *sort_scratch, cudaStream_t s) {
+                   uint32_t *sort_scratch, cudaStream_t s) {
     if (n == 0) return;
-    launch_morton_chunks(tri, n, hb, ctl, keys, epoch, sort_scratch, 0, sort_chunks(n), s);
+    launch_morton_chunks(tri, n, hb, ctl, keys, sort_scratch, 0, sort_chunks(n), s);
 }
 
 void launch_morton_chunks(const float4 *tri, uint32_t n, HostBounds hb, Control *ctl, uint32_t *keys,
-                          uint32_t *epoch, uint32_t *sort_scratch, uint32_t c0, uint32_t c1, cudaStream_t s) {
+                          uint32_t *sort_scratch, uint32_t c0, uint32_t c1, cudaStream_t s) {
     if (n == 0 || c1 <= c0) return;
-    k_morton<kSrcSoup><<<c1 - c0, kThreads, 0, s>>>(tri, n, hb, ctl, keys, epoch, sort_chunk_tiles(n),
+    k_morton<kSrcSoup><<<c1 - c0, kThreads, 0, s>>>(tri, n, hb, ctl, keys, sort_chunk_tiles(n),
                                                     sort_scratch, sort_chunk_sums(sort_scratch, n), nullptr, 0u,
                                                     c0);
 }
@@ -619,10 +605,10 @@ void launch_bounds_cen(const float4 *tri, uint32_t t0, uint32_t t1, float *cen, 
 }
 
 void launch_morton_cen(const float *cen, uint32_t cen_stride, uint32_t n, Control *ctl, uint32_t *keys,
-                       uint32_t *epoch, uint32_t *sort_scratch, cudaStream_t s) {
+                       uint32_t *sort_scratch, cudaStream_t s) {
     if (n == 0) return;
     launch_chained(chain_build(n), k_morton_cen, sort_chunks(n), kCenThreads, sizeof(CenSmem), s, cen, cen_stride, n, ctl, keys,
-                   epoch, sort_chunk_tiles(n), sort_scratch, sort_chunk_sums(sort_scratch, n));
+                   sort_chunk_tiles(n), sort_scratch, sort_chunk_sums(sort_scratch, n));
 }
 
 cudaError_t morton_init() {
@@ -639,9 +625,9 @@ void launch_bounds_mesh(const float4 *verts, uint32_t nverts, const uint32_t *id
 }
 
 void launch_morton_mesh(const float4 *verts, uint32_t nverts, const uint32_t *idx3, uint32_t n, HostBounds hb,
-                        Control *ctl, uint32_t *keys, uint32_t *epoch, uint32_t *sort_scratch, cudaStream_t s) {
+                        Control *ctl, uint32_t *keys, uint32_t *sort_scratch, cudaStream_t s) {
     if (n == 0) return;
-    k_morton<kSrcMesh><<<sort_chunks(n), kThreads, 0, s>>>(verts, n, hb, ctl, keys, epoch, sort_chunk_tiles(n),
+    k_morton<kSrcMesh><<<sort_chunks(n), kThreads, 0, s>>>(verts, n, hb, ctl, keys, sort_chunk_tiles(n),
                                                            sort_scratch, sort_chunk_sums(sort_scratch, n), idx3,
                                                            nverts, 0u);
 }
@@ -671,14 +657,14 @@ void launch_bounds_batch(const BatchPlan &bp, const float4 *tri, const float *ho
 
 void launch_morton_batch(const BatchPlan &bp, const float4 *tri, const float *host_bounds,
                          const uint32_t *seg_ord, uint32_t *seg_hist, Control *ctl,
-                         uint32_t *keys_out, uint32_t *epoch, cudaStream_t s) {
+                         uint32_t *keys_out, cudaStream_t s) {
     if (bp.tiles == 0) return;
     if (bp.digit_bits == kDigitBits32)
         k_morton_batch<kDigitBits32><<<bp.tiles, kThreads, 0, s>>>(tri, bp.rows, bp.tile_seg, host_bounds,
-                                                                   seg_ord, seg_hist, ctl, keys_out, epoch);
+                                                                   seg_ord, seg_hist, ctl, keys_out);
     else
         k_morton_batch<kDigitBits><<<bp.tiles, kThreads, 0, s>>>(tri, bp.rows, bp.tile_seg, host_bounds,
-                                                                 seg_ord, seg_hist, ctl, keys_out, epoch);
+                                                                 seg_ord, seg_hist, ctl, keys_out);
 }
 
 }  // namespace lvbh
