@@ -14,17 +14,24 @@ namespace lvbh {
 namespace {
 
 constexpr int kStack = 64;  // the reference's private stack holds 32 (:493)
-constexpr int kSmemStack = 32;  // the first entries of a ray's stack, in shared memory
 
-// A ray's stack: entries 0 .. kSmemStack - 1 in shared memory, entry i of thread t at [i][t] (a
-// warp's 32 entries of one depth in 32 banks); deeper entries (rare) in thread-local memory.
-template <int NT>
+// A stack entry: the node pushed and the distance of its box (a popped internal node whose box
+// begins at or past the closest hit so far has nothing to offer, see ray_step).
+struct StackEntry {
+    int32_t node;
+    float dist;
+};
+// A ray's stack: the first DEPTH entries in shared memory, entry i of thread t at [i][t]; deeper
+// entries (rare) in thread-local memory.
+template <int NT, int DEPTH>
 struct RayStack {
-    int32_t *s;     // &smem[0][threadIdx.x] of a [kSmemStack][NT] array
-    int32_t *deep;  // kStack - kSmemStack entries
-    __device__ __forceinline__ int32_t &operator[](int i) const {
-        return i < kSmemStack ? s[i * NT] : deep[i - kSmemStack];
+    StackEntry *s;     // &smem[0][threadIdx.x] of a [DEPTH][NT] array
+    StackEntry *deep;  // kStack - DEPTH entries
+    __device__ __forceinline__ void put(int i, StackEntry e) const {
+        if (i < DEPTH) s[i * NT] = e;
+        else deep[i - DEPTH] = e;
     }
+    __device__ __forceinline__ StackEntry get(int i) const { return i < DEPTH ? s[i * NT] : deep[i - DEPTH]; }
 };
 
 struct F3 { float x, y, z; };
@@ -42,6 +49,19 @@ __device__ __forceinline__ F3 cross3(F3 a, F3 b) {
             __fsub_rn(__fmul_rn(a.x, b.y), __fmul_rn(a.y, b.x))};
 }
 
+// Two consecutive float4: one 32-byte load (WIDE: p on a 32-byte boundary) or two of 16.
+template <bool WIDE>
+__device__ __forceinline__ void ldg_pair(const float4 *p, float4 &a, float4 &b) {
+    if constexpr (WIDE) {
+        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+            : "l"(p));
+    } else {
+        a = __ldg(p);
+        b = __ldg(p + 1);
+    }
+}
+
 // Where a leaf's three vertices come from: the 48-byte sorted soup, or the indexed leaf format
 // (three vertex indices per sorted leaf into 16-byte vertex rows; an index past the buffer
 // reads row 0).
@@ -52,6 +72,21 @@ struct SoupTris {
         a = __ldg(t);
         b = __ldg(t + 1);
         c = __ldg(t + 2);
+    }
+    // WIDE: the 48 bytes from the 32-byte boundary at or below them in two loads; the first and the
+    // last leaf, whose window could leave the buffer, by 16-byte loads.
+    template <bool WIDE>
+    __device__ __forceinline__ void get(uint32_t leaf, uint32_t n, float4 &a, float4 &b, float4 &c) const {
+        if (!WIDE || leaf == 0 || leaf == n - 1) {
+            get((int)leaf, a, b, c);
+            return;
+        }
+        const float4 *t = tris + 3ull * leaf;
+        const bool odd = (reinterpret_cast<uintptr_t>(t) & 16u) != 0;
+        float4 d;
+        ldg_pair<true>(t - odd, a, b);
+        ldg_pair<true>(t - odd + 2, c, d);
+        if (odd) { a = b; b = c; c = d; }
     }
 };
 struct MeshTris {
@@ -65,12 +100,13 @@ struct MeshTris {
         b = __ldg(verts + (i1 < nverts ? i1 : 0u));
         c = __ldg(verts + (i2 < nverts ? i2 : 0u));
     }
+    template <bool WIDE>
+    __device__ __forceinline__ void get(uint32_t leaf, uint32_t, float4 &a, float4 &b, float4 &c) const {
+        get((int)leaf, a, b, c);
+    }
 };
 
-template <class Tris>
-__device__ float tri_intersect(F3 o, F3 d, const Tris &tr, int leaf) {
-    float4 a, b, c;
-    tr.get(leaf, a, b, c);
+__device__ __forceinline__ float tri_intersect(F3 o, F3 d, float4 a, float4 b, float4 c) {
     const F3 v0 = {a.x, a.y, a.z}, v1 = {b.x, b.y, b.z}, v2 = {c.x, c.y, c.z};
     const F3 v0v1 = sub3(v1, v0), v0v2 = sub3(v2, v0);
     const F3 pvec = cross3(d, v0v2);
@@ -86,6 +122,8 @@ __device__ float tri_intersect(F3 o, F3 d, const Tris &tr, int leaf) {
     return __fmul_rn(dot3(v0v2, qvec), i_det);
 }
 
+// aabb_intersect (:621-628) with WGSL's min / max written as `a < b ? a : b`, which also fixes
+// what a NaN does.
 __device__ __forceinline__ float aabb_intersect(F3 lo, F3 hi, F3 o, F3 inv) {
     const float fx = __fmul_rn(__fsub_rn(hi.x, o.x), inv.x), nx = __fmul_rn(__fsub_rn(lo.x, o.x), inv.x);
     const float fy = __fmul_rn(__fsub_rn(hi.y, o.y), inv.y), ny = __fmul_rn(__fsub_rn(lo.y, o.y), inv.y);
@@ -93,6 +131,20 @@ __device__ __forceinline__ float aabb_intersect(F3 lo, F3 hi, F3 o, F3 inv) {
     const float t0 = wmax(wmin(fx, nx), wmax(wmin(fy, ny), wmin(fz, nz)));
     const float t1 = wmin(wmax(fx, nx), wmin(wmax(fy, ny), wmax(fz, nz)));
     return (t1 >= t0) ? ((t1 < 0.0f) ? -1e30f : t0) : -1e30f;
+}
+
+// The same for a ray and a box without NaN or infinity, where hardware min / max (one
+// instruction for two or three operands) differ from the above in the sign of a zero only, and
+// the result is only compared: the entry distance, and whether the box counts as entered.
+// (Finite o and non-zero finite inv make no NaN of a finite box: a difference may overflow, but
+// infinity times inv is infinity.)
+__device__ __forceinline__ bool aabb_enter(F3 lo, F3 hi, F3 o, F3 inv, float dist, float &t0) {
+    const float fx = __fmul_rn(__fsub_rn(hi.x, o.x), inv.x), nx = __fmul_rn(__fsub_rn(lo.x, o.x), inv.x);
+    const float fy = __fmul_rn(__fsub_rn(hi.y, o.y), inv.y), ny = __fmul_rn(__fsub_rn(lo.y, o.y), inv.y);
+    const float fz = __fmul_rn(__fsub_rn(hi.z, o.z), inv.z), nz = __fmul_rn(__fsub_rn(lo.z, o.z), inv.z);
+    t0 = fmaxf(fmaxf(fminf(fx, nx), fminf(fy, ny)), fminf(fz, nz));
+    const float t1 = fminf(fminf(fmaxf(fx, nx), fmaxf(fy, ny)), fmaxf(fz, nz));
+    return t1 >= t0 && t1 >= 0.0f && t0 < dist && t0 != -1e30f;
 }
 
 // One ray's traversal state.
@@ -103,6 +155,7 @@ struct RayState {
     int sp, node_idx;
     uint32_t deepest;
     uint32_t visits;  // node visits so far: a valid tree needs fewer than 2 N
+    bool odd;         // a component of the ray is NaN or infinite
 };
 
 __device__ __forceinline__ void ray_init(RayState &st, const float4 *__restrict__ rays, uint32_t r,
@@ -123,59 +176,109 @@ __device__ __forceinline__ void ray_init(RayState &st, const float4 *__restrict_
     st.node_idx = 0;
     st.deepest = 0;
     st.visits = 0;
+    st.odd = !(isfinite(ro.x) && isfinite(ro.y) && isfinite(ro.z) && isfinite(rd.x) && isfinite(rd.y) && isfinite(rd.z));
 }
 
-// One node visit of the reference's loop (pathtracer.js:505-581): a leaf is tested, an internal
-// node's children are tested and the nearer valid one is taken with the farther pushed.
-// Returns false once the ray's stack is empty.
-template <class Tris, class Stack>
-__device__ __forceinline__ bool ray_step(RayState &st, const Stack &stack, const float4 *__restrict__ nodes,
-                                         const Tris &tris, uint32_t n) {
-    if (st.sp < 0) return false;
-    const int node_idx = st.node_idx;
-    if ((node_idx < 0 ? (uint32_t)(-(node_idx + 1)) >= n : (uint32_t)node_idx >= n) ||
-        ++st.visits > 2u * n + 64u) {
-        st.sp = -1;  // a link outside the tree or a cycle: stop this ray (never on a built tree)
-        st.deepest = 0xFFFFFFFFu;
-        return false;
+// The reference's loop (pathtracer.js:505-581), one node visit at a time: a leaf is tested, an
+// internal node's children are tested and the nearer valid one is taken with the farther pushed.
+// st.sp < 0 once the ray's stack is empty (or its walk broke off).
+
+// The visit's row, checked; false when the walk breaks off: a link outside the tree or a cycle
+// (never on a built tree).
+__device__ __forceinline__ bool visit(RayState &st, uint32_t row, uint32_t n) {
+    if (row < n && ++st.visits <= 2u * n + 64u) return true;
+    st.sp = -1;
+    st.deepest = 0xFFFFFFFFu;
+    return false;
+}
+
+// The next node from the stack.  A popped internal node whose box begins at or past the closest
+// hit is skipped without a visit: its children's boxes lie inside its own and every operation of
+// the box test is monotone, so both would begin at or past the hit too and the visit would push
+// nothing.  (A popped leaf is tested: its triangle's distance is rounded differently from its
+// box's.)
+template <class Stack>
+__device__ __forceinline__ void pop(RayState &st, const Stack &stack) {
+    while (--st.sp >= 0) {
+        const StackEntry e = stack.get(st.sp);
+        st.node_idx = e.node;
+        if (e.node < 0 || e.dist < st.dist) break;
     }
-    if (node_idx < 0) {
-        const int leaf = -(node_idx + 1);
-        const float t = tri_intersect(st.o, st.d, tris, leaf);
-        if (t > 0.0f && t < st.dist) { st.dist = wmin(t, st.dist); st.prim = leaf; }
-        st.sp -= 1;
-        st.node_idx = st.sp >= 0 ? stack[st.sp] : 0;
-    } else {
-        const float4 *nd = nodes + 4ull * node_idx;
-        const float4 l0 = __ldg(nd), l1 = __ldg(nd + 1), r0 = __ldg(nd + 2), r1 = __ldg(nd + 3);
-        const float ld = aabb_intersect({l0.x, l0.y, l0.z}, {l1.x, l1.y, l1.z}, st.o, st.inv);
-        const float rdist = aabb_intersect({r0.x, r0.y, r0.z}, {r1.x, r1.y, r1.z}, st.o, st.inv);
-        const int lc = __float_as_int(l0.w), rc = __float_as_int(r0.w);
-        const bool lv = ld != -1e30f && ld < st.dist;
-        const bool rv = rdist != -1e30f && rdist < st.dist;
-        if (lv && rv) {
-            const bool near_left = ld < rdist;
-            if (st.sp >= kStack) { st.sp = -1; st.deepest = kStack + 1; return false; }
-            stack[st.sp] = near_left ? rc : lc;
-            st.sp += 1;
-            st.deepest = max(st.deepest, (uint32_t)st.sp);
-            st.node_idx = near_left ? lc : rc;
-        } else if (lv) {
-            st.node_idx = lc;
-        } else if (rv) {
-            st.node_idx = rc;
-        } else {
-            st.sp -= 1;
-            st.node_idx = st.sp >= 0 ? stack[st.sp] : 0;
-        }
+}
+
+template <bool WIDE, class Stack>
+__device__ __forceinline__ void visit_node(RayState &st, const Stack &stack, const float4 *__restrict__ nodes, uint32_t n) {
+    const uint32_t row = (uint32_t)st.node_idx;
+    if (!visit(st, row, n)) return;
+    const float4 *nd = nodes + 4ull * row;
+    float4 l0, l1, r0, r1;
+    ldg_pair<WIDE>(nd, l0, l1);
+    ldg_pair<WIDE>(nd + 2, r0, r1);
+    const int lc = __float_as_int(l0.w), rc = __float_as_int(r0.w);
+    float ld, rd;
+    bool lv = aabb_enter({l0.x, l0.y, l0.z}, {l1.x, l1.y, l1.z}, st.o, st.inv, st.dist, ld);
+    bool rv = aabb_enter({r0.x, r0.y, r0.z}, {r1.x, r1.y, r1.z}, st.o, st.inv, st.dist, rd);
+    if (st.odd) {  // the reference's comparisons, NaN included; nothing it pushes is skipped
+        ld = aabb_intersect({l0.x, l0.y, l0.z}, {l1.x, l1.y, l1.z}, st.o, st.inv);
+        rd = aabb_intersect({r0.x, r0.y, r0.z}, {r1.x, r1.y, r1.z}, st.o, st.inv);
+        lv = ld != -1e30f && ld < st.dist;
+        rv = rd != -1e30f && rd < st.dist;
     }
-    return st.sp >= 0;
+    if (!lv && !rv) {
+        pop(st, stack);
+        return;
+    }
+    const bool near_left = lv && (!rv || ld < rd);
+    st.node_idx = near_left ? lc : rc;
+    if (lv && rv) {
+        if (st.sp >= kStack) { st.sp = -1; st.deepest = kStack + 1; return; }
+        stack.put(st.sp, StackEntry{near_left ? rc : lc, st.odd ? -INFINITY : near_left ? rd : ld});
+        st.sp += 1;
+        st.deepest = max(st.deepest, (uint32_t)st.sp);
+    }
+}
+
+template <bool WIDE, class Tris, class Stack>
+__device__ __forceinline__ void visit_leaf(RayState &st, const Stack &stack, const Tris &tris, uint32_t n) {
+    const uint32_t row = (uint32_t)~st.node_idx;  // leaf i is linked as -(i + 1)
+    if (!visit(st, row, n)) return;
+    float4 a, b, c;
+    tris.template get<WIDE>(row, n, a, b, c);
+    const float t = tri_intersect(st.o, st.d, a, b, c);
+    if (t > 0.0f && t < st.dist) { st.dist = t; st.prim = (int)row; }
+    pop(st, stack);
+}
+
+// A ray's next visits: up to kNodeVisits internal nodes, then its leaf if it is at one.
+//
+// What bounds the walk: L1 requests (each lane's rows lie in lines of their own), then issue slots
+// with 13 to 17 of 32 lanes active, and at the end the longest rays (36 visits on average, 1,240 for
+// the longest of 4 M rays on the 2 M sphere, about 0.5 us a visit alone).  Kernel times on the
+// B200: 4 M rays on the 2 M sphere / 100,003 rays on a 131 K mesh / a 1080p bounce, from 2.85 ms /
+// 192 us / 598 us: internal nodes culled when popped 2.61 / 185 / 590; 32-byte row loads and 12
+// stack entries in shared memory 2.40 / 179 / 620; hardware min and max 2.31 / 173 / 598; up to
+// four node visits between leaf tests and refills, in a loop of the lane's own, 2.01 / 146 / 480.
+// Two, six and eight visits took 2.19, 2.00 and 2.04 ms (545, 522 and 563 us a bounce); leaves held
+// back until eight lanes have one 2.07 ms / 162 us / 535 us; both children's rows prefetched 2.73
+// ms / 198 us / 652 us; rays sorted by origin and direction beforehand save less than the sort costs.
+constexpr int kNodeVisits = 4;
+template <bool WIDE, class Tris, class Stack>
+__device__ __forceinline__ void ray_round(RayState &st, bool have, const Stack &stack, const float4 *__restrict__ nodes,
+                                          const Tris &tris, uint32_t n) {
+    for (int k = 0; k < kNodeVisits && have && st.sp >= 0 && st.node_idx >= 0; ++k)
+        visit_node<WIDE>(st, stack, nodes, n);
+    __syncwarp();
+    if (have && st.sp >= 0 && st.node_idx < 0) visit_leaf<WIDE>(st, stack, tris, n);
+    __syncwarp();
 }
 
 // Persistent traversal: each lane takes a new ray as soon as its current one is done (a warp
 // refills its idle lanes from a global counter once a quarter of them are idle), so a warp is
-// not held by its slowest ray.  Each ray's own walk is exactly the reference's.
-template <class Tris>
+// not held by its slowest ray.  Each ray's own walk is the reference's, in its order.
+// Stack entries in shared memory (the rest of the SM's 256 KB is L1): 8, 12 and 16 take 2.05,
+// 2.01 and 2.04 ms for the 4 M rays.
+constexpr int kTraceDepth = 12;
+template <bool WIDE, class Tris>
 __global__ void __launch_bounds__(128) k_trace(const float4 *__restrict__ nodes, Tris tris, uint32_t n,
                                                const float4 *__restrict__ rays, uint32_t num_rays,
                                                int32_t *__restrict__ hit_prim,
@@ -184,10 +287,9 @@ __global__ void __launch_bounds__(128) k_trace(const float4 *__restrict__ nodes,
                                                uint32_t *__restrict__ counter) {
     const int lane = threadIdx.x & 31;
     const uint32_t lt = lanemask_lt();
-    // the first kSmemStack entries in shared memory (1,515 -> 1,580 M rays/s on the 2 M sphere)
-    __shared__ int32_t sstack[kSmemStack][128];
-    int32_t deep[kStack - kSmemStack];
-    const RayStack<128> stack{&sstack[0][threadIdx.x], deep};
+    __shared__ StackEntry sstack[kTraceDepth][128];
+    StackEntry deep[kStack - kTraceDepth];
+    const RayStack<128, kTraceDepth> stack{&sstack[0][threadIdx.x], deep};
     RayState st;
     bool have = false, exhausted = false;
     uint32_t r = 0;
@@ -209,7 +311,8 @@ __global__ void __launch_bounds__(128) k_trace(const float4 *__restrict__ nodes,
         } else if (exhausted && idle == 0xFFFFFFFFu) {
             break;
         }
-        if (have && !ray_step(st, stack, nodes, tris, n)) {
+        ray_round<WIDE>(st, have, stack, nodes, tris, n);
+        if (have && st.sp < 0) {
             hit_prim[r] = st.dist == 1e30f ? -1 : st.prim;
             hit_t[r] = st.dist == 1e30f ? -1.0f : st.dist;
             if (max_stack) max_stack[r] = st.deepest;
@@ -386,9 +489,11 @@ __device__ __forceinline__ void pt_end(PixelPath &pp, const RayState &st, const 
     __stcs(out + 3 * plane + px, make_float4(b.x, b.y, b.z, 1.0f));
 }
 
+// Stack entries in shared memory: 8, 12 and 16 take 480, 491 and 489 us for the 1080p bounce.
 // One bounce of every pixel: persistent warps fetch pixels from *counter as lanes finish (the
 // traversal's dynamic fetch), each pixel's walk exactly the reference's.
-template <class Tris>
+constexpr int kPtDepth = 8;
+template <bool WIDE, class Tris>
 __global__ void __launch_bounds__(128) k_pt_step(const float4 *__restrict__ nodes, Tris tris,
                                                  uint32_t n, const float4 *__restrict__ in, float4 *__restrict__ out,
                                                  PtFrame f, uint32_t *__restrict__ counter) {
@@ -396,10 +501,9 @@ __global__ void __launch_bounds__(128) k_pt_step(const float4 *__restrict__ node
     const uint32_t lt = lanemask_lt();
     const uint32_t num = f.width * f.height;
     const size_t plane = num;
-    // thread-local stack: this kernel's node fetches gain more from the L1 it would share with
-    // a shared-memory stack (0.666 -> 0.700 ms per 1080p bounce with one) than the stack does
-    int32_t stack_mem[kStack];
-    int32_t *const stack = stack_mem;
+    __shared__ StackEntry sstack[kPtDepth][128];
+    StackEntry deep[kStack - kPtDepth];
+    const RayStack<128, kPtDepth> stack{&sstack[0][threadIdx.x], deep};
     RayState st;
     PixelPath pp;
     bool have = false, exhausted = false;
@@ -423,7 +527,8 @@ __global__ void __launch_bounds__(128) k_pt_step(const float4 *__restrict__ node
         } else if (exhausted && idle == 0xFFFFFFFFu) {
             break;
         }
-        if (have && !ray_step(st, stack, nodes, tris, n)) {
+        ray_round<WIDE>(st, have, stack, nodes, tris, n);
+        if (have && st.sp < 0) {
             pt_end(pp, st, tris, out, plane, f);
             have = false;
         }
@@ -432,51 +537,64 @@ __global__ void __launch_bounds__(128) k_pt_step(const float4 *__restrict__ node
 
 }  // namespace
 
+namespace {
+
+// Blocks of a persistent kernel over `items`: as many as fit on the device at most.
+template <class K>
+uint32_t persistent_grid(K kernel, uint32_t items, int &per_sm) {
+    if (!per_sm && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0) != cudaSuccess || per_sm < 1)) {
+        cudaGetLastError();
+        per_sm = 4;
+    }
+    const uint32_t want = (items + 127) / 128, cap = (uint32_t)(sm_count() * per_sm);
+    return want < cap ? want : cap;
+}
+
+template <bool WIDE, class Tris>
+void trace_impl(const float4 *nodes, Tris tris, uint32_t n, const float4 *rays, uint32_t num_rays, int32_t *hit_prim,
+                float *hit_t, uint32_t *max_stack, uint32_t *counter, cudaStream_t s) {
+    static int per_sm = 0;
+    const uint32_t grid = persistent_grid(k_trace<WIDE, Tris>, num_rays, per_sm);
+    k_trace<WIDE, Tris><<<grid, 128, 0, s>>>(nodes, tris, n, rays, num_rays, hit_prim, hit_t, max_stack, counter);
+}
+
+// The tree's 32-byte loads need node records on 32-byte boundaries (any torch tensor's; an entry
+// point asks for 16).
+bool wide(const float4 *nodes) { return (reinterpret_cast<uintptr_t>(nodes) & 31u) == 0; }
+
+}  // namespace
+
 void launch_trace(const float4 *nodes, const float4 *tris, uint32_t n, const float4 *rays,
                   uint32_t num_rays, int32_t *hit_prim, float *hit_t, uint32_t *max_stack,
                   uint32_t *counter, cudaStream_t s) {
     if (num_rays == 0) return;
-    static int per_sm = 0;
-    if (!per_sm && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace<SoupTris>, 128, 0) != cudaSuccess ||
-                    per_sm < 1)) {
-        cudaGetLastError();
-        per_sm = 4;
-    }
-    const uint32_t want = (num_rays + 127) / 128, cap = (uint32_t)(sm_count() * per_sm);
     cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-    k_trace<<<want < cap ? want : cap, 128, 0, s>>>(nodes, SoupTris{tris}, n, rays, num_rays, hit_prim, hit_t,
-                                                    max_stack, counter);
+    if (wide(nodes)) trace_impl<true>(nodes, SoupTris{tris}, n, rays, num_rays, hit_prim, hit_t, max_stack, counter, s);
+    else trace_impl<false>(nodes, SoupTris{tris}, n, rays, num_rays, hit_prim, hit_t, max_stack, counter, s);
 }
 
 void launch_trace_mesh(const float4 *nodes, const float4 *verts, uint32_t num_verts, const uint32_t *sidx, uint32_t n,
                        const float4 *rays, uint32_t num_rays, int32_t *hit_prim, float *hit_t,
                        uint32_t *max_stack, uint32_t *counter, cudaStream_t s) {
     if (num_rays == 0) return;
-    static int per_sm = 0;
-    if (!per_sm && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace<MeshTris>, 128, 0) != cudaSuccess ||
-                    per_sm < 1)) {
-        cudaGetLastError();
-        per_sm = 4;
-    }
-    const uint32_t want = (num_rays + 127) / 128, cap = (uint32_t)(sm_count() * per_sm);
     cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-    k_trace<<<want < cap ? want : cap, 128, 0, s>>>(nodes, MeshTris{verts, sidx, num_verts}, n, rays, num_rays,
-                                                    hit_prim, hit_t, max_stack, counter);
+    const MeshTris tris{verts, sidx, num_verts};
+    if (wide(nodes)) trace_impl<true>(nodes, tris, n, rays, num_rays, hit_prim, hit_t, max_stack, counter, s);
+    else trace_impl<false>(nodes, tris, n, rays, num_rays, hit_prim, hit_t, max_stack, counter, s);
 }
 
 void launch_pt_step(const float4 *nodes, const float4 *tris, uint32_t n, const float4 *state_in,
                     float4 *state_out, const PtFrame &f, uint32_t *counter, cudaStream_t s) {
     const uint32_t num = f.width * f.height;
     if (num == 0) return;
-    static int per_sm = 0;
-    if (!per_sm && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pt_step<SoupTris>, 128, 0) != cudaSuccess ||
-                    per_sm < 1)) {
-        cudaGetLastError();
-        per_sm = 4;
-    }
-    const uint32_t want = (num + 127) / 128, cap = (uint32_t)(sm_count() * per_sm);
     cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-    k_pt_step<<<want < cap ? want : cap, 128, 0, s>>>(nodes, SoupTris{tris}, n, state_in, state_out, f, counter);
+    static int per_wide = 0, per_narrow = 0;
+    if (wide(nodes))
+        k_pt_step<true, SoupTris><<<persistent_grid(k_pt_step<true, SoupTris>, num, per_wide), 128, 0, s>>>(
+            nodes, SoupTris{tris}, n, state_in, state_out, f, counter);
+    else
+        k_pt_step<false, SoupTris><<<persistent_grid(k_pt_step<false, SoupTris>, num, per_narrow), 128, 0, s>>>(
+            nodes, SoupTris{tris}, n, state_in, state_out, f, counter);
 }
 
 }  // namespace lvbh
