@@ -324,33 +324,42 @@ struct MeshIn {
 // bounds).
 enum Pre : int { kPreNone = 0, kPreCen = 1, kPreKeys = 2 };
 
-// An error: a launch could not be made (the tree pass's tensor map); the rest was enqueued.
+// An error: a launch could not be made (the small build's cluster, the tree pass's tensor map).
 cudaError_t enqueue_build(lvbh_ctx *ctx, const float4 *tri, uint32_t n, const HostBounds &hb,
                           const lvbh_result *out, cudaStream_t s, bool profile, const MeshIn *mesh = nullptr,
                           int pre = kPreNone) {
     if (profile) cudaEventRecord(ctx->ev[1], s);
-    if (pre == kPreNone)
-        cudaMemsetAsync(reinterpret_cast<char *>(ctx->ctl) + offsetof(Control, err), 0,
-                        sizeof(Control) - offsetof(Control, err), s);
-    // a soup whose box is reduced here: box and centroids in one pass, then the keys from the
-    // centroids
-    const bool cen_path = !hb.use && !mesh;
-    if (!hb.use && pre == kPreNone) {
-        if (mesh) launch_bounds_mesh(mesh->verts, mesh->nverts, mesh->idx3, n, ctx->ctl, s);
-        else launch_bounds_cen(tri, 0, n, ctx->cen, ctx->cap, ctx->ctl, s);
+    if (pre == kPreNone && small_build(n)) {
+        if (profile) { cudaEventRecord(ctx->ev[2], s); cudaEventRecord(ctx->ev[3], s); }  // all in the sort stage
+        uint32_t *kv = ctx->keys_b;  // vals_b follows it in the arena
+        const cudaError_t e = mesh ? launch_small_sort_mesh(mesh->verts, mesh->nverts, mesh->idx3, n, hb, ctx->ctl, kv,
+                                                            out->morton, out->leaf_index, s)
+                                   : launch_small_sort(tri, n, hb, ctx->ctl, kv, out->morton, out->leaf_index, s);
+        if (e != cudaSuccess) return e;
+    } else {
+        if (pre == kPreNone)
+            cudaMemsetAsync(reinterpret_cast<char *>(ctx->ctl) + offsetof(Control, err), 0,
+                            sizeof(Control) - offsetof(Control, err), s);
+        // a soup whose box is reduced here: box and centroids in one pass, then the keys from the
+        // centroids
+        const bool cen_path = !hb.use && !mesh;
+        if (!hb.use && pre == kPreNone) {
+            if (mesh) launch_bounds_mesh(mesh->verts, mesh->nverts, mesh->idx3, n, ctx->ctl, s);
+            else launch_bounds_cen(tri, 0, n, ctx->cen, ctx->cap, ctx->ctl, s);
+        }
+        if (profile) cudaEventRecord(ctx->ev[2], s);
+        // unsorted keys go to keys_a, so that the three passes ping-pong keys_a -> result ->
+        // scratch -> result
+        uint32_t *keys_a = ctx->keys_a;
+        if (mesh) launch_morton_mesh(mesh->verts, mesh->nverts, mesh->idx3, n, hb, ctx->ctl, keys_a,
+                                     ctx->lookback, s);
+        else if (cen_path) launch_morton_cen(ctx->cen, ctx->cap, n, ctx->ctl, keys_a, ctx->lookback, s);
+        else if (pre != kPreKeys) launch_morton(tri, n, hb, ctx->ctl, keys_a, ctx->lookback, s);
+        if (profile) cudaEventRecord(ctx->ev[3], s);
+        launch_sort_pass(keys_a, nullptr, out->morton, out->leaf_index, n, 0, true, ctx->ctl, ctx->lookback, s);
+        launch_sort_pass(out->morton, out->leaf_index, ctx->keys_b, ctx->vals_b, n, 1, false, ctx->ctl, ctx->lookback, s);
+        launch_sort_pass(ctx->keys_b, ctx->vals_b, out->morton, out->leaf_index, n, 2, false, ctx->ctl, ctx->lookback, s);
     }
-    if (profile) cudaEventRecord(ctx->ev[2], s);
-    // unsorted keys go to keys_a, so that the three passes ping-pong keys_a -> result ->
-    // scratch -> result
-    uint32_t *keys_a = ctx->keys_a;
-    if (mesh) launch_morton_mesh(mesh->verts, mesh->nverts, mesh->idx3, n, hb, ctx->ctl, keys_a,
-                                 ctx->lookback, s);
-    else if (cen_path) launch_morton_cen(ctx->cen, ctx->cap, n, ctx->ctl, keys_a, ctx->lookback, s);
-    else if (pre != kPreKeys) launch_morton(tri, n, hb, ctx->ctl, keys_a, ctx->lookback, s);
-    if (profile) cudaEventRecord(ctx->ev[3], s);
-    launch_sort_pass(keys_a, nullptr, out->morton, out->leaf_index, n, 0, true, ctx->ctl, ctx->lookback, s);
-    launch_sort_pass(out->morton, out->leaf_index, ctx->keys_b, ctx->vals_b, n, 1, false, ctx->ctl, ctx->lookback, s);
-    launch_sort_pass(ctx->keys_b, ctx->vals_b, out->morton, out->leaf_index, n, 2, false, ctx->ctl, ctx->lookback, s);
     if (profile) cudaEventRecord(ctx->ev[4], s);
     if (mesh) {
         uint32_t *sidx = static_cast<uint32_t *>(out->tris);
@@ -407,6 +416,11 @@ cudaError_t enqueue_batch(lvbh_ctx *ctx, const float4 *tri, const BatchPlan &bp,
                              profile ? ctx->ev + 5 : nullptr);
 }
 
+// A build enqueued kernel by kernel, or, when the build before it had the same buffers and sizes
+// (a program that rebuilds in place), as a graph: captured then, replayed from then on.  Capturing
+// for buffers seen once costs more than it saves: 1,024 meshes in rotating buffers took 3,768 us
+// with a graph made each time, 3,581 us launched directly (3,571 us replayed); 262,144 triangles
+// 131, 124 and 117 us.
 int launch_batch_graph(lvbh_ctx *ctx, const float4 *tri, const BatchPlan &bp, bool use_bounds,
                        const lvbh_result *out, cudaStream_t s) {
     BatchKey key;
@@ -440,6 +454,7 @@ int launch_batch_graph(lvbh_ctx *ctx, const float4 *tri, const BatchPlan &bp, bo
     return LVBH_OK;
 }
 
+// As launch_batch_graph, for one mesh.
 int launch_graph(lvbh_ctx *ctx, const float4 *tri, uint32_t n, const HostBounds &hb,
                  const lvbh_result *out, cudaStream_t s, const MeshIn *mesh, int pre) {
     GraphKey key;
@@ -523,10 +538,11 @@ int build_common(lvbh_ctx *ctx, const float4 *tri_dev, uint32_t n, const float *
     }
     int rc = LVBH_OK;
     if (profile && !profile_upload) cudaEventRecord(ctx->ev[0], s);
-    if (profile || (flags & LVBH_NO_GRAPH)) {
+    // a small build is three launches: cheaper than a graph's, and nothing to capture for new buffers
+    if (profile || (flags & LVBH_NO_GRAPH) || (pre == kPreNone && small_build(n))) {
         const cudaError_t qe = enqueue_build(ctx, tri_dev, n, hb, out, s, profile, mesh, pre);
         cudaError_t e = cudaGetLastError();
-        if (qe != cudaSuccess) return cuda_fail(ctx, qe, "tree pass tensor map");
+        if (qe != cudaSuccess) return cuda_fail(ctx, qe, "build launch");
         if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
     } else {
         rc = launch_graph(ctx, tri_dev, n, hb, out, s, mesh, pre);
@@ -667,7 +683,8 @@ int lvbh_create(lvbh_ctx **out, const lvbh_config *cfg) {
     for (auto &e : ctx->ev) {
         if (cudaEventCreate(&e) != cudaSuccess) { cudaGetLastError(); lvbh_destroy(ctx); return LVBH_ECUDA; }
     }
-    if (emit_init() != cudaSuccess || sort_init() != cudaSuccess || morton_init() != cudaSuccess) {
+    if (emit_init() != cudaSuccess || sort_init() != cudaSuccess || morton_init() != cudaSuccess ||
+        small_init() != cudaSuccess) {
         cudaGetLastError();
         lvbh_destroy(ctx);
         return LVBH_ECUDA;

@@ -169,6 +169,17 @@ void launch_bounds_cen(const float4 *tri, uint32_t t0, uint32_t t1, float *cen, 
 void launch_morton_cen(const float *cen, uint32_t cen_stride, uint32_t n, Control *ctl, uint32_t *keys,
                        uint32_t *sort_scratch, cudaStream_t s);
 cudaError_t morton_init();  // once per device, before the first launch
+// K1 + K2 of a small build in one cluster kernel (small.cu): box, keys, sorted keys and
+// permutation, and the control block's error word and box (nothing to clear before).  kv: 2 n words
+// of scratch, 8-byte aligned.
+constexpr uint32_t kSmallMax = 1u << 17;  // where the two paths take the same time (small.cu)
+bool small_build(uint32_t n);  // whether n triangles take it on this device
+cudaError_t small_init();      // once per device, before the first launch
+cudaError_t launch_small_sort(const float4 *tri, uint32_t n, const HostBounds &hb, Control *ctl, uint32_t *kv,
+                              uint32_t *keys, uint32_t *vals, cudaStream_t s);
+cudaError_t launch_small_sort_mesh(const float4 *verts, uint32_t nverts, const uint32_t *idx3, uint32_t n,
+                                   const HostBounds &hb, Control *ctl, uint32_t *kv, uint32_t *keys, uint32_t *vals,
+                                   cudaStream_t s);
 // K2: one reduce-then-scan pass over 10-bit digit `pass` (0..2) of 30-bit keys.  counted: the
 // tile histograms, chunk sums and global digit counts (ctl->hist_part) of this pass are there
 // already (K1b makes those of pass 0); otherwise the pass's tile-histogram kernel makes them
