@@ -131,7 +131,7 @@ struct lvbh_ctx {
     cudaEvent_t up_ev[1 + kUploadChunks] = {};
     // cached graph of the last build shape
     cudaStream_t cap_stream = nullptr;
-    GraphKey gkey;
+    GraphKey gkey, gseen;  // of gexec, and of the last build that could have replayed a graph
     cudaGraphExec_t gexec = nullptr;
     // batched builds: segment table, per-segment bounds and histograms, look-back words and
     // open items (device), and a pinned mirror of the table, host bounds and reduced bounds
@@ -149,7 +149,7 @@ struct lvbh_ctx {
     SegRow *bh_rows = nullptr;
     float *bh_bounds = nullptr;
     uint32_t *bh_ord = nullptr;
-    BatchKey bkey;
+    BatchKey bkey, bseen;  // as gkey, gseen
     cudaGraphExec_t bgexec = nullptr;
     // batched-build tunables: forced by the caller, or tuned per segment-size histogram
     bool forced = false;
@@ -161,6 +161,7 @@ struct lvbh_ctx {
     lvbh_result *last_out = nullptr;
     HostBounds last_hb{};
     bool pending = false;
+    bool last_gather = false;  // it began with the indexed-mesh gather, which may set aux_err
     bool last_batch = false;
     uint32_t last_segs = 0;
     float *last_bounds_out = nullptr;
@@ -437,7 +438,15 @@ int launch_batch_graph(lvbh_ctx *ctx, const float4 *tri, const BatchPlan &bp, bo
     key.tree_ctas = bp.tree_ctas_per_sm;
     key.outs[0] = out->nodes; key.outs[1] = out->tris; key.outs[2] = out->parents;
     key.outs[3] = out->leaf_index; key.outs[4] = out->morton;
+    const bool again = key == ctx->bseen;
+    ctx->bseen = key;
     if (!ctx->bgexec || !(key == ctx->bkey)) {
+        if (!again) {
+            const cudaError_t qe = enqueue_batch(ctx, tri, bp, use_bounds, out, s, false);
+            cudaError_t e = cudaGetLastError();
+            if (qe != cudaSuccess) return cuda_fail(ctx, qe, "build launch");
+            return e == cudaSuccess ? LVBH_OK : cuda_fail(ctx, e, "kernel launch");
+        }
         if (ctx->bgexec) { cudaGraphExecDestroy(ctx->bgexec); ctx->bgexec = nullptr; }
         if (!ctx->cap_stream) LVBH_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
         LVBH_CUDA(ctx, cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal));
@@ -470,13 +479,23 @@ int launch_graph(lvbh_ctx *ctx, const float4 *tri, uint32_t n, const HostBounds 
     key.pre = pre;
     key.outs[0] = out->nodes; key.outs[1] = out->tris; key.outs[2] = out->parents;
     key.outs[3] = out->leaf_index; key.outs[4] = out->morton;
+    // above kChainMaxTris the launches are not chained and a graph pays even for one replay (2^24
+    // triangles in rotating buffers: 1,666 us updated each time, 1,685 us launched directly)
+    const bool again = key == ctx->gseen || !chain_build(n);
+    ctx->gseen = key;
     if (!ctx->gexec || !(key == ctx->gkey)) {
+        if (!again) {
+            const cudaError_t qe = enqueue_build(ctx, tri, n, hb, out, s, false, mesh, pre);
+            cudaError_t e = cudaGetLastError();
+            if (qe != cudaSuccess) return cuda_fail(ctx, qe, "build launch");
+            return e == cudaSuccess ? LVBH_OK : cuda_fail(ctx, e, "kernel launch");
+        }
         if (!ctx->cap_stream) LVBH_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
         LVBH_CUDA(ctx, cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal));
         const cudaError_t qe = enqueue_build(ctx, tri, n, hb, out, ctx->cap_stream, false, mesh, pre);
         cudaGraph_t g = nullptr;
         LVBH_CUDA(ctx, cudaStreamEndCapture(ctx->cap_stream, &g));
-        if (qe != cudaSuccess) { cudaGraphDestroy(g); return cuda_fail(ctx, qe, "tree pass tensor map"); }
+        if (qe != cudaSuccess) { cudaGraphDestroy(g); return cuda_fail(ctx, qe, "build launch"); }
         bool updated = false;
         if (ctx->gexec) {
             cudaGraphExecUpdateResultInfo info;
@@ -723,13 +742,13 @@ int lvbh_build_soup(lvbh_ctx *ctx, const float *tri_array, uint32_t num_tris,
     if (num_tris && !tri_array) return fail(ctx, LVBH_EINVAL, "tri_array is NULL");
     DeviceGuard g(ctx->device);
     if (int rc = finish_pending(ctx)) return rc;
+    ctx->last_gather = false;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = check_out(ctx, num_tris, flags, out)) return rc;
     out->num_tris = out->num_nodes = num_tris;
     std::memset(out->bounds, 0, sizeof out->bounds);
     if (num_tris) {
         if (int rc = ensure_arena(ctx, num_tris)) return rc;
-        LVBH_CUDA(ctx, cudaMemsetAsync(&ctx->ctl->aux_err, 0, sizeof(uint32_t), s));
     }
     const float4 *tri = reinterpret_cast<const float4 *>(tri_array);
     bool profile_upload = false;
@@ -759,6 +778,7 @@ int lvbh_build_indexed(lvbh_ctx *ctx, const float *xyz, uint32_t num_verts, cons
     if (num_tris && (!xyz || !idx3 || !num_verts)) return fail(ctx, LVBH_EINVAL, "NULL vertex or index buffer");
     DeviceGuard g(ctx->device);
     if (int rc = finish_pending(ctx)) return rc;
+    ctx->last_gather = false;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = check_out(ctx, num_tris, flags, out)) return rc;
     out->num_tris = out->num_nodes = num_tris;
@@ -774,6 +794,7 @@ int lvbh_build_indexed(lvbh_ctx *ctx, const float *xyz, uint32_t num_verts, cons
     const bool host = (flags & LVBH_INPUT_HOST) != 0;
     if (int rc = ensure_arena(ctx, num_tris)) return rc;
     if (int rc = ensure_stage(ctx, soup + (host ? vb + ib : 0))) return rc;
+    ctx->last_gather = true;
     LVBH_CUDA(ctx, cudaMemsetAsync(&ctx->ctl->aux_err, 0, sizeof(uint32_t), s));
     char *st = static_cast<char *>(ctx->stage);
     bool profile_upload = false;
@@ -802,13 +823,13 @@ int lvbh_build_mesh(lvbh_ctx *ctx, const float *verts4, uint32_t num_verts, cons
         return fail(ctx, LVBH_EINVAL, "device vertex rows must be 16-byte aligned, indices 4-byte aligned");
     DeviceGuard g(ctx->device);
     if (int rc = finish_pending(ctx)) return rc;
+    ctx->last_gather = false;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = check_out(ctx, num_tris, flags, out, 12)) return rc;
     out->num_tris = out->num_nodes = num_tris;
     std::memset(out->bounds, 0, sizeof out->bounds);
     if (!num_tris) return build_common(ctx, nullptr, 0, model_bounds, flags, out, s, false);
     if (int rc = ensure_arena(ctx, num_tris)) return rc;
-    LVBH_CUDA(ctx, cudaMemsetAsync(&ctx->ctl->aux_err, 0, sizeof(uint32_t), s));
     bool profile_upload = false;
     if (host) {
         const size_t vb = align_up(16ull * num_verts), ib = align_up(12ull * num_tris);
@@ -865,6 +886,7 @@ int lvbh_build_batched(lvbh_ctx *ctx, const float *tri_array, const uint32_t *se
     if (total && !tri_array) return fail(ctx, LVBH_EINVAL, "tri_array is NULL");
     DeviceGuard g(ctx->device);
     if (int rc = finish_pending(ctx)) return rc;
+    ctx->last_gather = false;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = check_out(ctx, total, flags, out)) return rc;
     out->num_tris = out->num_nodes = total;
@@ -896,7 +918,6 @@ int lvbh_build_batched(lvbh_ctx *ctx, const float *tri_array, const uint32_t *se
         return BatchPlan{ctx->b_rows, ctx->b_tile_seg, ctx->b_blk_seg, ctx->b_grp_seg, num_segs,
                          (uint32_t)tiles, blk, total, grp, t.digit_bits, t.log_block, t.tree_ctas};
     };
-    LVBH_CUDA(ctx, cudaMemsetAsync(&ctx->ctl->aux_err, 0, sizeof(uint32_t), s));
     const float4 *tri = reinterpret_cast<const float4 *>(tri_array);
     const bool profile = (flags & LVBH_PROFILE) != 0;
     if (profile) cudaEventRecord(ctx->ev[0], s);
@@ -998,7 +1019,8 @@ int lvbh_sync(lvbh_ctx *ctx) {
     ctx->pending = false;
     cudaError_t e = cudaStreamSynchronize(ctx->last_stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamSynchronize");
-    const uint32_t err = ctx->host_ctl[offsetof(Control, aux_err) / 4] | ctx->host_ctl[offsetof(Control, err) / 4];
+    const uint32_t err = (ctx->last_gather ? ctx->host_ctl[offsetof(Control, aux_err) / 4] : 0u) |
+                         ctx->host_ctl[offsetof(Control, err) / 4];
     if (ctx->last_batch) {
         if (ctx->last_bounds_out) {
             for (uint64_t i = 0; i < ctx->last_segs * 6ull; ++i) {
@@ -1037,6 +1059,7 @@ int lvbh_test_stall_lookback(lvbh_ctx *ctx, uint32_t stall_tile, uint32_t spin_c
     if (!ctx) return LVBH_EINVAL;
     DeviceGuard g(ctx->device);
     if (int rc = finish_pending(ctx)) return rc;
+    ctx->last_gather = false;
     ctx->test_stall1 = stall_tile + 1u;  // UINT32_MAX -> 0: no tile stalls
     ctx->test_spin = spin_cycles;
     if (ctx->ctl) {
