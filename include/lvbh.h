@@ -380,6 +380,16 @@ LVBH_API int  lvbh_parse_obj(lvbh_ctx *ctx, const char *text, uint64_t bytes, ui
                              const float **tri_out, uint32_t *num_tris, double *bounds6,
                              uint64_t *err_line, void *stream);
 
+/* The same in two calls, for a caller that wants the soup in memory of its own: _begin checks the
+ * text and gives the number of triangles, _into writes them to `tri` (*num_tris x 12 floats of
+ * device memory, 16-byte aligned).  The text stays as it is in between, and no other parse runs
+ * on ctx; _into without a _begin that returned LVBH_OK is LVBH_EINVAL.  Other arguments and
+ * statuses as lvbh_parse_obj. */
+LVBH_API int  lvbh_parse_obj_begin(lvbh_ctx *ctx, const char *text, uint64_t bytes, uint32_t flags,
+                                   uint32_t *num_tris, uint64_t *err_line, void *stream);
+LVBH_API int  lvbh_parse_obj_into(lvbh_ctx *ctx, float *tri, double *bounds6, uint64_t *err_line,
+                                  void *stream);
+
 /* ---- test hook: a device wait that runs out --------------------------------------------
  * No counterpart in the reference (its shaders spin without a bound).  For tests of the
  * bounded waits: on this context, sort tile `stall_tile` (0-based, in the order tiles start) of

@@ -1183,8 +1183,35 @@ int lvbh_parse_obj(lvbh_ctx *ctx, const char *text, uint64_t bytes, uint32_t fla
     if (bytes > LVBH_OBJ_MAX_BYTES) return fail(ctx, LVBH_EINVAL, "text exceeds LVBH_OBJ_MAX_BYTES");
     DeviceGuard g(ctx->device);
     if (ctx->pending) LVBH_CUDA(ctx, cudaStreamSynchronize(ctx->last_stream));
-    return obj_parse(ctx->obj, text, bytes, (flags & LVBH_INPUT_HOST) != 0, tri_out, num_tris, bounds6,
-                     err_line, static_cast<cudaStream_t>(stream), ctx->err);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    uint32_t n = 0;
+    if (int rc = obj_scan(ctx->obj, text, bytes, (flags & LVBH_INPUT_HOST) != 0, &n, err_line, s, ctx->err)) return rc;
+    if (int rc = obj_emit(ctx->obj, nullptr, tri_out, bounds6, err_line, s, ctx->err)) return rc;
+    *num_tris = n;
+    return LVBH_OK;
+}
+
+int lvbh_parse_obj_begin(lvbh_ctx *ctx, const char *text, uint64_t bytes, uint32_t flags, uint32_t *num_tris,
+                         uint64_t *err_line, void *stream) {
+    if (!ctx) return LVBH_EINVAL;
+    if (!num_tris || !err_line) return fail(ctx, LVBH_EINVAL, "NULL output pointer");
+    *err_line = 0;
+    if (bytes && !text) return fail(ctx, LVBH_EINVAL, "text is NULL");
+    if (bytes > LVBH_OBJ_MAX_BYTES) return fail(ctx, LVBH_EINVAL, "text exceeds LVBH_OBJ_MAX_BYTES");
+    DeviceGuard g(ctx->device);
+    if (ctx->pending) LVBH_CUDA(ctx, cudaStreamSynchronize(ctx->last_stream));
+    return obj_scan(ctx->obj, text, bytes, (flags & LVBH_INPUT_HOST) != 0, num_tris, err_line,
+                    static_cast<cudaStream_t>(stream), ctx->err);
+}
+
+int lvbh_parse_obj_into(lvbh_ctx *ctx, float *tri, double *bounds6, uint64_t *err_line, void *stream) {
+    if (!ctx) return LVBH_EINVAL;
+    if (!tri || !bounds6 || !err_line) return fail(ctx, LVBH_EINVAL, "NULL output pointer");
+    *err_line = 0;
+    if (reinterpret_cast<uintptr_t>(tri) & 15u) return fail(ctx, LVBH_EINVAL, "tri must be 16-byte aligned");
+    DeviceGuard g(ctx->device);
+    if (ctx->pending) LVBH_CUDA(ctx, cudaStreamSynchronize(ctx->last_stream));
+    return obj_emit(ctx->obj, tri, nullptr, bounds6, err_line, static_cast<cudaStream_t>(stream), ctx->err);
 }
 
 }  // extern "C"

@@ -267,21 +267,37 @@ struct PtFrame {
 void launch_pt_step(const float4 *nodes, const float4 *tris, uint32_t n, const float4 *state_in,
                     float4 *state_out, const PtFrame &f, uint32_t *counter, cudaStream_t s);
 
-// OBJ ingest (obj.cu): device memory of one parse, grown on demand and held by the context.
+// OBJ ingest (obj.cu): device memory of one parse, grown on demand and held by the context, and
+// what obj_scan leaves to obj_emit.
 struct ObjScratch {
     void *text = nullptr;  // staged host text, newline counts, control block
     size_t text_bytes = 0;
     void *lines = nullptr;  // per-line arrays
     size_t lines_bytes = 0;
-    void *soup = nullptr;  // model-0 vertices (double) and the triangle soup
+    void *verts = nullptr;  // model 0's vertices
+    size_t verts_bytes = 0;
+    void *soup = nullptr;  // the triangle soup, when the caller gives no place for it
     size_t soup_bytes = 0;
     void *host = nullptr;  // pinned readback
+    bool scanned = false;
+    const char *src = nullptr;  // the caller's text, and the text on the device
+    const uint8_t *d_text = nullptr;
+    uint64_t src_bytes = 0;
+    bool host_text = false;
+    void *ctl = nullptr;
+    uint32_t *line_start = nullptr, *fans = nullptr;
+    uint8_t *type = nullptr;
+    unsigned long long *pre = nullptr;
 };
-// OBJ text -> triangle soup + bounds (lvbh_parse_obj).  *err_line: the 1-based line whose
-// statement the parser rejects, 0 for a failure found after parsing (LVBH_EINVAL for both).
-int obj_parse(ObjScratch &sc, const char *text, uint64_t bytes, bool host_text,
-              const float **tri_out, uint32_t *num_tris, double *bounds6, uint64_t *err_line,
-              cudaStream_t s, std::string &err);
+// OBJ text -> triangle soup + bounds (lvbh_parse_obj) in two steps: obj_scan finds the lines,
+// checks the statements and counts the triangles; obj_emit parses vertices and faces into dst
+// (*num_tris x 12 floats, 16-byte aligned; null: the scratch's own soup) and needs the text as
+// it was.  *err_line: the 1-based line whose statement the parser rejects, 0 for a failure found
+// after parsing (LVBH_EPARSE for both).
+int obj_scan(ObjScratch &sc, const char *text, uint64_t bytes, bool host_text, uint32_t *num_tris, uint64_t *err_line,
+             cudaStream_t s, std::string &err);
+int obj_emit(ObjScratch &sc, float *dst, const float **tri_out, double *bounds6, uint64_t *err_line, cudaStream_t s,
+             std::string &err);
 void obj_free(ObjScratch &sc);
 
 }  // namespace lvbh

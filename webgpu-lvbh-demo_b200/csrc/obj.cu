@@ -23,9 +23,13 @@
 //     (round to nearest even, the Float32Array of build-bvh.js:14-21), pad 3.1415; bounds are
 //     Math.min / Math.max over the faces' vertices in double (NaN absorbs, -0 below +0) from
 //     +-1e30, and two floor triangles lie at z_min + .01 (parse-obj.js:62-76).
-// Passes: newlines per 4 KB chunk -> scan -> line starts; per-line classify and check; the
-// model-0 line range; a 64-bit scan of (vertex count | triangle count) over it; vertices;
-// faces -> soup + bounds.  Each pass streams the text from HBM once; its bound is HBM.
+// Passes: newlines per 16 KB chunk -> scan -> line starts; per-line classify and check with a
+// (vertex | triangle) count per block of 256 lines; one block that finds model 0's line range
+// and scans those counts over it; vertices; faces -> soup; bounds over the vertices that faces
+// used, and the floor.  The per-line passes are bound by instructions per text byte, so the
+// forms that exporters write (single spaces, plain decimals, indices that start with 1 to 9) have
+// short loops of their own (fast_*), which leave every other line to the general scanners.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -33,6 +37,7 @@
 #include <vector>
 
 #include "lvbh.h"
+#include "lvbh_device.cuh"
 #include "lvbh_internal.h"
 
 namespace lvbh {
@@ -49,18 +54,15 @@ constexpr uint32_t kNone = 0xFFFFFFFFu;
 
 enum : uint8_t { LT_NONE = 0, LT_O, LT_G, LT_V, LT_VT, LT_VN, LT_L, LT_S, LT_F };
 
-// Device state of one parse (set to its initial values by the host before the passes).
+// Device state of one parse (set to its initial values by k_nl_count).
 struct ObjCtl {
     uint32_t err_line;    // smallest 0-based line whose statement throws (kNone: none)
-    uint32_t first_o;     // first `o` line (kNone: none)
-    uint32_t second_o;    // the next `o` line after it
-    uint32_t first_need;  // first v / vt / vn / l / f line (creates the default model)
     uint32_t bad_index;   // a model-0 face names no vertex
     uint32_t num_hard;    // vertex lines left to the host parser
     uint32_t newlines;
     uint32_t m0a, m0b;    // model 0's lines [m0a, m0b)
     uint32_t no_model;    // the text defines no model (output.models[0] is undefined)
-    uint32_t pad;
+    uint32_t done;        // blocks of the bounds pass that have finished
     unsigned long long totals;  // model-0 vertices (low 32 bits) and triangles (high 32 bits)
     unsigned long long bmin[3], bmax[3];  // ordered doubles (ord64)
     uint32_t nan_min[3], nan_max[3];
@@ -353,10 +355,10 @@ __device__ __forceinline__ bool parse_number(const uint8_t *b, uint32_t &i, uint
 }
 
 // Line l: its bytes [p, q) (without the '\n').
-__device__ __forceinline__ void line_bytes(uint64_t n, const uint64_t *line_start, uint32_t L, uint32_t l,
+__device__ __forceinline__ void line_bytes(uint64_t n, const uint32_t *line_start, uint32_t L, uint32_t l,
                                            uint64_t &p, uint64_t &q) {
     p = line_start[l];
-    q = l + 1 < L ? line_start[l + 1] - 1 : n;
+    q = l + 1 < L ? line_start[l + 1] - 1u : n;
 }
 
 constexpr int kLineBlock = 256;     // lines per block of the per-line kernels
@@ -365,9 +367,9 @@ constexpr int kWindow = 24 * 1024;  // text bytes a block stages in shared memor
 // Stages the text of lines [l0, l0 + cnt) into win (as much as fits, from the 16-byte boundary
 // at or below the first line's start) with coalesced 16-byte loads; [w0, w1) is what it holds.
 // Every thread of the block calls it.
-__device__ void stage_lines(const uint8_t *__restrict__ text, uint64_t n, const uint64_t *__restrict__ line_start,
+__device__ void stage_lines(const uint8_t *__restrict__ text, uint64_t n, const uint32_t *__restrict__ line_start,
                             uint32_t L, uint32_t l0, uint32_t cnt, uint8_t *win, uint64_t &w0, uint64_t &w1) {
-    const uint64_t a = line_start[l0] & ~15ull;
+    const uint64_t a = line_start[l0] & ~15u;
     const uint64_t z = l0 + cnt < L ? line_start[l0 + cnt] : n;
     const uint64_t e = z < a + kWindow ? z : a + kWindow;
     for (uint64_t c = a + 16ull * threadIdx.x; c < e; c += 16ull * blockDim.x) {
@@ -456,10 +458,16 @@ __device__ __forceinline__ uint32_t newlines64(const uint4 (&v)[4]) {
     return c;
 }
 
-// Newlines per kChunk bytes (64 per thread).
+// Newlines per kChunk bytes (64 per thread); the control block's initial values.
 __global__ void __launch_bounds__(kT) k_nl_count(const uint8_t *__restrict__ s, uint64_t n,
-                                                 uint32_t *__restrict__ cnt) {
+                                                 uint32_t *__restrict__ cnt, ObjCtl *__restrict__ ctl) {
     __shared__ uint32_t w[kT / 32];
+    if (blockIdx.x == 0) {
+        for (uint32_t i = threadIdx.x; i < sizeof(ObjCtl) / 4; i += kT) reinterpret_cast<uint32_t *>(ctl)[i] = 0u;
+        __syncthreads();
+        if (threadIdx.x == 0) ctl->err_line = kNone;
+        if (threadIdx.x < 3) ctl->bmin[threadIdx.x] = ~0ull;
+    }
     uint4 v[4];
     load64(s, n, (uint64_t)blockIdx.x * kChunk + threadIdx.x * 64ull, v);
     const uint32_t c = __reduce_add_sync(0xFFFFFFFFu, newlines64(v));
@@ -477,6 +485,7 @@ __global__ void __launch_bounds__(kT) k_nl_count(const uint8_t *__restrict__ s, 
 template <typename U>
 __global__ void __launch_bounds__(1024) k_scan_small(U *v, uint32_t n, U *total) {
     __shared__ U s_warp[32];
+    chain_wait();
     const uint32_t per = (n + 1023) / 1024, b = threadIdx.x * per, e = min(n, b + per);
     U sum = 0;
     for (uint32_t i = b; i < e; ++i) sum += v[i];
@@ -490,22 +499,25 @@ __global__ void __launch_bounds__(1024) k_scan_small(U *v, uint32_t n, U *total)
     if (threadIdx.x == 0) *total = all;
 }
 
-// Line starts: the newline at byte k (rank r over the text) starts line r + 1 at k + 1.
+// Line starts: the newline at byte k (rank r over the text) starts line r + 1 at k + 1.  At most
+// `cap` lines are written (the caller sees from the count that there are more).
 __global__ void __launch_bounds__(kT) k_nl_write(const uint8_t *__restrict__ s, uint64_t n,
-                                                 const uint32_t *__restrict__ base,
-                                                 uint64_t *__restrict__ line_start) {
+                                                 const uint32_t *__restrict__ base, uint32_t cap,
+                                                 uint32_t *__restrict__ line_start) {
     __shared__ uint32_t s_warp[kT / 32];
     const uint64_t p = (uint64_t)blockIdx.x * kChunk + threadIdx.x * 64ull;
     uint4 v[4];
     load64(s, n, p, v);
-    uint32_t r = base[blockIdx.x] + block_scan<uint32_t>(newlines64(v), s_warp, nullptr);
+    const uint32_t before = block_scan<uint32_t>(newlines64(v), s_warp, nullptr);
+    chain_wait();
+    uint32_t r = base[blockIdx.x] + before;
     const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         uint32_t m = ~(((w[j] ^ 0x0A0A0A0Au) & 0x7F7F7F7Fu) + 0x7F7F7F7Fu | (w[j] ^ 0x0A0A0A0Au) | 0x7F7F7F7Fu);
         while (m) {  // one bit (7, 15, 23 or 31) per newline byte, in text order
             const int byte = (__ffs(m) - 1) >> 3;
-            line_start[++r] = p + 4 * j + byte + 1;
+            if (++r < cap) line_start[r] = (uint32_t)(p + 4 * j + byte + 1);
             m &= m - 1;
         }
     }
@@ -528,7 +540,7 @@ __device__ __forceinline__ LineClass classify(const uint8_t *b, uint32_t len) {
     const uint32_t a = i;
     skip_token(b, i, e);
     const uint8_t t = keyword(b, a, i);
-    if (t == LT_NONE) return {LT_NONE, false, 0};
+    if (t == LT_NONE || t == LT_V || t == LT_VT || t == LT_VN || t == LT_O) return {t, false, 0};  // no checks
     uint32_t ntok = 1;
     bool bad = false;
     while (skip_ws(b, i, e)) {
@@ -552,44 +564,137 @@ __device__ __forceinline__ LineClass classify(const uint8_t *b, uint32_t len) {
     return {t, bad, fan};
 }
 
-// Per line: its class, and the first `o` and model-creating lines.  One block per kLineBlock
-// lines, their text staged in shared memory.
+// The class of a line in its common forms: empty, comment, `v ` / `vt ` / `vn ` (no checks), and
+// `f` with tokens apart by spaces that start with 1 to 9 (an index that parseInt makes neither 0
+// nor NaN) and hold ASCII without '#'.  b[len] is the line's '\n'.  False: classify() decides.
+__device__ __forceinline__ bool fast_class(const uint8_t *b, uint32_t len, LineClass &r) {
+    r = LineClass{LT_NONE, false, 0};
+    const uint32_t c0 = b[0];
+    if (c0 == '\n' || c0 == '#') return true;
+    const uint32_t c1 = b[1];  // at most the '\n'
+    if (c0 == 'v') {
+        if (c1 == ' ') { r.type = LT_V; return true; }
+        if ((c1 == 't' || c1 == 'n') && b[2] == ' ') { r.type = c1 == 't' ? LT_VT : LT_VN; return true; }
+        return false;
+    }
+    if (c0 != 'f' || c1 != ' ') return false;
+    r.type = LT_F;
+    uint32_t i = 1, ntok = 0, c = ' ';
+    for (;;) {
+        while (c == ' ') c = b[++i];
+        if (c == '\n') break;
+        if (c == '\r' && b[i + 1] == '\n') break;
+        if (c - '1' > 8u) return false;
+        ++ntok;
+        uint32_t slashes = 0;
+        do {
+            c = b[++i];
+            slashes += c == '/';
+        } while (c > ' ' && c < 0x80 && c != '#');
+        if (c != ' ' && c != '\n' && c != '\r') return false;
+        r.bad |= slashes > 2;
+    }
+    if (ntok < 3) r.bad = true;
+    else r.fan = ntok - 2;
+    return true;
+}
+
+// What k_lines leaves per block of kLineBlock lines: packed counts of all its lines (vertices in
+// the low, triangles in the high 32 bits), its first two `o` lines and its first model-creating one.
+struct LineBlock {
+    unsigned long long count;
+    uint32_t o1, o2, need, pad;
+};
+
+// Per line: its class.  One block per kLineBlock lines, their text staged in shared memory.
 __global__ void __launch_bounds__(kLineBlock) k_lines(const uint8_t *__restrict__ text, uint64_t n,
-                                                      const uint64_t *__restrict__ line_start, uint32_t L,
+                                                      const uint32_t *__restrict__ line_start, uint32_t cap,
                                                       uint8_t *__restrict__ type, uint32_t *__restrict__ fans,
-                                                      ObjCtl *__restrict__ ctl) {
+                                                      LineBlock *__restrict__ blocks, ObjCtl *__restrict__ ctl) {
     __shared__ __align__(16) uint8_t win[kWindow];
-    const uint32_t l0 = blockIdx.x * kLineBlock, l = l0 + threadIdx.x;
+    __shared__ unsigned long long s_count[kLineBlock / 32];
+    __shared__ uint32_t s_o[kLineBlock / 32], s_need[kLineBlock / 32];
+    chain_wait();
+    const uint32_t L = ctl->newlines + 1u, l0 = blockIdx.x * kLineBlock, l = l0 + threadIdx.x;
+    if (L > cap || l0 >= L) return;  // more lines than there is room for: the caller comes again
     uint64_t w0, w1;
     stage_lines(text, n, line_start, L, l0, min((uint32_t)kLineBlock, L - l0), win, w0, w1);
     LineClass c{LT_NONE, false, 0};
     if (l < L) {
         uint64_t p, q;
         line_bytes(n, line_start, L, l, p, q);
-        if (p >= w0 && q <= w1) c = classify(win + (p - w0), (uint32_t)(q - p));
-        else c = classify(text + p, (uint32_t)(q - p));
+        const uint32_t len = (uint32_t)(q - p);
+        if (p >= w0 && q < w1) {  // its newline too
+            if (!fast_class(win + (p - w0), len, c)) c = classify(win + (p - w0), len);
+        } else {
+            c = classify(text + p, len);
+        }
         type[l] = c.type;
         fans[l] = c.fan;
     }
     warp_min_into(c.bad ? l : kNone, &ctl->err_line);
-    warp_min_into(c.type == LT_O ? l : kNone, &ctl->first_o);
     const bool need = c.type == LT_V || c.type == LT_VT || c.type == LT_VN || c.type == LT_L || c.type == LT_F;
-    warp_min_into(need ? l : kNone, &ctl->first_need);
+    const uint32_t nv = __popc(__ballot_sync(0xFFFFFFFFu, c.type == LT_V));
+    const uint32_t nt = __reduce_add_sync(0xFFFFFFFFu, c.type == LT_F ? c.fan : 0u);
+    const uint32_t no = __ballot_sync(0xFFFFFFFFu, c.type == LT_O), nn = __ballot_sync(0xFFFFFFFFu, need);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) {
+        s_count[warp] = (unsigned long long)nt << 32 | nv;
+        s_o[warp] = no;
+        s_need[warp] = nn;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        LineBlock r{0ull, kNone, kNone, kNone, 0u};
+        for (int w = kLineBlock / 32 - 1; w >= 0; --w) {
+            r.count += s_count[w];
+            const uint32_t at = l0 + 32 * w, o = s_o[w];
+            if (s_need[w]) r.need = at + __ffs(s_need[w]) - 1;
+            if (o) {
+                const uint32_t rest = o & (o - 1);
+                r.o2 = rest ? at + __ffs(rest) - 1 : r.o1;
+                r.o1 = at + __ffs(o) - 1;
+            }
+        }
+        blocks[blockIdx.x] = r;
+    }
 }
 
-// The first `o` line after the first one.
-__global__ void __launch_bounds__(kT) k_second_o(const uint8_t *__restrict__ type, uint32_t L,
-                                                 ObjCtl *__restrict__ ctl) {
-    const uint32_t fo = ctl->first_o;
-    if (fo == kNone) return;
-    const uint32_t l = blockIdx.x * kT + threadIdx.x;
-    warp_min_into(l < L && l > fo && type[l] == LT_O ? l : kNone, &ctl->second_o);
+// Packed count of a model-0 line: one vertex (low 32 bits) or a face's triangles (high).
+__device__ __forceinline__ unsigned long long line_count(uint8_t t, uint32_t fan) {
+    return t == LT_V ? 1ull : t == LT_F ? (unsigned long long)fan << 32 : 0ull;
 }
 
-// Model 0's lines: the default model when a model-creating statement precedes the first `o`
+// Model 0's lines [a, b): the default model when a model-creating statement precedes the first `o`
 // (_currentModel, obj-file-parser.js:82-91), else the model that `o` opens, up to the next `o`.
-__global__ void k_model_range(uint32_t L, ObjCtl *__restrict__ ctl) {
-    const uint32_t fo = ctl->first_o, fn = ctl->first_need, so = ctl->second_o;
+// Then pre[block]: the packed counts of model 0's lines before the block.  One block of threads,
+// each over a run of consecutive line blocks; a line block that a or b cuts is counted line by line.
+__global__ void __launch_bounds__(1024) k_model(const LineBlock *__restrict__ blocks, const uint8_t *__restrict__ type,
+                                                const uint32_t *__restrict__ fans, uint32_t cap,
+                                                unsigned long long *__restrict__ pre, ObjCtl *__restrict__ ctl) {
+    __shared__ uint32_t s_min[3][32];
+    __shared__ unsigned long long s_warp[32];
+    chain_wait();
+    const uint32_t L = ctl->newlines + 1u;
+    if (L > cap) return;
+    const uint32_t nb = (L + (kLineBlock - 1)) / kLineBlock, per = (nb + 1023u) / 1024u;
+    const uint32_t b0 = min(nb, threadIdx.x * per), b1 = min(nb, b0 + per);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto block_min = [&](uint32_t v, int slot) {
+        v = __reduce_min_sync(0xFFFFFFFFu, v);
+        if (lane == 0) s_min[slot][warp] = v;
+        __syncthreads();
+        return __reduce_min_sync(0xFFFFFFFFu, s_min[slot][lane]);
+    };
+    uint32_t o1 = kNone, need = kNone;
+    for (uint32_t i = b0; i < b1; ++i) {
+        o1 = min(o1, blocks[i].o1);
+        need = min(need, blocks[i].need);
+    }
+    const uint32_t fo = block_min(o1, 0), fn = block_min(need, 1);
+    uint32_t o2 = kNone;
+    for (uint32_t i = b0; i < b1; ++i) o2 = min(o2, blocks[i].o1 == fo ? blocks[i].o2 : blocks[i].o1);
+    const uint32_t so = block_min(o2, 2);
     uint32_t a = 0, b = 0, none = 0;
     if (fn != kNone && (fo == kNone || fn < fo)) {
         b = fo == kNone ? L : fo;
@@ -599,54 +704,32 @@ __global__ void k_model_range(uint32_t L, ObjCtl *__restrict__ ctl) {
     } else {
         none = 1;
     }
-    ctl->m0a = a;
-    ctl->m0b = b;
-    ctl->no_model = none;
-}
-
-// Packed count of a model-0 line: one vertex (low 32 bits) or a face's triangles (high).
-__device__ __forceinline__ unsigned long long line_count(const uint8_t *type, const uint32_t *fans,
-                                                         uint32_t l) {
-    const uint8_t t = type[l];
-    return t == LT_V ? 1ull : t == LT_F ? (unsigned long long)fans[l] << 32 : 0ull;
-}
-
-// Tile sums of the packed counts of the L lines (zero outside model 0's [m0a, m0b)).
-__global__ void __launch_bounds__(kT) k_scan_up(const uint8_t *__restrict__ type,
-                                                const uint32_t *__restrict__ fans, uint32_t L,
-                                                const ObjCtl *__restrict__ ctl,
-                                                unsigned long long *__restrict__ sums) {
-    __shared__ unsigned long long s_warp[kT / 32];
-    const uint32_t a = ctl->m0a, b = ctl->m0b;
-    const uint64_t base = (uint64_t)blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    unsigned long long t = 0;
-    for (int k = 0; k < kScanItems; ++k)
-        if (base + k >= a && base + k < b) t += line_count(type, fans, (uint32_t)(base + k));
-    unsigned long long all;
-    block_scan<unsigned long long>(t, s_warp, &all);
-    if (threadIdx.x == 0) sums[blockIdx.x] = all;
-}
-
-// pre[l]: exclusive prefix of the packed counts at line l.
-__global__ void __launch_bounds__(kT) k_scan_down(const uint8_t *__restrict__ type,
-                                                  const uint32_t *__restrict__ fans, uint32_t L,
-                                                  const ObjCtl *__restrict__ ctl,
-                                                  const unsigned long long *__restrict__ sums,
-                                                  unsigned long long *__restrict__ pre) {
-    __shared__ unsigned long long s_warp[kT / 32];
-    const uint32_t a = ctl->m0a, b = ctl->m0b;
-    const uint64_t base = (uint64_t)blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    unsigned long long x[kScanItems], t = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        x[k] = (base + k >= a && base + k < b) ? line_count(type, fans, (uint32_t)(base + k)) : 0ull;
-        t += x[k];
+    // the line blocks that a and b lie in (the same one, or a is at its block's start, at times)
+    const uint32_t ba = a / kLineBlock, bb = b / kLineBlock;
+    auto cut = [&](uint32_t blk) {  // model 0's lines of one block
+        const uint32_t l = blk * kLineBlock + threadIdx.x;
+        unsigned long long c = 0;
+        if (threadIdx.x < kLineBlock && l >= a && l < b) c = line_count(type[l], fans[l]);
+        unsigned long long all;
+        block_scan<unsigned long long>(c, s_warp, &all);
+        return all;
+    };
+    const unsigned long long ca = cut(ba), cb = cut(bb);
+    auto count = [&](uint32_t i) {
+        return i < ba || i > bb ? 0ull : i == ba ? ca : i == bb ? cb : blocks[i].count;
+    };
+    unsigned long long sum = 0, all;
+    for (uint32_t i = b0; i < b1; ++i) sum += count(i);
+    unsigned long long run = block_scan<unsigned long long>(sum, s_warp, &all);
+    for (uint32_t i = b0; i < b1; ++i) {
+        pre[i] = run;
+        run += count(i);
     }
-    unsigned long long run = sums[blockIdx.x] + block_scan<unsigned long long>(t, s_warp, nullptr);
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        if (base + k < L) pre[base + k] = run;
-        run += x[k];
+    if (threadIdx.x == 0) {
+        ctl->m0a = a;
+        ctl->m0b = b;
+        ctl->no_model = none;
+        ctl->totals = all;
     }
 }
 
@@ -678,45 +761,38 @@ __device__ __forceinline__ VertexParse parse_vertex(const uint8_t *b, uint32_t l
     return r;
 }
 
-// Model-0 vertex lines -> doubles at their rank; numbers outside the device's exact range are
-// listed for the host.  One block per kLineBlock lines of model 0, its text staged when it holds
-// a vertex line.
-__global__ void __launch_bounds__(kLineBlock) k_vertices(const uint8_t *__restrict__ text, uint64_t n,
-                                                         const uint64_t *__restrict__ line_start, uint32_t L,
-                                                         const uint8_t *__restrict__ type, uint32_t a, uint32_t m,
-                                                         const unsigned long long *__restrict__ pre,
-                                                         double *__restrict__ verts, HardLine *__restrict__ hard,
-                                                         ObjCtl *__restrict__ ctl) {
-    __shared__ __align__(16) uint8_t win[kWindow];
-    const uint32_t i0 = blockIdx.x * kLineBlock, i = i0 + threadIdx.x;
-    const bool mine = i < m && type[a + i] == LT_V;
-    if (!__syncthreads_or(mine)) return;
-    uint64_t w0, w1;
-    stage_lines(text, n, line_start, L, a + i0, min((uint32_t)kLineBlock, m - i0), win, w0, w1);
-    if (!mine) return;
-    uint64_t p, q;
-    line_bytes(n, line_start, L, a + i, p, q);
-    VertexParse r;
-    if (p >= w0 && q <= w1) r = parse_vertex(win + (p - w0), (uint32_t)(q - p));
-    else r = parse_vertex(text + p, (uint32_t)(q - p));
-    const uint32_t vi = (uint32_t)(pre[a + i] & 0xFFFFFFFFull);
-    verts[3ull * vi] = r.x;
-    verts[3ull * vi + 1] = r.y;
-    verts[3ull * vi + 2] = r.z;
-    if (!r.ok) {
-        const uint32_t h = atomicAdd(&ctl->num_hard, 1u);
-        hard[h] = HardLine{p, p + r.end, vi, 0u, 0u, 0u};
+// The coordinates of a vertex line in its common form: `v`, then three plain decimals of at most
+// nine digits apart by spaces (value = digits / 10^k, one IEEE division of exact doubles, as
+// dec_to_double has it).  b[len] is the line's '\n'.  False: parse_vertex() decides.
+__device__ __forceinline__ bool fast_vertex(const uint8_t *b, double (&out)[3]) {
+    if (b[0] != 'v' || b[1] != ' ') return false;
+    uint32_t i = 1, c = ' ';
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (c != ' ') return false;
+        while (c == ' ') c = b[++i];
+        const bool neg = c == '-';
+        if (neg) c = b[++i];
+        uint32_t m = 0, nd = 0, k = 0, d;
+        while ((d = c - '0') <= 9u && nd < 10) {
+            m = m * 10 + d;
+            ++nd;
+            c = b[++i];
+        }
+        if (c == '.') {
+            c = b[++i];
+            while ((d = c - '0') <= 9u && nd < 10) {
+                m = m * 10 + d;
+                ++nd;
+                ++k;
+                c = b[++i];
+            }
+        }
+        if (nd == 0 || nd > 9 || (c != ' ' && c != '\n' && c != '\r')) return false;
+        const double v = k ? __ddiv_rn((double)m, kPow10[k]) : (double)m;
+        out[a] = neg ? -v : v;
     }
-}
-
-__global__ void __launch_bounds__(kT) k_patch(const HardFix *__restrict__ fix, uint32_t count,
-                                              double *__restrict__ verts) {
-    const uint32_t i = blockIdx.x * kT + threadIdx.x;
-    if (i >= count) return;
-    const HardFix f = fix[i];
-    verts[3ull * f.vi] = f.xyz[0];
-    verts[3ull * f.vi + 1] = f.xyz[1];
-    verts[3ull * f.vi + 2] = f.xyz[2];
+    return true;
 }
 
 // float32 of a coordinate as Float32Array stores it (NaN as the quiet NaN 0x7FC00000).
@@ -724,11 +800,198 @@ __device__ __forceinline__ float to_f32(double d) {
     return isnan(d) ? __int_as_float(0x7FC00000) : __double2float_rn(d);
 }
 
-// Running Math.min / Math.max of one thread's vertices (ordered doubles, NaN flags).
-struct BoundsAcc {
-    unsigned long long mn[3], mx[3];
-    bool nan[3];
-    __device__ __forceinline__ void add(const double (&c)[3]) {
+// A vertex as the soup holds it: x, the file's z as y and y as z, and the pad.
+__device__ __forceinline__ float4 soup_row(double x, double y, double z) {
+    return make_float4(to_f32(x), to_f32(z), to_f32(y), __double2float_rn(3.1415));
+}
+
+// Model 0's vertices by rank: their doubles, their soup rows, and whether a face names them.
+struct Verts {
+    double *xyz;
+    float4 *row;
+    uint8_t *used;
+};
+
+// Model-0 vertex lines -> doubles and soup rows at their rank; numbers outside the device's
+// exact range are listed for the host.  Block i has the lines of line block blk0 + i, its text
+// staged when it holds a vertex line of model 0's lines [a, b).
+__global__ void __launch_bounds__(kLineBlock) k_vertices(const uint8_t *__restrict__ text, uint64_t n,
+                                                         const uint32_t *__restrict__ line_start, uint32_t L,
+                                                         const uint8_t *__restrict__ type, uint32_t blk0, uint32_t a,
+                                                         uint32_t b, const unsigned long long *__restrict__ pre,
+                                                         Verts vs, HardLine *__restrict__ hard,
+                                                         ObjCtl *__restrict__ ctl) {
+    __shared__ __align__(16) uint8_t win[kWindow];
+    __shared__ uint32_t s_v[kLineBlock / 32];
+    const uint32_t blk = blk0 + blockIdx.x, l0 = blk * kLineBlock, l = l0 + threadIdx.x;
+    const bool mine = l >= a && l < b && type[l] == LT_V;
+    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, mine);
+    if ((threadIdx.x & 31) == 0) s_v[threadIdx.x >> 5] = __popc(bal);
+    if (!__syncthreads_or(mine)) return;
+    uint32_t vi = (uint32_t)pre[blk] + __popc(bal & lanemask_lt());
+    for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) vi += s_v[w];
+    uint64_t w0, w1;
+    stage_lines(text, n, line_start, L, l0, min((uint32_t)kLineBlock, L - l0), win, w0, w1);
+    if (!mine) return;
+    uint64_t p, q;
+    line_bytes(n, line_start, L, l, p, q);
+    double c[3];
+    if (!(p >= w0 && q < w1 && fast_vertex(win + (p - w0), c))) {
+        VertexParse r;
+        if (p >= w0 && q <= w1) r = parse_vertex(win + (p - w0), (uint32_t)(q - p));
+        else r = parse_vertex(text + p, (uint32_t)(q - p));
+        c[0] = r.x;
+        c[1] = r.y;
+        c[2] = r.z;
+        if (!r.ok) {
+            const uint32_t h = atomicAdd(&ctl->num_hard, 1u);
+            hard[h] = HardLine{p, p + r.end, vi, 0u, 0u, 0u};
+        }
+    }
+    vs.xyz[3ull * vi] = c[0];
+    vs.xyz[3ull * vi + 1] = c[1];
+    vs.xyz[3ull * vi + 2] = c[2];
+    vs.row[vi] = soup_row(c[0], c[1], c[2]);
+    vs.used[vi] = 0;
+}
+
+__global__ void __launch_bounds__(kT) k_patch(const HardFix *__restrict__ fix, uint32_t count, Verts vs) {
+    const uint32_t i = blockIdx.x * kT + threadIdx.x;
+    if (i >= count) return;
+    const HardFix f = fix[i];
+    vs.xyz[3ull * f.vi] = f.xyz[0];
+    vs.xyz[3ull * f.vi + 1] = f.xyz[1];
+    vs.xyz[3ull * f.vi + 2] = f.xyz[2];
+    vs.row[f.vi] = soup_row(f.xyz[0], f.xyz[1], f.xyz[2]);
+}
+
+// A face's fan, one vertex after the other: stores triangles (first, previous, current).
+struct Fan {
+    float4 first, prev;
+    float4 *tri;
+    uint32_t nv = 0;
+    // vertex vk (0-based, the model's): false when the model has no such vertex
+    __device__ __forceinline__ bool add(uint32_t vk, uint32_t nverts, const Verts &vs) {
+        if (vk >= nverts) return false;
+        vs.used[vk] = 1;
+        const float4 cur = vs.row[vk];
+        if (nv == 0) {
+            first = cur;
+        } else if (nv >= 2) {
+            tri[0] = first;
+            tri[1] = prev;
+            tri[2] = cur;
+            tri += 3;
+        }
+        prev = cur;
+        ++nv;
+        return true;
+    }
+};
+
+// The face line b[0, len): its vertices resolved (negative indices against `before`, the
+// model's vertices so far) and fanned; false when an index names no vertex.
+__device__ __forceinline__ bool emit_face(const uint8_t *b, uint32_t len, long long before, uint32_t nverts,
+                                          const Verts &vs, float4 *tri) {
+    uint32_t i = 0, e = len;
+    skip_ws(b, i, e);
+    skip_token(b, i, e);  // the keyword
+    Fan fan;
+    fan.tri = tri;
+    while (skip_ws(b, i, e)) {
+        long long v = parse_index(b, i, e);
+        skip_token(b, i, e);
+        if (v == kIdxNaN || v == kIdxHuge) return false;
+        if (v < 0) v = before + 1 + v;  // vertices.length + 1 + vertexIndex
+        const long long vk = v - 1;
+        if (vk < 0 || vk >= (long long)nverts) return false;
+        fan.add((uint32_t)vk, nverts, vs);
+    }
+    return true;
+}
+
+// The same for the common form (as fast_class has it, indices of at most nine digits); done:
+// false when emit_face has to do the line (again from its start: it stores the same triangles).
+__device__ __forceinline__ bool fast_face(const uint8_t *b, uint32_t nverts, const Verts &vs, float4 *tri, bool &done) {
+    done = false;
+    if (b[0] != 'f' || b[1] != ' ') return true;
+    Fan fan;
+    fan.tri = tri;
+    uint32_t i = 1, c = ' ';
+    for (;;) {
+        while (c == ' ') c = b[++i];
+        if (c == '\n') break;
+        if (c == '\r' && b[i + 1] == '\n') break;
+        uint32_t v = c - '0', d, nd = 1;
+        if (v - 1u > 8u) return true;
+        while ((d = (c = b[++i]) - '0') <= 9u && nd < 10) {
+            v = v * 10 + d;
+            ++nd;
+        }
+        if (nd > 9) return true;
+        if (c == '/') {
+            do c = b[++i];
+            while (c > ' ' && c < 0x80 && c != '#');
+        }
+        if (c != ' ' && c != '\n' && c != '\r') return true;
+        if (!fan.add(v - 1u, nverts, vs)) {
+            done = true;
+            return false;
+        }
+    }
+    done = true;
+    return true;
+}
+
+// Model-0 faces -> fan triangles (y and z swapped, float32, pad 3.1415), their vertices marked.
+// Blocks as k_vertices.
+__global__ void __launch_bounds__(kLineBlock) k_faces(const uint8_t *__restrict__ text, uint64_t n,
+                                                      const uint32_t *__restrict__ line_start, uint32_t L,
+                                                      const uint8_t *__restrict__ type,
+                                                      const uint32_t *__restrict__ fans, uint32_t blk0, uint32_t a,
+                                                      uint32_t b, const unsigned long long *__restrict__ pre,
+                                                      uint32_t nverts, Verts vs, float4 *__restrict__ tri,
+                                                      ObjCtl *__restrict__ ctl) {
+    __shared__ __align__(16) uint8_t win[kWindow];
+    __shared__ unsigned long long s_warp[kLineBlock / 32];
+    const uint32_t blk = blk0 + blockIdx.x, l0 = blk * kLineBlock, l = l0 + threadIdx.x;
+    const bool in = l >= a && l < b;
+    const uint8_t ty = in ? type[l] : (uint8_t)LT_NONE;
+    const bool mine = ty == LT_F;
+    if (!__syncthreads_or(mine)) return;
+    const unsigned long long at = pre[blk] + block_scan<unsigned long long>(line_count(ty, mine ? fans[l] : 0u), s_warp, nullptr);
+    uint64_t w0, w1;
+    stage_lines(text, n, line_start, L, l0, min((uint32_t)kLineBlock, L - l0), win, w0, w1);
+    chain_wait();  // the vertices
+    if (!mine) return;
+    uint64_t p, q;
+    line_bytes(n, line_start, L, l, p, q);
+    float4 *out = tri + 3ull * (at >> 32);
+    const long long before = (long long)(at & 0xFFFFFFFFull);  // model-0 vertices so far
+    bool ok = true, done = false;
+    if (p >= w0 && q < w1) ok = fast_face(win + (p - w0), nverts, vs, out, done);
+    if (!done) {
+        if (p >= w0 && q <= w1) ok = emit_face(win + (p - w0), (uint32_t)(q - p), before, nverts, vs, out);
+        else ok = emit_face(text + p, (uint32_t)(q - p), before, nverts, vs, out);
+    }
+    if (!ok) atomicOr(&ctl->bad_index, 1u);
+}
+
+// Math.min / Math.max over the vertices that faces name (x, the file's z, y; -0 below +0, NaN
+// absorbs), and, in the last block to finish, the floor (parse-obj.js:62-76): two triangles at
+// z_min + .01, 10000 out in x and y, after the model's triangles; z_min = Math.min from 1e30.
+__global__ void __launch_bounds__(kT) k_bounds_floor(Verts vs, uint32_t nverts, float4 *__restrict__ tri_floor,
+                                                     ObjCtl *__restrict__ ctl) {
+    __shared__ unsigned long long s_mn[3][kT / 32], s_mx[3][kT / 32];
+    __shared__ int s_nan[3][kT / 32];
+    __shared__ bool s_last;
+    chain_wait();
+    unsigned long long mn[3] = {~0ull, ~0ull, ~0ull}, mx[3] = {0ull, 0ull, 0ull};
+    bool nan[3] = {false, false, false};
+    for (uint32_t v = blockIdx.x * kT + threadIdx.x; v < nverts; v += gridDim.x * kT) {
+        if (!vs.used[v]) continue;
+        const double *p = vs.xyz + 3ull * v;
+        const double c[3] = {p[0], p[2], p[1]};
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
             if (isnan(c[ax])) {
@@ -740,77 +1003,10 @@ struct BoundsAcc {
             mx[ax] = o > mx[ax] ? o : mx[ax];
         }
     }
-};
-
-// The face line b[0, len): its vertices resolved (negative indices against `before`, the
-// model's vertices so far), fanned from the first, stored from triangle `out` on; false when an
-// index names no vertex.
-__device__ __forceinline__ bool emit_face(const uint8_t *b, uint32_t len, long long before, uint32_t nverts,
-                                          const double *__restrict__ verts, float4 *__restrict__ tri,
-                                          unsigned long long out, BoundsAcc &bd) {
-    uint32_t i = 0, e = len;
-    skip_ws(b, i, e);
-    skip_token(b, i, e);  // the keyword
-    const float pad = __double2float_rn(3.1415);
-    float4 r = make_float4(0.f, 0.f, 0.f, pad), prev = r;
-    int nv = 0;
-    while (skip_ws(b, i, e)) {
-        long long v = parse_index(b, i, e);
-        skip_token(b, i, e);
-        if (v == kIdxNaN || v == kIdxHuge) return false;
-        if (v < 0) v = before + 1 + v;  // vertices.length + 1 + vertexIndex
-        const long long vk = v - 1;
-        if (vk < 0 || vk >= (long long)nverts) return false;
-        const double *vp = verts + 3ull * (unsigned long long)vk;
-        const double c[3] = {vp[0], vp[2], vp[1]};  // x, then the file's z as y and y as z
-        bd.add(c);
-        const float4 cur = make_float4(to_f32(c[0]), to_f32(c[1]), to_f32(c[2]), pad);
-        if (nv == 0) {
-            r = cur;
-        } else if (nv >= 2) {
-            float4 *o = tri + 3ull * out;
-            o[0] = r;
-            o[1] = prev;
-            o[2] = cur;
-            ++out;
-        }
-        prev = cur;
-        ++nv;
-    }
-    return true;
-}
-
-// Model-0 faces -> fan triangles (y and z swapped, float32, pad 3.1415) and the bounds.  One
-// block per kLineBlock lines of model 0, its text staged when it holds a face line.
-__global__ void __launch_bounds__(kLineBlock) k_faces(const uint8_t *__restrict__ text, uint64_t n,
-                                                      const uint64_t *__restrict__ line_start, uint32_t L,
-                                                      const uint8_t *__restrict__ type, uint32_t a, uint32_t m,
-                                                      const unsigned long long *__restrict__ pre, uint32_t nverts,
-                                                      const double *__restrict__ verts, float4 *__restrict__ tri,
-                                                      ObjCtl *__restrict__ ctl) {
-    __shared__ __align__(16) uint8_t win[kWindow];
-    const uint32_t i0 = blockIdx.x * kLineBlock, i = i0 + threadIdx.x;
-    const bool mine = i < m && type[a + i] == LT_F;
-    if (!__syncthreads_or(mine)) return;
-    uint64_t w0, w1;
-    stage_lines(text, n, line_start, L, a + i0, min((uint32_t)kLineBlock, m - i0), win, w0, w1);
-    BoundsAcc bd{{~0ull, ~0ull, ~0ull}, {0ull, 0ull, 0ull}, {false, false, false}};
-    if (mine) {
-        uint64_t p, q;
-        line_bytes(n, line_start, L, a + i, p, q);
-        const long long before = (long long)(pre[a + i] & 0xFFFFFFFFull);  // model-0 vertices so far
-        const unsigned long long out = pre[a + i] >> 32;
-        bool ok;
-        if (p >= w0 && q <= w1) ok = emit_face(win + (p - w0), (uint32_t)(q - p), before, nverts, verts, tri, out, bd);
-        else ok = emit_face(text + p, (uint32_t)(q - p), before, nverts, verts, tri, out, bd);
-        if (!ok) atomicOr(&ctl->bad_index, 1u);
-    }
-    __shared__ unsigned long long s_mn[3][kLineBlock / 32], s_mx[3][kLineBlock / 32];
-    __shared__ int s_nan[3][kLineBlock / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int ax = 0; ax < 3; ++ax) {
-        unsigned long long lo = bd.mn[ax], hi = bd.mx[ax];
+        unsigned long long lo = mn[ax], hi = mx[ax];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const unsigned long long lo2 = __shfl_xor_sync(0xFFFFFFFFu, lo, o);
@@ -818,7 +1014,7 @@ __global__ void __launch_bounds__(kLineBlock) k_faces(const uint8_t *__restrict_
             lo = lo2 < lo ? lo2 : lo;
             hi = hi2 > hi ? hi2 : hi;
         }
-        const int nan_any = __any_sync(0xFFFFFFFFu, bd.nan[ax]);
+        const int nan_any = __any_sync(0xFFFFFFFFu, nan[ax]);
         if (lane == 0) { s_mn[ax][warp] = lo; s_mx[ax][warp] = hi; s_nan[ax][warp] = nan_any; }
     }
     __syncthreads();
@@ -826,31 +1022,31 @@ __global__ void __launch_bounds__(kLineBlock) k_faces(const uint8_t *__restrict_
         const int ax = threadIdx.x;
         unsigned long long lo = ~0ull, hi = 0ull;
         int nan_any = 0;
-        for (int w = 0; w < kLineBlock / 32; ++w) {
+        for (int w = 0; w < kT / 32; ++w) {
             lo = s_mn[ax][w] < lo ? s_mn[ax][w] : lo;
             hi = s_mx[ax][w] > hi ? s_mx[ax][w] : hi;
             nan_any |= s_nan[ax][w];
         }
-        if (lo != ~0ull && lo < *(volatile unsigned long long *)&ctl->bmin[ax]) atomicMin(&ctl->bmin[ax], lo);
-        if (hi != 0ull && hi > *(volatile unsigned long long *)&ctl->bmax[ax]) atomicMax(&ctl->bmax[ax], hi);
-        if (nan_any && !*(volatile uint32_t *)&ctl->nan_min[ax]) {
+        if (lo != ~0ull) atomicMin(&ctl->bmin[ax], lo);
+        if (hi != 0ull) atomicMax(&ctl->bmax[ax], hi);
+        if (nan_any) {
             atomicOr(&ctl->nan_min[ax], 1u);
             atomicOr(&ctl->nan_max[ax], 1u);
         }
     }
-}
-
-// The floor (parse-obj.js:62-76): two triangles at z_min + .01, 10000 out in x and y, after the
-// model's triangles; z_min = Math.min from 1e30 over the faces' vertices (NaN absorbs).
-__global__ void k_floor(const ObjCtl *__restrict__ ctl, float4 *__restrict__ tri_floor) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atom_add_acq_rel_gpu(&ctl->done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
     const int v = threadIdx.x;  // 6 vertices
+    if (v == 0) ctl->done = 0u;
     if (v >= 6) return;
+    const unsigned long long zo = __ldcg(&ctl->bmin[2]);
     double zmin = 1e30;
-    if (ctl->nan_min[2]) {
+    if (__ldcg(&ctl->nan_min[2])) {
         zmin = NAN;
-    } else if (ctl->bmin[2] != ~0ull) {
-        const unsigned long long o = ctl->bmin[2];
-        const double d = __longlong_as_double((long long)((o >> 63) ? (o & 0x7FFFFFFFFFFFFFFFull) : ~o));
+    } else if (zo != ~0ull) {
+        const double d = __longlong_as_double((long long)((zo >> 63) ? (zo & 0x7FFFFFFFFFFFFFFFull) : ~zo));
         zmin = d < 1e30 ? d : 1e30;
     }
     const float h = to_f32(__dadd_rn(zmin, .01)), f = 10000.0f, pad = __double2float_rn(3.1415);
@@ -908,30 +1104,37 @@ cudaError_t grow(void *&p, size_t &have, size_t need) {
 
 }  // namespace
 
-int obj_parse(ObjScratch &sc, const char *text, uint64_t bytes, bool host_text, const float **tri_out,
-              uint32_t *num_tris, double *bounds6, uint64_t *err_line, cudaStream_t s,
-              std::string &err) {
-    auto cuda = [&](cudaError_t e, const char *what) -> int {
-        if (e == cudaSuccess) return LVBH_OK;
-        cudaGetLastError();
-        err = std::string(what) + ": " + cudaGetErrorString(e);
-        return e == cudaErrorMemoryAllocation ? LVBH_ENOMEM : LVBH_ECUDA;
-    };
 #define OBJ_CUDA(call, what)                          \
     do {                                              \
         if (int rc_ = cuda((call), what)) return rc_; \
     } while (0)
+
+namespace {
+
+int obj_cuda(cudaError_t e, const char *what, std::string &err) {
+    if (e == cudaSuccess) return LVBH_OK;
+    cudaGetLastError();
+    err = std::string(what) + ": " + cudaGetErrorString(e);
+    return e == cudaErrorMemoryAllocation ? LVBH_ENOMEM : LVBH_ECUDA;
+}
+
+}  // namespace
+
+int obj_scan(ObjScratch &sc, const char *text, uint64_t bytes, bool host_text, uint32_t *num_tris, uint64_t *err_line,
+             cudaStream_t s, std::string &err) {
+    auto cuda = [&](cudaError_t e, const char *what) { return obj_cuda(e, what, err); };
     auto reject = [&](uint64_t line, const std::string &msg) {
         *err_line = line;
         err = msg;
         return LVBH_EPARSE;
     };
     *err_line = 0;
+    sc.scanned = false;
     if (!sc.host) OBJ_CUDA(cudaMallocHost(&sc.host, sizeof(ObjCtl)), "cudaMallocHost");
     ObjCtl *hc = static_cast<ObjCtl *>(sc.host);
     // text (staged when it is host memory or not 16-byte aligned), control block, newline
     // counts per chunk
-    const uint32_t chunks = (uint32_t)((bytes + kChunk - 1) / kChunk);
+    const uint32_t chunks = bytes ? (uint32_t)((bytes + kChunk - 1) / kChunk) : 1u;
     const bool stage = host_text || (reinterpret_cast<uintptr_t>(text) & 15u);
     const size_t text_part = stage ? align256(bytes) : 0;
     OBJ_CUDA(grow(sc.text, sc.text_bytes, text_part + align256(sizeof(ObjCtl)) + align256((chunks + 1) * 4ull)),
@@ -946,74 +1149,90 @@ int obj_parse(ObjScratch &sc, const char *text, uint64_t bytes, bool host_text, 
     }
     ObjCtl *ctl = reinterpret_cast<ObjCtl *>(c);
     uint32_t *cnt = reinterpret_cast<uint32_t *>(c + align256(sizeof(ObjCtl)));
-    std::memset(hc, 0, sizeof(ObjCtl));
-    hc->err_line = hc->first_o = hc->second_o = hc->first_need = kNone;
-    for (int a = 0; a < 3; ++a) hc->bmin[a] = ~0ull;
-    OBJ_CUDA(cudaMemcpyAsync(ctl, hc, sizeof(ObjCtl), cudaMemcpyHostToDevice, s), "cudaMemcpyAsync(ctl)");
-    if (chunks) {
-        k_nl_count<<<chunks, kT, 0, s>>>(d_text, bytes, cnt);
-        k_scan_small<uint32_t><<<1, 1024, 0, s>>>(cnt, chunks, &ctl->newlines);
-        OBJ_CUDA(cudaGetLastError(), "k_nl_count");
-        OBJ_CUDA(cudaMemcpyAsync(&hc->newlines, &ctl->newlines, 4, cudaMemcpyDeviceToHost, s), "readback");
+    k_nl_count<<<chunks, kT, 0, s>>>(d_text, bytes, cnt, ctl);
+    launch_chained(true, k_scan_small<uint32_t>, 1, 1024, 0, s, cnt, chunks, &ctl->newlines);
+    // lines, model 0 and the vertex / triangle prefixes in one stream-ordered run, for as many lines
+    // as a text of this size usually has at most; one with more of them (seen from the count)
+    // runs again
+    uint32_t cap = (uint32_t)std::min<uint64_t>(bytes / 16 + 4096, 0xFFFFFFFEull);
+    for (;;) {
+        const uint32_t nb = cap / kLineBlock + 1;
+        const size_t starts = align256((cap + 1ull) * 4), types = align256(cap), fan_part = align256(cap * 4ull);
+        const size_t blk_part = align256(nb * sizeof(LineBlock));
+        OBJ_CUDA(grow(sc.lines, sc.lines_bytes, starts + types + fan_part + blk_part + align256(nb * 8ull)),
+                 "cudaMalloc(obj lines)");
+        char *cl = static_cast<char *>(sc.lines);
+        sc.line_start = reinterpret_cast<uint32_t *>(cl);
+        sc.type = reinterpret_cast<uint8_t *>(cl + starts);
+        sc.fans = reinterpret_cast<uint32_t *>(cl + starts + types);
+        LineBlock *blocks = reinterpret_cast<LineBlock *>(cl + starts + types + fan_part);
+        sc.pre = reinterpret_cast<unsigned long long *>(cl + starts + types + fan_part + blk_part);
+        launch_chained(true, k_nl_write, chunks, kT, 0, s, d_text, bytes, cnt, cap, sc.line_start);
+        launch_chained(true, k_lines, (cap + kLineBlock - 1) / kLineBlock, kLineBlock, 0, s, d_text, bytes, sc.line_start,
+                       cap, sc.type, sc.fans, blocks, ctl);
+        launch_chained(true, k_model, 1, 1024, 0, s, blocks, sc.type, sc.fans, cap, sc.pre, ctl);
+        OBJ_CUDA(cudaGetLastError(), "k_lines");
+        OBJ_CUDA(cudaMemcpyAsync(hc, ctl, sizeof(ObjCtl), cudaMemcpyDeviceToHost, s), "readback");
+        OBJ_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        if (hc->newlines + 1ull <= cap) break;
+        cap = hc->newlines + 1u;  // at most LVBH_OBJ_MAX_BYTES + 1
     }
-    OBJ_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
-    const uint32_t L = hc->newlines + 1;
-    // per-line arrays: starts, types, fan counts; then (model-0 range only) prefixes
-    const size_t lines_need = align256((L + 1ull) * 8) + align256(L) + align256(L * 4ull) +
-                              align256(L * 8ull) + align256(((L + (uint64_t)kScanTile - 1) / kScanTile + 1) * 8);
-    OBJ_CUDA(grow(sc.lines, sc.lines_bytes, lines_need), "cudaMalloc(obj lines)");
-    char *cl = static_cast<char *>(sc.lines);
-    uint64_t *line_start = reinterpret_cast<uint64_t *>(cl);
-    cl += align256((L + 1ull) * 8);
-    uint8_t *type = reinterpret_cast<uint8_t *>(cl);
-    cl += align256(L);
-    uint32_t *fans = reinterpret_cast<uint32_t *>(cl);
-    cl += align256(L * 4ull);
-    unsigned long long *pre = reinterpret_cast<unsigned long long *>(cl);
-    cl += align256(L * 8ull);
-    unsigned long long *sums = reinterpret_cast<unsigned long long *>(cl);
-    if (chunks) k_nl_write<<<chunks, kT, 0, s>>>(d_text, bytes, cnt, line_start);
-    else OBJ_CUDA(cudaMemsetAsync(line_start, 0, 8, s), "cudaMemsetAsync");
-    const uint32_t lb = (uint32_t)((L + (uint64_t)kT - 1) / kT);
-    const uint32_t tiles = (uint32_t)((L + (uint64_t)kScanTile - 1) / kScanTile);
-    // lines, model 0 and the vertex / triangle prefixes in one stream-ordered run (the first
-    // `o`, the model range and the scan read what the kernels before them left in ctl)
-    k_lines<<<lb, kLineBlock, 0, s>>>(d_text, bytes, line_start, L, type, fans, ctl);
-    k_second_o<<<lb, kT, 0, s>>>(type, L, ctl);
-    k_model_range<<<1, 1, 0, s>>>(L, ctl);
-    k_scan_up<<<tiles, kT, 0, s>>>(type, fans, L, ctl, sums);
-    k_scan_small<unsigned long long><<<1, 1024, 0, s>>>(sums, tiles, &ctl->totals);
-    k_scan_down<<<tiles, kT, 0, s>>>(type, fans, L, ctl, sums, pre);
-    OBJ_CUDA(cudaGetLastError(), "k_lines");
-    OBJ_CUDA(cudaMemcpyAsync(hc, ctl, sizeof(ObjCtl), cudaMemcpyDeviceToHost, s), "readback");
-    OBJ_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
     if (hc->err_line != kNone)
         return reject(hc->err_line + 1ull, "line " + std::to_string(hc->err_line + 1ull) +
                                                 ": a statement the OBJ parser rejects");
     if (hc->no_model) return reject(0, "the OBJ text defines no model");
-    const uint32_t m0a = hc->m0a, m = hc->m0b - hc->m0a;
-    const uint32_t mb = (uint32_t)((m + (uint64_t)kLineBlock - 1) / kLineBlock);
-    const uint32_t nverts = (uint32_t)(hc->totals & 0xFFFFFFFFull);
     const uint64_t nfan = hc->totals >> 32;
     if (nfan + 2 > LVBH_MAX_TRIS) return reject(0, "the OBJ text makes more than LVBH_MAX_TRIS triangles");
-    const uint32_t ntri = (uint32_t)nfan + 2;
-    // the soup first (16-byte aligned), then the vertices and the hard-line slots
-    const size_t tbytes = align256(ntri * 48ull), vbytes = align256(nverts * 24ull);
-    OBJ_CUDA(grow(sc.soup, sc.soup_bytes, tbytes + vbytes + align256(nverts * (size_t)sizeof(HardLine))),
-             "cudaMalloc(obj soup)");
-    float4 *tri = static_cast<float4 *>(sc.soup);
-    double *verts = reinterpret_cast<double *>(static_cast<char *>(sc.soup) + tbytes);
-    HardLine *hard = reinterpret_cast<HardLine *>(static_cast<char *>(sc.soup) + tbytes + vbytes);
-    // vertices, faces and the floor, then one read-back; numbers the device left to the host
-    // (rare) are patched in and the faces and floor run again
-    auto faces_and_floor = [&]() {
-        if (nfan && mb)
-            k_faces<<<mb, kLineBlock, 0, s>>>(d_text, bytes, line_start, L, type, m0a, m, pre, nverts, verts, tri, ctl);
-        k_floor<<<1, 32, 0, s>>>(ctl, tri + 3ull * nfan);
+    *num_tris = (uint32_t)nfan + 2;
+    sc.scanned = true;
+    sc.src = text;
+    sc.d_text = d_text;
+    sc.src_bytes = bytes;
+    sc.host_text = host_text;
+    sc.ctl = ctl;
+    return LVBH_OK;
+}
+
+int obj_emit(ObjScratch &sc, float *dst, const float **tri_out, double *bounds6, uint64_t *err_line, cudaStream_t s,
+             std::string &err) {
+    auto cuda = [&](cudaError_t e, const char *what) { return obj_cuda(e, what, err); };
+    *err_line = 0;
+    if (!sc.scanned) {
+        err = "no scanned OBJ text";
+        return LVBH_EINVAL;
+    }
+    sc.scanned = false;
+    ObjCtl *hc = static_cast<ObjCtl *>(sc.host), *ctl = static_cast<ObjCtl *>(sc.ctl);
+    const uint32_t L = hc->newlines + 1u, a = hc->m0a, b = hc->m0b;
+    const uint32_t nverts = (uint32_t)(hc->totals & 0xFFFFFFFFull), nfan = (uint32_t)(hc->totals >> 32);
+    const uint32_t blk0 = a / kLineBlock, nblk = b > a ? (b - 1) / kLineBlock - blk0 + 1 : 0;
+    const size_t xyz = align256(nverts * 24ull), rows = align256(nverts * 16ull), used = align256(nverts);
+    OBJ_CUDA(grow(sc.verts, sc.verts_bytes, xyz + rows + used + align256(nverts * (size_t)sizeof(HardLine))),
+             "cudaMalloc(obj vertices)");
+    if (!dst) {
+        OBJ_CUDA(grow(sc.soup, sc.soup_bytes, align256((nfan + 2ull) * 48)), "cudaMalloc(obj soup)");
+        dst = static_cast<float *>(sc.soup);
+    }
+    char *cv = static_cast<char *>(sc.verts);
+    float4 *tri = reinterpret_cast<float4 *>(dst);
+    const Verts vs{reinterpret_cast<double *>(cv), reinterpret_cast<float4 *>(cv + xyz),
+                   reinterpret_cast<uint8_t *>(cv + xyz + rows)};
+    HardLine *hard = reinterpret_cast<HardLine *>(cv + xyz + rows + used);
+    const uint8_t *d_text = sc.d_text;
+    const uint64_t bytes = sc.src_bytes;
+    // vertices, faces, bounds and floor, then one read-back; numbers the device left to the host
+    // (rare) are patched in and the faces, bounds and floor run again
+    auto faces_bounds_floor = [&](bool chain) {
+        if (nfan)
+            launch_chained(chain && nverts, k_faces, nblk, kLineBlock, 0, s, d_text, bytes, sc.line_start, L, sc.type, sc.fans,
+                           blk0, a, b, sc.pre, nverts, vs, tri, ctl);
+        const uint32_t want = (nverts + kT - 1) / kT, most = (uint32_t)sm_count() * 4u;
+        const uint32_t grid = want < 1 ? 1 : want < most ? want : most;
+        launch_chained(true, k_bounds_floor, grid, kT, 0, s, vs, nverts, tri + 3ull * nfan, ctl);
     };
-    if (nverts && mb)
-        k_vertices<<<mb, kLineBlock, 0, s>>>(d_text, bytes, line_start, L, type, m0a, m, pre, verts, hard, ctl);
-    faces_and_floor();
+    if (nverts)
+        k_vertices<<<nblk, kLineBlock, 0, s>>>(d_text, bytes, sc.line_start, L, sc.type, blk0, a, b, sc.pre, vs, hard, ctl);
+    faces_bounds_floor(true);
     OBJ_CUDA(cudaGetLastError(), "k_faces");
     OBJ_CUDA(cudaMemcpyAsync(hc, ctl, sizeof(ObjCtl), cudaMemcpyDeviceToHost, s), "readback");
     OBJ_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
@@ -1026,8 +1245,8 @@ int obj_parse(ObjScratch &sc, const char *text, uint64_t bytes, bool host_text, 
         std::vector<uint8_t> buf;
         for (uint32_t h = 0; h < nh; ++h) {
             uint64_t len = hl[h].end - hl[h].start;
-            const uint8_t *ln = reinterpret_cast<const uint8_t *>(text) + hl[h].start;
-            if (!host_text) {
+            const uint8_t *ln = reinterpret_cast<const uint8_t *>(sc.src) + hl[h].start;
+            if (!sc.host_text) {
                 buf.resize(len);
                 if (len) OBJ_CUDA(cudaMemcpy(buf.data(), d_text + hl[h].start, len, cudaMemcpyDeviceToHost), "readback");
                 ln = buf.data();
@@ -1037,47 +1256,50 @@ int obj_parse(ObjScratch &sc, const char *text, uint64_t bytes, bool host_text, 
             uint64_t k = 0, ta = 0, tb = 0;
             next_token(ln, k, len, ta, tb);  // the keyword
             HardFix f{{0.0, 0.0, 0.0}, hl[h].vi, 0u};
-            for (int a = 0; a < 3; ++a) {
+            for (int ax = 0; ax < 3; ++ax) {
                 if (!next_token(ln, k, len, ta, tb)) break;
-                f.xyz[a] = host_parse_float(ln + ta, tb - ta);
+                f.xyz[ax] = host_parse_float(ln + ta, tb - ta);
             }
             fix[h] = f;
         }
         HardFix *dfix = reinterpret_cast<HardFix *>(hard);
         OBJ_CUDA(cudaMemcpyAsync(dfix, fix.data(), nh * sizeof(HardFix), cudaMemcpyHostToDevice, s),
                  "cudaMemcpyAsync(fix)");
-        k_patch<<<(nh + kT - 1) / kT, kT, 0, s>>>(dfix, nh, verts);
+        k_patch<<<(nh + kT - 1) / kT, kT, 0, s>>>(dfix, nh, vs);
         // the bounds and the index check start over
-        for (int a = 0; a < 3; ++a) {
-            hc->bmin[a] = ~0ull;
-            hc->bmax[a] = 0ull;
-            hc->nan_min[a] = hc->nan_max[a] = 0u;
+        for (int ax = 0; ax < 3; ++ax) {
+            hc->bmin[ax] = ~0ull;
+            hc->bmax[ax] = 0ull;
+            hc->nan_min[ax] = hc->nan_max[ax] = 0u;
         }
         hc->bad_index = 0u;
         OBJ_CUDA(cudaMemcpyAsync(ctl, hc, sizeof(ObjCtl), cudaMemcpyHostToDevice, s), "cudaMemcpyAsync(ctl)");
-        faces_and_floor();
+        faces_bounds_floor(false);
         OBJ_CUDA(cudaGetLastError(), "k_faces");
         OBJ_CUDA(cudaMemcpyAsync(hc, ctl, sizeof(ObjCtl), cudaMemcpyDeviceToHost, s), "readback");
         OBJ_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");  // also: `fix` is pageable
     }
-    if (hc->bad_index) return reject(0, "a face of model 0 names a vertex the model does not have");
-    // bounds: Math.min / Math.max from 1e30 / -1e30 over the faces' vertices
-    for (int a = 0; a < 3; ++a) {
-        const double lo = hc->bmin[a] == ~0ull ? 1e30 : ord64_inv(hc->bmin[a]);
-        const double hi = hc->bmax[a] == 0ull ? -1e30 : ord64_inv(hc->bmax[a]);
-        bounds6[a] = hc->nan_min[a] ? NAN : (lo < 1e30 ? lo : 1e30);
-        bounds6[3 + a] = hc->nan_max[a] ? NAN : (hi > -1e30 ? hi : -1e30);
+    if (hc->bad_index) {
+        err = "a face of model 0 names a vertex the model does not have";
+        return LVBH_EPARSE;
     }
-    *tri_out = reinterpret_cast<const float *>(tri);
-    *num_tris = ntri;
-#undef OBJ_CUDA
+    // bounds: Math.min / Math.max from 1e30 / -1e30 over the faces' vertices
+    for (int ax = 0; ax < 3; ++ax) {
+        const double lo = hc->bmin[ax] == ~0ull ? 1e30 : ord64_inv(hc->bmin[ax]);
+        const double hi = hc->bmax[ax] == 0ull ? -1e30 : ord64_inv(hc->bmax[ax]);
+        bounds6[ax] = hc->nan_min[ax] ? NAN : (lo < 1e30 ? lo : 1e30);
+        bounds6[3 + ax] = hc->nan_max[ax] ? NAN : (hi > -1e30 ? hi : -1e30);
+    }
+    if (tri_out) *tri_out = dst;
     return LVBH_OK;
 }
+#undef OBJ_CUDA
 
 void obj_free(ObjScratch &sc) {
     if (sc.text) cudaFree(sc.text);
     if (sc.lines) cudaFree(sc.lines);
     if (sc.soup) cudaFree(sc.soup);
+    if (sc.verts) cudaFree(sc.verts);
     if (sc.host) cudaFreeHost(sc.host);
     sc = ObjScratch{};
 }

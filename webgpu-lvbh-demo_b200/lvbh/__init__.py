@@ -433,17 +433,26 @@ class BVHBuilder:
                                         else np.asarray(text, dtype=np.uint8).reshape(-1))
             ptr, nbytes = keep.ctypes.data, keep.size
             flags = INPUT_HOST
-        tri = ctypes.c_void_p()
         n = ctypes.c_uint32()
         b6 = (ctypes.c_double * 6)()
         line = ctypes.c_uint64()
-        rc = _native.lib.lvbh_parse_obj(self._ctx, ctypes.c_void_p(ptr if nbytes else 0), nbytes, flags,
-                                        ctypes.byref(tri), ctypes.byref(n), b6, ctypes.byref(line),
-                                        _stream_ptr(stream, self.device))
+        sp = _stream_ptr(stream, self.device)
+        text_args = (self._ctx, ctypes.c_void_p(ptr if nbytes else 0), nbytes, flags)
+        if stream is None or stream == torch.cuda.current_stream(self.device):
+            # the soup straight into a tensor of the stream that the parse runs on
+            rc = _native.lib.lvbh_parse_obj_begin(*text_args, ctypes.byref(n), ctypes.byref(line), sp)
+            if rc == _native.OK:
+                soup = torch.empty((n.value, 12), dtype=torch.float32, device=self.device)
+                rc = _native.lib.lvbh_parse_obj_into(self._ctx, ctypes.c_void_p(soup.data_ptr()), b6,
+                                                     ctypes.byref(line), sp)
+        else:
+            tri = ctypes.c_void_p()
+            rc = _native.lib.lvbh_parse_obj(*text_args, ctypes.byref(tri), ctypes.byref(n), b6, ctypes.byref(line), sp)
+            if rc == _native.OK:
+                soup = _device_floats(tri.value, n.value * 12, self.device).clone().reshape(n.value, 12)
         if rc == _native.EPARSE:
             raise ObjError(int(line.value), _native.lib.lvbh_last_error(self._ctx).decode())
         _native.check(self._ctx, rc)
-        soup = _device_floats(tri.value, n.value * 12, self.device).clone().reshape(n.value, 12)
         return {"NUM_TRIS": n.value, "TRI_ARR": soup,
                 "BOUNDS": {"min": [b6[0], b6[1], b6[2]], "max": [b6[3], b6[4], b6[5]]}}
 
