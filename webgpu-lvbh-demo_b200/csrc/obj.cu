@@ -354,36 +354,43 @@ __device__ __forceinline__ bool parse_number(const uint8_t *b, uint32_t &i, uint
     return true;
 }
 
-// Line l: its bytes [p, q) (without the '\n').
-__device__ __forceinline__ void line_bytes(uint64_t n, const uint32_t *line_start, uint32_t L, uint32_t l,
-                                           uint64_t &p, uint64_t &q) {
-    p = line_start[l];
-    q = l + 1 < L ? line_start[l + 1] - 1u : n;
-}
-
 constexpr int kLineBlock = 256;     // lines per block of the per-line kernels
-constexpr int kWindow = 24 * 1024;  // text bytes a block stages in shared memory
+constexpr int kWindow = 16 * 1024;  // text bytes a block stages in shared memory
 
-// Stages the text of lines [l0, l0 + cnt) into win (as much as fits, from the 16-byte boundary
-// at or below the first line's start) with coalesced 16-byte loads; [w0, w1) is what it holds.
-// Every thread of the block calls it.
-__device__ void stage_lines(const uint8_t *__restrict__ text, uint64_t n, const uint32_t *__restrict__ line_start,
-                            uint32_t L, uint32_t l0, uint32_t cnt, uint8_t *win, uint64_t &w0, uint64_t &w1) {
-    const uint64_t a = line_start[l0] & ~15u;
-    const uint64_t z = l0 + cnt < L ? line_start[l0 + cnt] : n;
-    const uint64_t e = z < a + kWindow ? z : a + kWindow;
-    for (uint64_t c = a + 16ull * threadIdx.x; c < e; c += 16ull * blockDim.x) {
-        if (c + 16 <= n) {
-            *reinterpret_cast<uint4 *>(win + (c - a)) = __ldcs(reinterpret_cast<const uint4 *>(text + c));
-        } else {
-            for (int k = 0; k < 16; ++k)
-                if (c + k < n) win[c - a + k] = text[c + k];
-        }
+// A thread's line l of a block's lines [l0, l0 + kLineBlock), and the text the block stages:
+// positions fit 32 bits (LVBH_OBJ_MAX_BYTES).  Their loads depend on nothing but the line number,
+// so they are in flight together with a kernel's other first loads.
+struct LineText {
+    uint32_t p, q;    // the line's bytes [p, q) (without the '\n'; nothing past the last line)
+    uint32_t w0, w1;  // the window: from the 16-byte boundary at or below the first line's start, as
+                      // much of the block's text as fits
+    __device__ __forceinline__ LineText(const uint32_t *__restrict__ line_start, uint32_t L, uint32_t l0, uint64_t n) {
+        const uint32_t l = l0 + threadIdx.x, last = min(L, l0 + kLineBlock);
+        p = l < L ? line_start[l] : 0u;
+        q = l + 1 < L ? line_start[l + 1] - 1u : l < L ? (uint32_t)n : 0u;
+        w0 = line_start[l0] & ~15u;
+        const uint32_t z = last < L ? line_start[last] : (uint32_t)n;
+        w1 = w0 + min(z - w0, (uint32_t)kWindow);
     }
-    w0 = a;
-    w1 = e;
-    __syncthreads();
-}
+    // [w0, w1) of the text into win, all 16-byte copies in flight together.  Every thread calls it.
+    __device__ __forceinline__ void stage(const uint8_t *__restrict__ text, uint64_t n, uint8_t *win) const {
+        const uint32_t len = w1 - w0, rest = (uint32_t)n - w0;
+        for (uint32_t o = 16u * threadIdx.x; o < len; o += 16u * kLineBlock) {
+            if (o + 16u <= rest) {
+                cp_async16(win + o, text + w0 + o);
+            } else {
+                for (uint32_t k = 0; k < 16; ++k)
+                    if (o + k < rest) win[o + k] = text[w0 + o + k];
+            }
+        }
+        cp_async_commit();
+        cp_async_wait_all();
+        __syncthreads();
+    }
+    __device__ __forceinline__ uint32_t len() const { return q - p; }
+    __device__ __forceinline__ bool whole() const { return p >= w0 && q < w1; }  // the line and its newline
+    __device__ __forceinline__ bool body() const { return p >= w0 && q <= w1; }  // the line
+};
 
 __device__ __forceinline__ uint8_t lower(uint8_t c) { return (c >= 'A' && c <= 'Z') ? c + 32 : c; }
 
@@ -439,7 +446,7 @@ __device__ __forceinline__ void warp_min_into(uint32_t v, uint32_t *dst) {
 __device__ __forceinline__ void load64(const uint8_t *__restrict__ s, uint64_t n, uint64_t p, uint4 (&v)[4]) {
     if (p + 64 <= n) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = __ldcs(reinterpret_cast<const uint4 *>(s + p) + j);
+        for (int j = 0; j < 4; ++j) v[j] = __ldg(reinterpret_cast<const uint4 *>(s + p) + j);  // read again: keep it in L2
     } else {
         uint8_t *b = reinterpret_cast<uint8_t *>(v);
         for (int k = 0; k < 64; ++k) b[k] = p + k < n ? s[p + k] : 0;
@@ -449,6 +456,12 @@ __device__ __forceinline__ void load64(const uint8_t *__restrict__ s, uint64_t n
 __device__ __forceinline__ uint32_t newlines_in(uint32_t w) {
     const uint32_t x = w ^ 0x0A0A0A0Au;  // zero bytes where '\n' was
     return __popc(~(((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x | 0x7F7F7F7Fu));
+}
+
+// The newline bytes of w as four bits.
+__device__ __forceinline__ uint32_t newline_nibble(uint32_t w) {
+    const uint32_t x = w ^ 0x0A0A0A0Au, y = ~(((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x | 0x7F7F7F7Fu);
+    return ((y >> 7) * 0x10204080u) >> 28;  // bits 7, 15, 23, 31 -> 0, 1, 2, 3
 }
 
 __device__ __forceinline__ uint32_t newlines64(const uint4 (&v)[4]) {
@@ -508,18 +521,23 @@ __global__ void __launch_bounds__(kT) k_nl_write(const uint8_t *__restrict__ s, 
     const uint64_t p = (uint64_t)blockIdx.x * kChunk + threadIdx.x * 64ull;
     uint4 v[4];
     load64(s, n, p, v);
-    const uint32_t before = block_scan<uint32_t>(newlines64(v), s_warp, nullptr);
-    chain_wait();
-    uint32_t r = base[blockIdx.x] + before;
+    // bit k: byte k is a newline
+    unsigned long long m = 0;
     const uint32_t *w = reinterpret_cast<const uint32_t *>(v);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        uint32_t m = ~(((w[j] ^ 0x0A0A0A0Au) & 0x7F7F7F7Fu) + 0x7F7F7F7Fu | (w[j] ^ 0x0A0A0A0Au) | 0x7F7F7F7Fu);
-        while (m) {  // one bit (7, 15, 23 or 31) per newline byte, in text order
-            const int byte = (__ffs(m) - 1) >> 3;
-            if (++r < cap) line_start[r] = (uint32_t)(p + 4 * j + byte + 1);
-            m &= m - 1;
-        }
+    for (int h = 0; h < 2; ++h) {
+        uint32_t bits = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) bits |= newline_nibble(w[8 * h + j]) << (4 * j);
+        m |= (unsigned long long)bits << (32 * h);
+    }
+    const uint32_t before = block_scan<uint32_t>((uint32_t)__popcll((long long)m), s_warp, nullptr);
+    chain_wait();
+    uint32_t r = base[blockIdx.x] + before;
+    while (m) {
+        const int k = __ffsll((long long)m) - 1;
+        if (++r < cap) line_start[r] = (uint32_t)p + k + 1;
+        m &= m - 1;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) line_start[0] = 0;
 }
@@ -567,7 +585,7 @@ __device__ __forceinline__ LineClass classify(const uint8_t *b, uint32_t len) {
 // The class of a line in its common forms: empty, comment, `v ` / `vt ` / `vn ` (no checks), and
 // `f` with tokens apart by spaces that start with 1 to 9 (an index that parseInt makes neither 0
 // nor NaN) and hold ASCII without '#'.  b[len] is the line's '\n'.  False: classify() decides.
-__device__ __forceinline__ bool fast_class(const uint8_t *b, uint32_t len, LineClass &r) {
+__device__ __forceinline__ bool fast_class(const uint8_t *b, LineClass &r) {
     r = LineClass{LT_NONE, false, 0};
     const uint32_t c0 = b[0];
     if (c0 == '\n' || c0 == '#') return true;
@@ -586,48 +604,50 @@ __device__ __forceinline__ bool fast_class(const uint8_t *b, uint32_t len, LineC
         if (c == '\r' && b[i + 1] == '\n') break;
         if (c - '1' > 8u) return false;
         ++ntok;
-        uint32_t slashes = 0;
-        do {
-            c = b[++i];
-            slashes += c == '/';
-        } while (c > ' ' && c < 0x80 && c != '#');
+        do c = b[++i];
+        while (c - '0' <= 9u);
+        if (c == '/') {
+            uint32_t slashes = 1;
+            do {
+                c = b[++i];
+                slashes += c == '/';
+            } while (c > ' ' && c < 0x80 && c != '#');
+            r.bad |= slashes > 2;
+        }
         if (c != ' ' && c != '\n' && c != '\r') return false;
-        r.bad |= slashes > 2;
     }
     if (ntok < 3) r.bad = true;
     else r.fan = ntok - 2;
     return true;
 }
 
-// What k_lines leaves per block of kLineBlock lines: packed counts of all its lines (vertices in
-// the low, triangles in the high 32 bits), its first two `o` lines and its first model-creating one.
-struct LineBlock {
-    unsigned long long count;
-    uint32_t o1, o2, need, pad;
+// What k_lines leaves per block of kLineBlock lines (an array each): packed counts of all its
+// lines (vertices in the low, triangles in the high 32 bits), its first two `o` lines and its
+// first model-creating one (kNone: none).
+struct LineBlocks {
+    unsigned long long *count;
+    uint32_t *o1, *o2, *need;
 };
 
 // Per line: its class.  One block per kLineBlock lines, their text staged in shared memory.
-__global__ void __launch_bounds__(kLineBlock) k_lines(const uint8_t *__restrict__ text, uint64_t n,
+__global__ void __launch_bounds__(kLineBlock, 8) k_lines(const uint8_t *__restrict__ text, uint64_t n,
                                                       const uint32_t *__restrict__ line_start, uint32_t cap,
                                                       uint8_t *__restrict__ type, uint32_t *__restrict__ fans,
-                                                      LineBlock *__restrict__ blocks, ObjCtl *__restrict__ ctl) {
+                                                      LineBlocks blocks, ObjCtl *__restrict__ ctl) {
     __shared__ __align__(16) uint8_t win[kWindow];
     __shared__ unsigned long long s_count[kLineBlock / 32];
     __shared__ uint32_t s_o[kLineBlock / 32], s_need[kLineBlock / 32];
     chain_wait();
     const uint32_t L = ctl->newlines + 1u, l0 = blockIdx.x * kLineBlock, l = l0 + threadIdx.x;
     if (L > cap || l0 >= L) return;  // more lines than there is room for: the caller comes again
-    uint64_t w0, w1;
-    stage_lines(text, n, line_start, L, l0, min((uint32_t)kLineBlock, L - l0), win, w0, w1);
+    const LineText lt(line_start, L, l0, n);
+    lt.stage(text, n, win);
     LineClass c{LT_NONE, false, 0};
     if (l < L) {
-        uint64_t p, q;
-        line_bytes(n, line_start, L, l, p, q);
-        const uint32_t len = (uint32_t)(q - p);
-        if (p >= w0 && q < w1) {  // its newline too
-            if (!fast_class(win + (p - w0), len, c)) c = classify(win + (p - w0), len);
+        if (lt.whole()) {
+            if (!fast_class(win + (lt.p - lt.w0), c)) c = classify(win + (lt.p - lt.w0), lt.len());
         } else {
-            c = classify(text + p, len);
+            c = classify(text + lt.p, lt.len());
         }
         type[l] = c.type;
         fans[l] = c.fan;
@@ -645,18 +665,22 @@ __global__ void __launch_bounds__(kLineBlock) k_lines(const uint8_t *__restrict_
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        LineBlock r{0ull, kNone, kNone, kNone, 0u};
+        unsigned long long count = 0;
+        uint32_t o1 = kNone, o2 = kNone, first_need = kNone;
         for (int w = kLineBlock / 32 - 1; w >= 0; --w) {
-            r.count += s_count[w];
+            count += s_count[w];
             const uint32_t at = l0 + 32 * w, o = s_o[w];
-            if (s_need[w]) r.need = at + __ffs(s_need[w]) - 1;
+            if (s_need[w]) first_need = at + __ffs(s_need[w]) - 1;
             if (o) {
                 const uint32_t rest = o & (o - 1);
-                r.o2 = rest ? at + __ffs(rest) - 1 : r.o1;
-                r.o1 = at + __ffs(o) - 1;
+                o2 = rest ? at + __ffs(rest) - 1 : o1;
+                o1 = at + __ffs(o) - 1;
             }
         }
-        blocks[blockIdx.x] = r;
+        blocks.count[blockIdx.x] = count;
+        blocks.o1[blockIdx.x] = o1;
+        blocks.o2[blockIdx.x] = o2;
+        blocks.need[blockIdx.x] = first_need;
     }
 }
 
@@ -667,9 +691,9 @@ __device__ __forceinline__ unsigned long long line_count(uint8_t t, uint32_t fan
 
 // Model 0's lines [a, b): the default model when a model-creating statement precedes the first `o`
 // (_currentModel, obj-file-parser.js:82-91), else the model that `o` opens, up to the next `o`.
-// Then pre[block]: the packed counts of model 0's lines before the block.  One block of threads,
-// each over a run of consecutive line blocks; a line block that a or b cuts is counted line by line.
-__global__ void __launch_bounds__(1024) k_model(const LineBlock *__restrict__ blocks, const uint8_t *__restrict__ type,
+// Then pre[block]: the packed counts of model 0's lines before the block.  One block of threads;
+// a line block that a or b cuts is counted line by line.
+__global__ void __launch_bounds__(1024) k_model(LineBlocks blocks, const uint8_t *__restrict__ type,
                                                 const uint32_t *__restrict__ fans, uint32_t cap,
                                                 unsigned long long *__restrict__ pre, ObjCtl *__restrict__ ctl) {
     __shared__ uint32_t s_min[3][32];
@@ -677,8 +701,7 @@ __global__ void __launch_bounds__(1024) k_model(const LineBlock *__restrict__ bl
     chain_wait();
     const uint32_t L = ctl->newlines + 1u;
     if (L > cap) return;
-    const uint32_t nb = (L + (kLineBlock - 1)) / kLineBlock, per = (nb + 1023u) / 1024u;
-    const uint32_t b0 = min(nb, threadIdx.x * per), b1 = min(nb, b0 + per);
+    const uint32_t nb = (L + (kLineBlock - 1)) / kLineBlock;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     auto block_min = [&](uint32_t v, int slot) {
         v = __reduce_min_sync(0xFFFFFFFFu, v);
@@ -686,15 +709,19 @@ __global__ void __launch_bounds__(1024) k_model(const LineBlock *__restrict__ bl
         __syncthreads();
         return __reduce_min_sync(0xFFFFFFFFu, s_min[slot][lane]);
     };
-    uint32_t o1 = kNone, need = kNone;
-    for (uint32_t i = b0; i < b1; ++i) {
-        o1 = min(o1, blocks[i].o1);
-        need = min(need, blocks[i].need);
+    // a thread's two smallest first-`o` lines and its smallest model-creating line
+    uint32_t o1 = kNone, o2 = kNone, need = kNone;
+#pragma unroll 8
+    for (uint32_t i = threadIdx.x; i < nb; i += 1024) {
+        const uint32_t o = blocks.o1[i];
+        o2 = min(o2, max(o1, o));
+        o1 = min(o1, o);
+        need = min(need, blocks.need[i]);
     }
     const uint32_t fo = block_min(o1, 0), fn = block_min(need, 1);
-    uint32_t o2 = kNone;
-    for (uint32_t i = b0; i < b1; ++i) o2 = min(o2, blocks[i].o1 == fo ? blocks[i].o2 : blocks[i].o1);
-    const uint32_t so = block_min(o2, 2);
+    uint32_t so = o1 == fo ? o2 : o1;
+    if (threadIdx.x == 0 && fo != kNone) so = min(so, blocks.o2[fo / kLineBlock]);
+    so = block_min(so, 2);
     uint32_t a = 0, b = 0, none = 0;
     if (fn != kNone && (fo == kNone || fn < fo)) {
         b = fo == kNone ? L : fo;
@@ -706,24 +733,82 @@ __global__ void __launch_bounds__(1024) k_model(const LineBlock *__restrict__ bl
     }
     // the line blocks that a and b lie in (the same one, or a is at its block's start, at times)
     const uint32_t ba = a / kLineBlock, bb = b / kLineBlock;
-    auto cut = [&](uint32_t blk) {  // model 0's lines of one block
-        const uint32_t l = blk * kLineBlock + threadIdx.x;
-        unsigned long long c = 0;
-        if (threadIdx.x < kLineBlock && l >= a && l < b) c = line_count(type[l], fans[l]);
-        unsigned long long all;
-        block_scan<unsigned long long>(c, s_warp, &all);
-        return all;
-    };
-    const unsigned long long ca = cut(ba), cb = cut(bb);
-    auto count = [&](uint32_t i) {
-        return i < ba || i > bb ? 0ull : i == ba ? ca : i == bb ? cb : blocks[i].count;
-    };
-    unsigned long long sum = 0, all;
-    for (uint32_t i = b0; i < b1; ++i) sum += count(i);
-    unsigned long long run = block_scan<unsigned long long>(sum, s_warp, &all);
-    for (uint32_t i = b0; i < b1; ++i) {
-        pre[i] = run;
-        run += count(i);
+    // threads 0 .. 255 count block ba's lines of model 0, threads 256 .. 511 block bb's
+    const uint32_t half = threadIdx.x / kLineBlock, l = (half ? bb : ba) * kLineBlock + threadIdx.x % kLineBlock;
+    unsigned long long c = 0, ca = 0, cb = 0;
+    if (half < 2 && l >= a && l < b) c = line_count(type[l], fans[l]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
+    if (lane == 0) s_warp[warp] = c;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kLineBlock / 32; ++w) {
+        ca += s_warp[w];
+        cb += s_warp[kLineBlock / 32 + w];
+    }
+    __syncthreads();
+    // a warp's 512 line blocks in four rows of 128, four consecutive ones per lane (whole lines per
+    // access: with 16 consecutive ones per thread the one SM's requests took 16 us of the kernel's
+    // 21 for 12,300 line blocks)
+    constexpr int kRows = 4;
+    unsigned long long all = 0;
+    for (uint32_t base = 0; base < nb; base += 1024u * 4 * kRows) {
+        unsigned long long x[kRows][4], run[kRows], sum = 0;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            const uint32_t i = base + (warp * kRows + r) * 128u + 4u * lane;
+#pragma unroll
+            for (int k = 0; k < 4; k += 2) {
+                ulonglong2 v = make_ulonglong2(0ull, 0ull);
+                if (i + k + 1 < nb) v = *reinterpret_cast<const ulonglong2 *>(blocks.count + i + k);
+                else if (i + k < nb) v.x = blocks.count[i + k];
+                x[r][k] = v.x;
+                x[r][k + 1] = v.y;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            unsigned long long four = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t i = base + (warp * kRows + r) * 128u + 4u * lane + k;
+                if (i < ba || i > bb) x[r][k] = 0ull;
+                if (i == bb) x[r][k] = cb;
+                if (i == ba) x[r][k] = ca;
+                four += x[r][k];
+            }
+            unsigned long long incl = four;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            run[r] = sum + incl - four;  // before this lane's four, within the warp
+            sum += __shfl_sync(0xFFFFFFFFu, incl, 31);
+        }
+        if (lane == 0) s_warp[warp] = sum;
+        __syncthreads();
+        unsigned long long off = all;
+        for (int w = 0; w < 32; ++w) {
+            off += w < warp ? s_warp[w] : 0ull;
+            all += s_warp[w];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            const uint32_t i = base + (warp * kRows + r) * 128u + 4u * lane;
+            unsigned long long p4[4], c4 = off + run[r];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                p4[k] = c4;
+                c4 += x[r][k];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k += 2) {
+                if (i + k + 1 < nb) *reinterpret_cast<ulonglong2 *>(pre + i + k) = make_ulonglong2(p4[k], p4[k + 1]);
+                else if (i + k < nb) pre[i + k] = p4[k];
+            }
+        }
     }
     if (threadIdx.x == 0) {
         ctl->m0a = a;
@@ -773,22 +858,22 @@ __device__ __forceinline__ bool fast_vertex(const uint8_t *b, double (&out)[3]) 
         while (c == ' ') c = b[++i];
         const bool neg = c == '-';
         if (neg) c = b[++i];
-        uint32_t m = 0, nd = 0, k = 0, d;
-        while ((d = c - '0') <= 9u && nd < 10) {
+        uint32_t m = 0, d, at = i;  // (m wraps past nine digits: not used then)
+        while ((d = c - '0') <= 9u) {
             m = m * 10 + d;
-            ++nd;
             c = b[++i];
         }
+        uint32_t nd = i - at, k = 0;
         if (c == '.') {
-            c = b[++i];
-            while ((d = c - '0') <= 9u && nd < 10) {
+            c = b[at = ++i];
+            while ((d = c - '0') <= 9u) {
                 m = m * 10 + d;
-                ++nd;
-                ++k;
                 c = b[++i];
             }
+            k = i - at;
+            nd += k;
         }
-        if (nd == 0 || nd > 9 || (c != ' ' && c != '\n' && c != '\r')) return false;
+        if (nd - 1u > 8u || (c != ' ' && c != '\n' && c != '\r')) return false;
         const double v = k ? __ddiv_rn((double)m, kPow10[k]) : (double)m;
         out[a] = neg ? -v : v;
     }
@@ -815,7 +900,7 @@ struct Verts {
 // Model-0 vertex lines -> doubles and soup rows at their rank; numbers outside the device's
 // exact range are listed for the host.  Block i has the lines of line block blk0 + i, its text
 // staged when it holds a vertex line of model 0's lines [a, b).
-__global__ void __launch_bounds__(kLineBlock) k_vertices(const uint8_t *__restrict__ text, uint64_t n,
+__global__ void __launch_bounds__(kLineBlock, 8) k_vertices(const uint8_t *__restrict__ text, uint64_t n,
                                                          const uint32_t *__restrict__ line_start, uint32_t L,
                                                          const uint8_t *__restrict__ type, uint32_t blk0, uint32_t a,
                                                          uint32_t b, const unsigned long long *__restrict__ pre,
@@ -824,28 +909,27 @@ __global__ void __launch_bounds__(kLineBlock) k_vertices(const uint8_t *__restri
     __shared__ __align__(16) uint8_t win[kWindow];
     __shared__ uint32_t s_v[kLineBlock / 32];
     const uint32_t blk = blk0 + blockIdx.x, l0 = blk * kLineBlock, l = l0 + threadIdx.x;
+    const LineText lt(line_start, L, l0, n);
+    uint32_t vi = (uint32_t)pre[blk];
     const bool mine = l >= a && l < b && type[l] == LT_V;
     const uint32_t bal = __ballot_sync(0xFFFFFFFFu, mine);
     if ((threadIdx.x & 31) == 0) s_v[threadIdx.x >> 5] = __popc(bal);
     if (!__syncthreads_or(mine)) return;
-    uint32_t vi = (uint32_t)pre[blk] + __popc(bal & lanemask_lt());
-    for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) vi += s_v[w];
-    uint64_t w0, w1;
-    stage_lines(text, n, line_start, L, l0, min((uint32_t)kLineBlock, L - l0), win, w0, w1);
+    lt.stage(text, n, win);
     if (!mine) return;
-    uint64_t p, q;
-    line_bytes(n, line_start, L, l, p, q);
+    vi += __popc(bal & lanemask_lt());
+    for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) vi += s_v[w];
     double c[3];
-    if (!(p >= w0 && q < w1 && fast_vertex(win + (p - w0), c))) {
+    if (!(lt.whole() && fast_vertex(win + (lt.p - lt.w0), c))) {
         VertexParse r;
-        if (p >= w0 && q <= w1) r = parse_vertex(win + (p - w0), (uint32_t)(q - p));
-        else r = parse_vertex(text + p, (uint32_t)(q - p));
+        if (lt.body()) r = parse_vertex(win + (lt.p - lt.w0), lt.len());
+        else r = parse_vertex(text + lt.p, lt.len());
         c[0] = r.x;
         c[1] = r.y;
         c[2] = r.z;
         if (!r.ok) {
             const uint32_t h = atomicAdd(&ctl->num_hard, 1u);
-            hard[h] = HardLine{p, p + r.end, vi, 0u, 0u, 0u};
+            hard[h] = HardLine{lt.p, (unsigned long long)lt.p + r.end, vi, 0u, 0u, 0u};
         }
     }
     vs.xyz[3ull * vi] = c[0];
@@ -922,13 +1006,11 @@ __device__ __forceinline__ bool fast_face(const uint8_t *b, uint32_t nverts, con
         while (c == ' ') c = b[++i];
         if (c == '\n') break;
         if (c == '\r' && b[i + 1] == '\n') break;
-        uint32_t v = c - '0', d, nd = 1;
+        uint32_t v = c - '0', d;
+        const uint32_t at = i;
         if (v - 1u > 8u) return true;
-        while ((d = (c = b[++i]) - '0') <= 9u && nd < 10) {
-            v = v * 10 + d;
-            ++nd;
-        }
-        if (nd > 9) return true;
+        while ((d = (c = b[++i]) - '0') <= 9u) v = v * 10 + d;
+        if (i - at > 9) return true;  // v may have wrapped
         if (c == '/') {
             do c = b[++i];
             while (c > ' ' && c < 0x80 && c != '#');
@@ -945,7 +1027,7 @@ __device__ __forceinline__ bool fast_face(const uint8_t *b, uint32_t nverts, con
 
 // Model-0 faces -> fan triangles (y and z swapped, float32, pad 3.1415), their vertices marked.
 // Blocks as k_vertices.
-__global__ void __launch_bounds__(kLineBlock) k_faces(const uint8_t *__restrict__ text, uint64_t n,
+__global__ void __launch_bounds__(kLineBlock, 8) k_faces(const uint8_t *__restrict__ text, uint64_t n,
                                                       const uint32_t *__restrict__ line_start, uint32_t L,
                                                       const uint8_t *__restrict__ type,
                                                       const uint32_t *__restrict__ fans, uint32_t blk0, uint32_t a,
@@ -953,26 +1035,29 @@ __global__ void __launch_bounds__(kLineBlock) k_faces(const uint8_t *__restrict_
                                                       uint32_t nverts, Verts vs, float4 *__restrict__ tri,
                                                       ObjCtl *__restrict__ ctl) {
     __shared__ __align__(16) uint8_t win[kWindow];
-    __shared__ unsigned long long s_warp[kLineBlock / 32];
+    __shared__ uint32_t s_warp[kLineBlock / 32], s_v[kLineBlock / 32];
     const uint32_t blk = blk0 + blockIdx.x, l0 = blk * kLineBlock, l = l0 + threadIdx.x;
+    const LineText lt(line_start, L, l0, n);
+    const unsigned long long first = pre[blk];
     const bool in = l >= a && l < b;
     const uint8_t ty = in ? type[l] : (uint8_t)LT_NONE;
+    const uint32_t fan = in ? fans[l] : 0u;
     const bool mine = ty == LT_F;
+    const uint32_t vbal = __ballot_sync(0xFFFFFFFFu, ty == LT_V);
+    if ((threadIdx.x & 31) == 0) s_v[threadIdx.x >> 5] = __popc(vbal);
     if (!__syncthreads_or(mine)) return;
-    const unsigned long long at = pre[blk] + block_scan<unsigned long long>(line_count(ty, mine ? fans[l] : 0u), s_warp, nullptr);
-    uint64_t w0, w1;
-    stage_lines(text, n, line_start, L, l0, min((uint32_t)kLineBlock, L - l0), win, w0, w1);
+    const uint32_t at = (uint32_t)(first >> 32) + block_scan<uint32_t>(mine ? fan : 0u, s_warp, nullptr);
+    lt.stage(text, n, win);
     chain_wait();  // the vertices
     if (!mine) return;
-    uint64_t p, q;
-    line_bytes(n, line_start, L, l, p, q);
-    float4 *out = tri + 3ull * (at >> 32);
-    const long long before = (long long)(at & 0xFFFFFFFFull);  // model-0 vertices so far
+    float4 *out = tri + 3ull * at;
     bool ok = true, done = false;
-    if (p >= w0 && q < w1) ok = fast_face(win + (p - w0), nverts, vs, out, done);
+    if (lt.whole()) ok = fast_face(win + (lt.p - lt.w0), nverts, vs, out, done);
     if (!done) {
-        if (p >= w0 && q <= w1) ok = emit_face(win + (p - w0), (uint32_t)(q - p), before, nverts, vs, out);
-        else ok = emit_face(text + p, (uint32_t)(q - p), before, nverts, vs, out);
+        uint32_t before = (uint32_t)first + __popc(vbal & lanemask_lt());  // model-0 vertices so far
+        for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) before += s_v[w];
+        if (lt.body()) ok = emit_face(win + (lt.p - lt.w0), lt.len(), before, nverts, vs, out);
+        else ok = emit_face(text + lt.p, lt.len(), before, nverts, vs, out);
     }
     if (!ok) atomicOr(&ctl->bad_index, 1u);
 }
@@ -989,9 +1074,10 @@ __global__ void __launch_bounds__(kT) k_bounds_floor(Verts vs, uint32_t nverts, 
     unsigned long long mn[3] = {~0ull, ~0ull, ~0ull}, mx[3] = {0ull, 0ull, 0ull};
     bool nan[3] = {false, false, false};
     for (uint32_t v = blockIdx.x * kT + threadIdx.x; v < nverts; v += gridDim.x * kT) {
-        if (!vs.used[v]) continue;
+        const bool used = vs.used[v] != 0;  // (read with the coordinates: one wait)
         const double *p = vs.xyz + 3ull * v;
         const double c[3] = {p[0], p[2], p[1]};
+        if (!used) continue;
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
             if (isnan(c[ax])) {
@@ -1027,8 +1113,9 @@ __global__ void __launch_bounds__(kT) k_bounds_floor(Verts vs, uint32_t nverts, 
             hi = s_mx[ax][w] > hi ? s_mx[ax][w] : hi;
             nan_any |= s_nan[ax][w];
         }
-        if (lo != ~0ull) atomicMin(&ctl->bmin[ax], lo);
-        if (hi != 0ull) atomicMax(&ctl->bmax[ax], hi);
+        // (few blocks still move the words that all of them would queue on)
+        if (lo != ~0ull && lo < *(volatile unsigned long long *)&ctl->bmin[ax]) atomicMin(&ctl->bmin[ax], lo);
+        if (hi != 0ull && hi > *(volatile unsigned long long *)&ctl->bmax[ax]) atomicMax(&ctl->bmax[ax], hi);
         if (nan_any) {
             atomicOr(&ctl->nan_min[ax], 1u);
             atomicOr(&ctl->nan_max[ax], 1u);
@@ -1158,15 +1245,18 @@ int obj_scan(ObjScratch &sc, const char *text, uint64_t bytes, bool host_text, u
     for (;;) {
         const uint32_t nb = cap / kLineBlock + 1;
         const size_t starts = align256((cap + 1ull) * 4), types = align256(cap), fan_part = align256(cap * 4ull);
-        const size_t blk_part = align256(nb * sizeof(LineBlock));
-        OBJ_CUDA(grow(sc.lines, sc.lines_bytes, starts + types + fan_part + blk_part + align256(nb * 8ull)),
+        const size_t b8 = align256(nb * 8ull), b4 = align256(nb * 4ull);
+        OBJ_CUDA(grow(sc.lines, sc.lines_bytes, starts + types + fan_part + 2 * b8 + 3 * b4),
                  "cudaMalloc(obj lines)");
         char *cl = static_cast<char *>(sc.lines);
         sc.line_start = reinterpret_cast<uint32_t *>(cl);
         sc.type = reinterpret_cast<uint8_t *>(cl + starts);
         sc.fans = reinterpret_cast<uint32_t *>(cl + starts + types);
-        LineBlock *blocks = reinterpret_cast<LineBlock *>(cl + starts + types + fan_part);
-        sc.pre = reinterpret_cast<unsigned long long *>(cl + starts + types + fan_part + blk_part);
+        cl += starts + types + fan_part;
+        sc.pre = reinterpret_cast<unsigned long long *>(cl);
+        const LineBlocks blocks{reinterpret_cast<unsigned long long *>(cl + b8), reinterpret_cast<uint32_t *>(cl + 2 * b8),
+                                reinterpret_cast<uint32_t *>(cl + 2 * b8 + b4),
+                                reinterpret_cast<uint32_t *>(cl + 2 * b8 + 2 * b4)};
         launch_chained(true, k_nl_write, chunks, kT, 0, s, d_text, bytes, cnt, cap, sc.line_start);
         launch_chained(true, k_lines, (cap + kLineBlock - 1) / kLineBlock, kLineBlock, 0, s, d_text, bytes, sc.line_start,
                        cap, sc.type, sc.fans, blocks, ctl);
@@ -1226,7 +1316,7 @@ int obj_emit(ObjScratch &sc, float *dst, const float **tri_out, double *bounds6,
         if (nfan)
             launch_chained(chain && nverts, k_faces, nblk, kLineBlock, 0, s, d_text, bytes, sc.line_start, L, sc.type, sc.fans,
                            blk0, a, b, sc.pre, nverts, vs, tri, ctl);
-        const uint32_t want = (nverts + kT - 1) / kT, most = (uint32_t)sm_count() * 4u;
+        const uint32_t want = (nverts + kT - 1) / kT, most = (uint32_t)sm_count() * 8u;
         const uint32_t grid = want < 1 ? 1 : want < most ? want : most;
         launch_chained(true, k_bounds_floor, grid, kT, 0, s, vs, nverts, tri + 3ull * nfan, ctl);
     };
