@@ -12,29 +12,23 @@
 // s with a smaller d.  A node [L, R] is the LEFT child of split R when d[R] > d[L-1], else the
 // RIGHT child of split L-1 (adjacent d values always differ), so its Karras index is R or L
 // (0 for the root) - exactly the numbering compute_child_index produces - and its parent
-// follows from its own range alone.  The tree is therefore built bottom-up with the boxes:
-// every leaf climbs; at each split the first child to arrive parks, the second merges both
-// into the parent's record and climbs on.  No per-node binary search, N-1 box unions.
+// follows from its own range alone; its parent is the node of the larger of the two separators
+// around it.  So every node is found on its own thread from the separators, with its box as the
+// union of a range of leaves: no per-node binary search and no climb from child to parent.
 //
 // Passes.
 //   K3b (k_tree_climb)   blocks of 256 sorted leaves in shared memory, a persistent grid that
 //                        prefetches the next blocks: leaf k's triangle perm[k] arrives with
 //                        three others by one TMA gather of four 48-byte rows, goes to the
-//                        output soup at k and is reduced to its
-//                        box (exact-zero components nudged by 1e-8 as bvh-up-pass.js:209-210
-//                        does).  The climb runs in steps:
-//                        the items still climbing after a step are compacted into a queue, so
-//                        warps stay full while the number of items shrinks.  Parking and
-//                        merging use an arrival mask per split (shared-memory atomics) and
-//                        parked items in shared memory; records go straight to the node
-//                        buffer, parent links are staged and written coalesced.  An item
-//                        whose parent split lies outside the block, or whose sibling never
-//                        arrives (the parent straddles the block boundary), leaves as an
-//                        "open item" (at most 2 x 64 per block: they hang off the two boundary
-//                        paths of a tree at most 64 deep).
+//                        output soup at k and is reduced to its box (exact-zero components
+//                        nudged by 1e-8 as bvh-up-pass.js:209-210 does).  Then the nodes that lie
+//                        in the block, one thread each.  A subtree whose parent crosses the
+//                        block's edge leaves as an "open item" (at most 2 x 64 per block: they
+//                        hang off the two boundary paths of a tree at most 64 deep).
 //   K3c (k_top_group)    the nodes that straddle blocks (~3 % of them), from the open items: per
 //                        group of blocks in shared memory, each node on its own thread, then per
 //                        group of groups, up to the root (see below).
+#include <cstddef>
 #include <cstring>
 #include <cuda.h>  // CUtensorMap
 #include <cudaTypedefs.h>
@@ -53,19 +47,7 @@ template <int LOG>
 struct TreeGeo {
     static constexpr int EB = 1 << LOG;
     static constexpr int kCtasPerSm = LOG == 8 ? 4 : 8;
-    static_assert(2 * LOG + 14 <= 32, "packed item ranges");
-    // packed local range and end separators of a climbing item:
-    // l | r << LOG | (d[l-1] + 1) << 2 LOG | (d[r] + 1) << 2 LOG + 7   (d + 1 <= 64)
-    static __device__ __forceinline__ uint32_t pack(int l, int r, int dl, int dr) {
-        return (uint32_t)l | ((uint32_t)r << LOG) | ((uint32_t)(dl + 1) << (2 * LOG)) |
-               ((uint32_t)(dr + 1) << (2 * LOG + 7));
-    }
-    static __device__ __forceinline__ int rl(uint32_t p) { return (int)(p & (EB - 1)); }
-    static __device__ __forceinline__ int rr(uint32_t p) { return (int)((p >> LOG) & (EB - 1)); }
-    static __device__ __forceinline__ int rdl(uint32_t p) { return (int)((p >> (2 * LOG)) & 127u) - 1; }
-    static __device__ __forceinline__ int rdr(uint32_t p) { return (int)(p >> (2 * LOG + 7)) - 1; }
 };
-constexpr int kFreeClimb = 64;                 // K3b items left when compaction stops
 
 // Where a block of EB sorted leaves lives.  A batched build is a list of segments (meshes)
 // laid end to end; every block lies inside one segment and every index a kernel works with
@@ -82,7 +64,6 @@ struct OneSeg {
     int n;
     __device__ __forceinline__ int blocks() const { return (n + EB - 1) / EB; }
     __device__ __forceinline__ Span span(int blk) const { return Span{0, n, blk * EB}; }
-    __device__ __forceinline__ size_t item_base(int blk, int cap) const { return (size_t)blk * cap; }
 };
 
 template <int LOG>
@@ -98,11 +79,8 @@ struct ManySegs {
         const int first = (int)__ldg(&rows[sg].blk);
         return Span{t0, (int)(t1 - t0), (blk - first) * EB};
     }
-    __device__ __forceinline__ size_t item_base(int blk, int cap) const { return (size_t)blk * cap; }
 };
 
-// K3b shared memory.  A climbing item is two float4: box min + link (node index, or
-// -(leaf + 1)), box max + its packed local range and end separators (TreeGeo::pack).
 // Where the tree pass gets its leaves.  SoupLeaves: leaf t of a block is triangle perm[b0 + t]
 // of the 48-byte soup, copied to the output soup.  MeshLeaves (the indexed leaf format): leaf t
 // is the sorted triangle b0 + t, whose three vertex indices are already in sorted order
@@ -121,37 +99,54 @@ struct MeshLeaves {
     uint32_t nverts;
 };
 
-// The gathered triangles of this block and the next: buffer b holds leaves 4g .. 4g + 3 in
-// slot[b][g], four 48-byte rows (float4 0..11, one tensor gather each) in a 256-byte slot, so
-// that every gather's destination starts on a 128-byte boundary.  The slots' last 64 bytes
-// (float4 12..15), which no copy writes, hold the step queues: [queue][min/max][item] of the
-// items of the current and the next step (a step after the first has at most EB / 2: every
-// merge takes two items), entry f = (queue * 2 + min/max) * EB / 2 + item at flat slot f / 4,
-// float4 12 + f % 4.
-template <int EB, int PROW>
-struct ClimbSmem {
-    float4 slot[2][EB / 4][16];
-    float4 pend[2][2][EB];  // [side][min/max][split] the child parked at each split.  Split
-                            // index innermost keeps the 16-byte accesses of random splits off
-                            // each other's banks.
-    uint32_t key[EB + 2];   // keys of leaves b0-1 .. b0+EB
-    uint32_t mask[EB];      // arrivals at each split: bit 0 left child, bit 1 right child
-    int par[2 * EB];        // parent of internal node b0 + j at j, of leaf b0 + j at EB + j
-                            // (-1 = not set here)
-    uint32_t prow[PROW];    // soup, one segment: the rows of the block two ahead, staged for its gathers
-    Span sp2[2];            // soup: the span of the block two ahead of an iteration on buffer b
-    int cnt[3];             // item counters, rotating over the steps
-    int open[2];            // open items emitted, by buffer parity (a block's and the next's)
-    uint64_t bar[2];        // completion of the gathers into slot[0] / slot[1]
+// K3b shared memory.
+//
+// slot: the gathered triangles of this block and the next: buffer b holds leaves 4g .. 4g + 3 in
+// slot[b][g], four 48-byte rows (float4 0..11, one tensor gather each) in a 256-byte slot, so that
+// every gather's destination starts on a 128-byte boundary.  Once a block's rows are read, its
+// buffer holds the block's boxes of 16 leaves, until the copies of the block two ahead go there.
+// pool: the boxes of 1 and of 4 leaves from each leaf on ([0 .. EB) and [EB .. 2 EB) mins and maxes
+// of one, then of four); when every node has its box, the records: node of separator j at
+// [4 j .. 4 j + 3], each record's four words rotated (rec_at) so that the scattered writes of its
+// two halves spread over the banks.
+// key, perm: the keys of this block's leaves and the next's, the permutation entries (mesh: the
+// vertex indices) of the leaves two and three blocks ahead, all by 4-byte cp.async: held in registers
+// from one block to the next they spilled, and a spilled load waits for its value at once.
+template <int EB, bool MESH>
+struct TreeSmem {
+    static constexpr int kRow = MESH ? 3 : 4;      // float4 per leaf in a slot
+    static constexpr int kIdx = MESH ? 3 : 1;      // index words per leaf
+    float4 slot[2][EB * kRow];
+    float4 pool[4 * EB];
+    __align__(16) uint32_t plane[EB / 32][8];  // (16-byte loads) bit b of the separators before leaves
+                                               // 32 w .. 32 w + 31, at [w][b]
+    uint32_t key[2][EB + 2];      // keys of leaves b0-1 .. b0+EB, by buffer parity
+    uint32_t perm[2][kIdx * EB];  // as above: two blocks ahead of a block on buffer b at [b]
+    int P[EB];                    // separator j's node: its index less b0 (-1: not in this block)
+    Span ring[8];                 // spans of this CTA's blocks it .. it + 4 at [it % 8], several segments
+    uint64_t bar[2];              // completion of the gathers into slot[0] / slot[1]
+    uint8_t wmin[EB / 32];        // smallest separator of each warp's
+    uint8_t sep[EB + 1];          // separators (before each leaf and after the last; -1 as 0)
+    int open[2];                  // open items emitted, by buffer parity (a block's and the next's)
+    static __device__ __forceinline__ int rec_at(int j, int part) { return 4 * j + (part ^ ((j >> 1) & 3)); }
 };
 
-// Whether a tree pass issues its soup gathers late (see issue_next in k_tree_climb) and its
-// shared-memory layout.
-template <int LOG, class Segs, class Leaves>
-struct TreeLayout {
-    static constexpr bool kLate = !Leaves::kMesh && std::is_same<Segs, OneSeg<LOG>>::value;
-    using Smem = ClimbSmem<(1 << LOG), kLate ? (1 << LOG) : 1>;
-};
+// The lanes whose 6-bit value, given bit by bit in planes, is below v.
+__device__ __forceinline__ uint32_t lanes_below(const uint32_t (&plane)[6], uint32_t v) {
+    uint32_t lt = 0, eq = 0xFFFFFFFFu;
+#pragma unroll
+    for (int b = 5; b >= 0; --b) {
+        const uint32_t m = (uint32_t)((int32_t)(v << (31 - b)) >> 31);  // all ones when v has bit b
+        lt |= eq & m & ~plane[b];
+        eq &= ~(plane[b] ^ m);
+    }
+    return lt;
+}
+
+__device__ __forceinline__ void box_join(float4 &lo, float4 &hi, const float4 &l, const float4 &h) {
+    lo.x = fminf(lo.x, l.x); lo.y = fminf(lo.y, l.y); lo.z = fminf(lo.z, l.z);
+    hi.x = fmaxf(hi.x, h.x); hi.y = fmaxf(hi.y, h.y); hi.z = fmaxf(hi.z, h.z);
+}
 
 // K3b: leaf gather, rearrange and the tree over blocks of EB sorted leaves (see the pass list
 // above).  Leaf t of a block gathers triangle perm[b0 + t]: its index is loaded three blocks
@@ -160,6 +155,25 @@ struct TreeLayout {
 // rows, completing on the buffer's mbarrier; no registers held meanwhile), then written to the
 // output soup and reduced to the leaf box.  A mesh leaf's three 16-byte vertex rows (mostly L2
 // hits) come by cp.async instead (soup_map unused).
+//
+// Separator j of the block (the split before leaf j, j >= 1) has its node on thread j.  The node
+// covers leaves a .. b - 1 between the nearest smaller separators on either side; its parent is
+// the node of the larger of those two, its index follows from its range, its box is the union of
+// its leaves.  The nearest smaller separators come from bit planes (six ballots per warp: the
+// lanes below a value are a few bit operations on them; the warp to look in from the warps'
+// minima), the box from windows of 1, 4 and 16 leaves made by shuffles.  Node and leaf then hand
+// box and link to their parent's record in shared memory, and each record goes out by four
+// neighbouring threads.  A node with no smaller separator on one side within the block lies across
+// its edge; what hangs below such nodes leaves as open items.
+//
+// What bounds it: shared-memory wavefronts (65 % of the LSU pipe), four block barriers a block
+// and DRAM (220 B per triangle at 2^24, 50 %); issue slots are half used.  Before, every leaf
+// climbed: the first child at a split parked, the second merged and went on, step by step with
+// block barriers and then in dependent chains (13,000 cycles of a block's 19,000).  The pass,
+// climb -> this (B200): 2^24 clustered triangles 847 -> 803 us, 1,000,003 59 -> 53, the 2 M mesh
+// 118 -> 94, a 1,024-mesh batch of 33 M triangles 1,806 -> 1,476.  On the way there: prefetched
+// keys and indices in registers (spilled) 1,045 us at 2^24; windows of 4 and 16 leaves from
+// shared memory with a barrier each 829; both spilled in a batch 1,931.
 template <int LOG, class Segs, class Leaves = SoupLeaves>
 __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_tree_climb(Segs segs,
                                                     const uint32_t *__restrict__ keys_all,
@@ -167,126 +181,106 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
                                                     float4 *nodes_all, int32_t *parents_all,
                                                     OpenItem *out_items, uint32_t *out_counts,
                                                     Control *ctl, const __grid_constant__ CUtensorMap soup_map) {
-    using G = TreeGeo<LOG>;
-    constexpr int EB = G::EB;
-    constexpr int kFree = kFreeClimb < EB / 2 ? kFreeClimb : EB / 2;  // the free climb leaves threads
-                                                                     // EB / 2 .. 3 EB / 4 - 1 idle
-    // the soup gathers of a one-segment build issued late, by threads the free climb leaves idle
-    // (a batch keeps them in the refill: its extra state spilled there, 13.6 -> 14.1 ms a batch)
-    using Layout = TreeLayout<LOG, Segs, Leaves>;
-    constexpr bool kLate = Layout::kLate;
+    constexpr int EB = TreeGeo<LOG>::EB, W = EB / 32;
+    constexpr bool kOne = std::is_same<Segs, OneSeg<LOG>>::value;
+    // When a block's buffer is refilled: beside the hand-over, by two warps (one soup: its scattered
+    // rows come late enough as it is, 2^24 triangles 803 us against 842-867 at the end), or at the
+    // end, by every warp (meshes of a batch and mesh leaves, whose rows mostly hit L2: the copies'
+    // queueing holds up no barrier, a 33 M triangle batch 1,573 -> 1,475 us, the 2 M mesh 96 -> 94)
+    constexpr bool kLate = !kOne || Leaves::kMesh;
+    using Smem = TreeSmem<EB, Leaves::kMesh>;
+    static_assert(offsetof(Smem, plane) % 16 == 0 && offsetof(Smem, pool) % 16 == 0 && offsetof(Smem, bar) % 8 == 0, "aligned loads");
     extern __shared__ __align__(16) unsigned char smem[];
     // the layout from the first 128-byte boundary (the launch adds 128 bytes of slack)
-    typename Layout::Smem &S =
-        *reinterpret_cast<typename Layout::Smem *>(smem + ((128u - (smem_addr(smem) & 127u)) & 127u));
-    // leaf t's three rows in buffer b; entry f of the step queues (see ClimbSmem)
-    auto tri_row = [&](int b, int x) -> float4 * { return &S.slot[b][x >> 2][(x & 3) * 3]; };
-    auto qent = [&](int f) -> float4 & { return (&S.slot[0][0][0])[(f >> 2) * 16 + 12 + (f & 3)]; };
-    const int t = threadIdx.x, lane = t & 31;
+    Smem &S = *reinterpret_cast<Smem *>(smem + ((128u - (smem_addr(smem) & 127u)) & 127u));
+    // leaf t's three rows in buffer b
+    auto tri_row = [&](int b, int x) -> float4 * { return &S.slot[b][Leaves::kMesh ? 3 * x : (x >> 2) * 16 + (x & 3) * 3]; };
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     chain_wait();
     // a sort whose look-back gave up left unsorted keys: build nothing from them (uniform)
     if (ld_relaxed_gpu(&ctl->err) & ERR_LOOKBACK_TIMEOUT) return;
     const int nblk = segs.blocks();
     const uint32_t lt = lanemask_lt();
 
-    // Leaves come in three steps ahead of their block: this thread's permutation entry (its three
-    // vertex indices for a mesh) three blocks ahead, its triangle copied into slot[] two blocks
-    // ahead, its key one block ahead.  Two buffers, slot[0] and slot[1], serve the copies two
-    // blocks ahead: a block's buffer is refilled once its own leaf phase has read it (right after
-    // it, or for a one-segment soup during the block's free climb), so the copies of two blocks
-    // are in flight while a block climbs.
-    uint32_t pa = 0, pb = 0, pc = 0;
-    auto fetch_perm = [&](int blk) {
-        const Span sp = segs.span(blk);
-        if (sp.b0 + t < sp.n) {
-            if constexpr (Leaves::kMesh) {
-                const uint32_t *r = lv.sidx + 3ull * (sp.start + sp.b0 + t);
-                pa = __ldg(r);
-                pb = __ldg(r + 1);
-                pc = __ldg(r + 2);
-            } else {
-                pa = __ldg(lv.perm + sp.start + sp.b0 + t);
-            }
+    // Leaves come in three steps ahead of their block: the permutation entry (its three vertex
+    // indices for a mesh) three blocks ahead, its triangle copied into slot[] two blocks ahead, its
+    // key one block ahead.  Two buffers, slot[0] and slot[1], serve the copies two blocks ahead: a
+    // block's buffer is refilled once its boxes are used, so the copies of two blocks are in flight
+    // for most of a block.
+    const int grid = (int)gridDim.x;
+    // the span of this CTA's block `it` (a batch's, loads in a chain, by thread 0 an iteration before
+    // anyone needs it)
+    auto span_of = [&](int it) -> Span {
+        if constexpr (kOne) return segs.span(blockIdx.x + it * grid);
+        else return S.ring[it & 7];
+    };
+    auto find_span = [&](int it) {
+        if constexpr (!kOne)
+            if ((int)blockIdx.x + it * grid < nblk) S.ring[it & 7] = segs.span(blockIdx.x + it * grid);
+    };
+    auto fetch_perm = [&](const Span &sp, int b) {
+        if constexpr (Leaves::kMesh) {
+            const int words = 3 * min(EB, sp.n - sp.b0);
+            const uint32_t *r = lv.sidx + 3ull * (sp.start + sp.b0);
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                if (t + q * EB < words) cp_async4(&S.perm[b][t + q * EB], r + t + q * EB);
+        } else if (sp.b0 + t < sp.n) {
+            cp_async4(&S.perm[b][t], lv.perm + sp.start + sp.b0 + t);
         }
     };
     bool bad_perm = false;
-    // The block's triangles into slot[buf].  Soup: thread 4g issues one tile::gather4 copy of
-    // leaves 4g .. 4g+3 (rows sp.start + perm) on the buffer's mbarrier, whose phase expects 192
-    // bytes per group of four of the block (thread 0's arrival is its only one); a leaf past the
-    // segment in the last group repeats its group's first row (read, never used).  The copy
-    // engine takes about one small copy per 11 to 17 cycles per SM, which one 48-byte copy per
-    // leaf kept saturated; with four rows a copy and the tensor map's 64-byte L2 fills a random
-    // gather of 16.7 M rows takes 0.55 ms against 0.67 (B200; DRAM reads 154 -> 98 B per row).
-    // Mesh: the vertex rows (mostly in L2) by cp.async, one commit group per thread and block.
-    auto fetch_tri = [&](int blk, int buf) {
-        const Span sp = segs.span(blk);
-        const int b0 = sp.b0, n = sp.n, k = b0 + t;
+    // Mesh: the block's vertex rows (mostly in L2) by cp.async, one commit group per thread and block.
+    auto fetch_mesh = [&](const Span &sp, int buf) {
         if constexpr (Leaves::kMesh) {
-            if (k < n) {
+            if (sp.b0 + t < sp.n) {
                 // an index past the vertex buffer was reported by the Morton pass; read row 0
                 const uint32_t nv = lv.nverts;
+                const uint32_t *p = &S.perm[buf][3 * t];
                 float4 *d = tri_row(buf, t);
-                cp_async16(d, lv.verts + (pa < nv ? pa : 0u));
-                cp_async16(d + 1, lv.verts + (pb < nv ? pb : 0u));
-                cp_async16(d + 2, lv.verts + (pc < nv ? pc : 0u));
+#pragma unroll
+                for (int q = 0; q < 3; ++q) cp_async16(d + q, lv.verts + (p[q] < nv ? p[q] : 0u));
             }
             cp_async_commit();
-        } else {
-            if (t == 0) mbar_arrive_tx(&S.bar[buf], 192u * (uint32_t)((min(EB, n - b0) + 3) / 4));
-            uint32_t row = 0;
-            if (k < n) {
-                uint32_t ti = pa;
-                if (ti >= (uint32_t)n) { bad_perm = true; ti = 0; }
-                row = (uint32_t)(sp.start + ti);
-            }
-            const uint32_t r1 = __shfl_down_sync(0xFFFFFFFFu, row, 1), r2 = __shfl_down_sync(0xFFFFFFFFu, row, 2),
-                           r3 = __shfl_down_sync(0xFFFFFFFFu, row, 3);
-            if ((t & 3) == 0 && k < n)
-                gather4_g2s(tri_row(buf, t), &soup_map, row, k + 1 < n ? r1 : row, k + 2 < n ? r2 : row,
-                            k + 3 < n ? r3 : row, &S.bar[buf]);
         }
     };
-    // one block ahead: its span, this thread's key, the keys on either side of the block
-    Span nsp{0, 0, 0};
-    uint32_t nk = 0, nk_lo = 0, nk_hi = 0;
-    auto fetch_keys = [&](int blk) {
-        nsp = segs.span(blk);
-        const uint32_t *keys = keys_all + nsp.start;
-        const int b0 = nsp.b0, n = nsp.n, k = b0 + t;
-        if (k < n) nk = __ldg(keys + k);
-        if (t == 0) nk_lo = b0 > 0 ? __ldg(keys + b0 - 1) : 0u;
-        if (t == EB - 1) nk_hi = (b0 + EB < n) ? __ldg(keys + b0 + EB) : 0u;
-    };
-    const int grid = (int)gridDim.x;
-    // after every thread has read slot[buf] (a barrier between): load the permutation three
-    // ahead and, for mesh leaves, refill the buffer with the block two ahead
-    auto refill = [&](int blk, int buf) {
-        if (blk + 2 * grid >= nblk) return;
-        if constexpr (!kLate) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // reads above, copies below
-            fetch_tri(blk + 2 * grid, buf);
-        }
-        if (blk + 3 * grid < nblk) {
-            fetch_perm(blk + 3 * grid);
-            if (kLate && t == 0) S.sp2[buf ^ 1] = segs.span(blk + 3 * grid);  // the next iteration's
-        }
-    };
-    // Soup: the block two ahead's gathers into slot[buf] (read by now), group g of it (leaves
-    // 4g .. 4g+3, rows staged in prow).  Issued by threads that the free climb leaves idle: the
-    // 64 copies of a block queue on the copy engine for ~2,300 cycles, a stall that delayed the
-    // whole block's first climb step when every fourth thread issued them after the leaf phase
-    // (tree pass 0.90 -> 0.886 ms on 16.7 M).
-    auto issue_next = [&](int blk, int buf, int g) {
-        if (blk + 2 * grid >= nblk) return;
-        const Span s2 = S.sp2[buf];
-        const int m2 = min(EB, s2.n - s2.b0), ng = (m2 + 3) / 4;
+    // Soup: group g of a block's gathers into slot[buf] (leaves 4g .. 4g+3) as one tile::gather4 copy
+    // on the buffer's mbarrier, whose phase expects 192 bytes per group (group 0's arrival is its
+    // only one); a leaf past the segment repeats its group's first row (read, never used).  The copy
+    // engine takes about one small copy per 11 to 17 cycles per SM, which one 48-byte copy per leaf
+    // kept saturated; with four rows a copy and the tensor map's 64-byte L2 fills a random gather of
+    // 16.7 M rows takes 0.55 ms against 0.67 (B200; DRAM reads 154 -> 98 B per row).
+    auto gather_rows = [&](const Span &sp, int buf, int g) {
+        const int m2 = min(EB, sp.n - sp.b0), ng = (m2 + 3) / 4;
         if (g == 0) mbar_arrive_tx(&S.bar[buf], 192u * (uint32_t)ng);
         if (g < ng) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // reads above, copies below
-            const int x = 4 * g;  // a leaf past the segment repeats its group's first row
-            const uint32_t r0 = S.prow[x];
-            gather4_g2s(&S.slot[buf][g][0], &soup_map, r0, x + 1 < m2 ? S.prow[x + 1] : r0,
-                        x + 2 < m2 ? S.prow[x + 2] : r0, x + 3 < m2 ? S.prow[x + 3] : r0, &S.bar[buf]);
+            uint32_t row[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                uint32_t ti = S.perm[buf][4 * g + (4 * g + q < m2 ? q : 0)];
+                if (ti >= (uint32_t)sp.n) { bad_perm = true; ti = 0; }
+                row[q] = (uint32_t)(sp.start + ti);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // reads and writes above, copies below
+            gather4_g2s(&S.slot[buf][16 * g], &soup_map, row[0], row[1], row[2], row[3], &S.bar[buf]);
+        }
+    };
+    // one block ahead: the keys of its leaves and on either side of it
+    auto fetch_keys = [&](const Span &sp, int b) {
+        const uint32_t *keys = keys_all + sp.start;
+        const int b0 = sp.b0, n = sp.n, k = b0 + t;
+        if (k < n) cp_async4(&S.key[b][t + 1], keys + k);
+        if (t == 0 && b0 > 0) cp_async4(&S.key[b][0], keys + b0 - 1);
+        if (t == EB - 1 && b0 + EB < n) cp_async4(&S.key[b][EB + 1], keys + b0 + EB);
+    };
+    // The block two ahead's leaves into slot[buf], which no thread reads any more.
+    auto refill = [&](int blk, int it, int buf) {
+        if (blk + 2 * grid >= nblk) return;
+        if constexpr (Leaves::kMesh) {
+            fetch_mesh(span_of(it + 2), buf);
+        } else {
+            const int g = kLate ? 8 * warp + lane : t - EB / 2;
+            if (kLate ? lane < 8 : g >= 0 && g < EB / 4) gather_rows(span_of(it + 2), buf, g);
         }
     };
     int buf = 0;
@@ -294,26 +288,29 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
     bool copy_timeout = false;
     if (t < 2) mbar_init(&S.bar[t], 1);
     if (t < 2) S.open[t] = 0;
-    if (kLate && t == 0 && (int)blockIdx.x + 2 * grid < nblk) S.sp2[0] = segs.span(blockIdx.x + 2 * grid);
+    if (t < 4) find_span(t);
     mbar_init_fence();
     __syncthreads();
     if ((int)blockIdx.x < nblk) {
-        fetch_perm(blockIdx.x);
-        fetch_tri(blockIdx.x, 0);
-        fetch_keys(blockIdx.x);
-        if ((int)blockIdx.x + grid < nblk) {
-            fetch_perm(blockIdx.x + grid);
-            fetch_tri(blockIdx.x + grid, 1);
-            if ((int)blockIdx.x + 2 * grid < nblk) fetch_perm(blockIdx.x + 2 * grid);
+        // the first two blocks' leaves (uniform branches)
+        for (int k = 0; k < 2 && (int)blockIdx.x + k * grid < nblk; ++k) fetch_perm(span_of(k), k);
+        cp_async_commit();
+        cp_async_wait_all();
+        __syncthreads();
+        for (int k = 0; k < 2 && (int)blockIdx.x + k * grid < nblk; ++k) {
+            const Span sp = span_of(k);
+            if constexpr (Leaves::kMesh) fetch_mesh(sp, k);
+            else if (t < EB / 4) gather_rows(sp, k, t);
         }
+        __syncthreads();  // perm is read
+        fetch_keys(span_of(0), 0);
+        if ((int)blockIdx.x + 2 * grid < nblk) fetch_perm(span_of(2), 0);
+        cp_async_commit();
     }
 
     // Thread 0, after a barrier that follows the previous block's emissions: that block's count
     // of open items, and its counter cleared for the next block (the counters alternate with the
-    // buffers).  No barrier ends a block: every shared word a thread reads after the climb (its
-    // own mask, links and parked pair) it resets itself at the next block's start, and the next
-    // block touches anyone else's only after its leaf barrier (a barrier at the end of each
-    // block cost the pass 0.852 -> 0.890 ms on 16.7 M).
+    // buffers).
     auto settle_prev = [&](int blk, int buf) {
         if (blk - grid >= (int)blockIdx.x) {
             const int o = S.open[buf ^ 1];
@@ -323,36 +320,38 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
         }
         S.open[buf ^ 1] = 0;
     };
+    // after the barrier that ends a block's use of the other buffer's keys and indices: the next
+    // block's keys and the permutation three blocks ahead
+    auto fetch_next = [&](int blk, int it, int buf) {
+        if (blk + grid < nblk) fetch_keys(span_of(it + 1), buf ^ 1);
+        if (blk + 3 * grid < nblk) fetch_perm(span_of(it + 3), buf ^ 1);
+        cp_async_commit();
+    };
     int last = -1, last_buf = 0;
-    for (int blk = blockIdx.x; blk < nblk; blk += grid, buf ^= 1) {
+    for (int blk = blockIdx.x, it = 0; blk < nblk; blk += grid, ++it, buf ^= 1) {
         last = blk;
         last_buf = buf;
-        const Span sp = nsp;
+        const Span sp = span_of(it);
         const int b0 = sp.b0, n = sp.n;
         float4 *nodes = nodes_all + 4ull * sp.start;
         int32_t *parents = parents_all + 2ull * sp.start;
         const int m = min(EB, n - b0);
         const int k = b0 + t;
         const bool active = t < m;
-        S.key[t + 1] = active ? nk : 0u;
-        if (t == 0) S.key[0] = nk_lo;
-        if (t == EB - 1) S.key[EB + 1] = nk_hi;
-        S.mask[t] = 0;
-        S.par[t] = -1;
-        S.par[EB + t] = -1;
-        if (t < 3) S.cnt[t] = 0;
         // this leaf's triangle: to the output soup, and its box (exact-zero components nudged
         // by 1e-8 as bvh-up-pass.js:209-210 does)
         if constexpr (Leaves::kMesh) {
-            // the next block's group may still be in flight (the newest one), not this one's
-            if (blk + grid < nblk) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            // the rows of the next block may still be in flight (the newest group), not this one's; in
+            // the first turn the keys came last
+            if (blk + grid < nblk && blk != (int)blockIdx.x) asm volatile("cp.async.wait_group 1;" ::: "memory");
             else cp_async_wait_all();
         } else {
+            cp_async_wait_all();
             if (!mbar_wait(&S.bar[buf], (phase >> buf) & 1u)) copy_timeout = true;
             phase ^= 1u << buf;
         }
         float4 leaf_lo = make_float4(0.f, 0.f, 0.f, __int_as_float(-(k + 1)));
-        float4 leaf_hi0 = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 leaf_hi = make_float4(0.f, 0.f, 0.f, 0.f);
         if (active) {
             const float4 *tr = tri_row(buf, t);
             const float4 a = tr[0], b = tr[1], c = tr[2];
@@ -367,38 +366,27 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
             nx = nx == 0.0f ? -1e-8f : nx; ny = ny == 0.0f ? -1e-8f : ny; nz = nz == 0.0f ? -1e-8f : nz;
             xx = xx == 0.0f ? 1e-8f : xx;  xy = xy == 0.0f ? 1e-8f : xy;  xz = xz == 0.0f ? 1e-8f : xz;
             leaf_lo = make_float4(nx, ny, nz, __int_as_float(-(k + 1)));
-            leaf_hi0 = make_float4(xx, xy, xz, 0.f);
-        }
-        if (blk + grid < nblk) fetch_keys(blk + grid);
-        if constexpr (kLate) {  // this thread's row of the block two ahead
-            if (blk + 2 * grid < nblk) {
-                const Span s2 = S.sp2[buf];
-                uint32_t row = 0;
-                if (s2.b0 + t < s2.n) {
-                    uint32_t ti = pa;
-                    if (ti >= (uint32_t)s2.n) { bad_perm = true; ti = 0; }
-                    row = (uint32_t)(s2.start + ti);
-                }
-                S.prow[t] = row;
-            }
+            leaf_hi = make_float4(xx, xy, xz, 0.f);
         }
         if (n == 1) {  // one leaf, one arrival at node 0: left slot only, f_1 = 1
             if (t == 0) {
                 nodes[0] = make_float4(leaf_lo.x, leaf_lo.y, leaf_lo.z, __int_as_float(-1));
-                nodes[1] = make_float4(leaf_hi0.x, leaf_hi0.y, leaf_hi0.z, __int_as_float(1));
+                nodes[1] = make_float4(leaf_hi.x, leaf_hi.y, leaf_hi.z, __int_as_float(1));
                 nodes[2] = make_float4(0.f, 0.f, 0.f, 0.f);
                 nodes[3] = make_float4(0.f, 0.f, 0.f, 0.f);
                 parents[0] = 0;
                 parents[1] = 0;
-                out_counts[blk] = 0;
             }
-            // uniform across the block; no other thread reads what this one wrote.  The barrier
-            // keeps every thread's wait on this buffer's phase ahead of its next arming.
+            // uniform across the block.  The barrier keeps every thread's wait on this buffer's
+            // phase and its reads ahead of the refill.
             __syncthreads();
-            if (t == 0) settle_prev(blk, buf);
-            refill(blk, buf);
-            if constexpr (kLate)
-                if (t < EB / 4) issue_next(blk, buf, t);
+            if (t == 0) {
+                settle_prev(blk, buf);
+                find_span(it + 4);
+            }
+            fetch_next(blk, it, buf);
+            refill(blk, it, buf);
+            __syncthreads();  // perm is read
             continue;
         }
         if (k == 0) {  // the root has no parent; slot N-1 and record N-1 stay zero
@@ -408,130 +396,176 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
             float4 *last = nodes + 4ull * (n - 1);
             last[0] = z; last[1] = z; last[2] = z; last[3] = z;
         }
-        __syncthreads();  // every thread has waited on and read slot[buf]: it may be refilled
-        if (t == 0) settle_prev(blk, buf);
-        refill(blk, buf);
-        auto dval = [&](int x) -> int {  // d of split b0 + x, x in [-1, EB - 1]
+        __syncthreads();  // rows read, keys written; the block before is done with the pool
+        if (t == 0) {
+            settle_prev(blk, buf);
+            find_span(it + 4);
+        }
+        fetch_next(blk, it, buf);
+        // the separator before leaf t, as 6 bits: d of a split is 2 or more (keys below 2^30, indices
+        // below 2^30), -1 past the segment's ends is kept as 0; past the block's leaves 63
+        auto dval = [&](int x) -> uint32_t {  // separator after leaf b0 + x, x in [-1, EB - 1]
             const int g = b0 + x;
-            if (g < 0 || g >= n - 1) return -1;
-            const uint32_t a = S.key[x + 1], b = S.key[x + 2];
-            return a != b ? __clz(a ^ b) : 32 + __clz(g ^ (g + 1));
+            if (g < 0 || g >= n - 1) return 0u;
+            const uint32_t a = S.key[buf][x + 1], b = S.key[buf][x + 2];
+            return (uint32_t)(a != b ? __clz(a ^ b) : 32 + __clz(g ^ (g + 1)));
         };
+        const uint32_t sv = active ? dval(t - 1) : 63u;
+        uint32_t pl[6];
+        uint32_t mine = 0;
+#pragma unroll
+        for (int b = 0; b < 6; ++b) {
+            pl[b] = __ballot_sync(0xFFFFFFFFu, (sv >> b) & 1u);
+            mine = lane == b ? pl[b] : mine;
+        }
+        if (lane < 6) S.plane[warp][lane] = mine;
+        const uint32_t smallest = __reduce_min_sync(0xFFFFFFFFu, sv);
+        if (lane == 0) S.wmin[warp] = (uint8_t)smallest;
+        if (active) S.sep[t] = (uint8_t)sv;
+        if (t == m - 1) S.sep[m] = (uint8_t)dval(m - 1);
+        S.P[t] = -1;
+        float4 *lo1 = S.pool, *hi1 = S.pool + EB, *lo4 = S.pool + 2 * EB, *hi4 = S.pool + 3 * EB;
+        float4 *lo16 = S.slot[buf], *hi16 = lo16 + EB;
+        // boxes of 1, 4 and 16 leaves from each leaf on, cut at the warp's end
+        lo1[t] = leaf_lo;
+        hi1[t] = leaf_hi;
+        {
+            float4 lo = leaf_lo, hi = leaf_hi;
+            auto widen = [&](int d) {  // (past the warp's end a lane meets itself)
+                box_join(lo, hi, make_float4(__shfl_down_sync(0xFFFFFFFFu, lo.x, d), __shfl_down_sync(0xFFFFFFFFu, lo.y, d),
+                                             __shfl_down_sync(0xFFFFFFFFu, lo.z, d), 0.f),
+                         make_float4(__shfl_down_sync(0xFFFFFFFFu, hi.x, d), __shfl_down_sync(0xFFFFFFFFu, hi.y, d),
+                                     __shfl_down_sync(0xFFFFFFFFu, hi.z, d), 0.f));
+            };
+            widen(1);
+            widen(2);
+            lo4[t] = lo;
+            hi4[t] = hi;
+            widen(4);
+            widen(8);
+            lo16[t] = lo;
+            hi16[t] = hi;
+        }
+        __syncthreads();
+        int na = -1, nb = m + 1;  // separator t's node: leaves na .. nb - 1 (-1, m + 1: none in the block)
+        if (t >= 1 && active) {
+            const uint32_t below = lanes_below(pl, sv);
+            const uint32_t ml = below & lt, mr = below & ~lt;  // (bit t itself is never set)
+            uint32_t wb = 0;  // the warps with a separator below this one
+#pragma unroll
+            for (int w = 0; w < W; ++w) wb |= (uint32_t)(S.wmin[w] < sv) << w;
+            auto search = [&](int w) {
+                const uint4 x = *reinterpret_cast<const uint4 *>(&S.plane[w][0]);
+                const uint2 y = *reinterpret_cast<const uint2 *>(&S.plane[w][4]);
+                const uint32_t p6[6] = {x.x, x.y, x.z, x.w, y.x, y.y};
+                return lanes_below(p6, sv);
+            };
+            if (ml) {
+                na = 32 * warp + 31 - __clz(ml);
+            } else {
+                const uint32_t wl = wb & ((1u << warp) - 1u);
+                if (wl) {
+                    const int w = 31 - __clz(wl);
+                    na = 32 * w + 31 - __clz(search(w));
+                }
+            }
+            if (mr) {
+                nb = 32 * warp + __ffs(mr) - 1;
+            } else {
+                const uint32_t wr = wb & ~((2u << warp) - 1u);
+                if (wr) {
+                    const int w = __ffs(wr) - 1;
+                    nb = 32 * w + __ffs(search(w)) - 1;
+                } else if (S.sep[m] < sv) {
+                    nb = m;
+                }
+            }
+        }
+        // the node: index, box, and the record its parent has (separator np, 0 and m: not here)
+        const bool in = na >= 0 && nb <= m && t >= 1 && active;
+        float4 nlo, nhi;
+        int np = 0, P = 0;
+        bool nleft = false, root = false;
+        if (in) {
+            nleft = S.sep[nb] > S.sep[na];
+            root = b0 + na == 0 && b0 + nb == n;
+            P = root ? 0 : nleft ? nb - 1 : na;  // (the root's block begins the segment: b0 == 0)
+            np = nleft ? nb : na;
+            S.P[t] = P;
+            // its leaves warp by warp: a node that goes on past its first warp takes that warp's
+            // leaves as one cut window of 16 (two from 17 leaves on); any other piece is at most
+            // four windows, the last one ending with it
+            int u = na, e = min(nb, (na | 31) + 1);
+            if (e < nb) {
+                nlo = lo16[na];
+                nhi = hi16[na];
+                if (e - na > 16) box_join(nlo, nhi, lo16[e - 16], hi16[e - 16]);
+                u = e;
+                e = min(nb, u + 32);
+            } else {
+                nlo = lo1[na];
+                nhi = hi1[na];
+                u = na + 1;
+            }
+            for (;;) {
+                const int len = e - u, step = len >= 16 ? 16 : len >= 4 ? 4 : 1, z = e - step;
+                const float4 *slo = len >= 16 ? lo16 : len >= 4 ? lo4 : lo1, *shi = len >= 16 ? hi16 : len >= 4 ? hi4 : hi1;
+                box_join(nlo, nhi, slo[z], shi[z]);
+                for (int i = u; i < z; i += step) box_join(nlo, nhi, slo[i], shi[i]);
+                if (e == nb) break;
+                u = e;
+                e = min(nb, e + 32);
+            }
+            nlo.w = __int_as_float(b0 + P);
+        }
+        const bool lleft = active && S.sep[t + 1] > sv;  // the leaf is its parent's left child
+        const int ip = lleft ? t + 1 : t;
+        leaf_lo = lo1[t];  // (read back rather than held through the search)
+        leaf_hi = hi1[t];
+        __syncthreads();
+        // hand over: side 0 in words 0 and 1 of the record, side 1 in 2 and 3 (f_1 = 2, f_2 = 0)
+        auto hand = [&](int j, bool left, float4 lo, float4 hi) {
+            hi.w = __int_as_float(left ? 2 : 0);
+            S.pool[Smem::rec_at(j, left ? 0 : 2)] = lo;
+            S.pool[Smem::rec_at(j, left ? 1 : 3)] = hi;
+        };
+        if (in && !root && np > 0 && np < m) hand(np, nleft, nlo, nhi);
+        if (active && ip > 0 && ip < m) hand(ip, lleft, leaf_lo, leaf_hi);
+        if (!kLate) refill(blk, it, buf);
+        __syncthreads();
+        // parent links, and what leaves the block for K3c
         OpenItem *out = out_items + (size_t)blk * kOpenCap;
-        auto emit = [&](float4 lo, float4 hi) {  // an item leaves the block for K3c
-            const uint32_t pk = __float_as_uint(hi.w);
+        auto emit = [&](float4 lo, float4 hi, int a, int b) {
+            const int dl = S.sep[a], dr = S.sep[b];
             OpenItem it;
             it.lo = lo;
-            it.hi = make_float4(hi.x, hi.y, hi.z, __int_as_float(G::rdr(pk)));
-            it.xl = b0 + G::rl(pk);
-            it.xr = b0 + G::rr(pk);
-            it.pad0 = G::rdl(pk);
+            it.hi = make_float4(hi.x, hi.y, hi.z, __int_as_float(dr ? dr : -1));
+            it.xl = b0 + a;
+            it.xr = b0 + b - 1;
+            it.pad0 = dl ? dl : -1;
             it.pad1 = 0;
             const int at = atomicAdd(&S.open[buf], 1);
             if (at < kOpenCap) out[at] = it;
             else atomicOr(&ctl->err, ERR_CLIMB);
         };
-        // One step of an item: leave the block, park at its parent split, or merge with the
-        // parked sibling into the parent (returned in nlo/nhi, true unless it is the root).
-        auto climb = [&](float4 lo, float4 hi, float4 &nlo, float4 &nhi) -> bool {
-            const uint32_t pk = __float_as_uint(hi.w);
-            const int l = G::rl(pk), r = G::rr(pk), dl = G::rdl(pk), dr = G::rdr(pk);
-            const bool is_left = dr > dl;
-            const int s = is_left ? r : l - 1;
-            if (s < 0 || s > m - 2) {
-                emit(lo, hi);
-                return false;
-            }
-            const int side = is_left ? 0 : 1;
-            S.pend[side][0][s] = lo;
-            S.pend[side][1][s] = hi;
-            if (atom_or_acq_rel_cta(&S.mask[s], 1u << side) == 0u) return false;  // first parks
-            const float4 slo = S.pend[side ^ 1][0][s], shi = S.pend[side ^ 1][1][s];
-            const uint32_t spk = __float_as_uint(shi.w);
-            const int L = is_left ? l : G::rl(spk), R = is_left ? G::rr(spk) : r;
-            const int ndl = is_left ? dl : G::rdl(spk), ndr = is_left ? G::rdr(spk) : dr;
-            const bool root = (b0 + L == 0) && (b0 + R == n - 1);
-            const int P = root ? 0 : (ndr > ndl ? b0 + R : b0 + L);
-            // the record: this child in slot `side`, the sibling in the other (f_1 = 2, f_2 = 0)
-            float4 *rc = nodes + 4ull * P;
-            rc[2 * side] = lo;
-            rc[2 * side + 1] = make_float4(hi.x, hi.y, hi.z, __int_as_float(2 - 2 * side));
-            rc[2 - 2 * side] = slo;
-            rc[3 - 2 * side] = make_float4(shi.x, shi.y, shi.z, __int_as_float(2 * side));
-            const int mref = __float_as_int(lo.w), sref = __float_as_int(slo.w);
-            S.par[mref >= 0 ? mref - b0 : EB - 1 - b0 - mref] = P;
-            S.par[sref >= 0 ? sref - b0 : EB - 1 - b0 - sref] = P;
-            if (root) return false;
-            nlo = make_float4(fminf(lo.x, slo.x), fminf(lo.y, slo.y), fminf(lo.z, slo.z), __int_as_float(P));
-            nhi = make_float4(fmaxf(hi.x, shi.x), fmaxf(hi.y, shi.y), fmaxf(hi.z, shi.z),
-                              __uint_as_float(G::pack(L, R, ndl, ndr)));
-            return true;
-        };
-        // the items that climb on go to queue oq, counted in S.cnt[oc] (warp-aggregated)
-        auto append = [&](bool cont, float4 nlo, float4 nhi, int oq, int oc) {
-            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, cont);
-            int base = 0;
-            if (lane == 0 && bal) base = atomicAdd(&S.cnt[oc], __popc(bal));
-            base = __shfl_sync(0xFFFFFFFFu, base, 0);
-            if (cont) {
-                const int at = base + __popc(bal & lt);
-                qent((oq * 2) * (EB / 2) + at) = nlo;
-                qent((oq * 2 + 1) * (EB / 2) + at) = nhi;
-            }
-        };
-
-        // step 0: the leaves
-        float4 nlo = make_float4(0.f, 0.f, 0.f, 0.f), nhi = nlo;
-        bool cont = false;
-        if (active)
-            cont = climb(leaf_lo, make_float4(leaf_hi0.x, leaf_hi0.y, leaf_hi0.z,
-                                              __uint_as_float(G::pack(t, t, dval(t - 1), dval(t)))),
-                         nlo, nhi);
-        append(cont, nlo, nhi, 0, 0);
-        // later steps: the merged parents, compacted.  Once at most kFree items are left,
-        // each takes one thread of the first warps and climbs on its own, item in registers,
-        // without block barriers (the park / merge handshake works across warps).
-        int cur = 0, c = 0;
-        bool issued = false;  // the block two ahead's gathers (uniform)
-        for (int guard = 0; guard < 2 * EB; ++guard) {
-            __syncthreads();
-            const int count = S.cnt[c];
-            if (count <= kFree) {
-                if (t < count) {
-                    float4 lo = qent((cur * 2) * (EB / 2) + t), hi = qent((cur * 2 + 1) * (EB / 2) + t);
-                    for (int g2 = 0; g2 < 2 * EB; ++g2) {
-                        if (!climb(lo, hi, nlo, nhi)) break;
-                        lo = nlo;
-                        hi = nhi;
-                    }
-                } else if (kLate && t >= EB / 2 && t < EB / 2 + EB / 4) {
-                    issue_next(blk, buf, t - EB / 2);  // count <= kFree <= EB / 2
-                }
-                issued = true;
-                break;
-            }
-            const int nc = c == 2 ? 0 : c + 1, rc = nc == 2 ? 0 : nc + 1;
-            cont = false;
-            if (t < count) cont = climb(qent((cur * 2) * (EB / 2) + t), qent((cur * 2 + 1) * (EB / 2) + t), nlo, nhi);
-            append(cont, nlo, nhi, cur ^ 1, nc);
-            if (t == 0) S.cnt[rc] = 0;
-            cur ^= 1;
-            c = nc;
+        if (active) {
+            const int q = ip > 0 && ip < m ? S.P[ip] : -1;
+            if (q >= 0) parents[n + k] = b0 + q;
+            else emit(leaf_lo, leaf_hi, t, t + 1);
         }
-        if (kLate && !issued && t < EB / 4) issue_next(blk, buf, t);
-        __syncthreads();
-        // a child parked at a split whose sibling never came: the parent straddles the block
-        if (t < m - 1) {
-            const uint32_t mk = S.mask[t];
-            if (mk == 1u || mk == 2u) {
-                const int side = mk == 1u ? 0 : 1;
-                emit(S.pend[side][0][t], S.pend[side][1][t]);
-            }
+        if (in && !root) {
+            const int q = np > 0 && np < m ? S.P[np] : -1;
+            if (q >= 0) parents[b0 + P] = b0 + q;
+            else emit(nlo, nhi, na, nb);
         }
-        if (active) {  // the climb is over (barrier above): the staged links are final
-            if (S.par[t] >= 0) parents[k] = S.par[t];
-            if (S.par[EB + t] >= 0) parents[n + k] = S.par[EB + t];
+        // the records, four threads each
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int j = r * (EB / 4) + (t >> 2), part = t & 3;
+            const int q = S.P[j];
+            if (q >= 0) nodes[4ull * (b0 + q) + part] = S.pool[Smem::rec_at(j, part)];
         }
+        if (kLate) refill(blk, it, buf);
     }
     __syncthreads();  // the last block's open items are counted
     if (t == 0 && last >= 0) {
@@ -588,11 +622,6 @@ struct RunSmem {
     int warp[kRunWarps];
     int take, last;
 };
-
-__device__ __forceinline__ void box_join(float4 &lo, float4 &hi, const float4 &l, const float4 &h) {
-    lo.x = fminf(lo.x, l.x); lo.y = fminf(lo.y, l.y); lo.z = fminf(lo.z, l.z);
-    hi.x = fmaxf(hi.x, h.x); hi.y = fmaxf(hi.y, h.y); hi.z = fmaxf(hi.z, h.z);
-}
 
 // The union of items [u, v): at most four windows of the largest length that fits (the last one
 // ends at v, overlapping the one before), their loads all in flight.
@@ -914,7 +943,7 @@ __global__ void __launch_bounds__(kRunCap, Groups::kCtas) k_top_group(Groups gro
 
 // the layout plus the slack that puts it on a 128-byte boundary
 template <int LOG, class Segs, class Leaves>
-inline size_t leaves_smem_bytes() { return sizeof(typename TreeLayout<LOG, Segs, Leaves>::Smem) + 128; }
+inline size_t leaves_smem_bytes() { return sizeof(TreeSmem<(1 << LOG), Leaves::kMesh>) + 128; }
 
 // The soup as a 2-D tensor of `rows` rows of 12 floats, 48 bytes apart, for the tree pass's
 // tile::gather4 copies: one-row boxes of a whole row, the L2 filling 64 bytes per DRAM request

@@ -50,15 +50,6 @@ __device__ __forceinline__ uint32_t quantise(float bmin, float bmax, float umin,
     return quantise_cen(centroid(bmin, bmax), umin, umax);
 }
 
-// Common-prefix length delta(i, j) of the sorted keys (radix-tree.js:160-185): -1 when j is
-// out of range, clz(k_i ^ k_j) when the keys differ, else 32 + clz(i ^ j) (index tie-break).
-// i must be in range.
-__device__ __forceinline__ int delta(const uint32_t *__restrict__ keys, int n, int i, int j) {
-    if (j < 0 || j >= n) return -1;
-    const uint32_t a = __ldg(keys + i), b = __ldg(keys + j);
-    return a != b ? __clz(a ^ b) : 32 + __clz(i ^ j);
-}
-
 // Monotone float <-> uint32 maps for atomic min/max reductions.  `ord_lo` orders floats
 // ascending; atomicMax on ord_hi(x) = ~ord_lo(x) keeps the minimum, atomicMax on ord_lo(x)
 // keeps the maximum, so an all-zero word is the identity of both.
@@ -83,16 +74,6 @@ __device__ __forceinline__ bool finite3(float4 v) {
 // waiting blocks that let in cost more than the launch they hid (a 2^20-triangle build 0.235
 // -> 0.250 ms, against 0.232 ms without the early signal).
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-// Shared-memory atomic OR with acquire-release semantics at CTA scope: the caller's earlier
-// writes are visible to a thread that later sees its bit, and what the caller reads after it
-// includes the writes of threads whose bits it saw.
-__device__ __forceinline__ uint32_t atom_or_acq_rel_cta(uint32_t *p, uint32_t v) {
-    uint32_t old;
-    asm volatile("atom.acq_rel.cta.shared.or.b32 %0, [%1], %2;"
-                 : "=r"(old) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v) : "memory");
-    return old;
-}
 
 // Global-memory atomic add with acquire-release semantics at GPU scope: after a block barrier it
 // publishes the whole block's writes to a thread that later reads a value at least as new.
