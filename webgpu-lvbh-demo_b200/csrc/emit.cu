@@ -107,8 +107,7 @@ struct MeshLeaves {
 // buffer holds the block's boxes of 16 leaves, until the copies of the block two ahead go there.
 // pool: the boxes of 1 and of 4 leaves from each leaf on ([0 .. EB) and [EB .. 2 EB) mins and maxes
 // of one, then of four); when every node has its box, the records: node of separator j at
-// [4 j .. 4 j + 3], each record's four words rotated (rec_at) so that the scattered writes of its
-// two halves spread over the banks.
+// [4 j .. 4 j + 3] (rec_at).
 // key, perm: the keys of this block's leaves and the next's, the permutation entries (mesh: the
 // vertex indices) of the leaves two and three blocks ahead, all by 4-byte cp.async: held in registers
 // from one block to the next they spilled, and a spilled load waits for its value at once.
@@ -128,7 +127,6 @@ struct TreeSmem {
     uint8_t wmin[EB / 32];        // smallest separator of each warp's
     uint8_t sep[EB + 1];          // separators (before each leaf and after the last; -1 as 0)
     int open[2];                  // open items emitted, by buffer parity (a block's and the next's)
-    static __device__ __forceinline__ int rec_at(int j, int part) { return 4 * j + (part ^ ((j >> 1) & 3)); }
 };
 
 // The lanes whose 6-bit value, given bit by bit in planes, is below v.
@@ -146,6 +144,125 @@ __device__ __forceinline__ uint32_t lanes_below(const uint32_t (&plane)[6], uint
 __device__ __forceinline__ void box_join(float4 &lo, float4 &hi, const float4 &l, const float4 &h) {
     lo.x = fminf(lo.x, l.x); lo.y = fminf(lo.y, l.y); lo.z = fminf(lo.z, l.z);
     hi.x = fmaxf(hi.x, h.x); hi.y = fmaxf(hi.y, h.y); hi.z = fmaxf(hi.z, h.z);
+}
+
+// The separators of up to 32 W consecutive leaves or items as bit planes: bit b of those before
+// 32 w .. 32 w + 31 at plane[w][b], each warp's smallest at wmin[w], each one at sep[i] (6 bits: -1,
+// past a segment's ends, as 0; other separators are 2 or more).
+//
+// The nearest smaller separators of sv, the one before this thread's leaf or item, among the m + 1
+// around and between m of them: na before it (-1: none), nb after it (m + 1: none).
+template <int W>
+__device__ __forceinline__ void nearest_smaller(const uint32_t (*plane)[8], const uint8_t *wmin, const uint8_t *sep,
+                                                const uint32_t (&own)[6], uint32_t sv, int m, int &na, int &nb) {
+    const int warp = threadIdx.x >> 5;
+    const uint32_t below = lanes_below(own, sv), lt = lanemask_lt();
+    const uint32_t ml = below & lt, mr = below & ~lt;  // (this lane's own bit is never set)
+    uint32_t wb = 0;  // the warps with a separator below this one
+#pragma unroll
+    for (int w = 0; w < W; ++w) wb |= (uint32_t)(wmin[w] < sv) << w;
+    auto search = [&](int w) {
+        const uint4 x = *reinterpret_cast<const uint4 *>(&plane[w][0]);
+        const uint2 y = *reinterpret_cast<const uint2 *>(&plane[w][4]);
+        const uint32_t p6[6] = {x.x, x.y, x.z, x.w, y.x, y.y};
+        return lanes_below(p6, sv);
+    };
+    na = -1;
+    nb = m + 1;
+    if (ml) {
+        na = 32 * warp + 31 - __clz(ml);
+    } else {
+        const uint32_t wl = wb & ((1u << warp) - 1u);
+        if (wl) {
+            const int w = 31 - __clz(wl);
+            na = 32 * w + 31 - __clz(search(w));
+        }
+    }
+    if (mr) {
+        nb = 32 * warp + __ffs(mr) - 1;
+    } else {
+        const uint32_t wr = wb & ~((2u << warp) - 1u);
+        if (wr) {
+            const int w = __ffs(wr) - 1;
+            nb = 32 * w + __ffs(search(w)) - 1;
+        } else if (sep[m] < sv) {
+            nb = m;
+        }
+    }
+}
+
+// This thread's bit-plane words (all lanes call it) and what the block sees of them.
+__device__ __forceinline__ void put_planes(uint32_t sv, uint32_t (&own)[6], uint32_t (*plane)[8], uint8_t *wmin) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t mine = 0;
+#pragma unroll
+    for (int b = 0; b < 6; ++b) {
+        own[b] = __ballot_sync(0xFFFFFFFFu, (sv >> b) & 1u);
+        mine = lane == b ? own[b] : mine;
+    }
+    if (lane < 6) plane[warp][lane] = mine;
+    const uint32_t smallest = __reduce_min_sync(0xFFFFFFFFu, sv);
+    if (lane == 0) wmin[warp] = (uint8_t)smallest;
+}
+
+// Boxes of 1, 4 and 16 consecutive leaves or items from each one on, cut at the warp's end.
+struct Windows {
+    float4 *lo1, *hi1, *lo4, *hi4, *lo16, *hi16;
+    // this thread's 4 and 16 (all lanes call it; lo, hi: its own box)
+    __device__ __forceinline__ void put(float4 lo, float4 hi) const {
+        const int t = threadIdx.x;
+        auto widen = [&](int d) {  // (past the warp's end a lane meets itself)
+            box_join(lo, hi, make_float4(__shfl_down_sync(0xFFFFFFFFu, lo.x, d), __shfl_down_sync(0xFFFFFFFFu, lo.y, d),
+                                         __shfl_down_sync(0xFFFFFFFFu, lo.z, d), 0.f),
+                     make_float4(__shfl_down_sync(0xFFFFFFFFu, hi.x, d), __shfl_down_sync(0xFFFFFFFFu, hi.y, d),
+                                 __shfl_down_sync(0xFFFFFFFFu, hi.z, d), 0.f));
+        };
+        widen(1);
+        widen(2);
+        lo4[t] = lo;
+        hi4[t] = hi;
+        widen(4);
+        widen(8);
+        lo16[t] = lo;
+        hi16[t] = hi;
+    }
+    // The union of a .. b - 1 (at least two), warp by warp: a range that goes on past its first warp
+    // takes that warp's part as one cut window of 16 (two from 17 on); any other piece is at most
+    // four windows, the last one ending with it.
+    __device__ __forceinline__ void get(int a, int b, float4 &lo, float4 &hi) const {
+        int u = a, e = min(b, (a | 31) + 1);
+        if (e < b) {
+            lo = lo16[a];
+            hi = hi16[a];
+            if (e - a > 16) box_join(lo, hi, lo16[e - 16], hi16[e - 16]);
+            u = e;
+            e = min(b, u + 32);
+        } else {
+            lo = lo1[a];
+            hi = hi1[a];
+            u = a + 1;
+        }
+        for (;;) {
+            const int len = e - u, step = len >= 16 ? 16 : len >= 4 ? 4 : 1, z = e - step;
+            const float4 *slo = len >= 16 ? lo16 : len >= 4 ? lo4 : lo1, *shi = len >= 16 ? hi16 : len >= 4 ? hi4 : hi1;
+            box_join(lo, hi, slo[z], shi[z]);
+            for (int i = u; i < z; i += step) box_join(lo, hi, slo[i], shi[i]);
+            if (e == b) break;
+            u = e;
+            e = min(b, e + 32);
+        }
+    }
+};
+
+// Word `part` of the record of separator j in a pool of records, each record's four words rotated
+// so that the scattered writes of its two halves spread over the banks.
+__device__ __forceinline__ int rec_at(int j, int part) { return 4 * j + (part ^ ((j >> 1) & 3)); }
+// Box and link of a child into its parent's record: side 0 in words 0 and 1, side 1 in 2 and 3
+// (f_1 = 2, f_2 = 0).
+__device__ __forceinline__ void hand_over(float4 *pool, int j, bool left, float4 lo, float4 hi) {
+    hi.w = __int_as_float(left ? 2 : 0);
+    pool[rec_at(j, left ? 0 : 2)] = lo;
+    pool[rec_at(j, left ? 1 : 3)] = hi;
 }
 
 // K3b: leaf gather, rearrange and the tree over blocks of EB sorted leaves (see the pass list
@@ -200,7 +317,6 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
     // a sort whose look-back gave up left unsorted keys: build nothing from them (uniform)
     if (ld_relaxed_gpu(&ctl->err) & ERR_LOOKBACK_TIMEOUT) return;
     const int nblk = segs.blocks();
-    const uint32_t lt = lanemask_lt();
 
     // Leaves come in three steps ahead of their block: the permutation entry (its three vertex
     // indices for a mesh) three blocks ahead, its triangle copied into slot[] two blocks ahead, its
@@ -412,75 +528,17 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
         };
         const uint32_t sv = active ? dval(t - 1) : 63u;
         uint32_t pl[6];
-        uint32_t mine = 0;
-#pragma unroll
-        for (int b = 0; b < 6; ++b) {
-            pl[b] = __ballot_sync(0xFFFFFFFFu, (sv >> b) & 1u);
-            mine = lane == b ? pl[b] : mine;
-        }
-        if (lane < 6) S.plane[warp][lane] = mine;
-        const uint32_t smallest = __reduce_min_sync(0xFFFFFFFFu, sv);
-        if (lane == 0) S.wmin[warp] = (uint8_t)smallest;
+        put_planes(sv, pl, S.plane, S.wmin);
         if (active) S.sep[t] = (uint8_t)sv;
         if (t == m - 1) S.sep[m] = (uint8_t)dval(m - 1);
         S.P[t] = -1;
-        float4 *lo1 = S.pool, *hi1 = S.pool + EB, *lo4 = S.pool + 2 * EB, *hi4 = S.pool + 3 * EB;
-        float4 *lo16 = S.slot[buf], *hi16 = lo16 + EB;
-        // boxes of 1, 4 and 16 leaves from each leaf on, cut at the warp's end
-        lo1[t] = leaf_lo;
-        hi1[t] = leaf_hi;
-        {
-            float4 lo = leaf_lo, hi = leaf_hi;
-            auto widen = [&](int d) {  // (past the warp's end a lane meets itself)
-                box_join(lo, hi, make_float4(__shfl_down_sync(0xFFFFFFFFu, lo.x, d), __shfl_down_sync(0xFFFFFFFFu, lo.y, d),
-                                             __shfl_down_sync(0xFFFFFFFFu, lo.z, d), 0.f),
-                         make_float4(__shfl_down_sync(0xFFFFFFFFu, hi.x, d), __shfl_down_sync(0xFFFFFFFFu, hi.y, d),
-                                     __shfl_down_sync(0xFFFFFFFFu, hi.z, d), 0.f));
-            };
-            widen(1);
-            widen(2);
-            lo4[t] = lo;
-            hi4[t] = hi;
-            widen(4);
-            widen(8);
-            lo16[t] = lo;
-            hi16[t] = hi;
-        }
+        const Windows win{S.pool, S.pool + EB, S.pool + 2 * EB, S.pool + 3 * EB, S.slot[buf], S.slot[buf] + EB};
+        win.lo1[t] = leaf_lo;
+        win.hi1[t] = leaf_hi;
+        win.put(leaf_lo, leaf_hi);
         __syncthreads();
         int na = -1, nb = m + 1;  // separator t's node: leaves na .. nb - 1 (-1, m + 1: none in the block)
-        if (t >= 1 && active) {
-            const uint32_t below = lanes_below(pl, sv);
-            const uint32_t ml = below & lt, mr = below & ~lt;  // (bit t itself is never set)
-            uint32_t wb = 0;  // the warps with a separator below this one
-#pragma unroll
-            for (int w = 0; w < W; ++w) wb |= (uint32_t)(S.wmin[w] < sv) << w;
-            auto search = [&](int w) {
-                const uint4 x = *reinterpret_cast<const uint4 *>(&S.plane[w][0]);
-                const uint2 y = *reinterpret_cast<const uint2 *>(&S.plane[w][4]);
-                const uint32_t p6[6] = {x.x, x.y, x.z, x.w, y.x, y.y};
-                return lanes_below(p6, sv);
-            };
-            if (ml) {
-                na = 32 * warp + 31 - __clz(ml);
-            } else {
-                const uint32_t wl = wb & ((1u << warp) - 1u);
-                if (wl) {
-                    const int w = 31 - __clz(wl);
-                    na = 32 * w + 31 - __clz(search(w));
-                }
-            }
-            if (mr) {
-                nb = 32 * warp + __ffs(mr) - 1;
-            } else {
-                const uint32_t wr = wb & ~((2u << warp) - 1u);
-                if (wr) {
-                    const int w = __ffs(wr) - 1;
-                    nb = 32 * w + __ffs(search(w)) - 1;
-                } else if (S.sep[m] < sv) {
-                    nb = m;
-                }
-            }
-        }
+        if (t >= 1 && active) nearest_smaller<W>(S.plane, S.wmin, S.sep, pl, sv, m, na, nb);
         // the node: index, box, and the record its parent has (separator np, 0 and m: not here)
         const bool in = na >= 0 && nb <= m && t >= 1 && active;
         float4 nlo, nhi;
@@ -492,45 +550,16 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
             P = root ? 0 : nleft ? nb - 1 : na;  // (the root's block begins the segment: b0 == 0)
             np = nleft ? nb : na;
             S.P[t] = P;
-            // its leaves warp by warp: a node that goes on past its first warp takes that warp's
-            // leaves as one cut window of 16 (two from 17 leaves on); any other piece is at most
-            // four windows, the last one ending with it
-            int u = na, e = min(nb, (na | 31) + 1);
-            if (e < nb) {
-                nlo = lo16[na];
-                nhi = hi16[na];
-                if (e - na > 16) box_join(nlo, nhi, lo16[e - 16], hi16[e - 16]);
-                u = e;
-                e = min(nb, u + 32);
-            } else {
-                nlo = lo1[na];
-                nhi = hi1[na];
-                u = na + 1;
-            }
-            for (;;) {
-                const int len = e - u, step = len >= 16 ? 16 : len >= 4 ? 4 : 1, z = e - step;
-                const float4 *slo = len >= 16 ? lo16 : len >= 4 ? lo4 : lo1, *shi = len >= 16 ? hi16 : len >= 4 ? hi4 : hi1;
-                box_join(nlo, nhi, slo[z], shi[z]);
-                for (int i = u; i < z; i += step) box_join(nlo, nhi, slo[i], shi[i]);
-                if (e == nb) break;
-                u = e;
-                e = min(nb, e + 32);
-            }
+            win.get(na, nb, nlo, nhi);
             nlo.w = __int_as_float(b0 + P);
         }
         const bool lleft = active && S.sep[t + 1] > sv;  // the leaf is its parent's left child
         const int ip = lleft ? t + 1 : t;
-        leaf_lo = lo1[t];  // (read back rather than held through the search)
-        leaf_hi = hi1[t];
+        leaf_lo = win.lo1[t];  // (read back rather than held through the search)
+        leaf_hi = win.hi1[t];
         __syncthreads();
-        // hand over: side 0 in words 0 and 1 of the record, side 1 in 2 and 3 (f_1 = 2, f_2 = 0)
-        auto hand = [&](int j, bool left, float4 lo, float4 hi) {
-            hi.w = __int_as_float(left ? 2 : 0);
-            S.pool[Smem::rec_at(j, left ? 0 : 2)] = lo;
-            S.pool[Smem::rec_at(j, left ? 1 : 3)] = hi;
-        };
-        if (in && !root && np > 0 && np < m) hand(np, nleft, nlo, nhi);
-        if (active && ip > 0 && ip < m) hand(ip, lleft, leaf_lo, leaf_hi);
+        if (in && !root && np > 0 && np < m) hand_over(S.pool, np, nleft, nlo, nhi);
+        if (active && ip > 0 && ip < m) hand_over(S.pool, ip, lleft, leaf_lo, leaf_hi);
         if (!kLate) refill(blk, it, buf);
         __syncthreads();
         // parent links, and what leaves the block for K3c
@@ -563,7 +592,7 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
         for (int r = 0; r < 4; ++r) {
             const int j = r * (EB / 4) + (t >> 2), part = t & 3;
             const int q = S.P[j];
-            if (q >= 0) nodes[4ull * (b0 + q) + part] = S.pool[Smem::rec_at(j, part)];
+            if (q >= 0) nodes[4ull * (b0 + q) + part] = S.pool[rec_at(j, part)];
         }
         if (kLate) refill(blk, it, buf);
     }
@@ -610,29 +639,20 @@ constexpr int kRunWarps = kRunCap / 32;
 static_assert(kRunCap >= 2 * kOpenCap && kGroupBlocks <= 32 && kFan <= 32, "a run takes two children; one warp counts them");
 
 struct RunSmem {
-    float4 lo[4][kRunCap], hi[4][kRunCap];    // boxes of 1, 4, 16 and 64 items from each item on
-    float4 clo[2][kRunCap], chi[2][kRunCap];  // left and right child of each separator's node: box, link
-    uint32_t below[64][kRunWarps];  // separators below v among 32 w .. 32 w + 31, at [v][w]
-    int xl[kRunCap + 1];            // first leaf of each item, then the end of the last one
-    int sep[kRunCap + 1];           // the separators around and between the items
-    int out[kRunCap];               // what leaves the run from item i on: -1 nothing, 0 the item,
-                                    // else the node of separator out[i]
-    uint8_t done[kRunCap];          // separators whose node lies in the run
-    int cstart[33];                 // the children's first items among those loaded together
+    float4 lo[3][kRunCap], hi[3][kRunCap];  // Windows; when every node has its box, [1] holds those of
+                                            // the nodes that leave (box, link and end item)
+    float4 rec[4 * kRunCap];                // the separators' records (rec_at)
+    __align__(16) uint32_t plane[kRunWarps][8];
+    int xl[kRunCap + 1];     // first leaf of each item, then the end of the last one
+    int P[kRunCap];          // the separators' nodes (-1: not in this run)
+    int out[kRunCap];        // what leaves the run from item i on: -1 nothing, 0 the item, else the node
+                             // of separator out[i]
+    int cstart[33];          // the children's first items among those loaded together
     int warp[kRunWarps];
     int take, last;
+    uint8_t wmin[kRunWarps];
+    uint8_t sep[kRunCap + 1];  // the separators around and between the items (-1 as 0)
 };
-
-// The union of items [u, v): at most four windows of the largest length that fits (the last one
-// ends at v, overlapping the one before), their loads all in flight.
-__device__ __forceinline__ void run_box(const RunSmem &S, int u, int v, float4 &lo, float4 &hi) {
-    const int len = v - u, w = len >= 64 ? 3 : len >= 16 ? 2 : len >= 4 ? 1 : 0, step = 1 << (2 * w), z = v - step;
-    lo = S.lo[w][z];
-    hi = S.hi[w][z];
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        if (u + k * step < z) box_join(lo, hi, S.lo[w][u + k * step], S.hi[w][u + k * step]);
-}
 
 // The open item of leaves [xl, xr]; dl, dr: the separators before and after it.
 __device__ __forceinline__ OpenItem open_item(float4 lo, float4 hi, int ref, int xl, int xr, int dl, int dr) {
@@ -650,129 +670,85 @@ __device__ __forceinline__ OpenItem open_item(float4 lo, float4 hi, int ref, int
 // set, a barrier since): records and parent links to memory; the run's own open items, in leaf
 // order, to dst (at most kOpenCap of them) or, when dst is null, back to S as the next run.
 // Returns their number (uniform).  ok: false when an index lies outside the segment (nothing is
-// written for it).
-//
-// Thread j: the node of separator j (split xl[j] - 1), which covers items a .. b - 1 between the
-// nearest smaller separators a, b on either side; it takes the node's box as the union of those
-// items and hands box and index to its parent's node (that of the larger of separators a, b).
-// Thread i also hands item i to its parent's node.
+// written for it).  Thread t has item t and the node of separator t, as in the tree pass.
 __device__ __forceinline__ int reduce_run(RunSmem &S, int M, int n, float4 *nodes, int32_t *parents, OpenItem *dst,
                                           bool &ok) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int mysep = t < M ? S.sep[t] : 64;
-    // which separators lie below each value, one ballot per value
-    uint32_t keep0 = 0, keep1 = 0;  // the ballots of v = lane and v = 32 + lane
-    if (32 * warp < M) {
-#pragma unroll 8
-        for (int v = 0; v < 32; ++v) {
-            const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, mysep < v), b1 = __ballot_sync(0xFFFFFFFFu, mysep < 32 + v);
-            keep0 = lane == v ? b0 : keep0;
-            keep1 = lane == v ? b1 : keep1;
-        }
-    }
-    S.below[lane][warp] = keep0;
-    S.below[32 + lane][warp] = keep1;
+    const bool active = t < M;
+    const Windows win{S.lo[0], S.hi[0], S.lo[1], S.hi[1], S.lo[2], S.hi[2]};
+    const uint32_t sv = active ? S.sep[t] : 63u;
+    uint32_t pl[6];
+    put_planes(sv, pl, S.plane, S.wmin);
+    const float4 ilo = S.lo[0][t], ihi = S.hi[0][t];  // (past the run's end: not used)
+    win.put(ilo, ihi);
     S.out[t] = -1;
-    // windows of 4, 16 and 64 items
-#pragma unroll
-    for (int w = 1; w < 4; ++w) {
-        const int len = 1 << (2 * w), part = len / 4;
-        if (M < len) break;  // uniform
-        if (t + len <= M) {
-            float4 lo = S.lo[w - 1][t], hi = S.hi[w - 1][t];
-#pragma unroll
-            for (int k = 1; k < 4; ++k) box_join(lo, hi, S.lo[w - 1][t + k * part], S.hi[w - 1][t + k * part]);
-            S.lo[w][t] = lo;
-            S.hi[w][t] = hi;
-        }
-        __syncthreads();
-    }
-    if (M < 4) __syncthreads();  // (the ballots)
-    const int j = t;
-    int na = -1, nb = 0, P = 0, np = 0, ip = 0;  // node's ends, index, its and the item's parent separator
-    float4 nlo, nhi;
-    if (j >= 1 && j < M) {
-        if (mysep < 0) ok = false;  // only a segment's ends have separator -1
-        const uint4 *row = reinterpret_cast<const uint4 *>(S.below[max(mysep, 0)]);
-        uint32_t wd[kRunWarps];
-#pragma unroll
-        for (int w = 0; w < kRunWarps; w += 4) {
-            const uint4 r = row[w / 4];
-            wd[w] = r.x; wd[w + 1] = r.y; wd[w + 2] = r.z; wd[w + 3] = r.w;
-        }
-        int a = -1, b = S.sep[M] < mysep ? M : M + 1;  // -1 and M + 1: none in the run
-#pragma unroll
-        for (int w = 0; w < kRunWarps; ++w) {  // the words below j's, the last non-zero one wins
-            const uint32_t m = w < warp ? wd[w] : w == warp ? wd[w] & lanemask_lt() : 0u;
-            if (m) a = 32 * w + 31 - __clz(m);
-        }
-#pragma unroll
-        for (int w = kRunWarps - 1; w >= 0; --w) {  // and above (bit j itself is never set)
-            const uint32_t m = w > warp ? wd[w] : w == warp ? wd[w] & ~lanemask_lt() : 0u;
-            if (m) b = 32 * w + __ffs(m) - 1;
-        }
-        const bool in = a >= 0 && b <= M;
-        S.done[j] = in;
-        if (in) {
-            na = a;
-            nb = b;
-            const int L = S.xl[a], R = S.xl[b] - 1;
-            const bool left = S.sep[b] > S.sep[a];  // the node is its parent's left child
-            const bool root = L == 0 && R == n - 1;
-            P = root ? 0 : left ? R : L;
-            np = root ? -1 : left ? b : a;
-            run_box(S, a, b, nlo, nhi);
-            nlo.w = __int_as_float(P);
-            if (np > 0 && np < M) {
-                S.clo[left ? 0 : 1][np] = nlo;
-                S.chi[left ? 0 : 1][np] = nhi;
-            }
-        }
-    }
-    if (t < M) {
-        const bool left = S.sep[t + 1] > mysep;
-        ip = left ? t + 1 : t;
-        if (ip > 0 && ip < M) {
-            S.clo[left ? 0 : 1][ip] = S.lo[0][t];
-            S.chi[left ? 0 : 1][ip] = S.hi[0][t];
-        }
-    }
+    S.P[t] = -1;
     __syncthreads();
-    // the records; and what leaves: items and nodes of the run whose parent's node does not lie in it
-    auto leaves = [&](int p) { return p == 0 || p == M || (p > 0 && !S.done[p]); };
-    if (t < M && leaves(ip)) S.out[t] = 0;
-    if (na >= 0) {
-        const float4 ll = S.clo[0][j], lh = S.chi[0][j], rl = S.clo[1][j], rh = S.chi[1][j];
-        const int lref = __float_as_int(ll.w), rref = __float_as_int(rl.w);
-        if ((uint32_t)P < (uint32_t)(n - 1) && lref >= -n && lref < n - 1 && rref >= -n && rref < n - 1) {
-            float4 *rec = nodes + 4ull * P;
-            rec[0] = ll;
-            rec[1] = make_float4(lh.x, lh.y, lh.z, __int_as_float(2));
-            rec[2] = rl;
-            rec[3] = make_float4(rh.x, rh.y, rh.z, __int_as_float(0));
-            parents[lref >= 0 ? lref : n - (lref + 1)] = P;
-            parents[rref >= 0 ? rref : n - (rref + 1)] = P;
-        } else {
+    int na = -1, nb = M + 1, P = 0, np = 0;
+    float4 nlo, nhi;
+    bool in = false, root = false;
+    const int ref = __float_as_int(ilo.w);
+    if (active && (ref < -n || ref >= n - 1)) ok = false;
+    if (t >= 1 && active) {
+        nearest_smaller<kRunWarps>(S.plane, S.wmin, S.sep, pl, sv, M, na, nb);
+        in = na >= 0 && nb <= M;
+    }
+    if (in) {
+        const int L = S.xl[na], R = S.xl[nb] - 1;
+        const bool left = S.sep[nb] > S.sep[na];
+        root = L == 0 && R == n - 1;
+        P = root ? 0 : left ? R : L;
+        np = left ? nb : na;
+        if ((uint32_t)P >= (uint32_t)(n - 1)) {
             ok = false;
+            in = false;
+        } else {
+            S.P[t] = P;
+            win.get(na, nb, nlo, nhi);
+            nlo.w = __int_as_float(P);
+            if (!root && np > 0 && np < M) hand_over(S.rec, np, left, nlo, nhi);
         }
-        if (leaves(np)) {
-            S.out[na] = j;
+    }
+    const bool ileft = active && S.sep[t + 1] > sv;
+    const int ip = ileft ? t + 1 : t;
+    if (active && ip > 0 && ip < M) hand_over(S.rec, ip, ileft, ilo, ihi);
+    __syncthreads();
+    // parent links; what leaves: items and nodes of the run whose parent's node does not lie in it
+    if (active) {
+        const int q = ip > 0 && ip < M ? S.P[ip] : -1;
+        if (q < 0) S.out[t] = 0;
+        else if (ref >= -n && ref < n - 1) parents[ref >= 0 ? ref : n - (ref + 1)] = q;
+    }
+    if (in && !root) {
+        const int q = np > 0 && np < M ? S.P[np] : -1;
+        if (q >= 0) {
+            parents[P] = q;
+        } else {
+            S.out[na] = t;
             nhi.w = __int_as_float(nb);
-            S.lo[1][j] = nlo;  // the windows are read
-            S.hi[1][j] = nhi;
+            S.lo[1][t] = nlo;  // the windows are read
+            S.hi[1][t] = nhi;
         }
+    }
+    // the records, four threads each
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int j = r * (kRunCap / 4) + (t >> 2), part = t & 3;
+        if (r * (kRunCap / 4) >= M) break;  // uniform
+        const int q = S.P[j];
+        if (q >= 0) nodes[4ull * q + part] = S.rec[rec_at(j, part)];
     }
     __syncthreads();
     const int o = S.out[t];
     const uint32_t bal = __ballot_sync(0xFFFFFFFFu, o >= 0);
     if (lane == 0) S.warp[warp] = __popc(bal);
     float4 lo, hi;
-    int ref = 0, xl = 0, xr = 0, dl = 0, dr = 0;
+    int oref = 0, xl = 0, xr = 0, dl = 0, dr = 0;
     if (o >= 0) {
         lo = S.lo[o ? 1 : 0][o ? o : t];
         hi = S.hi[o ? 1 : 0][o ? o : t];
         const int b = o ? __float_as_int(hi.w) : t + 1;
-        ref = __float_as_int(lo.w);
+        oref = __float_as_int(lo.w);
         xl = S.xl[t];
         xr = S.xl[b] - 1;
         dl = S.sep[t];
@@ -788,17 +764,16 @@ __device__ __forceinline__ int reduce_run(RunSmem &S, int M, int n, float4 *node
         total += c;
     }
     if (dst) {
-        if (o >= 0 && at < kOpenCap) dst[at] = open_item(lo, hi, ref, xl, xr, dl, dr);
+        if (o >= 0 && at < kOpenCap) dst[at] = open_item(lo, hi, oref, xl, xr, dl ? dl : -1, dr ? dr : -1);
         return total;
     }
     if (o >= 0) {
-        lo.w = __int_as_float(ref);
         S.lo[0][at] = lo;
         S.hi[0][at] = hi;
         S.xl[at] = xl;
-        S.sep[at] = dl;
+        S.sep[at] = (uint8_t)dl;
     }
-    if (t == 0) { S.xl[total] = end_xl; S.sep[total] = end_sep; }
+    if (t == 0) { S.xl[total] = end_xl; S.sep[total] = (uint8_t)end_sep; }
     __syncthreads();
     return total;
 }
@@ -904,7 +879,7 @@ __global__ void __launch_bounds__(kRunCap, Groups::kCtas) k_top_group(Groups gro
                     it.pad0 = x.z;
                     S.out[t] = x.x;
                     // every first leaf inside the segment: what is derived from it then is too
-                    if (x.x < 0 || x.y < x.x || x.y >= n || x.z < -1 || x.z > 63) ok = false;
+                    if (x.x < 0 || x.y < x.x || x.y >= n) ok = false;
                 }
                 if (level == 1) {  // uniform
                     __syncthreads();
@@ -919,10 +894,10 @@ __global__ void __launch_bounds__(kRunCap, Groups::kCtas) k_top_group(Groups gro
                     S.lo[0][x] = it.lo;
                     S.hi[0][x] = it.hi;
                     S.xl[x] = it.xl;
-                    S.sep[x] = it.pad0;
+                    S.sep[x] = (uint8_t)min(max(it.pad0, 0), 63);
                     if (at == add - 1) {  // the run's end
                         S.xl[x + 1] = it.xr + 1;
-                        S.sep[x + 1] = __float_as_int(it.hi.w);
+                        S.sep[x + 1] = (uint8_t)min(max(__float_as_int(it.hi.w), 0), 63);
                     }
                 }
                 M += add;
