@@ -619,21 +619,24 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
 //
 // One block reduces a group of kGroupBlocks tree blocks; the last of kFan neighbouring groups to
 // finish (a counter per parent, nothing waits) goes on with what those groups left as one run,
-// and so on up to the root: three levels at 2^20 triangles, four at 2^24.  Latency bounds it: a
-// level is about eight block barriers and four dependent L2 accesses, 5 to 6 us.  Before, each
-// open item climbed one level of the tree at a time, parking and merging through shared-memory
-// hashes and then arrival words in L2 (0.5 to 2.6 us a level, up to 31 levels).  The pass, climbs
-// -> runs (B200): 4,098 triangles 19 -> 6 us, 65,536 uniform 35 -> 11, 1,000,003 clustered 63 ->
-// 26, the 2 M sphere 65 -> 34, 2^24 clustered 130 -> 91, 1,024 meshes of 33 M triangles 203 ->
-// 155; the scratch of arrival words and parked children (37 B per triangle) is gone.
+// and so on up to the root: three levels at 2^20 triangles, four at 2^24.  Latency bounds it: a level
+// is six block barriers and four dependent L2 accesses, about 4 us.  Before, each open item
+// climbed one level of the tree at a time, parking and merging through shared-memory hashes and
+// then arrival words in L2 (0.5 to 2.6 us a level, up to 31 levels).  The pass, climbs -> runs
+// (B200): 4,098 triangles 19 -> 5 us, 65,536 uniform 35 -> 10, 1,000,003 clustered 63 -> 22, the
+// 2 M sphere 65 -> 27, 2^24 clustered 130 -> 70, 1,024 meshes of 33 M triangles 203 -> 117; the
+// scratch of arrival words and parked children (37 B per triangle) is gone.  (Its first form found
+// separators with one ballot per value and had its windows from shared memory, a barrier each:
+// 11, 26, 35, 91 and 155 us.)
 //
 // Sizes: a run holds at most 256 items, one per thread: a child's open items (<= kOpenCap) always
 // fit beside what the children before it left (<= kOpenCap), so a run that would be longer is
 // reduced a few children at a time.  A tree block leaves 8.1 items on average (uniform and
 // clustered triangles), so a group of 24 blocks leaves 60 of 256 threads idle and rarely needs a
-// second turn.  24 blocks against 16 (more levels, more idle threads) at 2^24 and the batch:
-// 91 and 155 us against 109 and 173; 512 threads and 32 blocks: 117 and 231; 384 and 24: 110 and
-// 207 (fewer, longer blocks hide each other's latency less).
+// second turn.  16 blocks (more levels, more idle threads) take 89 us at 2^24 and 142 for the
+// batch, 28 blocks and 14 groups 68 and 109 but 23.1 (22.0) at 1,000,003 and 29.5 (27.3) for the
+// sphere; in the first form 512 threads and 32 blocks were slower than 256 and 24 (fewer, longer
+// blocks hide each other's latency less).
 constexpr int kRunCap = 256;
 constexpr int kRunWarps = kRunCap / 32;
 static_assert(kRunCap >= 2 * kOpenCap && kGroupBlocks <= 32 && kFan <= 32, "a run takes two children; one warp counts them");
@@ -786,14 +789,14 @@ struct GroupSpan {
 };
 template <int LOG>
 struct OneSegGroups {
-    static constexpr int kCtas = 3;  // 80 registers
+    static constexpr int kCtas = 3;  // 80 registers: 70 us at 2^24 either way, 22.0 against 23.3 at 1,000,003
     int n;
     __device__ __forceinline__ GroupSpan group(int g) const {
         return GroupSpan{0, n, 0, (n + (1 << LOG) - 1) >> LOG, g};
     }
 };
 struct ManySegGroups {  // groups never cross a segment; each starts at its segment's first group
-    static constexpr int kCtas = 4;  // many runs at once: 173 us at 4 against 185 at 3
+    static constexpr int kCtas = 4;  // many runs at once: 117 us at 4 against 122 at 3
     const SegRow *rows;
     const uint32_t *grp_seg;
     __device__ __forceinline__ GroupSpan group(int g) const {
