@@ -251,3 +251,18 @@ def test_lookback_wait_runs_out_then_clean_build(builder):
             assert_same(mesh_np(got, i), mesh_np(ref, i), f"mesh {i} after the timed-out build")
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("sizes,bits", [
+    ([4096] * 3, 10),                    # one sort tile each
+    ([4096, 4097, 8192, 1], 10),         # 6 tiles of 4 meshes
+    ([4097, 4097, 0, 1], 10),            # 5 tiles, an empty mesh
+    ([4097] * 3, 8),                     # two tiles each: the line
+    ([20_481, 1, 5, 4096], 8),           # one mesh holds most tiles
+])
+def test_batched_default_digits_follow_the_tiles(builder, sizes, bits):
+    import torch
+    tri, offs = make_batch(sizes, seed=47)
+    res = builder.build_batched(torch.from_numpy(tri).cuda(), offs)
+    assert builder.tunables()["digit_bits"] == bits
+    check_against_plain(builder, tri, offs, res)
