@@ -266,3 +266,29 @@ def test_batched_default_digits_follow_the_tiles(builder, sizes, bits):
     res = builder.build_batched(torch.from_numpy(tri).cuda(), offs)
     assert builder.tunables()["digit_bits"] == bits
     check_against_plain(builder, tri, offs, res)
+
+
+@pytest.mark.parametrize("digit_bits", [8, 10])
+@pytest.mark.parametrize("n", [8192, 12_288 - 31, 12_288 + 33, 20_000])
+@pytest.mark.parametrize("kind", ["equal", "runs", "half"])
+def test_batched_crowded_digits(builder, digit_bits, n, kind):
+    """Rows of 32 keys that share digits (peers above and below the crowd line), whole and ragged
+    sort tiles: equal triangles, runs of 3 to 40 equal ones, and every other row of 32 equal."""
+    import torch
+    from lvbh import scenes
+    tri = scenes.uniform_soup(n, seed=n, lo=(-1, -1, -1), hi=(1, 1, 1)).reshape(n, 12)
+    rng = np.random.default_rng(n)
+    if kind == "equal":
+        src = np.zeros(n, np.int64)
+    elif kind == "runs":
+        src = np.repeat(np.arange(n), rng.integers(3, 41, n))[:n]
+    else:
+        src = np.where((np.arange(n) // 32) % 2 == 0, 7, np.arange(n))
+    tri = np.concatenate([tri[src], tri[:5], tri[src][::-1]])
+    offs = np.array([0, n, n + 5, 2 * n + 5], np.int64)
+    builder.set_tunables(digit_bits=digit_bits, tree_block=256)
+    try:
+        res = builder.build_batched(torch.from_numpy(np.ascontiguousarray(tri)).cuda(), offs)
+    finally:
+        builder.set_tunables()
+    check_against_plain(builder, tri, offs, res)

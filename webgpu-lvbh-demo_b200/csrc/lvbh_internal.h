@@ -27,8 +27,8 @@ constexpr int kSortTile = kSortThreads * kSortItems; // keys per tile (4096)
 
 __host__ __device__ inline uint32_t sort_tiles(uint32_t n) { return (n + kSortTile - 1) / kSortTile; }
 
-// The plain build's sort scratch: per tile of kSortTile keys its kDigits counts of the pass's
-// digit, per chunk of sort_chunk_tiles(n) tiles their sum, per chunk the output offsets.  A
+// The plain build's sort scratch: per tile of kSortTile keys the kDigits counts of the pass's
+// digit over the chunk's earlier tiles, per chunk of sort_chunk_tiles(n) tiles their sum, per chunk the output offsets.  A
 // chunk is one block of the per-chunk kernels (Morton keys, tile histograms): 8 tiles when that
 // still gives kChunkFill blocks (two per SM), fewer for smaller sorts.
 constexpr int kSortChunkTiles = 8;

@@ -140,9 +140,9 @@ __global__ void __launch_bounds__(kThreads) k_bounds_cen(const float4 *__restric
 // K1b: per triangle box, centroid, quantisation and 30-bit Morton key, written in input order.
 // One block per chunk of sort_chunk_tiles(n) sort tiles: per tile each warp takes chunks of 32
 // triangles (96 consecutive float4, three coalesced 512-byte loads, transposed through shared
-// memory so that each lane owns a triangle); the digit counts of all three sort passes
-// accumulate over the block, and the counts of the first pass's digit per tile and per chunk
-// go straight to the sort's scratch, so the first sort pass starts from them.
+// memory so that each lane owns a triangle); the counts of the first pass's digit, per tile those
+// of the chunk's earlier tiles and per chunk their sum, go straight to the sort's scratch, so the
+// first sort pass starts from them.
 // kSrcMesh: the triangles are index triples into a buffer of 16-byte vertex rows (the indexed
 // leaf format's input); each lane gathers its triangle's three rows, an index past the buffer
 // reads row 0 and sets ERR_BAD_INDEX.  The centroids K1a stored are quantised by k_morton_cen.
@@ -253,9 +253,8 @@ __global__ void __launch_bounds__(THREADS) k_morton(const float4 *__restrict__ t
         uint32_t *row = tile_hist + (size_t)tile * kDigits + threadIdx.x * P;
 #pragma unroll
         for (int j = 0; j < P; ++j) {
-            const uint32_t c = th[threadIdx.x * P + j];
-            row[j] = c;
-            acc[j] += c;
+            row[j] = acc[j];  // of the chunk's earlier tiles
+            acc[j] += th[threadIdx.x * P + j];
         }
         __syncthreads();
     }
@@ -348,9 +347,8 @@ __global__ void __launch_bounds__(kCenThreads) k_morton_cen(const float *__restr
         uint32_t *row = tile_hist + (size_t)tile * kDigits + threadIdx.x * P;
 #pragma unroll
         for (int j = 0; j < P; ++j) {
-            const uint32_t c = th[b][threadIdx.x * P + j];
-            row[j] = c;
-            acc[j] += c;
+            row[j] = acc[j];  // of the chunk's earlier tiles
+            acc[j] += th[b][threadIdx.x * P + j];
         }
         // no barrier here: the next tile counts into th[b ^ 1], which this tile's first barrier
         // found read, and refills buffer b ^ 1 only, read before this tile's second barrier

@@ -9,9 +9,9 @@
 //   * the global digit counts of a pass are summed by its tile-histogram kernel (pass 0's by the
 //     Morton kernel, which writes pass 0's tile histograms with the keys);
 //   * a tile of 4096 keys (256 threads x 16) is ranked in shared memory: each warp walks its
-//     keys in input order; the lanes holding the same digit (its peers) are found with one
-//     ballot per digit bit, and the peers' lane order plus a per-warp running count in a
-//     16-bit shared counter gives each key its stable rank;
+//     keys in input order, finds the lanes holding the same digit (its peers, rank_warp), and the
+//     peers' lane order plus a per-warp running count in a 16-bit shared counter gives each key
+//     its stable rank;
 //   * the tile's digit counts are combined with earlier tiles by decoupled look-back: tiles
 //     are numbered by an atomic counter in launch order, each publishes its counts (flag
 //     AGGREGATE) and then its inclusive prefix (flag PREFIX) in one 32-bit word per digit, and
@@ -25,15 +25,23 @@
 // The plain build sorts one array of up to 2^29 keys, thousands of tiles long.  There a
 // look-back over 1024 digits would read 4 KB per predecessor tile and walk back about half a
 // wave of resident tiles, so its pass runs reduce-then-scan instead, with no waits at all:
-//   k_tile_hist   per tile of 4096 keys its digit counts, per chunk of 8 tiles their sum;
+//   k_tile_hist   per tile of 4096 keys the digit counts of its chunk's earlier tiles, per chunk
+//                 of 8 tiles their sum;
 //   k_chunk_scan  per chunk and digit the global output offset of the chunk's first key
 //                 (exclusive scan over chunks plus the digit's global start);
-//   k_scatter     ranks its tile as above, adds the counts of the earlier tiles of its chunk
-//                 (at most 7 rows of 4 KB, already final) to the chunk offset, and scatters.
+//   k_scatter     ranks its tile as above, adds its row of counts (4 KB, already final) to the
+//                 chunk offset, and scatters.
 // The batched build's segments span at most 64 tiles, so it keeps the one-kernel look-back.
 //
-// HBM-bound: per key one 4-byte key read (+4-byte value read after the first pass) and two
-// 4-byte writes (+ the 4-byte key read of k_tile_hist when reducing first).
+// Per key one 4-byte key read (+4-byte value read after the first pass) and two 4-byte writes (+
+// the 4-byte key read of k_tile_hist when reducing first), 41 us a pass of 2^24 keys at the copy
+// rate.  k_scatter takes 112 us (three passes 379 -> 337 us, 1,000,003 keys 39 -> 36, 2 M 64 -> 57):
+// it was issue-bound, 155 warp instructions per row of 32 keys, and is 123 since the counts are
+// read and prefixed two to a word, whole tiles skip the tests for the array's end, and a tile reads
+// one row of counts instead of up to seven; integer and shared-memory pipes are now busy about
+// two thirds of the time each (the scattered stores, 16 bytes to a run, take a quarter of the
+// latter).  Five or six blocks per SM instead of four, with the counts inside the staging buffers:
+// 351 and 383 us.
 #include "lvbh_device.cuh"
 #include "lvbh_internal.h"
 
@@ -102,13 +110,172 @@ struct ManySegSort {
 template <int BITS>
 struct SortSmem {
     static constexpr int D = 1 << BITS;
-    uint32_t keys[kSortTile];
-    uint32_t vals[kSortTile];
+    static constexpr bool kPeers = BITS == 8;
+    union {
+        struct {
+            uint32_t keys[kSortTile];
+            uint32_t vals[kSortTile];
+        };
+        uint32_t peers[kPeers ? W : 1][kPeers ? D : 1];  // while ranking: the lanes of a warp's row that hold a digit
+    };
     uint16_t whist[W][D];  // per-warp digit counts, then per-warp staging offsets
     uint32_t out[D];       // output position of staged index 0 of each digit
     uint32_t warp[W];
     uint32_t tile;
 };
+
+// Each warp clears its own counts and peer words (nothing else in the block touches them before
+// the barrier that ends the ranking).
+template <int BITS>
+__device__ __forceinline__ void clear_warp(SortSmem<BITS> &S, int warp, int lane) {
+    constexpr int D = 1 << BITS;
+    uint4 *h = reinterpret_cast<uint4 *>(S.whist[warp]);
+#pragma unroll
+    for (int i = 0; i < D / 8 / 32; ++i) h[32 * i + lane] = make_uint4(0u, 0u, 0u, 0u);
+    if constexpr (SortSmem<BITS>::kPeers) {
+        uint4 *m = reinterpret_cast<uint4 *>(S.peers[warp]);
+#pragma unroll
+        for (int i = 0; i < D / 4 / 32; ++i) m[32 * i + lane] = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+
+// Stable in-warp ranking, keys visited in input order (row-major, then lane): of the lanes holding
+// the same digit (its peers) the highest adds their number to the warp's count of the digit.  Peers
+// are found with one ballot per digit bit (five instructions each), or, with 8-bit digits, from a word
+// per digit into which each lane ORs its bit.  Ballots load the integer pipe and words the
+// shared-memory pipe, so three rows in four take words: four passes over 33.5 M keys in 1,024 meshes
+// took 802 us with ballots alone, 756, 717, 702 and 724 with one, two, three and four rows in four by
+// words.  Peers OR into their word one after the other, so after a ballot row with more than
+// kCrowd of them the next three rows use ballots too (720 us in all).  10-bit digits keep to ballots: their words
+// (32 KB a block) cost 375 us instead of 343 over the three passes of 2^24 keys.
+constexpr int kCrowd = 8;
+template <int BITS, bool FULL>
+__device__ __forceinline__ void rank_warp(SortSmem<BITS> &S, const uint32_t (&k)[IPT], uint32_t (&rank)[IPT / 2],
+                                          uint32_t wbase, uint32_t n, int shift, int warp, int lane) {
+    constexpr int D = 1 << BITS;
+    const uint32_t lt = lanemask_lt(), me = 1u << lane;
+    bool words = false;
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+        const bool valid = FULL || wbase + i * 32 + lane < n;
+        const uint32_t d = (k[i] >> shift) & (D - 1);
+        uint32_t peers = 0, cnt = 0;
+        if (valid) cnt = S.whist[warp][d];
+        if (SortSmem<BITS>::kPeers && i % 4 != 0 && words) {
+            uint32_t *w = &S.peers[warp][SortSmem<BITS>::kPeers ? d : 0];
+            if (valid) atomicOr(w, me);
+            __syncwarp();
+            if (valid) peers = *w;
+            __syncwarp();
+            if (peers >> lane == 1u) *w = 0;
+        } else {
+            peers = FULL ? 0xFFFFFFFFu : __ballot_sync(0xFFFFFFFFu, valid);
+#pragma unroll
+            for (int b = 0; b < BITS; ++b) {
+                const uint32_t bit = (d >> b) & 1u;
+                const uint32_t vote = __ballot_sync(0xFFFFFFFFu, bit);
+                peers &= bit ? vote : ~vote;
+            }
+            if (!valid) peers = 0;
+            if (SortSmem<BITS>::kPeers && i % 4 == 0) words = !__any_sync(0xFFFFFFFFu, __popc(peers) > kCrowd);
+            __syncwarp();
+        }
+        if (peers >> lane == 1u) S.whist[warp][d] = (uint16_t)(cnt + __popc(peers));
+        __syncwarp();
+        const uint32_t rk = cnt + __popc(peers & lt);
+        if (i & 1) rank[i / 2] |= rk << 16; else rank[i / 2] = rk;
+    }
+}
+
+// Thread tid owns digits tid * P .. tid * P + P - 1, whose 16-bit counts it takes two to a word (a
+// count or staging offset is at most kSortTile, so halves never carry).  The counts are read twice:
+// kept in registers in between they made k_scatter spill (357 us instead of 341 on 2^24 keys).
+template <int BITS>
+struct WarpCounts {
+    static constexpr int D = 1 << BITS, P = D / T, Q = (P + 1) / 2;
+    static_assert(P == 1 || P == 4, "one halfword or one 8-byte word per warp");
+    static __device__ __forceinline__ void ld(const SortSmem<BITS> &S, int w, int tid, uint32_t (&x)[Q]) {
+        if constexpr (P == 1) {
+            x[0] = S.whist[w][tid];
+        } else {
+            const uint2 v = *reinterpret_cast<const uint2 *>(&S.whist[w][tid * P]);
+            x[0] = v.x; x[Q - 1] = v.y;
+        }
+    }
+    // the tile's counts
+    static __device__ __forceinline__ void total(const SortSmem<BITS> &S, int tid, uint32_t (&cnt)[P]) {
+        uint32_t run[Q] = {};
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            uint32_t x[Q];
+            ld(S, w, tid, x);
+#pragma unroll
+            for (int q = 0; q < Q; ++q) run[q] += x[q];
+        }
+#pragma unroll
+        for (int j = 0; j < P; ++j) cnt[j] = (run[j / 2] >> (16 * (j & 1))) & 0xFFFFu;
+    }
+    // counts -> the staging position of each warp's first key of each digit; tst[j] is the tile's
+    static __device__ __forceinline__ void place(SortSmem<BITS> &S, int tid, const uint32_t (&tst)[P]) {
+        uint32_t run[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) run[q] = P == 1 ? tst[0] : tst[2 * q] | tst[(2 * q + 1) % P] << 16;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            uint32_t x[Q];
+            ld(S, w, tid, x);
+            if constexpr (P == 1) S.whist[w][tid] = (uint16_t)run[0];
+            else *reinterpret_cast<uint2 *>(&S.whist[w][tid * P]) = make_uint2(run[0], run[Q - 1]);
+#pragma unroll
+            for (int q = 0; q < Q; ++q) run[q] += x[q];
+        }
+    }
+};
+
+// Keys and values into digit order in shared memory.  Values go straight from global memory to their
+// slots by 4-byte asynchronous copies: all of a thread's copies are in flight at once and hold no
+// registers (loads followed by shared stores waited for each value in turn).
+template <int BITS, bool FULL>
+__device__ __forceinline__ void stage_tile(SortSmem<BITS> &S, const uint32_t (&k)[IPT], const uint32_t (&rank)[IPT / 2],
+                                           const uint32_t *__restrict__ vals_in, uint32_t wbase, uint32_t n, int shift,
+                                           int warp, int lane) {
+    constexpr int D = 1 << BITS;
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+        const uint32_t idx = wbase + i * 32 + lane;
+        if (FULL || idx < n) {
+            const uint32_t d = (k[i] >> shift) & (D - 1);
+            const uint32_t pos = S.whist[warp][d] + ((rank[i / 2] >> (16 * (i & 1))) & 0xFFFFu);
+            S.keys[pos] = k[i];
+            if (vals_in) cp_async4(&S.vals[pos], vals_in + idx);
+            else S.vals[pos] = idx;
+        }
+    }
+    cp_async_commit();
+}
+
+// The staged tile to its places: consecutive threads write consecutive words of each digit's run.
+template <int BITS, bool FULL>
+__device__ __forceinline__ void write_tile(const SortSmem<BITS> &S, uint32_t *__restrict__ keys_out,
+                                           uint32_t *__restrict__ vals_out, uint32_t tile_n, uint32_t n, int shift,
+                                           int tid, Control *ctl) {
+    constexpr int D = 1 << BITS;
+    bool oob = false;
+#pragma unroll (FULL ? 8 : 1)
+    for (int i = 0; i < IPT; ++i) {
+        const uint32_t j = i * T + tid;
+        if (!FULL && j >= tile_n) break;
+        const uint32_t key = S.keys[j];
+        const uint32_t o = S.out[(key >> shift) & (D - 1)] + j;
+        if (o < n) {  // always true for consistent counts (a look-back wait that gave up leaves others)
+            keys_out[o] = key;
+            vals_out[o] = S.vals[j];
+        } else {
+            oob = true;
+        }
+    }
+    if (oob) atomicOr(&ctl->err, ERR_SORT_RANGE);
+}
 
 template <int BITS, class Segs>
 __global__ void __launch_bounds__(T, 4) k_onesweep(Segs segs, const uint32_t *__restrict__ keys_all,
@@ -128,7 +295,7 @@ __global__ void __launch_bounds__(T, 4) k_onesweep(Segs segs, const uint32_t *__
     // test hook words (zero in normal use): a tile that publishes nothing, the wait bound
     const uint32_t stall1 = ctl->test_stall_tile1;
     const long long spin_limit = ctl->test_spin_limit ? (long long)ctl->test_spin_limit : kSpinLimitCycles;
-    for (int i = tid; i < W * D / 2; i += T) reinterpret_cast<uint32_t *>(&S.whist[0][0])[i] = 0;
+    clear_warp<BITS>(S, warp, lane);
     __syncthreads();
     const uint32_t tile = S.tile;
     const TileSpan sp = segs.span(tile);
@@ -150,45 +317,15 @@ __global__ void __launch_bounds__(T, 4) k_onesweep(Segs segs, const uint32_t *__
     if (vals_in && lane < IPT && wbase + lane * 32 < n)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(vals_in + wbase + lane * 32));
 
-    // Stable in-warp ranking, keys visited in input order (item-major, then lane).
+    const bool full = tile_base + (uint32_t)kSortTile <= n;
     uint32_t rank[IPT / 2];  // two 16-bit ranks per word
-    const uint32_t lt = lanemask_lt();
-#pragma unroll
-    for (int i = 0; i < IPT; ++i) {
-        const uint32_t idx = wbase + i * 32 + lane;
-        const bool valid = idx < n;
-        const uint32_t d = (k[i] >> shift) & (D - 1);
-        uint32_t peers = __ballot_sync(0xFFFFFFFFu, valid);
-#pragma unroll
-        for (int b = 0; b < BITS; ++b) {
-            const uint32_t bit = (d >> b) & 1u;
-            const uint32_t vote = __ballot_sync(0xFFFFFFFFu, bit);
-            peers &= bit ? vote : ~vote;
-        }
-        uint32_t cnt = 0;
-        if (valid) cnt = S.whist[warp][d];
-        __syncwarp();
-        if (valid && lane == 31 - __clz(peers)) S.whist[warp][d] = (uint16_t)(cnt + __popc(peers));
-        __syncwarp();
-        const uint32_t rk = cnt + __popc(peers & lt);
-        if (i & 1) rank[i / 2] |= rk << 16; else rank[i / 2] = rk;
-    }
+    if (full) rank_warp<BITS, true>(S, k, rank, wbase, n, shift, warp, lane);
+    else rank_warp<BITS, false>(S, k, rank, wbase, n, shift, warp, lane);
     __syncthreads();
 
-    // Per digit (thread tid owns digits tid*P .. tid*P+P-1): warp-exclusive prefixes (in place)
-    // and the tile's counts.
+    // The tile's counts (thread tid owns digits tid*P .. tid*P+P-1).
     uint32_t cnt[P];
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-        uint32_t c = 0;
-#pragma unroll
-        for (int w = 0; w < W; ++w) {
-            const uint32_t x = S.whist[w][tid * P + j];
-            S.whist[w][tid * P + j] = (uint16_t)c;
-            c += x;
-        }
-        cnt[j] = c;
-    }
+    WarpCounts<BITS>::total(S, tid, cnt);
 
     // Publish the tile's counts at once (its inclusive prefix when it is the segment's first
     // tile), so that later tiles can look back past it while it stages its keys.
@@ -205,29 +342,13 @@ __global__ void __launch_bounds__(T, 4) k_onesweep(Segs segs, const uint32_t *__
     for (int j = 0; j < P; ++j) tsum += cnt[j];
     uint32_t tstart = block_exclusive_scan(tsum, S.warp);
 #pragma unroll
-    for (int j = 0; j < P; ++j) {
-        const int dg = tid * P + j;
-        tst[j] = tstart;
-#pragma unroll
-        for (int w = 0; w < W; ++w) S.whist[w][dg] = (uint16_t)(S.whist[w][dg] + tstart);
-        tstart += cnt[j];
-    }
+    for (int j = 0; j < P; ++j) { tst[j] = tstart; tstart += cnt[j]; }
+    WarpCounts<BITS>::place(S, tid, tst);
     __syncthreads();
 
-    // Stage keys and values in digit order (values by 4-byte asynchronous copies, in flight
-    // during the look-back).
-#pragma unroll
-    for (int i = 0; i < IPT; ++i) {
-        const uint32_t idx = wbase + i * 32 + lane;
-        if (idx < n) {
-            const uint32_t d = (k[i] >> shift) & (D - 1);
-            const uint32_t pos = S.whist[warp][d] + ((rank[i / 2] >> (16 * (i & 1))) & 0xFFFFu);
-            S.keys[pos] = k[i];
-            if (vals_in) cp_async4(&S.vals[pos], vals_in + idx);
-            else S.vals[pos] = idx;
-        }
-    }
-    cp_async_commit();
+    // Stage keys and values in digit order; the values' copies are in flight during the look-back.
+    if (full) stage_tile<BITS, true>(S, k, rank, vals_in, wbase, n, shift, warp, lane);
+    else stage_tile<BITS, false>(S, k, rank, vals_in, wbase, n, shift, warp, lane);
 
     // Decoupled look-back across tiles, all P digits together: read kLookback predecessors
     // per digit at a time (independent loads), add their counts newest first until a PREFIX.
@@ -294,24 +415,12 @@ __global__ void __launch_bounds__(T, 4) k_onesweep(Segs segs, const uint32_t *__
     cp_async_wait_all();
     __syncthreads();
 
-    const uint32_t tile_n = min((uint32_t)kSortTile, n - tile_base);
-    bool oob = false;
-    for (uint32_t j = tid; j < tile_n; j += T) {
-        const uint32_t key = S.keys[j];
-        const uint32_t o = S.out[(key >> shift) & (D - 1)] + j;
-        if (o < n) {  // always true unless a look-back wait gave up or the counts are wrong
-            keys_out[o] = key;
-            vals_out[o] = S.vals[j];
-        } else {
-            oob = true;
-        }
-    }
-    if (oob) atomicOr(&ctl->err, ERR_SORT_RANGE);
+    if (full) write_tile<BITS, true>(S, keys_out, vals_out, (uint32_t)kSortTile, n, shift, tid, ctl);
+    else write_tile<BITS, false>(S, keys_out, vals_out, n - tile_base, n, shift, tid, ctl);
 }
 
-
-// Reduce: digit counts of every tile (tile_hist[tile][digit]) and of every chunk of chunk_tiles
-// tiles (chunk_sum[chunk][digit]), added up into the pass's global counts (ghist: kHistParts
+// Reduce: digit counts of the tiles before every tile in its chunk (tile_hist[tile][digit]) and of
+// every chunk of chunk_tiles tiles (chunk_sum[chunk][digit]), added up into the pass's global counts (ghist: kHistParts
 // partial rows, zero before; the chunk goes to row chunk % kHistParts).  One block per chunk;
 // each thread owns P contiguous digits.
 template <int BITS>
@@ -358,12 +467,9 @@ __global__ void __launch_bounds__(T) k_tile_hist(const uint32_t *__restrict__ ke
             else if (valid) atomicAdd(&h[d], 1u);
         }
         __syncthreads();
-        uint32_t c[P];
-#pragma unroll
-        for (int j = 0; j < P; ++j) { c[j] = h[tid * P + j]; acc[j] += c[j]; }
         uint32_t *row = tile_hist + (size_t)tile * D + tid * P;
 #pragma unroll
-        for (int j = 0; j < P; ++j) row[j] = c[j];
+        for (int j = 0; j < P; ++j) { row[j] = acc[j]; acc[j] += h[tid * P + j]; }
         __syncthreads();
     }
     uint32_t *row = chunk_sum + (size_t)blockIdx.x * D + tid * P;
@@ -439,7 +545,7 @@ __global__ void __launch_bounds__(T, 4) k_scatter(const uint32_t *__restrict__ k
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // each warp clears its own counts: the ranking below touches only those, so the warp starts it
     // without waiting for the block (a block barrier there cost about 1 us of the three passes)
-    for (int i = lane; i < D / 2; i += 32) reinterpret_cast<uint32_t *>(&S.whist[warp][0])[i] = 0;
+    clear_warp<BITS>(S, warp, lane);
     chain_wait();
     const uint32_t tile = blockIdx.x, tile_base = tile * (uint32_t)kSortTile;
     const int shift = pass * BITS;
@@ -455,106 +561,42 @@ __global__ void __launch_bounds__(T, 4) k_scatter(const uint32_t *__restrict__ k
     // them into L2 now (one 128-byte line of 32 values per lane)
     if (vals_in && lane < IPT && wbase + lane * 32 < n)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(vals_in + wbase + lane * 32));
-    // the digit prefixes of this tile (final values: independent 16-byte loads, all in flight
-    // with the keys), parked in S.out until the tile's own starts are known
+    // the digit prefixes of this tile (final values: two independent 16-byte loads, in flight with
+    // the keys), parked in S.out until the tile's own starts are known
     {
         static_assert(P == 4, "one 16-byte load per row");
-        const uint32_t chunk = tile / chunk_tiles, t0c = chunk * chunk_tiles;
-        uint4 acc = __ldg(reinterpret_cast<const uint4 *>(chunk_off + (size_t)chunk * D + tid * P));
-        uint4 row[kSortChunkTiles - 1];
-#pragma unroll
-        for (int q = 0; q < kSortChunkTiles - 1; ++q)
-            row[q] = t0c + q < tile ? __ldg(reinterpret_cast<const uint4 *>(tile_hist + (size_t)(t0c + q) * D + tid * P))
-                                    : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-        for (int q = 0; q < kSortChunkTiles - 1; ++q) {
-            acc.x += row[q].x; acc.y += row[q].y; acc.z += row[q].z; acc.w += row[q].w;
-        }
-        const uint32_t pre[P] = {acc.x, acc.y, acc.z, acc.w};
-#pragma unroll
-        for (int j = 0; j < P; ++j) S.out[tid * P + j] = pre[j];  // read after the barriers below
+        const uint4 c = __ldg(reinterpret_cast<const uint4 *>(chunk_off + (size_t)(tile / chunk_tiles) * D + tid * P));
+        const uint4 t = __ldg(reinterpret_cast<const uint4 *>(tile_hist + (size_t)tile * D + tid * P));
+        *reinterpret_cast<uint4 *>(&S.out[tid * P]) = make_uint4(c.x + t.x, c.y + t.y, c.z + t.z, c.w + t.w);
     }
     __syncwarp();
 
+    const bool full = tile_base + (uint32_t)kSortTile <= n;
     uint32_t rank[IPT / 2];
-    const uint32_t lt = lanemask_lt();
-#pragma unroll
-    for (int i = 0; i < IPT; ++i) {
-        const uint32_t idx = wbase + i * 32 + lane;
-        const bool valid = idx < n;
-        const uint32_t d = (k[i] >> shift) & (D - 1);
-        uint32_t peers = __ballot_sync(0xFFFFFFFFu, valid);
-#pragma unroll
-        for (int b = 0; b < BITS; ++b) {
-            const uint32_t bit = (d >> b) & 1u;
-            const uint32_t vote = __ballot_sync(0xFFFFFFFFu, bit);
-            peers &= bit ? vote : ~vote;
-        }
-        uint32_t cnt = 0;
-        if (valid) cnt = S.whist[warp][d];
-        __syncwarp();
-        if (valid && lane == 31 - __clz(peers)) S.whist[warp][d] = (uint16_t)(cnt + __popc(peers));
-        __syncwarp();
-        const uint32_t rk = cnt + __popc(peers & lt);
-        if (i & 1) rank[i / 2] |= rk << 16; else rank[i / 2] = rk;
-    }
+    if (full) rank_warp<BITS, true>(S, k, rank, wbase, n, shift, warp, lane);
+    else rank_warp<BITS, false>(S, k, rank, wbase, n, shift, warp, lane);
     __syncthreads();
 
-    uint32_t cnt[P], tsum = 0;
+    uint32_t cnt[P], tst[P], tsum = 0;
+    WarpCounts<BITS>::total(S, tid, cnt);
 #pragma unroll
-    for (int j = 0; j < P; ++j) {
-        uint32_t c = 0;
-#pragma unroll
-        for (int w = 0; w < W; ++w) {
-            const uint32_t x = S.whist[w][tid * P + j];
-            S.whist[w][tid * P + j] = (uint16_t)c;
-            c += x;
-        }
-        cnt[j] = c;
-        tsum += c;
-    }
+    for (int j = 0; j < P; ++j) tsum += cnt[j];
     uint32_t tstart = block_exclusive_scan(tsum, S.warp);
 #pragma unroll
     for (int j = 0; j < P; ++j) {
-        const int dg = tid * P + j;
-#pragma unroll
-        for (int w = 0; w < W; ++w) S.whist[w][dg] = (uint16_t)(S.whist[w][dg] + tstart);
-        S.out[dg] -= tstart;
+        tst[j] = tstart;
+        S.out[tid * P + j] -= tstart;
         tstart += cnt[j];
     }
+    WarpCounts<BITS>::place(S, tid, tst);
     __syncthreads();
 
-    // the values go straight from global memory to their staged slots by 4-byte asynchronous
-    // copies: all of a thread's copies are in flight at once and hold no registers (loads
-    // followed by shared stores waited for each value in turn)
-#pragma unroll
-    for (int i = 0; i < IPT; ++i) {
-        const uint32_t idx = wbase + i * 32 + lane;
-        if (idx < n) {
-            const uint32_t d = (k[i] >> shift) & (D - 1);
-            const uint32_t pos = S.whist[warp][d] + ((rank[i / 2] >> (16 * (i & 1))) & 0xFFFFu);
-            S.keys[pos] = k[i];
-            if (vals_in) cp_async4(&S.vals[pos], vals_in + idx);
-            else S.vals[pos] = idx;
-        }
-    }
-    cp_async_commit();
+    if (full) stage_tile<BITS, true>(S, k, rank, vals_in, wbase, n, shift, warp, lane);
+    else stage_tile<BITS, false>(S, k, rank, vals_in, wbase, n, shift, warp, lane);
     cp_async_wait_all();
     __syncthreads();
-
-    const uint32_t tile_n = min((uint32_t)kSortTile, n - tile_base);
-    bool oob = false;
-    for (uint32_t j = tid; j < tile_n; j += T) {
-        const uint32_t key = S.keys[j];
-        const uint32_t o = S.out[(key >> shift) & (D - 1)] + j;
-        if (o < n) {  // always true for consistent counts
-            keys_out[o] = key;
-            vals_out[o] = S.vals[j];
-        } else {
-            oob = true;
-        }
-    }
-    if (oob) atomicOr(&ctl->err, ERR_SORT_RANGE);
+    if (full) write_tile<BITS, true>(S, keys_out, vals_out, (uint32_t)kSortTile, n, shift, tid, ctl);
+    else write_tile<BITS, false>(S, keys_out, vals_out, n - tile_base, n, shift, tid, ctl);
 }
 
 template <int BITS, class Segs>
