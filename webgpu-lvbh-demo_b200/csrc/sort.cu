@@ -482,9 +482,9 @@ __global__ void __launch_bounds__(T) k_tile_hist(const uint32_t *__restrict__ ke
 
 // Scan: chunk_off[c][d] = start of digit d in the pass's output (exclusive scan of the global
 // counts over digits, the kHistParts partial rows of ghist summed) + counts of digit d in chunks
-// before c.  Block b covers digits
-// 32b .. 32b+31 (lane = digit); its 32 warps split the chunks.
+// before c.  Block b covers digits 32b .. 32b+31 (lane = digit); its 32 warps split the chunks.
 constexpr int kScanThreads = 1024;
+constexpr int kScanKeep = 16;  // 512 chunks: every sort up to 2^24 keys
 template <int BITS>
 __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(const uint32_t *__restrict__ chunk_sum,
                                                              uint32_t chunks,
@@ -497,6 +497,14 @@ __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(const uint32_t *__r
     __shared__ uint32_t s_part[SW][32];
     chain_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // a warp's chunks, the first kScanKeep of them held in registers for both sweeps: their loads
+    // are in flight together, and with the global counts
+    const uint32_t per = (chunks + SW - 1) / SW;
+    const uint32_t c0 = warp * per, c1 = min(chunks, c0 + per);
+    const int d0 = blockIdx.x * 32, d = d0 + lane;
+    uint32_t keep[kScanKeep], sum = 0;
+#pragma unroll
+    for (int i = 0; i < kScanKeep; ++i) keep[i] = c0 + i < c1 ? __ldg(chunk_sum + (size_t)(c0 + i) * D + d) : 0u;
     // digit starts: exclusive scan of the global counts, one digit per thread
     uint32_t g = 0;
 #pragma unroll
@@ -511,18 +519,20 @@ __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(const uint32_t *__r
     __syncthreads();
     uint32_t woff = 0;
     for (int w = 0; w < warp; ++w) woff += s_wsum[w];
-    const int d0 = blockIdx.x * 32;
     if (tid >= d0 && tid < d0 + 32) s_base[tid - d0] = woff + incl - g;
-    const uint32_t per = (chunks + SW - 1) / SW;
-    const uint32_t c0 = warp * per, c1 = min(chunks, c0 + per);
-    const int d = d0 + lane;
-    uint32_t sum = 0;
-    for (uint32_t c = c0; c < c1; ++c) sum += __ldg(chunk_sum + (size_t)c * D + d);
+    for (uint32_t c = c0 + kScanKeep; c < c1; ++c) sum += __ldg(chunk_sum + (size_t)c * D + d);
+#pragma unroll
+    for (int i = 0; i < kScanKeep; ++i) sum += keep[i];
     s_part[warp][lane] = sum;
     __syncthreads();
     uint32_t off = s_base[lane];
     for (int w = 0; w < warp; ++w) off += s_part[w][lane];
-    for (uint32_t c = c0; c < c1; ++c) {
+#pragma unroll
+    for (int i = 0; i < kScanKeep; ++i) {
+        if (c0 + i < c1) chunk_off[(size_t)(c0 + i) * D + d] = off;
+        off += keep[i];
+    }
+    for (uint32_t c = c0 + kScanKeep; c < c1; ++c) {
         chunk_off[(size_t)c * D + d] = off;
         off += __ldg(chunk_sum + (size_t)c * D + d);
     }
