@@ -1,4 +1,4 @@
-"""The one-kernel front of small builds (up to 131,072 triangles) at the edges of its blocks and keys
+"""The one-kernel front of small builds (65,536 triangles and fewer) at the edges of its blocks and keys
 per thread, and builds in buffers that repeat, alternate and change (launched directly or as a graph)."""
 import numpy as np
 import pytest

@@ -172,7 +172,7 @@ cudaError_t morton_init();  // once per device, before the first launch
 // K1 + K2 of a small build in one cluster kernel (small.cu): box, keys, sorted keys and
 // permutation, and the control block's error word and box (nothing to clear before).  kv: 2 n words
 // of scratch, 8-byte aligned.
-constexpr uint32_t kSmallMax = 1u << 17;  // where the two paths take the same time (small.cu)
+constexpr uint32_t kSmallMax = 1u << 16;  // both sides measured: small.cu
 bool small_build(uint32_t n);  // whether n triangles take it on this device
 cudaError_t small_init();      // once per device, before the first launch
 cudaError_t launch_small_sort(const float4 *tri, uint32_t n, const HostBounds &hb, Control *ctl, uint32_t *kv,

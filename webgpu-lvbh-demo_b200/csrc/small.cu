@@ -9,15 +9,16 @@
 // distributed shared memory and the keys through L2, with two cluster barriers per pass.  Results
 // are those of the general path (morton.cu, sort.cu).
 //
-// What bounds it: 16 SMs.  Of 61,000 cycles at 65,536 triangles (4 keys a thread) ranking takes
-// 21,000 (ALU: about 150 cycles a warp, key and scheduler), moving the keys 18,000, the rest is
-// reading triangles, quantising and barriers; 17 us at 4,098 triangles, 32 at 65,536.  Whole calls
-// in kept buffers, general path -> this one (B200): 64 triangles 72 -> 49 us, 1,000 83 -> 52,
-// 4,098 85 -> 56, 65,536 101 -> 81, 98,304 108 -> 101, 131,072 110 -> 107, 163,840 121 -> 132; so
-// kSmallMax is 131,072.  Measured on it: keys scattered through distributed shared memory
-// instead of L2 8,700 cycles a pass instead of 4,300 (two cycles a store either way until the keys
-// are put in digit order first), three 10-bit passes 35 us instead of 32, __match_any_sync for
-// the ballots 40 us.
+// What bounds it: 16 SMs.  Of 61,000 cycles at 65,536 triangles (4 keys a thread) ranking by ballots
+// took 21,000 (integer pipe: about 150 cycles a warp, key and scheduler), moving the keys 18,000,
+// the rest was reading triangles, quantising and barriers; with three rows in four ranked by words
+// (k_onesweep's mix, sort.cu) the kernel takes 29 us instead of 32, 17 at 4,098 triangles.  Whole
+// calls in kept buffers, general path -> this one (B200, clustered): 1,000 triangles 81 -> 55 us,
+// 4,098 83 -> 62, 20,000 93 -> 74, 50,000 95 -> 86, 65,536 95 -> 86 (uniform 93 -> 79), 81,920 98 ->
+// 100, 131,072 106 -> 122 (eight keys a thread); so kSmallMax is 65,536.  Measured on it: keys
+// scattered through distributed shared memory instead of L2 8,700 cycles a pass instead of 4,300
+// (two cycles a store either way until the keys are put in digit order first), three 10-bit passes
+// 35 us instead of 32, __match_any_sync for the ballots 40 us.
 #include <cooperative_groups.h>
 
 #include "lvbh_device.cuh"
@@ -40,6 +41,7 @@ constexpr int D = kDigits32, kPasses = kSortPasses32, kBits = kDigitBits32;
 // words of eight rows, every fourth row) then meet 32 different banks.
 constexpr int kRow = D / 2 + 1;
 constexpr int kParts = T / (D / 2), kPartRows = W / kParts;
+constexpr int kCrowd = 8;  // peers in a ballot row above which the next three rows use ballots too
 static_assert(kParts == 8 && kPartRows == 4, "one thread per word and group of four warps");
 
 // IPT keys per thread.
@@ -54,6 +56,8 @@ struct SmallSmem {
                                       // block's digit
         };
     };
+    uint32_t peers[IPT > 1 ? W : 1][IPT > 1 ? D : 4];  // the lanes of a warp's row that hold a digit (zero
+                                                       // between rows)
     uint32_t cnt[D / 2];    // the block's digit counts, two to a word ...
     uint32_t all[kMaxBlocks][D / 2];  // ... and every block's (each writes its row in all blocks: reading
                                       // the other blocks' rows took 4,200 cycles a pass instead)
@@ -175,6 +179,10 @@ __global__ void __launch_bounds__(T) k_small_sort(const float4 *__restrict__ row
     }
     __syncthreads();  // the centroids are read; keys and counts take their place
 
+    if constexpr (IPT > 1) {
+#pragma unroll
+        for (int i = 0; i < D / 32; ++i) S.peers[warp][32 * i + lane] = 0u;
+    }
     uint16_t *own = reinterpret_cast<uint16_t *>(S.whist[warp]);  // digit d at own[d]
     const uint32_t mine = min((uint32_t)(IPT * T), n - min(n, rank * (IPT * T)));  // the block's keys
     for (int pass = 0; pass < kPasses; ++pass) {
@@ -182,22 +190,35 @@ __global__ void __launch_bounds__(T) k_small_sort(const float4 *__restrict__ row
 #pragma unroll
         for (int i = 0; i < D / 64; ++i) S.whist[warp][32 * i + lane] = 0u;
         __syncwarp();
-        // stable ranks within the warp, as in k_scatter
+        // stable ranks within the warp, as in k_onesweep: after a ballot row, up to three by words
+        bool words = false;
         uint32_t rk[(IPT + 1) / 2];
 #pragma unroll
         for (int i = 0; i < IPT; ++i) {
             const bool valid = base + 32 * i < n;
             const uint32_t d = (k[i] >> shift) & (D - 1);
-            uint32_t peers = __ballot_sync(0xFFFFFFFFu, valid);
-#pragma unroll
-            for (int b = 0; b < kBits; ++b) {
-                const uint32_t bit = (d >> b) & 1u;
-                const uint32_t vote = __ballot_sync(0xFFFFFFFFu, bit);
-                peers &= bit ? vote : ~vote;
-            }
             const uint32_t c = own[d];  // (of digit 0 for a lane past the end: not used)
-            __syncwarp();
-            if (valid && lane == 31 - __clz(peers)) own[d] = (uint16_t)(c + __popc(peers));
+            uint32_t peers = 0;
+            if (IPT > 1 && i % 4 != 0 && words) {
+                uint32_t *w = &S.peers[IPT > 1 ? warp : 0][IPT > 1 ? d : 0];
+                if (valid) atomicOr(w, 1u << lane);
+                __syncwarp();
+                if (valid) peers = *w;
+                __syncwarp();
+                if (peers >> lane == 1u) *w = 0u;
+            } else {
+                peers = __ballot_sync(0xFFFFFFFFu, valid);
+#pragma unroll
+                for (int b = 0; b < kBits; ++b) {
+                    const uint32_t bit = (d >> b) & 1u;
+                    const uint32_t vote = __ballot_sync(0xFFFFFFFFu, bit);
+                    peers &= bit ? vote : ~vote;
+                }
+                if (!valid) peers = 0;
+                if (IPT > 1 && i % 4 == 0) words = !__any_sync(0xFFFFFFFFu, __popc(peers) > kCrowd);
+                __syncwarp();
+            }
+            if (peers >> lane == 1u) own[d] = (uint16_t)(c + __popc(peers));
             __syncwarp();
             const uint32_t x = c + __popc(peers & lt);
             if (i & 1) rk[i / 2] |= x << 16; else rk[i / 2] = x;
@@ -343,9 +364,8 @@ cudaError_t launch_src(const float4 *rows, const uint32_t *idx3, uint32_t nverts
     const uint32_t per = (n + kMaxBlocks * T - 1) / (kMaxBlocks * T);
     if (per <= 1) return launch_ipt<SRC, 1>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, s);
     if (per <= 2) return launch_ipt<SRC, 2>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, s);
-    if (per <= 4) return launch_ipt<SRC, 4>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, s);
-    static_assert(kSmallMax <= 8 * kMaxBlocks * T, "eight keys per thread are enough");
-    return launch_ipt<SRC, 8>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, s);
+    static_assert(kSmallMax <= 4 * kMaxBlocks * T, "four keys per thread are enough");
+    return launch_ipt<SRC, 4>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, s);
 }
 
 int g_small_ok[64];  // per device: 1 when a full cluster of every form fits
@@ -364,11 +384,9 @@ cudaError_t small_init() {
     cudaError_t e = small_attrs<kSoup, 1>(&c);
     if (e == cudaSuccess) e = small_attrs<kSoup, 2>(&c);
     if (e == cudaSuccess) e = small_attrs<kSoup, 4>(&c);
-    if (e == cudaSuccess) e = small_attrs<kSoup, 8>(&c);
     if (e == cudaSuccess) e = small_attrs<kMesh, 1>(&c);
     if (e == cudaSuccess) e = small_attrs<kMesh, 2>(&c);
     if (e == cudaSuccess) e = small_attrs<kMesh, 4>(&c);
-    if (e == cudaSuccess) e = small_attrs<kMesh, 8>(&c);
     if (e == cudaSuccess && dev >= 0 && dev < 64) g_small_ok[dev] = c > 0;
     return e;
 }
