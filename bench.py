@@ -66,8 +66,10 @@ MODEL_BYTES = {"bounds": 48, "morton": 52, "sort": 48, "gather": 0, "tree": 192,
 KERNELS = {"bounds": ("k_bounds_cen", 1), "morton": ("k_morton_cen", 1), "sort": ("k_scatter", 3),
            "gather": (None, 0), "tree": ("k_tree_climb", 1), "top": ("k_top_group", 1)}
 # box and centroids, Morton keys (+ the first pass's tile histograms), 3 sort passes x (chunk
-# scan, scatter) and 2 tile-histogram passes, tree, straddling pass (group level, then global)
+# scan, scatter) and 2 tile-histogram passes, tree, straddling pass; up to SMALL_BUILD triangles
+# the stages before the tree are one kernel
 LAUNCHES_PER_BUILD = 12
+SMALL_BUILD = 65_536
 MODEL_TOTAL = sum(MODEL_BYTES.values())  # 340 B per triangle
 
 
@@ -457,7 +459,7 @@ def run_ours(args, world, rank, local):
             "config": {"workload": wname, "num_tris": n, "parallelism": "replicas" if world > 1 else "single",
                        "bounds": "reduced on the device over all vertices",
                        "l2": "input soup 805 MB > 126 MB L2; no flush", "graph": True},
-            "gpu_launches": LAUNCHES_PER_BUILD * args.steps,
+            "gpu_launches": (LAUNCHES_PER_BUILD if n > SMALL_BUILD else 3) * args.steps,
             "roofline": roofline, "stage_ms": stage_ms, "cpu_baseline": cpu, "e2e": e2e_line,
             "clocks": clock_summary, "batched": batched, "served": served, "trace": trace, "obj": obj,
             "pt": pt, "mesh": mesh}

@@ -2,8 +2,9 @@
 //
 // Replaces the reference's host orchestration (scripts/bvh/build-bvh.js:12-66 and each kernel
 // module's execute(): 69 queue submits and 20 host waits per build) with one stream-ordered
-// chain of 8 kernels and a memset, replayed as a cached CUDA graph when the same build shape
-// repeats, and a single host wait at the end (none with LVBH_ASYNC).
+// chain of kernels (12 and a memset; 3 for up to kSmallMax triangles), replayed as a cached CUDA
+// graph when a build repeats in its buffers, and a single host wait at the end (none with
+// LVBH_ASYNC).
 #include <algorithm>
 #include <cmath>
 #include <cstddef>

@@ -10,7 +10,7 @@ namespace lvbh {
 enum : uint32_t {
     ERR_NONFINITE = 1u,         // a vertex coordinate is NaN or +-Inf
     ERR_LOOKBACK_TIMEOUT = 2u,  // a decoupled look-back wait exceeded its bound
-    ERR_CLIMB = 4u,             // a refit climb exceeded the depth any valid tree has
+    ERR_CLIMB = 4u,             // a block or run left more open items than a valid tree can
     ERR_BAD_INDEX = 8u,         // an indexed-mesh vertex index is out of range
     ERR_COPY_TIMEOUT = 16u,     // a copy wait (mbarrier) exceeded its bound
     ERR_SORT_RANGE = 32u,       // a radix sort scatter target fell outside the array (digit
