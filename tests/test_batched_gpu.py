@@ -254,11 +254,11 @@ def test_lookback_wait_runs_out_then_clean_build(builder):
 
 
 @pytest.mark.parametrize("sizes,bits", [
-    ([4096] * 3, 10),                    # one sort tile each
-    ([4096, 4097, 8192, 1], 10),         # 6 tiles of 4 meshes
-    ([4097, 4097, 0, 1], 10),            # 5 tiles, an empty mesh
-    ([4097] * 3, 8),                     # two tiles each: the line
-    ([20_481, 1, 5, 4096], 8),           # one mesh holds most tiles
+    ([64] * 63, 10),                        # 63 sort tiles
+    ([64] * 62 + [0, 4096], 10),            # an empty mesh has none
+    ([64] * 62 + [4097], 8),                # 64: the line
+    ([258_048], 10),                        # one mesh of 63 tiles
+    ([258_049, 1], 8),                      # of 64, and a mesh of one triangle
 ])
 def test_batched_default_digits_follow_the_tiles(builder, sizes, bits):
     import torch

@@ -930,12 +930,13 @@ int lvbh_build_batched(lvbh_ctx *ctx, const float *tri_array, const uint32_t *se
         return fail(ctx, LVBH_EINVAL, "device tri_array must be 16-byte aligned");
     }
     // the tunables: forced, tuned before for this size histogram, tuned now, or the defaults: digits
-    // of 10 bits (three passes) where meshes are mostly one sort tile, else of 8 (four passes, whose
-    // look-back reads a quarter of the words per tile): 512 meshes of one tile 190 us with 10 bits,
-    // 192 with 8; 64 meshes of 3 tiles on average 171 and 169; 1,024 of 3 tiles 1,056 and 1,037,
-    // of 8 tiles 3,212 and 3,027
+    // of 8 bits (four passes, a quarter of the counts to clear, look back over and hold a tile) from 64
+    // sort tiles on, below them of 10 (three passes: one launch less).  10 bits against 8 (B200): 8
+    // meshes 93 and 94 us, 64 of one tile or two 130 and 130, 64 of three 174 and 165, 512 of one 188
+    // and 179, 4,096 of up to 256 triangles 478 and 402, 1,024 of three tiles 1,042 and 995, of eight
+    // 3,214 and 2,898
     Tuned choice;
-    choice.t.digit_bits = tiles >= 2ull * num_segs ? kDigitBits32 : kDigitBits;
+    choice.t.digit_bits = tiles >= 64 ? kDigitBits32 : kDigitBits;
     if (ctx->forced) {
         choice.t = ctx->forced_t;
     } else if (flags & LVBH_AUTOTUNE) {
