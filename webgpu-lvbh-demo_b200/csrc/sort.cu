@@ -107,16 +107,15 @@ struct ManySegSort {
     }
 };
 
-template <int BITS>
+template <int BITS, bool WORDS = BITS == 8>  // WORDS: room for the peer words of rank_warp
 struct SortSmem {
     static constexpr int D = 1 << BITS;
-    static constexpr bool kPeers = BITS == 8;
     union {
         struct {
             uint32_t keys[kSortTile];
             uint32_t vals[kSortTile];
         };
-        uint32_t peers[kPeers ? W : 1][kPeers ? D : 1];  // while ranking: the lanes of a warp's row that hold a digit
+        uint32_t peers[WORDS ? W : 1][WORDS ? D : 1];  // while ranking: the lanes of a warp's row that hold a digit
     };
     uint16_t whist[W][D];  // per-warp digit counts, then per-warp staging offsets
     uint32_t out[D];       // output position of staged index 0 of each digit
@@ -126,13 +125,13 @@ struct SortSmem {
 
 // Each warp clears its own counts and peer words (nothing else in the block touches them before
 // the barrier that ends the ranking).
-template <int BITS>
-__device__ __forceinline__ void clear_warp(SortSmem<BITS> &S, int warp, int lane) {
+template <int BITS, bool WORDS>
+__device__ __forceinline__ void clear_warp(SortSmem<BITS, WORDS> &S, int warp, int lane) {
     constexpr int D = 1 << BITS;
     uint4 *h = reinterpret_cast<uint4 *>(S.whist[warp]);
 #pragma unroll
     for (int i = 0; i < D / 8 / 32; ++i) h[32 * i + lane] = make_uint4(0u, 0u, 0u, 0u);
-    if constexpr (SortSmem<BITS>::kPeers) {
+    if constexpr (WORDS) {
         uint4 *m = reinterpret_cast<uint4 *>(S.peers[warp]);
 #pragma unroll
         for (int i = 0; i < D / 4 / 32; ++i) m[32 * i + lane] = make_uint4(0u, 0u, 0u, 0u);
@@ -146,11 +145,12 @@ __device__ __forceinline__ void clear_warp(SortSmem<BITS> &S, int warp, int lane
 // shared-memory pipe, so three rows in four take words: four passes over 33.5 M keys in 1,024 meshes
 // took 802 us with ballots alone, 756, 717, 702 and 724 with one, two, three and four rows in four by
 // words.  Peers OR into their word one after the other, so after a ballot row with more than
-// kCrowd of them the next three rows use ballots too (720 us in all).  10-bit digits keep to ballots: their words
-// (32 KB a block) cost 375 us instead of 343 over the three passes of 2^24 keys.
+// kCrowd of them the next three rows use ballots too (720 us in all).  With 10-bit
+// digits (32 KB of words a block) words are taken up to kWordTiles tiles (launch_sort_pass).
 constexpr int kCrowd = 8;
-template <int BITS, bool FULL>
-__device__ __forceinline__ void rank_warp(SortSmem<BITS> &S, const uint32_t (&k)[IPT], uint32_t (&rank)[IPT / 2],
+constexpr uint32_t kWordTiles = 512;
+template <int BITS, bool FULL, bool WORDS>
+__device__ __forceinline__ void rank_warp(SortSmem<BITS, WORDS> &S, const uint32_t (&k)[IPT], uint32_t (&rank)[IPT / 2],
                                           uint32_t wbase, uint32_t n, int shift, int warp, int lane) {
     constexpr int D = 1 << BITS;
     const uint32_t lt = lanemask_lt(), me = 1u << lane;
@@ -161,8 +161,8 @@ __device__ __forceinline__ void rank_warp(SortSmem<BITS> &S, const uint32_t (&k)
         const uint32_t d = (k[i] >> shift) & (D - 1);
         uint32_t peers = 0, cnt = 0;
         if (valid) cnt = S.whist[warp][d];
-        if (SortSmem<BITS>::kPeers && i % 4 != 0 && words) {
-            uint32_t *w = &S.peers[warp][SortSmem<BITS>::kPeers ? d : 0];
+        if (WORDS && i % 4 != 0 && words) {
+            uint32_t *w = &S.peers[warp][WORDS ? d : 0];
             if (valid) atomicOr(w, me);
             __syncwarp();
             if (valid) peers = *w;
@@ -177,7 +177,7 @@ __device__ __forceinline__ void rank_warp(SortSmem<BITS> &S, const uint32_t (&k)
                 peers &= bit ? vote : ~vote;
             }
             if (!valid) peers = 0;
-            if (SortSmem<BITS>::kPeers && i % 4 == 0) words = !__any_sync(0xFFFFFFFFu, __popc(peers) > kCrowd);
+            if (WORDS && i % 4 == 0) words = !__any_sync(0xFFFFFFFFu, __popc(peers) > kCrowd);
             __syncwarp();
         }
         if (peers >> lane == 1u) S.whist[warp][d] = (uint16_t)(cnt + __popc(peers));
@@ -194,7 +194,8 @@ template <int BITS>
 struct WarpCounts {
     static constexpr int D = 1 << BITS, P = D / T, Q = (P + 1) / 2;
     static_assert(P == 1 || P == 4, "one halfword or one 8-byte word per warp");
-    static __device__ __forceinline__ void ld(const SortSmem<BITS> &S, int w, int tid, uint32_t (&x)[Q]) {
+    template <class Smem>
+    static __device__ __forceinline__ void ld(const Smem &S, int w, int tid, uint32_t (&x)[Q]) {
         if constexpr (P == 1) {
             x[0] = S.whist[w][tid];
         } else {
@@ -203,7 +204,8 @@ struct WarpCounts {
         }
     }
     // the tile's counts
-    static __device__ __forceinline__ void total(const SortSmem<BITS> &S, int tid, uint32_t (&cnt)[P]) {
+    template <class Smem>
+    static __device__ __forceinline__ void total(const Smem &S, int tid, uint32_t (&cnt)[P]) {
         uint32_t run[Q] = {};
 #pragma unroll
         for (int w = 0; w < W; ++w) {
@@ -216,7 +218,8 @@ struct WarpCounts {
         for (int j = 0; j < P; ++j) cnt[j] = (run[j / 2] >> (16 * (j & 1))) & 0xFFFFu;
     }
     // counts -> the staging position of each warp's first key of each digit; tst[j] is the tile's
-    static __device__ __forceinline__ void place(SortSmem<BITS> &S, int tid, const uint32_t (&tst)[P]) {
+    template <class Smem>
+    static __device__ __forceinline__ void place(Smem &S, int tid, const uint32_t (&tst)[P]) {
         uint32_t run[Q];
 #pragma unroll
         for (int q = 0; q < Q; ++q) run[q] = P == 1 ? tst[0] : tst[2 * q] | tst[(2 * q + 1) % P] << 16;
@@ -235,8 +238,8 @@ struct WarpCounts {
 // Keys and values into digit order in shared memory.  Values go straight from global memory to their
 // slots by 4-byte asynchronous copies: all of a thread's copies are in flight at once and hold no
 // registers (loads followed by shared stores waited for each value in turn).
-template <int BITS, bool FULL>
-__device__ __forceinline__ void stage_tile(SortSmem<BITS> &S, const uint32_t (&k)[IPT], const uint32_t (&rank)[IPT / 2],
+template <int BITS, bool FULL, bool WORDS>
+__device__ __forceinline__ void stage_tile(SortSmem<BITS, WORDS> &S, const uint32_t (&k)[IPT], const uint32_t (&rank)[IPT / 2],
                                            const uint32_t *__restrict__ vals_in, uint32_t wbase, uint32_t n, int shift,
                                            int warp, int lane) {
     constexpr int D = 1 << BITS;
@@ -255,8 +258,8 @@ __device__ __forceinline__ void stage_tile(SortSmem<BITS> &S, const uint32_t (&k
 }
 
 // The staged tile to its places: consecutive threads write consecutive words of each digit's run.
-template <int BITS, bool FULL>
-__device__ __forceinline__ void write_tile(const SortSmem<BITS> &S, uint32_t *__restrict__ keys_out,
+template <int BITS, bool FULL, bool WORDS>
+__device__ __forceinline__ void write_tile(const SortSmem<BITS, WORDS> &S, uint32_t *__restrict__ keys_out,
                                            uint32_t *__restrict__ vals_out, uint32_t tile_n, uint32_t n, int shift,
                                            int tid, Control *ctl) {
     constexpr int D = 1 << BITS;
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(T, 4) k_onesweep(Segs segs, const uint32_t *__
     // test hook words (zero in normal use): a tile that publishes nothing, the wait bound
     const uint32_t stall1 = ctl->test_stall_tile1;
     const long long spin_limit = ctl->test_spin_limit ? (long long)ctl->test_spin_limit : kSpinLimitCycles;
-    clear_warp<BITS>(S, warp, lane);
+    clear_warp(S, warp, lane);
     __syncthreads();
     const uint32_t tile = S.tile;
     const TileSpan sp = segs.span(tile);
@@ -542,7 +545,7 @@ __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(const uint32_t *__r
 
 // Scatter: the ranking and staging of k_onesweep; the prefix of each digit is the chunk's
 // offset plus the counts of the chunk's earlier tiles.  Tile = blockIdx.x, no waits.
-template <int BITS>
+template <int BITS, bool WORDS>
 __global__ void __launch_bounds__(T, 4) k_scatter(const uint32_t *__restrict__ keys_in,
                                                const uint32_t *__restrict__ vals_in,
                                                uint32_t *__restrict__ keys_out,
@@ -553,11 +556,11 @@ __global__ void __launch_bounds__(T, 4) k_scatter(const uint32_t *__restrict__ k
     constexpr int D = 1 << BITS;
     constexpr int P = D / T;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    SortSmem<BITS> &S = *reinterpret_cast<SortSmem<BITS> *>(smem_raw);
+    SortSmem<BITS, WORDS> &S = *reinterpret_cast<SortSmem<BITS, WORDS> *>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // each warp clears its own counts: the ranking below touches only those, so the warp starts it
     // without waiting for the block (a block barrier there cost about 1 us of the three passes)
-    clear_warp<BITS>(S, warp, lane);
+    clear_warp(S, warp, lane);
     chain_wait();
     const uint32_t tile = blockIdx.x, tile_base = tile * (uint32_t)kSortTile;
     const int shift = pass * BITS;
@@ -632,8 +635,11 @@ cudaError_t sort_init() {
     if (e == cudaSuccess) e = allow_smem<kDigitBits32, ManySegSort<kDigitBits32>>();
     if (e == cudaSuccess) e = allow_smem<kDigitBits32, OneSegSort>();
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_scatter<kDigitBits>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(SortSmem<kDigitBits>));
+        e = cudaFuncSetAttribute(k_scatter<kDigitBits, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(SortSmem<kDigitBits, false>));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_scatter<kDigitBits, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(SortSmem<kDigitBits, true>));
     return e;
 }
 
@@ -653,8 +659,16 @@ void launch_sort_pass(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t
     if (!counted)
         launch_chained(chain, k_tile_hist<kDigitBits>, chunks, T, 0, s, keys_in, n, pass, ct, tile_hist, chunk_sum, ghist);
     launch_chained(chain, k_chunk_scan<kDigitBits>, kDigits / 32, kScanThreads, 0, s, chunk_sum, chunks, ghist, chunk_off);
-    launch_chained(chain, k_scatter<kDigitBits>, tiles, T, sizeof(SortSmem<kDigitBits>), s, keys_in, vals_in, keys_out,
-                   vals_out, n, pass, tile_hist, chunk_off, ct, ctl);
+    // a single wave of tiles is bound by one tile's latency, which words shorten (rank_warp); more
+    // tiles by the shared-memory pipe, which words load.  Sort stage,
+    // ballots against words: 180,000 triangles 43.5 and 41.0 us, 1,000,003 58.3 and 54.2 (clustered
+    // 56.4 and 54.2), 2,090,000 89.1 and 87.0; three passes over 2^24 343 and 375
+    if (tiles <= kWordTiles)
+        launch_chained(chain, k_scatter<kDigitBits, true>, tiles, T, sizeof(SortSmem<kDigitBits, true>), s, keys_in, vals_in,
+                       keys_out, vals_out, n, pass, tile_hist, chunk_off, ct, ctl);
+    else
+        launch_chained(chain, k_scatter<kDigitBits, false>, tiles, T, sizeof(SortSmem<kDigitBits, false>), s, keys_in, vals_in,
+                       keys_out, vals_out, n, pass, tile_hist, chunk_off, ct, ctl);
 }
 
 void launch_onesweep32(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out,
