@@ -513,7 +513,8 @@ __global__ void __launch_bounds__(1024) k_scan_small(U *v, uint32_t n, U *total)
 }
 
 // Line starts: the newline at byte k (rank r over the text) starts line r + 1 at k + 1.  At most
-// `cap` lines are written (the caller sees from the count that there are more).
+// `cap` lines are written (the caller sees from the count that there are more).  Before chain_wait it
+// reads the text only, complete before k_nl_count began, for which k_scan_small has waited.
 __global__ void __launch_bounds__(kT) k_nl_write(const uint8_t *__restrict__ s, uint64_t n,
                                                  const uint32_t *__restrict__ base, uint32_t cap,
                                                  uint32_t *__restrict__ line_start) {
@@ -1026,7 +1027,9 @@ __device__ __forceinline__ bool fast_face(const uint8_t *b, uint32_t nverts, con
 }
 
 // Model-0 faces -> fan triangles (y and z swapped, float32, pad 3.1415), their vertices marked.
-// Blocks as k_vertices.
+// Blocks as k_vertices.  Before chain_wait it reads the text and what obj_scan's kernels wrote (lines,
+// types, fans, prefixes): the host has waited for those before it launched k_vertices, which writes
+// none of them.
 __global__ void __launch_bounds__(kLineBlock, 8) k_faces(const uint8_t *__restrict__ text, uint64_t n,
                                                       const uint32_t *__restrict__ line_start, uint32_t L,
                                                       const uint8_t *__restrict__ type,
@@ -1045,10 +1048,12 @@ __global__ void __launch_bounds__(kLineBlock, 8) k_faces(const uint8_t *__restri
     const bool mine = ty == LT_F;
     const uint32_t vbal = __ballot_sync(0xFFFFFFFFu, ty == LT_V);
     if ((threadIdx.x & 31) == 0) s_v[threadIdx.x >> 5] = __popc(vbal);
-    if (!__syncthreads_or(mine)) return;
-    const uint32_t at = (uint32_t)(first >> 32) + block_scan<uint32_t>(mine ? fan : 0u, s_warp, nullptr);
-    lt.stage(text, n, win);
-    chain_wait();  // the vertices
+    uint32_t at = 0;
+    if (__syncthreads_or(mine)) {
+        at = (uint32_t)(first >> 32) + block_scan<uint32_t>(mine ? fan : 0u, s_warp, nullptr);
+        lt.stage(text, n, win);
+    }
+    chain_wait();  // the vertices; every block's, so that k_bounds_floor's wait stands for k_vertices too
     if (!mine) return;
     float4 *out = tri + 3ull * at;
     bool ok = true, done = false;
