@@ -381,12 +381,18 @@ LVBH_API int  lvbh_parse_obj(lvbh_ctx *ctx, const char *text, uint64_t bytes, ui
                              uint64_t *err_line, void *stream);
 
 /* The same in two calls, for a caller that wants the soup in memory of its own: _begin checks the
- * text and gives the number of triangles, _into writes them to `tri` (*num_tris x 12 floats of
- * device memory, 16-byte aligned).  The text stays as it is in between, and no other parse runs
- * on ctx; _into without a _begin that returned LVBH_OK is LVBH_EINVAL.  Other arguments and
- * statuses as lvbh_parse_obj. */
+ * text and gives the number of triangles, _store writes them to `tri` (max_tris x 12 floats of
+ * device memory, 16-byte aligned).  max_tris below *num_tris is LVBH_EINVAL, with nothing written;
+ * _store may then be called again.  The text stays as it is in between, and no other parse runs
+ * on ctx; _store without a _begin that returned LVBH_OK is LVBH_EINVAL.  Other arguments and
+ * statuses as lvbh_parse_obj.
+ * _into is _store with all that the device allocation holds from `tri` on as max_tris: for a tri
+ * that has an allocation of its own.  Inside a larger one (a pool's, torch's) it cannot see where
+ * the caller's part ends; _store can. */
 LVBH_API int  lvbh_parse_obj_begin(lvbh_ctx *ctx, const char *text, uint64_t bytes, uint32_t flags,
                                    uint32_t *num_tris, uint64_t *err_line, void *stream);
+LVBH_API int  lvbh_parse_obj_store(lvbh_ctx *ctx, float *tri, uint32_t max_tris, double *bounds6,
+                                   uint64_t *err_line, void *stream);
 LVBH_API int  lvbh_parse_obj_into(lvbh_ctx *ctx, float *tri, double *bounds6, uint64_t *err_line,
                                   void *stream);
 

@@ -10,6 +10,8 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <map>
 #include <string>
 
@@ -662,6 +664,26 @@ int finish_pending(lvbh_ctx *ctx) {
     return rc;
 }
 
+// Triangles of 48 bytes from `tri` to the end of the device allocation it lies in (UINT32_MAX where the
+// driver names none).
+uint32_t tris_to_end(const float *tri) {
+    static const PFN_cuMemGetAddressRange_v3020 range = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(f);
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr p = reinterpret_cast<CUdeviceptr>(tri);
+    if (!tri || !range || range(&base, &size, p) != CUDA_SUCCESS) return UINT32_MAX;
+    return (uint32_t)std::min<uint64_t>((base + size - p) / 48, UINT32_MAX);
+}
+
 }  // namespace
 
 namespace lvbh {
@@ -1193,7 +1215,7 @@ int lvbh_parse_obj(lvbh_ctx *ctx, const char *text, uint64_t bytes, uint32_t fla
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     uint32_t n = 0;
     if (int rc = obj_scan(ctx->obj, text, bytes, (flags & LVBH_INPUT_HOST) != 0, &n, err_line, s, ctx->err)) return rc;
-    if (int rc = obj_emit(ctx->obj, nullptr, tri_out, bounds6, err_line, s, ctx->err)) return rc;
+    if (int rc = obj_emit(ctx->obj, nullptr, 0, tri_out, bounds6, err_line, s, ctx->err)) return rc;
     *num_tris = n;
     return LVBH_OK;
 }
@@ -1213,12 +1235,18 @@ int lvbh_parse_obj_begin(lvbh_ctx *ctx, const char *text, uint64_t bytes, uint32
 
 int lvbh_parse_obj_into(lvbh_ctx *ctx, float *tri, double *bounds6, uint64_t *err_line, void *stream) {
     if (!ctx) return LVBH_EINVAL;
+    DeviceGuard g(ctx->device);
+    return lvbh_parse_obj_store(ctx, tri, tris_to_end(tri), bounds6, err_line, stream);
+}
+
+int lvbh_parse_obj_store(lvbh_ctx *ctx, float *tri, uint32_t max_tris, double *bounds6, uint64_t *err_line, void *stream) {
+    if (!ctx) return LVBH_EINVAL;
     if (!tri || !bounds6 || !err_line) return fail(ctx, LVBH_EINVAL, "NULL output pointer");
     *err_line = 0;
     if (reinterpret_cast<uintptr_t>(tri) & 15u) return fail(ctx, LVBH_EINVAL, "tri must be 16-byte aligned");
     DeviceGuard g(ctx->device);
     if (ctx->pending) LVBH_CUDA(ctx, cudaStreamSynchronize(ctx->last_stream));
-    return obj_emit(ctx->obj, tri, nullptr, bounds6, err_line, static_cast<cudaStream_t>(stream), ctx->err);
+    return obj_emit(ctx->obj, tri, max_tris, nullptr, bounds6, err_line, static_cast<cudaStream_t>(stream), ctx->err);
 }
 
 }  // extern "C"

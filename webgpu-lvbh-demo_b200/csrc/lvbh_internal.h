@@ -291,13 +291,13 @@ struct ObjScratch {
 };
 // OBJ text -> triangle soup + bounds (lvbh_parse_obj) in two steps: obj_scan finds the lines,
 // checks the statements and counts the triangles; obj_emit parses vertices and faces into dst
-// (*num_tris x 12 floats, 16-byte aligned; null: the scratch's own soup) and needs the text as
-// it was.  *err_line: the 1-based line whose statement the parser rejects, 0 for a failure found
+// (room for max_tris x 12 floats, 16-byte aligned: fewer than *num_tris are refused; null: the
+// scratch's own soup) and needs the text as it was.  *err_line: the 1-based line whose statement the parser rejects, 0 for a failure found
 // after parsing (LVBH_EPARSE for both).
 int obj_scan(ObjScratch &sc, const char *text, uint64_t bytes, bool host_text, uint32_t *num_tris, uint64_t *err_line,
              cudaStream_t s, std::string &err);
-int obj_emit(ObjScratch &sc, float *dst, const float **tri_out, double *bounds6, uint64_t *err_line, cudaStream_t s,
-             std::string &err);
+int obj_emit(ObjScratch &sc, float *dst, uint32_t max_tris, const float **tri_out, double *bounds6, uint64_t *err_line,
+             cudaStream_t s, std::string &err);
 void obj_free(ObjScratch &sc);
 
 }  // namespace lvbh

@@ -1288,18 +1288,22 @@ int obj_scan(ObjScratch &sc, const char *text, uint64_t bytes, bool host_text, u
     return LVBH_OK;
 }
 
-int obj_emit(ObjScratch &sc, float *dst, const float **tri_out, double *bounds6, uint64_t *err_line, cudaStream_t s,
-             std::string &err) {
+int obj_emit(ObjScratch &sc, float *dst, uint32_t max_tris, const float **tri_out, double *bounds6, uint64_t *err_line,
+             cudaStream_t s, std::string &err) {
     auto cuda = [&](cudaError_t e, const char *what) { return obj_cuda(e, what, err); };
     *err_line = 0;
     if (!sc.scanned) {
         err = "no scanned OBJ text";
         return LVBH_EINVAL;
     }
-    sc.scanned = false;
     ObjCtl *hc = static_cast<ObjCtl *>(sc.host), *ctl = static_cast<ObjCtl *>(sc.ctl);
     const uint32_t L = hc->newlines + 1u, a = hc->m0a, b = hc->m0b;
     const uint32_t nverts = (uint32_t)(hc->totals & 0xFFFFFFFFull), nfan = (uint32_t)(hc->totals >> 32);
+    if (dst && nfan + 2u > max_tris) {  // the scan stays: the caller may come again with more room
+        err = "the soup has " + std::to_string(nfan + 2u) + " triangles, the caller's memory holds " + std::to_string(max_tris);
+        return LVBH_EINVAL;
+    }
+    sc.scanned = false;
     const uint32_t blk0 = a / kLineBlock, nblk = b > a ? (b - 1) / kLineBlock - blk0 + 1 : 0;
     const size_t xyz = align256(nverts * 24ull), rows = align256(nverts * 16ull), used = align256(nverts);
     OBJ_CUDA(grow(sc.verts, sc.verts_bytes, xyz + rows + used + align256(nverts * (size_t)sizeof(HardLine))),

@@ -443,8 +443,8 @@ class BVHBuilder:
             rc = _native.lib.lvbh_parse_obj_begin(*text_args, ctypes.byref(n), ctypes.byref(line), sp)
             if rc == _native.OK:
                 soup = torch.empty((n.value, 12), dtype=torch.float32, device=self.device)
-                rc = _native.lib.lvbh_parse_obj_into(self._ctx, ctypes.c_void_p(soup.data_ptr()), b6,
-                                                     ctypes.byref(line), sp)
+                rc = _native.lib.lvbh_parse_obj_store(self._ctx, ctypes.c_void_p(soup.data_ptr()), n.value, b6,
+                                                      ctypes.byref(line), sp)
         else:
             tri = ctypes.c_void_p()
             rc = _native.lib.lvbh_parse_obj(*text_args, ctypes.byref(tri), ctypes.byref(n), b6, ctypes.byref(line), sp)

@@ -146,6 +146,8 @@ def _load():
     L.lvbh_parse_obj_begin.restype = i32
     L.lvbh_parse_obj_begin.argtypes = [vp, vp, ctypes.c_uint64, u32, ctypes.POINTER(u32),
                                        ctypes.POINTER(ctypes.c_uint64), vp]
+    L.lvbh_parse_obj_store.restype = i32
+    L.lvbh_parse_obj_store.argtypes = [vp, vp, u32, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_uint64), vp]
     L.lvbh_parse_obj_into.restype = i32
     L.lvbh_parse_obj_into.argtypes = [vp, vp, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_uint64), vp]
     return L
