@@ -82,7 +82,9 @@ extern "C" {
  * about 100 GB of device memory). */
 #define LVBH_MAX_TRIS  ((uint32_t)1 << 29)
 
-/* Stage indices for lvbh_stage_times(). */
+/* Stage indices for lvbh_stage_times().  One kernel makes BOUNDS to SORT of a build of up to 65,536
+ * triangles; its time is divided by its own clock, and with bounds supplied reading the triangles
+ * counts as MORTON. */
 #define LVBH_STAGE_UPLOAD  0  /* host->device copy of the input (LVBH_INPUT_HOST only) */
 #define LVBH_STAGE_BOUNDS  1  /* scene box reduction with the triangle centroids (skipped when bounds are supplied) */
 #define LVBH_STAGE_MORTON  2  /* triangle centroid -> 30-bit Morton key + digit histograms */

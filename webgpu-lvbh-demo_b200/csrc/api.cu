@@ -129,6 +129,7 @@ struct lvbh_ctx {
     ObjScratch obj;                     // OBJ ingest buffers (the parsed soup among them)
     cudaEvent_t ev[LVBH_NUM_STAGES + 1] = {};
     bool ev_valid = false;
+    bool ev_small = false, ev_given = false;  // the profiled build's front was one kernel; its bounds were given
     // chunked upload of a host soup: its copy stream and events (start, one per chunk)
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t up_ev[1 + kUploadChunks] = {};
@@ -334,11 +335,10 @@ cudaError_t enqueue_build(lvbh_ctx *ctx, const float4 *tri, uint32_t n, const Ho
                           int pre = kPreNone) {
     if (profile) cudaEventRecord(ctx->ev[1], s);
     if (pre == kPreNone && small_build(n)) {
-        if (profile) { cudaEventRecord(ctx->ev[2], s); cudaEventRecord(ctx->ev[3], s); }  // all in the sort stage
         uint32_t *kv = ctx->keys_b;  // vals_b follows it in the arena
         const cudaError_t e = mesh ? launch_small_sort_mesh(mesh->verts, mesh->nverts, mesh->idx3, n, hb, ctx->ctl, kv,
-                                                            out->morton, out->leaf_index, s)
-                                   : launch_small_sort(tri, n, hb, ctx->ctl, kv, out->morton, out->leaf_index, s);
+                                                            out->morton, out->leaf_index, profile, s)
+                                   : launch_small_sort(tri, n, hb, ctx->ctl, kv, out->morton, out->leaf_index, profile, s);
         if (e != cudaSuccess) return e;
     } else {
         if (pre == kPreNone)
@@ -571,6 +571,8 @@ int build_common(lvbh_ctx *ctx, const float4 *tri_dev, uint32_t n, const float *
         if (rc) return rc;
     }
     ctx->ev_valid = profile;
+    ctx->ev_small = pre == kPreNone && small_build(n);
+    ctx->ev_given = hb.use != 0;
     // fetch the error words and the device-reduced bounds with the build
     LVBH_CUDA(ctx, cudaMemcpyAsync(ctx->host_ctl, ctx->ctl, offsetof(Control, pad1),
                                    cudaMemcpyDeviceToHost, s));
@@ -1120,11 +1122,22 @@ int lvbh_stage_times(lvbh_ctx *ctx, float *ms_out) {
     for (int i = 0; i < LVBH_NUM_STAGES; ++i) ms_out[i] = 0.0f;
     if (!ctx->ev_valid) return fail(ctx, LVBH_EINVAL, "no profiled build to report");
     DeviceGuard g(ctx->device);
-    for (int i = 0; i < LVBH_NUM_STAGES; ++i) {
+    auto between = [&](int a, int b) {
         float ms = 0.0f;
-        cudaError_t e = cudaEventElapsedTime(&ms, ctx->ev[i], ctx->ev[i + 1]);
-        if (e != cudaSuccess) { cudaGetLastError(); ms = 0.0f; }
-        ms_out[i] = ms;
+        if (cudaEventElapsedTime(&ms, ctx->ev[a], ctx->ev[b]) != cudaSuccess) { cudaGetLastError(); ms = 0.0f; }
+        return ms;
+    };
+    for (int i = 0; i < LVBH_NUM_STAGES; ++i) {
+        const bool front = i >= LVBH_STAGE_BOUNDS && i <= LVBH_STAGE_SORT;
+        if (!(ctx->ev_small && front)) ms_out[i] = between(i, i + 1);
+    }
+    if (ctx->ev_small) {  // box, keys and sort are one kernel (small.cu): its time in the shares it took
+        const float all = between(LVBH_STAGE_BOUNDS, LVBH_STAGE_SORT + 1);
+        const uint32_t *front = ctx->host_ctl + offsetof(Control, front) / 4;
+        const float box = ctx->ev_given ? 0.0f : (float)front[0] / 65536.0f, keys = (float)front[1] / 65536.0f;
+        ms_out[LVBH_STAGE_BOUNDS] = all * box;
+        ms_out[LVBH_STAGE_MORTON] = all * (keys - box);
+        ms_out[LVBH_STAGE_SORT] = all * (1.0f - keys);
     }
     return LVBH_OK;
 }

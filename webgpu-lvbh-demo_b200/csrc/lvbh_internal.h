@@ -81,7 +81,8 @@ struct Control {
     uint32_t aux_err;
     uint32_t err;
     uint32_t tile_counter[kSortPasses32];
-    uint32_t pad0[2];
+    uint32_t front[2];  // the small build's one kernel, when profiled: of 65,536 parts of its time, those until
+                        // the box was known and until the keys were
     uint32_t bounds_ord[6];   // scene min (ord_hi) and max (ord_lo), see lvbh_device.cuh
     uint32_t pad1[2];
     uint32_t hist[kHistWords];  // global digit counts of the unsorted keys, pass-major
@@ -171,15 +172,15 @@ void launch_morton_cen(const float *cen, uint32_t cen_stride, uint32_t n, Contro
 cudaError_t morton_init();  // once per device, before the first launch
 // K1 + K2 of a small build in one cluster kernel (small.cu): box, keys, sorted keys and
 // permutation, and the control block's error word and box (nothing to clear before).  kv: 2 n words
-// of scratch, 8-byte aligned.
+// of scratch, 8-byte aligned.  stamps: also ctl->front.
 constexpr uint32_t kSmallMax = 1u << 16;  // both sides measured: small.cu
 bool small_build(uint32_t n);  // whether n triangles take it on this device
 cudaError_t small_init();      // once per device, before the first launch
 cudaError_t launch_small_sort(const float4 *tri, uint32_t n, const HostBounds &hb, Control *ctl, uint32_t *kv,
-                              uint32_t *keys, uint32_t *vals, cudaStream_t s);
+                              uint32_t *keys, uint32_t *vals, bool stamps, cudaStream_t s);
 cudaError_t launch_small_sort_mesh(const float4 *verts, uint32_t nverts, const uint32_t *idx3, uint32_t n,
                                    const HostBounds &hb, Control *ctl, uint32_t *kv, uint32_t *keys, uint32_t *vals,
-                                   cudaStream_t s);
+                                   bool stamps, cudaStream_t s);
 // K2: one reduce-then-scan pass over 10-bit digit `pass` (0..2) of 30-bit keys.  counted: the
 // tile histograms, chunk sums and global digit counts (ctl->hist_part) of this pass are there
 // already (K1b makes those of pass 0); otherwise the pass's tile-histogram kernel makes them

@@ -68,6 +68,7 @@ struct SmallSmem {
     uint32_t ord[7];        // the block's box as ordered words, and its error bits ...
     uint32_t ords[kMaxBlocks][8];  // ... and every block's
     uint32_t box[7];        // the cluster's
+    uint32_t stamp[3];      // profiled: the clock at the start, with the box and with the keys
 };
 
 // A cluster barrier in two halves, the triangles' loads in between.
@@ -76,7 +77,8 @@ __device__ __forceinline__ void cluster_started_wait() { asm volatile("barrier.c
 
 // Key i of a thread is key (block IPT T) + warp 32 IPT + 32 i + lane: input order is (block, warp,
 // i, lane), the order the stable ranks count in.
-template <int SRC, int IPT>
+// STAMPS (a profiled build): the first block's first thread reads the clock between the stages.
+template <int SRC, int IPT, bool STAMPS>
 __global__ void __launch_bounds__(T) k_small_sort(const float4 *__restrict__ rows, const uint32_t *__restrict__ idx3,
                                                   uint32_t nverts, uint32_t n, HostBounds hb,
                                                   Control *__restrict__ ctl, uint2 *kv,
@@ -88,6 +90,8 @@ __global__ void __launch_bounds__(T) k_small_sort(const float4 *__restrict__ row
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t lt = lanemask_lt();
     const uint32_t local = warp * (32 * IPT) + lane, base = rank * (IPT * T) + local;
+    const bool stamps = STAMPS && rank == 0 && tid == 0;
+    if (stamps) S.stamp[0] = (uint32_t)clock();
 
     cluster_started_arrive();
     // boxes and centroids (aabb-z-idx.js:186-191)
@@ -161,6 +165,7 @@ __global__ void __launch_bounds__(T) k_small_sort(const float4 *__restrict__ row
         }
     }
     __syncthreads();
+    if (stamps) S.stamp[1] = (uint32_t)clock();
     float umin[3], umax[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -178,6 +183,7 @@ __global__ void __launch_bounds__(T) k_small_sort(const float4 *__restrict__ row
                            quantise_cen(S.cen[2][local + 32 * i], umin[2], umax[2]));
     }
     __syncthreads();  // the centroids are read; keys and counts take their place
+    if (stamps) S.stamp[2] = (uint32_t)clock();
 
     if constexpr (IPT > 1) {
 #pragma unroll
@@ -315,14 +321,24 @@ __global__ void __launch_bounds__(T) k_small_sort(const float4 *__restrict__ row
             vals_out[t] = v[i];
         }
     }
+    if (stamps) {
+        const float all = (float)((uint32_t)clock() - S.stamp[0]);
+        ctl->front[0] = (uint32_t)((float)(S.stamp[1] - S.stamp[0]) / all * 65536.0f);
+        ctl->front[1] = (uint32_t)((float)(S.stamp[2] - S.stamp[0]) / all * 65536.0f);
+    }
+}
+
+template <int SRC, int IPT, bool STAMPS>
+cudaError_t allow_cluster() {
+    auto k = k_small_sort<SRC, IPT, STAMPS>;
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallSmem<IPT>));
+    return e == cudaSuccess ? cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : e;
 }
 
 template <int SRC, int IPT>
 cudaError_t small_attrs(int *clusters) {
-    auto k = k_small_sort<SRC, IPT>;
-    const int smem = (int)sizeof(SmallSmem<IPT>);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaError_t e = allow_cluster<SRC, IPT, false>();
+    if (e == cudaSuccess) e = allow_cluster<SRC, IPT, true>();
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -331,18 +347,18 @@ cudaError_t small_attrs(int *clusters) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = kMaxBlocks;
     cfg.blockDim = T;
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = sizeof(SmallSmem<IPT>);
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int c = 0;
-    e = cudaOccupancyMaxActiveClusters(&c, k, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&c, k_small_sort<SRC, IPT, false>, &cfg);
     if (c < *clusters) *clusters = c;
     return e;
 }
 
 template <int SRC, int IPT>
 cudaError_t launch_ipt(const float4 *rows, const uint32_t *idx3, uint32_t nverts, uint32_t n, const HostBounds &hb,
-                       Control *ctl, uint32_t *kv, uint32_t *keys, uint32_t *vals, cudaStream_t s) {
+                       Control *ctl, uint32_t *kv, uint32_t *keys, uint32_t *vals, bool stamps, cudaStream_t s) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (n + IPT * T - 1) / (IPT * T);
@@ -354,18 +370,19 @@ cudaError_t launch_ipt(const float4 *rows, const uint32_t *idx3, uint32_t nverts
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_small_sort<SRC, IPT>, rows, idx3, nverts, n, hb, ctl, reinterpret_cast<uint2 *>(kv), keys, vals);
+    auto k = stamps ? k_small_sort<SRC, IPT, true> : k_small_sort<SRC, IPT, false>;
+    return cudaLaunchKernelEx(&cfg, k, rows, idx3, nverts, n, hb, ctl, reinterpret_cast<uint2 *>(kv), keys, vals);
 }
 
 // The fewest keys per thread with which at most 16 blocks hold n.
 template <int SRC>
 cudaError_t launch_src(const float4 *rows, const uint32_t *idx3, uint32_t nverts, uint32_t n, const HostBounds &hb,
-                       Control *ctl, uint32_t *kv, uint32_t *keys, uint32_t *vals, cudaStream_t s) {
+                       Control *ctl, uint32_t *kv, uint32_t *keys, uint32_t *vals, bool stamps, cudaStream_t s) {
     const uint32_t per = (n + kMaxBlocks * T - 1) / (kMaxBlocks * T);
-    if (per <= 1) return launch_ipt<SRC, 1>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, s);
-    if (per <= 2) return launch_ipt<SRC, 2>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, s);
+    if (per <= 1) return launch_ipt<SRC, 1>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, stamps, s);
+    if (per <= 2) return launch_ipt<SRC, 2>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, stamps, s);
     static_assert(kSmallMax <= 4 * kMaxBlocks * T, "four keys per thread are enough");
-    return launch_ipt<SRC, 4>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, s);
+    return launch_ipt<SRC, 4>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, stamps, s);
 }
 
 int g_small_ok[64];  // per device: 1 when a full cluster of every form fits
@@ -392,14 +409,14 @@ cudaError_t small_init() {
 }
 
 cudaError_t launch_small_sort(const float4 *tri, uint32_t n, const HostBounds &hb, Control *ctl, uint32_t *kv,
-                              uint32_t *keys, uint32_t *vals, cudaStream_t s) {
-    return launch_src<kSoup>(tri, nullptr, 0u, n, hb, ctl, kv, keys, vals, s);
+                              uint32_t *keys, uint32_t *vals, bool stamps, cudaStream_t s) {
+    return launch_src<kSoup>(tri, nullptr, 0u, n, hb, ctl, kv, keys, vals, stamps, s);
 }
 
 cudaError_t launch_small_sort_mesh(const float4 *verts, uint32_t nverts, const uint32_t *idx3, uint32_t n,
                                    const HostBounds &hb, Control *ctl, uint32_t *kv, uint32_t *keys, uint32_t *vals,
-                                   cudaStream_t s) {
-    return launch_src<kMesh>(verts, idx3, nverts, n, hb, ctl, kv, keys, vals, s);
+                                   bool stamps, cudaStream_t s) {
+    return launch_src<kMesh>(verts, idx3, nverts, n, hb, ctl, kv, keys, vals, stamps, s);
 }
 
 }  // namespace lvbh
