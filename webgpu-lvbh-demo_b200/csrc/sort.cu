@@ -146,9 +146,9 @@ __device__ __forceinline__ void clear_warp(SortSmem<BITS, WORDS> &S, int warp, i
 // took 802 us with ballots alone, 756, 717, 702 and 724 with one, two, three and four rows in four by
 // words.  Peers OR into their word one after the other, so after a ballot row with more than
 // kCrowd of them the next three rows use ballots too (720 us in all).  With 10-bit
-// digits (32 KB of words a block) words are taken up to kWordTiles tiles (launch_sort_pass).
+// digits (32 KB of words a block) words are taken while the tiles are one wave (launch_sort_pass).
 constexpr int kCrowd = 8;
-constexpr uint32_t kWordTiles = 512;
+constexpr int kBlocksPerSm = 4;  // of the kernels that rank
 template <int BITS, bool FULL, bool WORDS>
 __device__ __forceinline__ void rank_warp(SortSmem<BITS, WORDS> &S, const uint32_t (&k)[IPT], uint32_t (&rank)[IPT / 2],
                                           uint32_t wbase, uint32_t n, int shift, int warp, int lane) {
@@ -281,7 +281,7 @@ __device__ __forceinline__ void write_tile(const SortSmem<BITS, WORDS> &S, uint3
 }
 
 template <int BITS, class Segs>
-__global__ void __launch_bounds__(T, 4) k_onesweep(Segs segs, const uint32_t *__restrict__ keys_all,
+__global__ void __launch_bounds__(T, kBlocksPerSm) k_onesweep(Segs segs, const uint32_t *__restrict__ keys_all,
                                                 const uint32_t *__restrict__ vals_all,
                                                 uint32_t *__restrict__ keys_out_all,
                                                 uint32_t *__restrict__ vals_out_all, int pass,
@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(const uint32_t *__r
 // Scatter: the ranking and staging of k_onesweep; the prefix of each digit is the chunk's
 // offset plus the counts of the chunk's earlier tiles.  Tile = blockIdx.x, no waits.
 template <int BITS, bool WORDS>
-__global__ void __launch_bounds__(T, 4) k_scatter(const uint32_t *__restrict__ keys_in,
+__global__ void __launch_bounds__(T, kBlocksPerSm) k_scatter(const uint32_t *__restrict__ keys_in,
                                                const uint32_t *__restrict__ vals_in,
                                                uint32_t *__restrict__ keys_out,
                                                uint32_t *__restrict__ vals_out, uint32_t n,
@@ -660,10 +660,13 @@ void launch_sort_pass(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t
         launch_chained(chain, k_tile_hist<kDigitBits>, chunks, T, 0, s, keys_in, n, pass, ct, tile_hist, chunk_sum, ghist);
     launch_chained(chain, k_chunk_scan<kDigitBits>, kDigits / 32, kScanThreads, 0, s, chunk_sum, chunks, ghist, chunk_off);
     // a single wave of tiles is bound by one tile's latency, which words shorten (rank_warp); more
-    // tiles by the shared-memory pipe, which words load.  Sort stage,
-    // ballots against words: 180,000 triangles 43.5 and 41.0 us, 1,000,003 58.3 and 54.2 (clustered
-    // 56.4 and 54.2), 2,090,000 89.1 and 87.0; three passes over 2^24 343 and 375
-    if (tiles <= kWordTiles)
+    // tiles by the shared-memory pipe, which words load.  Sort stage on 148 SMs (a wave is 592 tiles), words
+    // against ballots, us: 200 tiles uniform 53 and 57, clustered 54 and 56, 396 of a mesh 67 and 69,
+    // 450 uniform 83 and 85, 512 88 and 89, 513 of a mesh 79 and 83, 560 uniform 92 and 93, 591 of a
+    // mesh 85 and 87, 592 uniform and clustered the same (87, 85); 620 clustered 98 and 95, 680 uniform 99
+    // and 98, 704 of a mesh the same (93), 880 118 and 115, 1,000 133 and 128, 2,300 277 and 260, 4,096 452
+    // and 425
+    if (tiles <= (uint32_t)(kBlocksPerSm * sm_count()))
         launch_chained(chain, k_scatter<kDigitBits, true>, tiles, T, sizeof(SortSmem<kDigitBits, true>), s, keys_in, vals_in,
                        keys_out, vals_out, n, pass, tile_hist, chunk_off, ct, ctl);
     else
