@@ -727,12 +727,12 @@ int lvbh_create(lvbh_ctx **out, const lvbh_config *cfg) {
     for (auto &e : ctx->ev) {
         if (cudaEventCreate(&e) != cudaSuccess) { cudaGetLastError(); lvbh_destroy(ctx); return LVBH_ECUDA; }
     }
-    if (emit_init() != cudaSuccess || sort_init() != cudaSuccess || morton_init() != cudaSuccess ||
-        small_init() != cudaSuccess) {
+    if (emit_init() != cudaSuccess || sort_init() != cudaSuccess || morton_init() != cudaSuccess) {
         cudaGetLastError();
         lvbh_destroy(ctx);
         return LVBH_ECUDA;
     }
+    small_init();
     if (cfg && cfg->reserve_tris) {
         if (cfg->reserve_tris > LVBH_MAX_TRIS) { lvbh_destroy(ctx); return LVBH_EINVAL; }
         if (int rc = ensure_arena(ctx, cfg->reserve_tris)) { lvbh_destroy(ctx); return rc; }

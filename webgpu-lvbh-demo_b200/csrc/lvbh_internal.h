@@ -175,7 +175,7 @@ cudaError_t morton_init();  // once per device, before the first launch
 // of scratch, 8-byte aligned.  stamps: also ctl->front.
 constexpr uint32_t kSmallMax = 1u << 16;  // both sides measured: small.cu
 bool small_build(uint32_t n);  // whether n triangles take it on this device
-cudaError_t small_init();      // once per device, before the first launch
+void small_init();             // once per device, before the first launch
 cudaError_t launch_small_sort(const float4 *tri, uint32_t n, const HostBounds &hb, Control *ctl, uint32_t *kv,
                               uint32_t *keys, uint32_t *vals, bool stamps, cudaStream_t s);
 cudaError_t launch_small_sort_mesh(const float4 *verts, uint32_t nverts, const uint32_t *idx3, uint32_t n,

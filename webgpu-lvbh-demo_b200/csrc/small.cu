@@ -19,6 +19,7 @@
 // scattered through distributed shared memory instead of L2 8,700 cycles a pass instead of 4,300
 // (two cycles a store either way until the keys are put in digit order first), three 10-bit passes
 // 35 us instead of 32, __match_any_sync for the ballots 40 us.
+#include <atomic>
 #include <cooperative_groups.h>
 
 #include "lvbh_device.cuh"
@@ -385,17 +386,19 @@ cudaError_t launch_src(const float4 *rows, const uint32_t *idx3, uint32_t nverts
     return launch_ipt<SRC, 4>(rows, idx3, nverts, n, hb, ctl, kv, keys, vals, stamps, s);
 }
 
-int g_small_ok[64];  // per device: 1 when a full cluster of every form fits
+std::atomic<int> g_small_ok[64];  // per device: 1 when a full cluster of every form fits
 
 }  // namespace
 
 bool small_build(uint32_t n) {
     int dev = 0;
     cudaGetDevice(&dev);
-    return n <= kSmallMax && dev >= 0 && dev < 64 && g_small_ok[dev];
+    return n <= kSmallMax && dev >= 0 && dev < 64 && g_small_ok[dev].load(std::memory_order_relaxed);
 }
 
-cudaError_t small_init() {
+// A device (or part of one) on which clusters of 16 such blocks cannot run answers the query with zero or
+// with an error; either way its small builds take the general path.
+void small_init() {
     int dev = 0, c = 1;
     cudaGetDevice(&dev);
     cudaError_t e = small_attrs<kSoup, 1>(&c);
@@ -404,8 +407,8 @@ cudaError_t small_init() {
     if (e == cudaSuccess) e = small_attrs<kMesh, 1>(&c);
     if (e == cudaSuccess) e = small_attrs<kMesh, 2>(&c);
     if (e == cudaSuccess) e = small_attrs<kMesh, 4>(&c);
-    if (e == cudaSuccess && dev >= 0 && dev < 64) g_small_ok[dev] = c > 0;
-    return e;
+    if (e != cudaSuccess) cudaGetLastError();
+    if (dev >= 0 && dev < 64) g_small_ok[dev].store(e == cudaSuccess && c > 0, std::memory_order_relaxed);
 }
 
 cudaError_t launch_small_sort(const float4 *tri, uint32_t n, const HostBounds &hb, Control *ctl, uint32_t *kv,
