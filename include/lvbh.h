@@ -64,7 +64,7 @@ extern "C" {
 #define LVBH_ETIMEOUT  3  /* a device-side wait gave up after its bound (error word set by a kernel) */
 #define LVBH_ECUDA     4  /* a CUDA runtime call failed; lvbh_last_error() has the text */
 #define LVBH_EBUSY     5  /* serving: queue full / request not finished yet */
-#define LVBH_EDEVICE   6  /* a kernel reported an inconsistent structure (bounded climb exceeded) */
+#define LVBH_EDEVICE   6  /* a kernel reported an inconsistent structure (open items, permutation, digit counts) */
 #define LVBH_ERANGE    7  /* a size beyond a fixed capacity (lvbh_sort_pairs_noalloc) */
 #define LVBH_EPARSE    8  /* lvbh_parse_obj: the text is one the reference's OBJ parser throws on */
 
@@ -73,7 +73,7 @@ extern "C" {
 #define LVBH_ASYNC         0x2u  /* return after enqueueing; call lvbh_sync() before reading results/status */
 #define LVBH_OUT_CALLER    0x4u  /* result pointers in *out are caller-owned device buffers to fill */
 #define LVBH_PROFILE       0x8u  /* record per-stage CUDA events; read them with lvbh_stage_times() */
-#define LVBH_NO_GRAPH      0x10u /* launch stage by stage instead of replaying a cached CUDA graph */
+#define LVBH_NO_GRAPH      0x10u /* launch kernel by kernel even where a cached CUDA graph would be replayed */
 #define LVBH_AUTOTUNE      0x20u /* lvbh_build_batched: pick the tunables by timing the candidates
                                     on the first batch of each mesh-size histogram (cached) */
 
@@ -159,7 +159,8 @@ LVBH_API int  lvbh_build_mesh(lvbh_ctx *ctx, const float *verts4, uint32_t num_v
                         uint32_t flags, lvbh_result *out, void *stream);
 
 /* Batched build: num_segs independent meshes laid end to end in one triangle soup, built in
- * one stream-ordered launch sequence (replayed as a cached CUDA graph) instead of one
+ * one stream-ordered launch sequence (from the second call in the same buffers with the same
+ * sizes on a cached CUDA graph) instead of one
  * build(TRI_ARRAY, NUM_TRIS, MODEL_BOUNDS) per mesh (scripts/bvh/build-bvh.js:12-66 called
  * num_segs times).
  *   tri_array    12 floats per triangle for all meshes (host memory with LVBH_INPUT_HOST).
@@ -187,8 +188,8 @@ LVBH_API int  lvbh_build_batched(lvbh_ctx *ctx, const float *tri_array, const ui
  * size histogram (per power-of-two size class, the bit length of the number of meshes in it),
  * and on the first batch with a new key times each candidate - digit width {10, 8} x tree block
  * {256, 128} - on that batch itself, then builds every batch with that key with the fastest.
- * Without it the defaults are used (10-bit digits, 256-leaf blocks).  Every choice gives the
- * same result words. */
+ * Without it the defaults are used: 256-leaf blocks; 8-bit digits when the meshes make 64 sort
+ * tiles (of up to 4,096 keys, each of one mesh) or more in all, 10-bit digits below.  Every choice gives the same result words. */
 typedef struct lvbh_tunables {
     uint32_t digit_bits;        /* radix sort digit width: 10 (three passes) or 8 (four passes) */
     uint32_t tree_block;        /* sorted leaves per tree block: 256 or 128 */

@@ -2,9 +2,10 @@
 //
 // Replaces the reference's host orchestration (scripts/bvh/build-bvh.js:12-66 and each kernel
 // module's execute(): 69 queue submits and 20 host waits per build) with one stream-ordered
-// chain of kernels (12 and a memset; 3 for up to kSmallMax triangles), replayed as a cached CUDA
-// graph when a build repeats in its buffers, and a single host wait at the end (none with
-// LVBH_ASYNC).
+// chain of kernels (12 and a memset; up to kSmallMax triangles 3), replayed as a cached CUDA graph
+// when a build repeats in its buffers (larger builds: always), and a single host wait at the end
+// (none with LVBH_ASYNC).  The indexed leaf format has one kernel more (leaf indices), a 12-byte
+// indexed mesh a memset and a gather.
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -560,7 +561,8 @@ int build_common(lvbh_ctx *ctx, const float4 *tri_dev, uint32_t n, const float *
     }
     int rc = LVBH_OK;
     if (profile && !profile_upload) cudaEventRecord(ctx->ev[0], s);
-    // a small build is three launches: cheaper than a graph's, and nothing to capture for new buffers
+    // a small build is three launches (a mesh's four): cheaper than a graph's, and nothing to capture
+    // for new buffers
     if (profile || (flags & LVBH_NO_GRAPH) || (pre == kPreNone && small_build(n))) {
         const cudaError_t qe = enqueue_build(ctx, tri_dev, n, hb, out, s, profile, mesh, pre);
         cudaError_t e = cudaGetLastError();
@@ -571,7 +573,7 @@ int build_common(lvbh_ctx *ctx, const float4 *tri_dev, uint32_t n, const float *
         if (rc) return rc;
     }
     ctx->ev_valid = profile;
-    ctx->ev_small = pre == kPreNone && small_build(n);
+    ctx->ev_small = profile && pre == kPreNone && small_build(n);
     ctx->ev_given = hb.use != 0;
     // fetch the error words and the device-reduced bounds with the build
     LVBH_CUDA(ctx, cudaMemcpyAsync(ctx->host_ctl, ctx->ctl, offsetof(Control, pad1),
@@ -1080,7 +1082,8 @@ int lvbh_sync(lvbh_ctx *ctx) {
     if (err & ERR_NONFINITE) return fail(ctx, LVBH_EINVAL, "non-finite vertex coordinate in the input");
     if (err & ERR_LOOKBACK_TIMEOUT) return fail(ctx, LVBH_ETIMEOUT, "radix sort look-back wait exceeded its bound");
     if (err & ERR_COPY_TIMEOUT) return fail(ctx, LVBH_ETIMEOUT, "leaf gather copy wait exceeded its bound");
-    if (err & ERR_CLIMB) return fail(ctx, LVBH_EDEVICE, "refit climb exceeded the maximum tree depth");
+    if (err & ERR_TREE)
+        return fail(ctx, LVBH_EDEVICE, "tree pass met a permutation entry out of range or open items no radix tree leaves");
     if (err & ERR_SORT_RANGE)
         return fail(ctx, LVBH_EDEVICE, "radix sort scatter target out of range (digit counts inconsistent with the keys)");
     return LVBH_OK;
@@ -1090,7 +1093,6 @@ int lvbh_test_stall_lookback(lvbh_ctx *ctx, uint32_t stall_tile, uint32_t spin_c
     if (!ctx) return LVBH_EINVAL;
     DeviceGuard g(ctx->device);
     if (int rc = finish_pending(ctx)) return rc;
-    ctx->last_gather = false;
     ctx->test_stall1 = stall_tile + 1u;  // UINT32_MAX -> 0: no tile stalls
     ctx->test_spin = spin_cycles;
     if (ctx->ctl) {

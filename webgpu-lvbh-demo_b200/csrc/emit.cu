@@ -284,13 +284,10 @@ __device__ __forceinline__ void hand_over(float4 *pool, int j, bool left, float4
 // its edge; what hangs below such nodes leaves as open items.
 //
 // What bounds it: shared-memory wavefronts (65 % of the LSU pipe), four block barriers a block
-// and DRAM (220 B per triangle at 2^24, 50 %); issue slots are half used.  Before, every leaf
-// climbed: the first child at a split parked, the second merged and went on, step by step with
-// block barriers and then in dependent chains (13,000 cycles of a block's 19,000).  The pass,
+// and DRAM (220 B per triangle at 2^24, 50 %); issue slots are half used.  Leaves that climb from
+// child to parent instead wait in dependent chains (13,000 cycles of a block's 19,000).  The pass,
 // climb -> this (B200): 2^24 clustered triangles 847 -> 803 us, 1,000,003 59 -> 53, the 2 M mesh
-// 118 -> 94, a 1,024-mesh batch of 33 M triangles 1,806 -> 1,476.  On the way there: prefetched
-// keys and indices in registers (spilled) 1,045 us at 2^24; windows of 4 and 16 leaves from
-// shared memory with a barrier each 829; both spilled in a batch 1,931.
+// 118 -> 94, a 1,024-mesh batch of 33 M triangles 1,806 -> 1,476.
 template <int LOG, class Segs, class Leaves = SoupLeaves>
 __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_tree_climb(Segs segs,
                                                     const uint32_t *__restrict__ keys_all,
@@ -432,7 +429,7 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
             const int o = S.open[buf ^ 1];
             out_counts[blk - grid] = (uint32_t)min(o, kOpenCap);
             out_counts[nblk + blk - grid] = 0u;  // a counter of the straddling pass
-            if (o > kOpenCap) atomicOr(&ctl->err, ERR_CLIMB);
+            if (o > kOpenCap) atomicOr(&ctl->err, ERR_TREE);
         }
         S.open[buf ^ 1] = 0;
     };
@@ -575,7 +572,7 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
             it.pad1 = 0;
             const int at = atomicAdd(&S.open[buf], 1);
             if (at < kOpenCap) out[at] = it;
-            else atomicOr(&ctl->err, ERR_CLIMB);
+            else atomicOr(&ctl->err, ERR_TREE);
         };
         if (active) {
             const int q = ip > 0 && ip < m ? S.P[ip] : -1;
@@ -601,9 +598,9 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
         const int o = S.open[last_buf];
         out_counts[last] = (uint32_t)min(o, kOpenCap);
         out_counts[nblk + last] = 0u;
-        if (o > kOpenCap) atomicOr(&ctl->err, ERR_CLIMB);
+        if (o > kOpenCap) atomicOr(&ctl->err, ERR_TREE);
     }
-    if (bad_perm) atomicOr(&ctl->err, ERR_CLIMB);
+    if (bad_perm) atomicOr(&ctl->err, ERR_TREE);
     if (copy_timeout) atomicOr(&ctl->err, ERR_COPY_TIMEOUT);
 }
 
@@ -620,14 +617,10 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
 // One block reduces a group of kGroupBlocks tree blocks; the last of kFan neighbouring groups to
 // finish (a counter per parent, nothing waits) goes on with what those groups left as one run,
 // and so on up to the root: three levels at 2^20 triangles, four at 2^24.  Latency bounds it: a level
-// is six block barriers and four dependent L2 accesses, about 4 us.  Before, each open item
-// climbed one level of the tree at a time, parking and merging through shared-memory hashes and
-// then arrival words in L2 (0.5 to 2.6 us a level, up to 31 levels).  The pass, climbs -> runs
-// (B200): 4,098 triangles 19 -> 5 us, 65,536 uniform 35 -> 10, 1,000,003 clustered 63 -> 22, the
-// 2 M sphere 65 -> 27, 2^24 clustered 130 -> 70, 1,024 meshes of 33 M triangles 203 -> 117; the
-// scratch of arrival words and parked children (37 B per triangle) is gone.  (Its first form found
-// separators with one ballot per value and had its windows from shared memory, a barrier each:
-// 11, 26, 35, 91 and 155 us.)
+// is six block barriers and four dependent L2 accesses, about 4 us (an item that climbs pays 0.5 to
+// 2.6 us for each of up to 31 levels of the tree).  The pass, climbs -> runs (B200): 4,098 triangles
+// 19 -> 5 us, 65,536 uniform 35 -> 10, 1,000,003 clustered 63 -> 22, the 2 M sphere 65 -> 27, 2^24
+// clustered 130 -> 70, 1,024 meshes of 33 M triangles 203 -> 117.
 //
 // Sizes: a run holds at most 256 items, one per thread: a child's open items (<= kOpenCap) always
 // fit beside what the children before it left (<= kOpenCap), so a run that would be longer is
@@ -635,8 +628,7 @@ __global__ void __launch_bounds__(TreeGeo<LOG>::EB, TreeGeo<LOG>::kCtasPerSm) k_
 // clustered triangles), so a group of 24 blocks leaves 60 of 256 threads idle and rarely needs a
 // second turn.  16 blocks (more levels, more idle threads) take 89 us at 2^24 and 142 for the
 // batch, 28 blocks and 14 groups 68 and 109 but 23.1 (22.0) at 1,000,003 and 29.5 (27.3) for the
-// sphere; in the first form 512 threads and 32 blocks were slower than 256 and 24 (fewer, longer
-// blocks hide each other's latency less).
+// sphere.
 constexpr int kRunCap = 256;
 constexpr int kRunWarps = kRunCap / 32;
 static_assert(kRunCap >= 2 * kOpenCap && kGroupBlocks <= 32 && kFan <= 32, "a run takes two children; one warp counts them");
@@ -916,7 +908,7 @@ __global__ void __launch_bounds__(kRunCap, Groups::kCtas) k_top_group(Groups gro
             }
         }
     }
-    if (!ok) atomicOr(&ctl->err, ERR_CLIMB);
+    if (!ok) atomicOr(&ctl->err, ERR_TREE);
 }
 
 // the layout plus the slack that puts it on a 128-byte boundary

@@ -10,7 +10,8 @@ namespace lvbh {
 enum : uint32_t {
     ERR_NONFINITE = 1u,         // a vertex coordinate is NaN or +-Inf
     ERR_LOOKBACK_TIMEOUT = 2u,  // a decoupled look-back wait exceeded its bound
-    ERR_CLIMB = 4u,             // a block or run left more open items than a valid tree can
+    ERR_TREE = 4u,              // a block or run left more open items than a valid tree can, or an entry
+                                // of the permutation or an open item names no leaf of its segment
     ERR_BAD_INDEX = 8u,         // an indexed-mesh vertex index is out of range
     ERR_COPY_TIMEOUT = 16u,     // a copy wait (mbarrier) exceeded its bound
     ERR_SORT_RANGE = 32u,       // a radix sort scatter target fell outside the array (digit
@@ -69,7 +70,8 @@ __device__ __forceinline__ bool finite3(float4 v) {
 // every block of the kernel before it on the stream has exited, before that kernel's
 // completion is flushed; chain_wait blocks until the kernel before has completed and its
 // memory is visible (and so, transitively, every earlier one).  Every chained kernel calls it
-// before its first access to global memory that a kernel before it on the stream may write.  Launched the ordinary way it returns at once.
+// before its first access to global memory that a kernel before it on the stream may write.  Launched
+// the ordinary way it returns at once.
 // No kernel signals its dependents early (griddepcontrol.launch_dependents at its start): the
 // waiting blocks that let in cost more than the launch they hid (a 2^20-triangle build 0.235
 // -> 0.250 ms, against 0.232 ms without the early signal).

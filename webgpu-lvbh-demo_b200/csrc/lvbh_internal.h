@@ -28,8 +28,8 @@ constexpr int kSortTile = kSortThreads * kSortItems; // keys per tile (4096)
 __host__ __device__ inline uint32_t sort_tiles(uint32_t n) { return (n + kSortTile - 1) / kSortTile; }
 
 // The plain build's sort scratch: per tile of kSortTile keys the kDigits counts of the pass's
-// digit over the chunk's earlier tiles, per chunk of sort_chunk_tiles(n) tiles their sum, per chunk the output offsets.  A
-// chunk is one block of the per-chunk kernels (Morton keys, tile histograms): 8 tiles when that
+// digit over the chunk's earlier tiles, per chunk of sort_chunk_tiles(n) tiles their sum, per chunk
+// the output offsets.  A chunk is one block of the per-chunk kernels (Morton keys, tile histograms): 8 tiles when that
 // still gives kChunkFill blocks (two per SM), fewer for smaller sorts.
 constexpr int kSortChunkTiles = 8;
 constexpr uint32_t kChunkFill = 296;
@@ -151,8 +151,6 @@ inline bool chain_build(uint32_t n) { return n <= kChainMaxTris; }
 int ctx_reserve_batch(lvbh_ctx *ctx, uint32_t max_tris, uint32_t max_segs);
 size_t ctx_device_bytes(const lvbh_ctx *ctx);
 
-// K1a: scene box over every vertex of the 48-byte triangle soup.
-void launch_bounds(const float4 *tri, uint32_t n, Control *ctl, cudaStream_t s);
 // K1b: triangle box centroid -> Morton key (input order), the first sort pass's tile
 // histograms, chunk sums (sort_scratch) and global digit counts (ctl->hist_part, zero before); flags
 // non-finite vertices in ctl->err.

@@ -26,48 +26,6 @@ __device__ __forceinline__ void warp_minmax(float (&mn)[3], float (&mx)[3]) {
     }
 }
 
-// K1a: min / max of every vertex coordinate.  Vertices are the float4 of the soup; the pad
-// word is ignored.  fminf/fmaxf skip NaN (K1b reports non-finite input separately).
-__global__ void __launch_bounds__(kThreads) k_bounds(const float4 *__restrict__ v, uint64_t nv,
-                                                     Control *__restrict__ ctl) {
-    float mn[3] = {INFINITY, INFINITY, INFINITY};
-    float mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-    const uint64_t stride = (uint64_t)gridDim.x * kThreads;
-    uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    for (; i + 3 * stride < nv; i += 4 * stride) {
-        float4 p[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) p[u] = ld_stream(v + i + u * stride);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            mn[0] = fminf(mn[0], p[u].x); mx[0] = fmaxf(mx[0], p[u].x);
-            mn[1] = fminf(mn[1], p[u].y); mx[1] = fmaxf(mx[1], p[u].y);
-            mn[2] = fminf(mn[2], p[u].z); mx[2] = fmaxf(mx[2], p[u].z);
-        }
-    }
-    for (; i < nv; i += stride) {
-        const float4 p = ld_stream(v + i);
-        mn[0] = fminf(mn[0], p.x); mx[0] = fmaxf(mx[0], p.x);
-        mn[1] = fminf(mn[1], p.y); mx[1] = fmaxf(mx[1], p.y);
-        mn[2] = fminf(mn[2], p.z); mx[2] = fmaxf(mx[2], p.z);
-    }
-    warp_minmax(mn, mx);
-    __shared__ float s[kWarps][6];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) { s[warp][a] = mn[a]; s[warp][3 + a] = mx[a]; }
-    }
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        const int a = threadIdx.x;
-        float r = s[0][a];
-        for (int w = 1; w < kWarps; ++w) r = a < 3 ? fminf(r, s[w][a]) : fmaxf(r, s[w][a]);
-        if (a < 3) atomicMax(&ctl->bounds_ord[a], ~ord_lo(r));
-        else atomicMax(&ctl->bounds_ord[a], ord_lo(r));
-    }
-}
-
 // K1a for a soup whose box is reduced on the device: the box and every triangle's centroid in
 // one read of triangles [t0, t1).  A warp loads a row of 32 triangles as three coalesced
 // 512-byte loads (its next row in flight meanwhile), transposes it through shared memory so
@@ -286,7 +244,8 @@ struct CenSmem {
 };
 __global__ void __launch_bounds__(kCenThreads) k_morton_cen(const float *__restrict__ cen, uint32_t cen_stride,
                                                             uint32_t n, Control *__restrict__ ctl,
-                                                            uint32_t *__restrict__ keys, uint32_t chunk_tiles, uint32_t *__restrict__ tile_hist,
+                                                            uint32_t *__restrict__ keys, uint32_t chunk_tiles,
+                                                            uint32_t *__restrict__ tile_hist,
                                                             uint32_t *__restrict__ chunk_sum) {
     constexpr int WARPS = kCenThreads / 32, P = kDigits / kCenThreads, R = kSortTile / 32 / WARPS;
     static_assert(R * WARPS * 32 == kSortTile && P * kCenThreads == kDigits, "whole rows and digits");
@@ -569,15 +528,6 @@ __global__ void k_gather_indexed(const float *__restrict__ xyz, uint32_t num_ver
 }
 
 }  // namespace
-
-void launch_bounds(const float4 *tri, uint32_t n, Control *ctl, cudaStream_t s) {
-    const uint64_t nv = 3ull * n;
-    uint64_t blocks = (nv + kThreads * 4 - 1) / (kThreads * 4);
-    const uint64_t cap = (uint64_t)sm_count() * 8;
-    if (blocks > cap) blocks = cap;
-    if (blocks == 0) blocks = 1;
-    k_bounds<<<(unsigned)blocks, kThreads, 0, s>>>(tri, nv, ctl);
-}
 
 void launch_morton(const float4 *tri, uint32_t n, HostBounds hb, Control *ctl, uint32_t *keys,
                    uint32_t *sort_scratch, cudaStream_t s) {

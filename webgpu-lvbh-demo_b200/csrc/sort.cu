@@ -31,7 +31,8 @@
 //                 (exclusive scan over chunks plus the digit's global start);
 //   k_scatter     ranks its tile as above, adds its row of counts (4 KB, already final) to the
 //                 chunk offset, and scatters.
-// The batched build's segments span at most 64 tiles, so it keeps the one-kernel look-back.
+// The batched build's segments mostly span few tiles (64 in the workloads it is made for; any size
+// works), so it keeps the one-kernel look-back.
 //
 // Per key one 4-byte key read (+4-byte value read after the first pass) and two 4-byte writes (+
 // the 4-byte key read of k_tile_hist when reducing first), 41 us a pass of 2^24 keys at the copy
@@ -423,8 +424,8 @@ __global__ void __launch_bounds__(T, kBlocksPerSm) k_onesweep(Segs segs, const u
 }
 
 // Reduce: digit counts of the tiles before every tile in its chunk (tile_hist[tile][digit]) and of
-// every chunk of chunk_tiles tiles (chunk_sum[chunk][digit]), added up into the pass's global counts (ghist: kHistParts
-// partial rows, zero before; the chunk goes to row chunk % kHistParts).  One block per chunk;
+// every chunk of chunk_tiles tiles (chunk_sum[chunk][digit]), added up into the pass's global counts
+// (ghist: kHistParts partial rows, zero before; the chunk goes to row chunk % kHistParts).  One block per chunk;
 // each thread owns P contiguous digits.
 template <int BITS>
 __global__ void __launch_bounds__(T) k_tile_hist(const uint32_t *__restrict__ keys, uint32_t n, int pass,
@@ -489,7 +490,9 @@ __global__ void __launch_bounds__(T) k_tile_hist(const uint32_t *__restrict__ ke
 // counts over digits, the kHistParts partial rows of ghist summed) + counts of digit d in chunks
 // before c.  Block b covers digits 32b .. 32b+31 (lane = digit); its 32 warps split the chunks.
 constexpr int kScanThreads = 1024;
-constexpr int kScanKeep = 16;  // 512 chunks: every sort up to 2^24 keys
+// 512 chunks in registers; of more (513 to 592 just below 592, 1,184 and 2,368 tiles, any number above
+// 4,096 tiles) the rest is read once a sweep
+constexpr int kScanKeep = 16;
 template <int BITS>
 __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(const uint32_t *__restrict__ chunk_sum,
                                                              uint32_t chunks,

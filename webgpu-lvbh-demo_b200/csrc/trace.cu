@@ -257,7 +257,9 @@ __device__ __forceinline__ void visit_leaf(RayState &st, const Stack &stack, con
 // B200: 4 M rays on the 2 M sphere / 100,003 rays on a 131 K mesh / a 1080p bounce, from 2.85 ms /
 // 192 us / 598 us: internal nodes culled when popped 2.61 / 185 / 590; 32-byte row loads and 12
 // stack entries in shared memory 2.40 / 179 / 620; hardware min and max 2.31 / 173 / 598; up to
-// four node visits between leaf tests and refills, in a loop of the lane's own, 2.01 / 146 / 480.
+// four node visits between leaf tests and refills, in a loop of the lane's own, 2.01 / 146 / 480.  (The
+// bounce is one camera's; whole calls at eight cameras went from 570 .. 863 to 442 .. 709 us, each
+// camera's passes within 4 %.)
 // Two, six and eight visits took 2.19, 2.00 and 2.04 ms (545, 522 and 563 us a bounce); leaves held
 // back until eight lanes have one 2.07 ms / 162 us / 535 us; both children's rows prefetched 2.73
 // ms / 198 us / 652 us; rays sorted by origin and direction beforehand save less than the sort costs.
