@@ -389,9 +389,9 @@ LVBH_API int  lvbh_parse_obj(lvbh_ctx *ctx, const char *text, uint64_t bytes, ui
  * _store may then be called again.  The text stays as it is in between, and no other parse runs
  * on ctx; _store without a _begin that returned LVBH_OK is LVBH_EINVAL.  Other arguments and
  * statuses as lvbh_parse_obj.
- * _into is _store with all that the device allocation holds from `tri` on as max_tris: for a tri
- * that has an allocation of its own.  Inside a larger one (a pool's, torch's) it cannot see where
- * the caller's part ends; _store can. */
+ * _into is _store with all that the cudaMalloc allocation holds from `tri` on as max_tris: for a tri
+ * that has an allocation of its own.  Inside a larger one (torch's), or in memory of another kind, it
+ * cannot see where the caller's part ends; _store can. */
 LVBH_API int  lvbh_parse_obj_begin(lvbh_ctx *ctx, const char *text, uint64_t bytes, uint32_t flags,
                                    uint32_t *num_tris, uint64_t *err_line, void *stream);
 LVBH_API int  lvbh_parse_obj_store(lvbh_ctx *ctx, float *tri, uint32_t max_tris, double *bounds6,

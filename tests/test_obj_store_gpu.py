@@ -1,5 +1,8 @@
 """The two-call OBJ parse into memory of the caller knows where that memory ends."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -48,3 +51,28 @@ def test_into_refuses_an_allocation_that_ends_too_early(builder):
     assert into(end - 48 * (n.value - 1)) == _native.EINVAL
     assert into(end - 48) == _native.EINVAL
     assert into(keep.data_ptr()) == _native.OK
+
+
+def test_into_takes_pool_memory(builder):
+    """Memory whose end is not told (a stream-ordered pool's) is the caller's word, as it was."""
+    import lvbh
+    here, pkg = os.path.dirname(os.path.abspath(__file__)), os.path.dirname(os.path.dirname(os.path.abspath(lvbh.__file__)))
+    code = (
+        "import sys, ctypes; sys.path[:0] = [%r, %r]\n"
+        "import torch, lvbh\n"
+        "from lvbh import _native\n"
+        "from test_obj_store_gpu import TEXT, begin\n"
+        "b = lvbh.BVHBuilder(0)\n"
+        "want = b.parse_obj(TEXT)['TRI_ARR']\n"
+        "n, b6 = ctypes.c_uint32(), (ctypes.c_double * 6)()\n"
+        "line = begin(b, n)\n"
+        "tri = torch.empty((n.value, 12), device='cuda')\n"
+        "rc = _native.lib.lvbh_parse_obj_into(b.ctx, ctypes.c_void_p(tri.data_ptr()), b6, ctypes.byref(line), None)\n"
+        "assert rc == _native.OK and torch.equal(tri.view(torch.int32), want.view(torch.int32))\n"
+        "big = torch.empty((1 << 21, 12), device='cuda')\n"
+        "line = begin(b, n)\n"
+        "rc = _native.lib.lvbh_parse_obj_into(b.ctx, ctypes.c_void_p(big[(1 << 21) - 12].data_ptr()), b6, ctypes.byref(line), None)\n"
+        "assert rc == _native.OK and torch.equal(big[-12:].view(torch.int32), want.view(torch.int32))\n"
+        % (pkg, here))
+    for conf in ("backend:cudaMallocAsync", "expandable_segments:True"):
+        subprocess.run([sys.executable, "-c", code], check=True, env=dict(os.environ, PYTORCH_CUDA_ALLOC_CONF=conf), timeout=300)

@@ -668,23 +668,30 @@ int finish_pending(lvbh_ctx *ctx) {
     return rc;
 }
 
-// Triangles of 48 bytes from `tri` to the end of the device allocation it lies in (UINT32_MAX where the
-// driver names none).
+template <class F>
+F driver_entry(const char *name) {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        f = nullptr;
+    }
+    return reinterpret_cast<F>(f);
+}
+
+// Triangles of 48 bytes from `tri` to the end of the cudaMalloc allocation it lies in; UINT32_MAX for
+// other memory (of a pool, or mapped piece by piece, where a range's end need not be the memory's).
 uint32_t tris_to_end(const float *tri) {
-    static const PFN_cuMemGetAddressRange_v3020 range = [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess) {
-            cudaGetLastError();
-            f = nullptr;
-        }
-        return reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(f);
-    }();
+    static const auto attribute = driver_entry<PFN_cuPointerGetAttribute_v4000>("cuPointerGetAttribute");
+    static const auto range = driver_entry<PFN_cuMemGetAddressRange_v3020>("cuMemGetAddressRange");
+    int legacy = 0;
     CUdeviceptr base = 0;
     size_t size = 0;
     const CUdeviceptr p = reinterpret_cast<CUdeviceptr>(tri);
-    if (!tri || !range || range(&base, &size, p) != CUDA_SUCCESS) return UINT32_MAX;
+    if (!tri || !attribute || !range ||
+        attribute(&legacy, CU_POINTER_ATTRIBUTE_IS_LEGACY_CUDA_IPC_CAPABLE, p) != CUDA_SUCCESS || !legacy ||
+        range(&base, &size, p) != CUDA_SUCCESS)
+        return UINT32_MAX;
     return (uint32_t)std::min<uint64_t>((base + size - p) / 48, UINT32_MAX);
 }
 
