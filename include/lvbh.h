@@ -73,7 +73,8 @@ extern "C" {
 #define LVBH_ASYNC         0x2u  /* return after enqueueing; call lvbh_sync() before reading results/status */
 #define LVBH_OUT_CALLER    0x4u  /* result pointers in *out are caller-owned device buffers to fill */
 #define LVBH_PROFILE       0x8u  /* record per-stage CUDA events; read them with lvbh_stage_times() */
-#define LVBH_NO_GRAPH      0x10u /* launch kernel by kernel even where a cached CUDA graph would be replayed */
+#define LVBH_NO_GRAPH      0x10u /* launch kernel by kernel even where a cached CUDA graph would be replayed;
+                                    without it a build on a stream that is being captured is LVBH_ECUDA */
 #define LVBH_AUTOTUNE      0x20u /* lvbh_build_batched: pick the tunables by timing the candidates
                                     on the first batch of each mesh-size histogram (cached) */
 

@@ -668,6 +668,17 @@ int finish_pending(lvbh_ctx *ctx) {
     return rc;
 }
 
+// A build that may replay a graph cannot be captured; one that is launched directly all the same (a small
+// one, buffers seen once) is refused there too, so that a caller's graph does not come to hold the
+// context's buffers by its size or by what was built before.  LVBH_NO_GRAPH and LVBH_PROFILE ask for
+// plain launches.
+int refuse_capture(lvbh_ctx *ctx, uint32_t n, uint32_t flags, cudaStream_t s) {
+    if (!n || (flags & (LVBH_NO_GRAPH | LVBH_PROFILE))) return LVBH_OK;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) cudaGetLastError();  // (the launches meet it again)
+    return st == cudaStreamCaptureStatusActive ? cuda_fail(ctx, cudaErrorStreamCaptureUnsupported, "build") : LVBH_OK;
+}
+
 template <class F>
 F driver_entry(const char *name) {
     void *f = nullptr;
@@ -779,6 +790,7 @@ int lvbh_build_soup(lvbh_ctx *ctx, const float *tri_array, uint32_t num_tris,
     ctx->last_gather = false;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = check_out(ctx, num_tris, flags, out)) return rc;
+    if (int rc = refuse_capture(ctx, num_tris, flags, s)) return rc;
     out->num_tris = out->num_nodes = num_tris;
     std::memset(out->bounds, 0, sizeof out->bounds);
     if (num_tris) {
@@ -815,6 +827,7 @@ int lvbh_build_indexed(lvbh_ctx *ctx, const float *xyz, uint32_t num_verts, cons
     ctx->last_gather = false;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = check_out(ctx, num_tris, flags, out)) return rc;
+    if (int rc = refuse_capture(ctx, num_tris, flags, s)) return rc;
     out->num_tris = out->num_nodes = num_tris;
     std::memset(out->bounds, 0, sizeof out->bounds);
     if (!num_tris) return build_common(ctx, nullptr, 0, model_bounds, flags, out, s, false);
@@ -860,6 +873,7 @@ int lvbh_build_mesh(lvbh_ctx *ctx, const float *verts4, uint32_t num_verts, cons
     ctx->last_gather = false;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = check_out(ctx, num_tris, flags, out, 12)) return rc;
+    if (int rc = refuse_capture(ctx, num_tris, flags, s)) return rc;
     out->num_tris = out->num_nodes = num_tris;
     std::memset(out->bounds, 0, sizeof out->bounds);
     if (!num_tris) return build_common(ctx, nullptr, 0, model_bounds, flags, out, s, false);
@@ -923,6 +937,7 @@ int lvbh_build_batched(lvbh_ctx *ctx, const float *tri_array, const uint32_t *se
     ctx->last_gather = false;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (int rc = check_out(ctx, total, flags, out)) return rc;
+    if (int rc = refuse_capture(ctx, total, flags, s)) return rc;
     out->num_tris = out->num_nodes = total;
     std::memset(out->bounds, 0, sizeof out->bounds);
     if (total == 0) {
